@@ -162,15 +162,19 @@ def _cumulative(lens):
     return torch.tensor(cu, dtype=torch.int32).cuda()
 
 
+def _block_inputs(r, cfg):
+    params = {n: r.normal(*shape, std=0.1, mean=1.0) if n.startswith("norm") else r.normal(*shape, std=0.02)
+              for n, shape in cfg.param_shapes().items()}
+    return params, r.normal(cfg.tokens, cfg.hidden), r.normal(cfg.tokens, cfg.hidden)
+
+
 def prepare(case, seed):
     r = _Random(seed)
     kind = case["kind"]
     s = {"case": case}
     if kind in ("block", "block_mx"):
         cfg = _config(case)
-        params = {n: r.normal(*shape, std=0.1, mean=1.0) if n.startswith("norm") else r.normal(*shape, std=0.02)
-                  for n, shape in cfg.param_shapes().items()}
-        s["x"], s["dy"] = r.normal(cfg.tokens, cfg.hidden), r.normal(cfg.tokens, cfg.hidden)
+        params, s["x"], s["dy"] = _block_inputs(r, cfg)
         if kind == "block_mx":
             s["block"] = cdl.sky1_mx.Sky1BlockMX(cfg, params)
         elif case["seqs"]:
@@ -310,3 +314,105 @@ def tolerance(case):
         return {"rel": 1e-6}
     return {"rel": {"block": 2.5e-2, "block_mx": 0.12, "lm": 5e-2, "linear": 7e-3, "attention": 1e-2, "rmsnorm": 7e-3,
                     "layernorm": 7e-3}[kind]}
+
+
+# --------------------------------------------------------------------------- the same in 64 bits
+def exact(case, seed):
+    """None: block_mx (its products are of quantized values) and lm (its state moves from pass to
+    pass)."""
+    kind = case["kind"]
+    if kind in ("block_mx", "lm"):
+        return None
+    if kind == "block":
+        return _exact_block(case, seed)
+    s = prepare(case, seed)
+    if kind == "linear":
+        x, w, dy = s["x"].double(), s["w"].double(), s["dy"].double()
+        return {"y": x @ w, "dx": dy @ w.T, "gw": x.T @ dy}
+    if kind == "attention":
+        return _exact_attention(case, s)
+    x = s["x"].double()
+    eps = s["opts"].eps
+    if kind == "rmsnorm":
+        dy, scale = s["dy"].double(), s["scale"].double()
+        r = (x.square().mean(1) + eps).rsqrt()
+        xh, g = x * r[:, None], dy * scale
+        dx = r[:, None] * (g - xh * (g * xh).mean(1, keepdim=True)) + s["res"].double()
+        return {"y": xh * scale, "r_inv": r, "dx": dx, "dscale": (dy * xh).sum(0)}
+    mean = x.mean(1)
+    r = ((x - mean[:, None]).square().mean(1) + eps).rsqrt()
+    y = (x - mean[:, None]) * r[:, None] * s["opts"].scale.double() + s["opts"].bias.double()
+    return {"y": y, "mean": mean, "r_inv": r}
+
+
+def _spans(case):
+    """(first row, rows) of every sequence, rows counted over the whole batch."""
+    lens = _lengths(case) if case["seqs"] else [case["seq"]] * case["batch"]
+    return [(sum(lens[:i]), n) for i, n in enumerate(lens)]
+
+
+def _scores(q, k, causal):
+    """q [n, heads, D], k [n, kv_heads, D] -> scaled (masked) scores [heads, n, n]."""
+    k = k.repeat_interleave(q.shape[1] // k.shape[1], 1)
+    sc = torch.einsum("qhd,khd->hqk", q, k) / math.sqrt(HEAD_DIM)
+    if causal:
+        sc = sc.masked_fill(torch.ones(sc.shape[1:], dtype=torch.bool, device=sc.device).triu(1), -math.inf)
+    return sc
+
+
+def _exact_attention(case, s):
+    def rows(t):
+        return t.reshape(-1, t.shape[-2], HEAD_DIM).double()
+
+    q, k, v, do = (rows(s[n]) for n in ("q", "k", "v", "do"))
+    out, dq, dk, dv = torch.zeros_like(q), torch.zeros_like(q), torch.zeros_like(k), torch.zeros_like(v)
+    lse = torch.zeros(q.shape[1], q.shape[0], dtype=torch.float64, device="cuda")
+    for first, n in _spans(case):
+        r = slice(first, first + n)
+        with torch.enable_grad():
+            qi, ki, vi = (t[r].clone().requires_grad_() for t in (q, k, v))
+            sc = _scores(qi, ki, case["causal"])
+            o = torch.einsum("hqk,khd->qhd", sc.softmax(-1), vi.repeat_interleave(q.shape[1] // v.shape[1], 1))
+            dq[r], dk[r], dv[r] = torch.autograd.grad(o, (qi, ki, vi), do[r])
+        out[r], lse[:, r] = o.detach(), sc.detach().logsumexp(-1)
+    if case["seqs"]:
+        n = s["rows"]
+        return {"out": out[:n], "lse": lse[:, :n], "dq": dq[:n], "dk": dk[:n], "dv": dv[:n]}
+    lse = lse.reshape(-1, case["batch"], case["seq"]).transpose(0, 1)
+    return {"out": out.reshape(s["q"].shape), "lse": lse, "dq": dq.reshape(s["q"].shape),
+            "dk": dk.reshape(s["k"].shape), "dv": dv.reshape(s["v"].shape)}
+
+
+def _exact_block(case, seed):
+    cfg = _config(case)
+    params, x, dy = _block_inputs(_Random(seed), cfg)
+    spans = _spans(case)
+    dy = dy.double()
+    dy[sum(n for _, n in spans):] = 0
+    w = {n: p.double().requires_grad_() for n, p in params.items()}
+    x = x.double().requires_grad_()
+
+    def norm(t, gain):
+        return t * (t.square().mean(1, keepdim=True) + cfg.eps).rsqrt() * gain
+
+    def rotated(t):
+        angle = torch.outer(torch.arange(len(t), dtype=torch.float64, device="cuda"),
+                            cfg.rope_base ** (-torch.arange(0, HEAD_DIM, 2, dtype=torch.float64, device="cuda") / HEAD_DIM))
+        c, sn = angle.cos()[:, None], angle.sin()[:, None]
+        lo, hi = t.chunk(2, -1)
+        return torch.cat([lo * c - hi * sn, hi * c + lo * sn], -1)
+
+    with torch.enable_grad():
+        qkv = (norm(x, w["norm1"]) @ w["wqkv"]).view(cfg.tokens, -1, HEAD_DIM)
+        parts = []
+        for first, n in spans:
+            q, k, v = qkv[first:first + n].split([cfg.heads, cfg.kv_heads, cfg.kv_heads], 1)
+            p = _scores(rotated(q), rotated(k), True).softmax(-1)
+            parts.append(torch.einsum("hqk,khd->qhd", p, v.repeat_interleave(cfg.heads // cfg.kv_heads, 1)))
+        attn = torch.cat(parts).reshape(-1, cfg.heads * HEAD_DIM)
+        attn = torch.nn.functional.pad(attn, (0, 0, 0, cfg.tokens - len(attn)))
+        o = attn @ w["wo"] + x
+        h = norm(o, w["norm2"])
+        out = (torch.nn.functional.silu(h @ w["wgate"]) * (h @ w["wup"])) @ w["wdown"] + o
+        grads = torch.autograd.grad(out, [x, *w.values()], dy)
+    return {"out": out.detach(), "dx": grads[0], "grads": dict(zip(w, grads[1:]))}
