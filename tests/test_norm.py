@@ -244,3 +244,22 @@ def test_general_path_shapes(cdl, gpu_ok, norm_type):
     _general_case(cdl, 50, 3000, norm_type, BF16, BF16, BF16, None, eps=1e-3)
     _general_case(cdl, 13, 100, norm_type, BF16, BF16, BF16, BF16)
     _general_case(cdl, 20, 96, norm_type, BF16, F32, None, None, col_stride=2)
+
+
+@pytest.mark.parametrize("norm_type", ["rms", "layer"])
+@pytest.mark.parametrize("cols", [1, 2, 31, 255, 256, 258, 1021, 1024, 1026, 2050, 4095, 4096, 4100, 8190, 8192])
+def test_register_rows_column_edges(cdl, gpu_ok, norm_type, cols):
+    """Rows kept in registers (norm_rows_kernel): both sides of every capacity, each access width
+    (4, 2 and 1 columns), row counts off the CTA's eight, rows with a stride of their own."""
+    _general_case(cdl, 13, cols, norm_type, F32, F32, F32, F32)
+    _general_case(cdl, 5, cols, norm_type, F32, BF16, BF16, None)
+    if cols < 8192:
+        gen = torch.Generator().manual_seed(3)
+        x = torch.randn(11, cols + 3, generator=gen).cuda()[:, 1:cols + 1]
+        out = cdl.ops.norm_fwd(x, cdl.ops.NormFwdOpts(save_stats=True, norm_type=norm_type, out=F32))
+        if norm_type == "layer":
+            y_ref, _, r_ref = layernorm_reference(to_f32(x), None, None, 1e-6)
+        else:
+            y_ref, r_ref = oracle.rmsnorm_fwd(to_f32(x), None, None, 1e-6)
+        assert_all_close("y", to_f32(out.y), y_ref, oracle.abs_rel_tolerance(y_ref, 1e-5, 1e-4))
+        assert_all_close("r_inv", to_f32(out.r_inv), r_ref, oracle.abs_rel_tolerance(r_ref, 1e-6, 1e-4))
