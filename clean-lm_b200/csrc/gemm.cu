@@ -17,6 +17,7 @@
 // Both operands may be K-major (K contiguous) or MN-major (M or N contiguous); that covers
 // forward (A row-major, B row-major), dgrad (B transposed view) and wgrad (A transposed view)
 // without copies.  M/N/K tails rely on TMA zero fill for loads and on predicated stores.
+#include "gemm_rows.cuh"
 #include "host.h"
 #include "ops.h"
 #include "ptx.cuh"
@@ -39,48 +40,11 @@ constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int THREADS = 320;  // warp 0 TMA, warp 1 MMA, warps 2-9 epilogue (two per TMEM lane quadrant)
 constexpr int EPI_WARPS = 8;
 constexpr int TMEM_COLS = 512;
-constexpr int RASTER_W = 8;  // N tiles per raster panel (upper bound; see Params::raster_w)
 // L2 budget for A plus one raster panel of B (see the raster_w computation on the host).
 #ifndef CDL_GEMM_RASTER_BUDGET_MB
 #define CDL_GEMM_RASTER_BUDGET_MB 96
 #endif
 constexpr size_t SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + 256;
-
-struct Params {
-  int M, N, K, batch;
-  int num_m_tiles, num_n_tiles, num_tiles, k_blocks;
-  int raster_w;        // N tiles per raster panel, 1 .. RASTER_W
-  int a_mn, b_mn;      // 1 = operand is MN-major (M or N contiguous)
-  int out_f32, c_mode; // c_mode: 0 none, 1 bf16, 2 f32
-  void* d;
-  const void* c;
-  long long ldd, ldc, d_batch, c_batch;  // in elements
-  int d_vec, c_vec;                      // 1 = rows are 16-byte aligned, vector access allowed
-  float alpha, beta;
-  int split_k;     // K slices per tile (pair kernel, accumulate-in-place form only); 1 = none
-  int atomic_out;  // 1 = add alpha * partial into D with red.global.add (D already holds C)
-  // Fused SwiGLU epilogues (bf16 [M, N] operands, 16-byte aligned rows):
-  //   1: D = G (the product),           out2 = SiLU(G) * aux0           (aux0 = up projection)
-  //   2: D = SiLU(aux0) * R,            out2 = R * aux1 * dSiLU(aux0)   (R = product, aux0 = gate, aux1 = up)
-  int wide;  // 1 = D, C and the fused operands all have 32-byte aligned rows: 256-bit accesses
-  int epi_mode;
-  const __nv_bfloat16* aux0;
-  const __nv_bfloat16* aux1;
-  __nv_bfloat16* out2;
-  long long ld_aux0, ld_aux1, ld_out2;
-  // Epilogue mode 3, rotate-half RoPE on the heads (128 columns each) below rope_cols:
-  //   d[r, h 128 + i]      = x[i] cos(pos, i) - x[i + 64] sin(pos, i)
-  //   d[r, h 128 + i + 64] = x[i + 64] cos(pos, i) + x[i] sin(pos, i)        (i < 64)
-  // with x the product's row, pos = r % rope_seqlen, or r - cu_seqlens[b] for the sequence b that
-  // holds row r of a ragged batch; the table is f32 [positions, 128] = cos | sin.
-  const float* rope_table;
-  const int* rope_cu;  // cu_seqlens of a ragged batch (device), or nullptr
-  int rope_seqlen, rope_cols, rope_nseq;
-  // Pair kernel: counter of the work units handed out beyond every cluster's first one (zero
-  // between launches; one counter per device and stream).
-  unsigned int* sched_counter;
-  int* status;
-};
 
 struct Barriers {
   uint64_t full[STAGES];
@@ -90,31 +54,6 @@ struct Barriers {
   uint32_t tmem_base;
   int abort_word;
 };
-
-__device__ __forceinline__ void tile_coords(const Params& p, int tile, int& b, int& m, int& n) {
-  const int per_batch = p.num_m_tiles * p.num_n_tiles;
-  b = tile / per_batch;
-  int r = tile - b * per_batch;
-  const int panel_tiles = p.raster_w * p.num_m_tiles;
-  const int panel = r / panel_tiles;
-  const int first_n = panel * p.raster_w;
-  const int width = min(p.raster_w, p.num_n_tiles - first_n);
-  r -= panel * panel_tiles;
-  m = r / width;
-  n = first_n + (r - m * width);
-}
-
-// sigmoid(x) = 0.5 + 0.5 tanh(x / 2): one MUFU operation per element (tanh.approx, relative error
-// about 2^-11, below the bf16 rounding of the outputs).  The reference's fused epilogues use
-// rcp.approx(1 + ex2.approx(-x log2 e)) (crates/cleandl/rust-kernels/src/sky_matmul/
-// tcgen05_bf16.rs:851-854), two MUFU operations; at 16 per clock per SM the 65536 elements of a
-// 256 x 256 tile then cost half the time of the tile's main loop, and the epilogue warps, not the
-// tensor pipe, set the pace of the fused GEMMs.
-__device__ __forceinline__ float fast_sigmoid(float x) {
-  float t;
-  asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(0.5f * x));
-  return fmaf(0.5f, t, 0.5f);
-}
 
 // 32 consecutive columns of one output row, all operands 32-byte aligned: C read, fused
 // SwiGLU or plain conversion, 256-bit stores.

@@ -1,98 +1,426 @@
-// General matmul for the operands the tensor-memory kernels of gemm.cu cannot take: pointers or
-// leading dimensions that are not 16-byte aligned (TMA cannot describe them; the reference hands
-// them to cuBLASLt, tests `unaligned_operands`, crates/cleandl/tests/matmul.rs:604-630) and f32
-// inputs (`f32_tf32_matmul`, tests/matmul.rs:243-265: the reference computes those with TF32
-// tensor cores, 10 mantissa bits; here the products are full f32, which its tolerance contains).
+// Matmul for the operands TMA cannot bring to the tensor cores as they are: bf16 pointers or leading
+// dimensions off the 16-byte grid (the reference hands them to cuBLASLt, tests `unaligned_operands`,
+// crates/cleandl/tests/matmul.rs:604-630) and f32 inputs (`f32_tf32_matmul`, tests/matmul.rs:243-265:
+// the reference computes those with TF32 tensor cores, 10 mantissa bits; here the products are full
+// f32, which its tolerance contains).
 //
-// D = alpha * A . B + beta * C with arbitrary element strides for A and B, f32 accumulation on
-// the CUDA cores.  This is the completeness path, not a fast one: a 64 x 64 tile per CTA of 256
-// threads, 4 x 4 outputs per thread, K in steps of 16 through shared memory with scalar loads.
+// D = alpha * A . B + beta * C, f32 accumulation.  128 x 128 tiles; the K range of a tile is shared by
+// a cluster of 1, 2, 4 or 8 CTAs whose partial sums meet in distributed shared memory (gemm_rows.cuh).
+//   warp 0       issues the tcgen05.mma (M128 N128 K16)
+//   16 loader warps: a warp takes a row of 64 consecutive elements, a lane two of
+//                them, with plain loads of any alignment, and writes them as bf16 into the
+//                128-byte-swizzled tile the tensor core reads; the loads of the next K block are in
+//                flight meanwhile
+//   4 sum warps  add the tensor core's sums of a few K blocks (Params::sum_blocks) to the running sums
+//
+// f32 operands.  A f32 value is the exact sum of three bf16 values (8 significant bits each):
+// x = h + m + l.  Of the nine products of two such sums the six of h.h, h.m, m.h, m.m, h.l and l.h are
+// taken; the others are below 2^-24 of the product.  bf16 products are exact in f32.  The tensor core
+// truncates when it adds, so it only ever sums one K block of 64, the small terms first; the blocks
+// are added with round-to-nearest.
+// A value whose pieces leave bf16's range (inf, NaN, the largest and the smallest magnitudes) has no
+// such sum: a CTA that met one computes its part of the tile again with plain FMAs.
+// Measured error (2-norm, against f64) 1.2e-7 at K = 1024 .. 2048, where a chain of FMAs has 5.7e-7 .. 8.1e-7.
+//
+// What bounds it: the loaders and the shared memory they share with the tensor core (f32: 96 KiB of
+// pieces written and 192 KiB read per K block of 64).  1024 x 2048 x 1536 f32 74 us (87 TFLOP/s; 64 x 64
+// tiles of FMAs on the CUDA cores: 460 us, 14 TFLOP/s); 1500 x 1027 x 2051 bf16 with odd rows 52 us
+// (310 us).
+#include "gemm_rows.cuh"
 #include "host.h"
 #include "ops.h"
 #include "ptx.cuh"
 
+#include <mutex>
+
 namespace cdl {
 namespace gemm_general {
 
-struct Params {
-  const void* a;
-  const void* b;
-  const void* c;  // nullable
-  void* d;
-  long long a_batch, a_row, a_col;  // element strides of A [batch, M, K]
-  long long b_batch, b_row, b_col;  // B [batch, K, N]
-  long long c_batch, c_row;         // C [batch, M, N], last dimension contiguous
-  long long d_batch, d_row;
-  int M, N, K;
-  int c_f32, d_f32;
-  float alpha, beta;
+using gemm::Params;
+
+constexpr int TILE = 128, BK = 64;
+constexpr int PIECE_BYTES = TILE * BK * 2;
+
+// One operand: element (i, k), i an index of M or N, at ptr + batch * s_batch + i * s_mn + k * s_k.
+struct Operand {
+  const void* ptr;
+  long long s_batch, s_mn, s_k;
+  int mn;        // extent of M or N
+  int mn_major;  // 1: rows of the tile run along M or N (contiguous there), 0: along K
+  int pairs;     // 1: every row starts on a pair of elements and is contiguous: one load for two
 };
 
-constexpr int TILE = 64;
-constexpr int KSTEP = 16;
+template <typename T>
+struct Traits;
+template <>
+struct Traits<float> {
+  static constexpr int PIECES = 3, STAGES = 2;
+};
+template <>
+struct Traits<__nv_bfloat16> {
+  static constexpr int PIECES = 1, STAGES = 6;
+};
+constexpr int MAX_STAGES = 6;
+// 21 warps leave 80 registers a thread: a loader holds its 8 rows of A and of B for the next K block.
+constexpr int LOADERS = 16, ROWS = TILE / LOADERS;
+constexpr int WARPS = 1 + LOADERS + 4, THREADS = WARPS * 32;
+constexpr int TMEM_COLS = 512;  // two accumulators and the running sums, 128 columns each
+template <typename T>
+constexpr int stage_bytes() { return 2 * Traits<T>::PIECES * PIECE_BYTES; }
+template <typename T>
+constexpr size_t smem_bytes() { return 1024 + Traits<T>::STAGES * stage_bytes<T>() + 256; }
 
-__device__ __forceinline__ float load_as_f32(const float* p) { return *p; }
-__device__ __forceinline__ float load_as_f32(const __nv_bfloat16* p) { return __bfloat162float(*p); }
+struct Barriers {
+  uint64_t full[MAX_STAGES];
+  uint64_t empty[MAX_STAGES];
+  uint64_t acc_full[2];
+  uint64_t acc_empty[2];
+  uint32_t tmem_base;
+  int abort_word;
+  int outside;  // f32: an element without an exact sum of three bf16 values was met
+};
+static_assert(sizeof(Barriers) <= 256, "barriers fit behind the stages");
+
+// Two elements of a row, as loaded.  Predicated loads in straight-line code: a row's loads wait for
+// nothing, so all of a block's are in flight at once.
+struct PairF32 { uint32_t x, y; };
+struct PairBf16 { uint32_t x, y; };  // x | y << 16 (x: both elements where one load takes them)
+__device__ __forceinline__ uint32_t load32_if(const void* p, int positive) {
+  uint32_t v;
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.gt.s32 p, %2, 0;\n\tmov.b32 %0, 0;\n\t@p ld.global.b32 %0, [%1];\n\t}\n"
+               : "=r"(v)
+               : "l"(p), "r"(positive));
+  return v;
+}
+__device__ __forceinline__ uint32_t load16_if(const void* p, int positive) {
+  uint32_t v;
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.gt.s32 p, %2, 0;\n\tmov.b32 %0, 0;\n\t@p ld.global.u16 %0, [%1];\n\t}\n"
+               : "=r"(v)
+               : "l"(p), "r"(positive));
+  return v;
+}
+__device__ __forceinline__ void load_pair_if(const float* p, PairF32& v, int positive) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.gt.s32 p, %3, 0;\n\tmov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\t"
+      "@p ld.global.v2.b32 {%0, %1}, [%2];\n\t}\n"
+      : "=r"(v.x), "=r"(v.y)
+      : "l"(p), "r"(positive));
+}
+__device__ __forceinline__ void load_pair_if(const __nv_bfloat16* p, PairBf16& v, int positive) {
+  v.x = load32_if(p, positive);
+  v.y = 0;
+}
+__device__ __forceinline__ uint32_t load_one_if(const float* p, int positive) { return load32_if(p, positive); }
+__device__ __forceinline__ uint32_t load_one_if(const __nv_bfloat16* p, int positive) { return load16_if(p, positive); }
+template <typename T>
+struct PairOf { using type = PairF32; };
+template <>
+struct PairOf<__nv_bfloat16> { using type = PairBf16; };
+
+// A loader warp's rows of one operand's tile.
+template <typename T>
+struct RowSource {
+  const T* p;               // this lane's first element of row 0 of the next K block
+  long long row_step, in_step, block_step;
+  int rows, inner;          // rows, and elements of a row, that exist (K-dependent one: of the next block)
+  int mn_major, pairs;
+  __device__ __forceinline__ void init(const Operand& o, int batch, int mn0, int k0, int K, int w, int lane) {
+    mn_major = o.mn_major;
+    pairs = o.pairs;
+    const int r0 = w * ROWS;
+    long long i, k;
+    if (mn_major) {  // rows: 64 K indices of two 64-wide panels
+      i = mn0 + (r0 & ~63) + 2 * lane;
+      k = k0 + (r0 & 63);
+      row_step = o.s_k;
+      in_step = o.s_mn;
+      rows = K - static_cast<int>(k);
+      inner = o.mn - (mn0 + (r0 & ~63));
+    } else {
+      i = mn0 + r0;
+      k = k0 + 2 * lane;
+      row_step = o.s_mn;
+      in_step = o.s_k;
+      rows = o.mn - static_cast<int>(i);
+      inner = K - k0;
+    }
+    block_step = BK * o.s_k;
+    p = static_cast<const T*>(o.ptr) + batch * o.s_batch + i * o.s_mn + k * o.s_k;
+  }
+  // Loads the rows of the next K block (zeros outside the operand) and moves on.
+  __device__ __forceinline__ void load(typename PairOf<T>::type (&v)[ROWS], int lane) {
+    // rows this lane's first and second element exist in
+    const int first = 2 * lane < inner ? rows : 0, second = 2 * lane + 1 < inner ? rows : 0;
+    const T* q = p;
+    if (pairs && (inner >= BK || (inner & 1) == 0)) {
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i, q += row_step) load_pair_if(q, v[i], second - i);
+    } else {
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i, q += row_step) {
+        v[i].x = load_one_if(q, first - i);
+        v[i].y = load_one_if(q + in_step, second - i);
+      }
+    }
+    p += block_step;
+    if (mn_major) rows -= BK;
+    else inner -= BK;
+  }
+};
+
+// Writes a warp's rows into the swizzled tile: row r is 128 bytes, its 16-byte chunk c at c ^ (r & 7).
+// Returns false for an element that is not the sum of its bf16 pieces.
+__device__ __forceinline__ bool store_rows(uint32_t tile, int lane, const PairBf16 (&v)[ROWS]) {
+  const uint32_t chunk = (lane >> 2) << 4, in = (lane & 3) << 2;
+#pragma unroll
+  for (int i = 0; i < ROWS; ++i)
+    asm volatile("st.shared.b32 [%0], %1;" ::"r"(tile + i * 128 + (chunk ^ ((i & 7) << 4)) + in),
+                 "r"(v[i].x | (v[i].y << 16))
+                 : "memory");
+  return true;
+}
+__device__ __forceinline__ bool store_rows(uint32_t tile, int lane, const PairF32 (&v)[ROWS]) {
+  const uint32_t chunk = (lane >> 2) << 4, in = (lane & 3) << 2;
+  bool exact = true;
+#pragma unroll
+  for (int i = 0; i < ROWS; ++i) {
+    const uint32_t at = tile + i * 128 + (chunk ^ ((i & 7) << 4)) + in;
+    const float x = __uint_as_float(v[i].x), y = __uint_as_float(v[i].y);
+    const uint32_t h = pack_bf16x2(x, y);
+    const float rx = x - bf16_lo(h), ry = y - bf16_hi(h);
+    const uint32_t m = pack_bf16x2(rx, ry);
+    const float tx = rx - bf16_lo(m), ty = ry - bf16_hi(m);
+    const uint32_t l = pack_bf16x2(tx, ty);
+    exact = exact && bf16_lo(l) == tx && bf16_hi(l) == ty;  // false for NaN (inf leaves one)
+    asm volatile("st.shared.b32 [%0], %1;" ::"r"(at), "r"(h) : "memory");
+    asm volatile("st.shared.b32 [%0], %1;" ::"r"(at + PIECE_BYTES), "r"(m) : "memory");
+    asm volatile("st.shared.b32 [%0], %1;" ::"r"(at + 2 * PIECE_BYTES), "r"(l) : "memory");
+  }
+  return exact;
+}
+
+// The CTA's part of the tile with plain FMAs (see the top of the file).
+__device__ __noinline__ void partial_by_fma(const Params& p, const Operand& oa, const Operand& ob, int b, int m0,
+                                            int n0, int k_begin, int k_end, float* part) {
+  const float* a = static_cast<const float*>(oa.ptr) + b * oa.s_batch;
+  const float* bb = static_cast<const float*>(ob.ptr) + b * ob.s_batch;
+  for (int e = threadIdx.x; e < TILE * TILE; e += blockDim.x) {
+    const int r = e / TILE, c = e % TILE;
+    if (m0 + r >= p.M || n0 + c >= p.N) continue;
+    const float* ar = a + (m0 + r) * oa.s_mn;
+    const float* bc = bb + (n0 + c) * ob.s_mn;
+    float acc = 0.f;
+    for (int k = k_begin; k < k_end; ++k) acc = fmaf(ar[k * oa.s_k], bc[k * ob.s_k], acc);
+    part[r * gemm::PART_LD + c] = acc;
+  }
+}
+
+template <int S, int W>
+__device__ __forceinline__ void store_out(const Params& p, const float* part, int rank, int warp, int b, int m0,
+                                          int n0) {
+  gemm::TileOut<S, W> out;
+  out.prefetch(p, rank, warp, b, m0, n0);
+  out.finish(p, part, rank, warp, b, m0, n0);
+}
 
 template <typename T>
-__global__ void __launch_bounds__(256) gemm_general_kernel(const Params p) {
-  __shared__ float s_a[KSTEP][TILE + 1];  // [k][m]
-  __shared__ float s_b[KSTEP][TILE + 1];  // [k][n]
-  const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;  // outputs rows ty * 4 .., columns tx * 4 ..
-  const int m0 = blockIdx.y * TILE, n0 = blockIdx.x * TILE;
-  const long long batch = blockIdx.z;
-  const T* a = static_cast<const T*>(p.a) + batch * p.a_batch;
-  const T* b = static_cast<const T*>(p.b) + batch * p.b_batch;
-  float acc[4][4] = {};
-  for (int k0 = 0; k0 < p.K; k0 += KSTEP) {
-    // 64 x 16 elements of each operand, four per thread; a warp walks the operand's rows (A) or
-    // columns (B), whichever index the tile's 64 runs over, so that contiguous operands coalesce
-    // in at least one of their two layouts.
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int e = tid + i * 256;
-      const int kk = e >> 6, mn = e & 63;
-      const int k = k0 + kk;
-      const int m = m0 + mn, n = n0 + mn;
-      s_a[kk][mn] = (k < p.K && m < p.M) ? load_as_f32(a + m * p.a_row + k * p.a_col) : 0.f;
-      s_b[kk][mn] = (k < p.K && n < p.N) ? load_as_f32(b + k * p.b_row + n * p.b_col) : 0.f;
+__global__ void __launch_bounds__(THREADS, 1)
+    gemm_general_kernel(const Params p, const Operand oa, const Operand ob) {
+  using Tr = Traits<T>;
+  constexpr bool F32 = Tr::PIECES == 3;
+  constexpr int STAGES = Tr::STAGES;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                             ~static_cast<uintptr_t>(1023));
+  Barriers* bars = reinterpret_cast<Barriers*>(smem + STAGES * stage_bytes<T>());
+  volatile int* abort_word = &bars->abort_word;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(&bars->full[s], LOADERS);
+      mbar_init(&bars->empty[s], 1);
     }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < KSTEP; ++kk) {
-      float av[4], bv[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        av[i] = s_a[kk][ty * 4 + i];
-        bv[i] = s_b[kk][tx * 4 + i];
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&bars->acc_full[i], 1);
+      mbar_init(&bars->acc_empty[i], 4);
     }
-    __syncthreads();
+    bars->abort_word = 0;
+    bars->outside = 0;
+    fence_mbar_init();
   }
+  if (warp == 0) {
+    tmem_alloc(&bars->tmem_base, TMEM_COLS);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = bars->tmem_base;
+  grid_dep_wait();  // the set-up above overlaps the previous kernel's tail
+  grid_dep_launch();
+
+  const int rank = p.split_k > 1 ? static_cast<int>(cluster_ctarank()) : 0;
+  int b, tm, tn;
+  gemm::tile_coords(p, static_cast<int>(blockIdx.x) / p.split_k, b, tm, tn);
+  const int m0 = tm * TILE, n0 = tn * TILE;
+  const int kb0 = static_cast<int>(static_cast<long long>(rank) * p.k_blocks / p.split_k);
+  const int kb1 = static_cast<int>(static_cast<long long>(rank + 1) * p.k_blocks / p.split_k);
+  const int blocks = kb1 - kb0;  // at least 1: the host never takes more slices than K blocks
+  float* part = reinterpret_cast<float*>(smem);
+
+  if (warp == 0) {
+    // ------------------------------------------------------------ MMA issuer
+    if (elect_one()) {
+      const uint32_t idesc = make_idesc_bf16(TILE, TILE, oa.mn_major, ob.mn_major);
+      const uint32_t a_lbo = oa.mn_major ? 8192u : 16u, b_lbo = ob.mn_major ? 8192u : 16u;
+      const uint32_t a_kstep = oa.mn_major ? 2048u : 32u, b_kstep = ob.mn_major ? 2048u : 32u;
+      for (int it = 0; it < blocks; ++it) {
+        const int s = it % STAGES, group = it / p.sum_blocks, acc = group & 1;
+        const bool first = it == group * p.sum_blocks, last = it + 1 == blocks || it + 1 == (group + 1) * p.sum_blocks;
+        if ((first && !mbar_wait(&bars->acc_empty[acc], ((group >> 1) & 1) ^ 1, abort_word, 231)) ||
+            !mbar_wait(&bars->full[s], (it / STAGES) & 1, abort_word, 232))
+          break;
+        tc_fence_after();
+        const uint32_t sa = smem_u32(smem + s * stage_bytes<T>()), sb = sa + Tr::PIECES * PIECE_BYTES;
+        const uint32_t d = tmem_base + acc * TILE;
+        // pieces (of A, of B), the smallest products first: l.h h.l m.m m.h h.m h.h
+        constexpr int terms = F32 ? 6 : 1;
+        constexpr int pa[6] = {F32 ? 2 : 0, 0, 1, 1, 0, 0}, pb[6] = {0, 2, 1, 0, 1, 0};
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int m = m0 + ty * 4 + i;
-    if (m >= p.M) continue;
+        for (int t = 0; t < terms; ++t)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int n = n0 + tx * 4 + j;
-      if (n >= p.N) continue;
-      float v = p.alpha * acc[i][j];
-      if (p.c != nullptr) {
-        const long long ci = batch * p.c_batch + m * p.c_row + n;
-        v += p.beta * (p.c_f32 ? static_cast<const float*>(p.c)[ci]
-                               : __bfloat162float(static_cast<const __nv_bfloat16*>(p.c)[ci]));
+          for (int k = 0; k < BK / 16; ++k)
+            umma_ss(d, smem_desc_sw128(sa + pa[t] * PIECE_BYTES + k * a_kstep, a_lbo, 1024),
+                    smem_desc_sw128(sb + pb[t] * PIECE_BYTES + k * b_kstep, b_lbo, 1024), idesc,
+                    (!first || (t | k) != 0) ? 1u : 0u);
+        umma_commit(&bars->empty[s]);
+        if (last) umma_commit(&bars->acc_full[acc]);
       }
-      const long long di = batch * p.d_batch + m * p.d_row + n;
-      if (p.d_f32) static_cast<float*>(p.d)[di] = v;
-      else static_cast<__nv_bfloat16*>(p.d)[di] = __float2bfloat16_rn(v);
+    }
+  } else if (warp <= LOADERS) {
+    // ------------------------------------------------------------ loaders
+    const int w = warp - 1;
+    RowSource<T> ra, rb;
+    ra.init(oa, b, m0, kb0 * BK, p.K, w, lane);
+    rb.init(ob, b, n0, kb0 * BK, p.K, w, lane);
+    typename PairOf<T>::type va[ROWS], vb[ROWS];
+    bool exact = true;
+    ra.load(va, lane);
+    rb.load(vb, lane);
+    for (int it = 0; it < blocks; ++it) {
+      const int s = it % STAGES;
+      if (!mbar_wait(&bars->empty[s], ((it / STAGES) & 1) ^ 1, abort_word, 131)) break;
+      const uint32_t sa = smem_u32(smem + s * stage_bytes<T>()) + w * ROWS * 128;
+      exact = store_rows(sa, lane, va) && exact;
+      if (it + 1 < blocks) ra.load(va, lane);
+      exact = store_rows(sa + Tr::PIECES * PIECE_BYTES, lane, vb) && exact;
+      if (it + 1 < blocks) rb.load(vb, lane);
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars->full[s]);
+    }
+    if (!exact) bars->outside = 1;
+  }
+  if (warp > LOADERS) {
+    // ------------------------------------------------------------ running sums: thread = row
+    // They live in tensor memory beside the two accumulators of the K blocks: 128 columns per thread
+    // in registers would leave the loader warps too few.
+    const int quad = warp & 3;
+    const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
+    const int groups = (blocks + p.sum_blocks - 1) / p.sum_blocks;
+    for (int g = 0; g < groups; ++g) {
+      const int acc = g & 1;
+      if (!mbar_wait(&bars->acc_full[acc], (g >> 1) & 1, abort_word, 331)) break;
+      tc_fence_after();
+      const bool last = g + 1 == groups;
+#pragma unroll
+      for (int c = 0; c < TILE; c += 32) {
+        uint32_t r[32], t[32];
+        tmem_ld32(t_row + acc * TILE + c, r);
+        if (g > 0) {
+          tmem_ld32(t_row + 2 * TILE + c, t);
+          tmem_wait_ld();
+#pragma unroll
+          for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(t[j]) + __uint_as_float(r[j]));
+        } else {
+          tmem_wait_ld();
+        }
+        if (last) {
+          // Every product is done and every stage read: the partial tile takes their place.
+          float v[32];
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+          gemm::store_partial(part, quad * 32 + lane, c, v);
+        } else {
+          tmem_st32(t_row + 2 * TILE + c, r);
+        }
+      }
+      tmem_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars->acc_empty[acc]);
     }
   }
+  __syncwarp();
+  if (F32) {
+    __syncthreads();
+    if (bars->outside != 0)
+      partial_by_fma(p, oa, ob, b, m0, n0, kb0 * BK, min(kb1 * BK, p.K), part);
+  }
+  if (p.split_k > 1) cluster_sync_all();
+  else __syncthreads();
+  if (warp >= 1) {
+    switch (p.split_k) {
+      case 1: store_out<1, WARPS - 1>(p, part, rank, warp - 1, b, m0, n0); break;
+      case 2: store_out<2, WARPS - 1>(p, part, rank, warp - 1, b, m0, n0); break;
+      case 4: store_out<4, WARPS - 1>(p, part, rank, warp - 1, b, m0, n0); break;
+      default: store_out<8, WARPS - 1>(p, part, rank, warp - 1, b, m0, n0); break;
+    }
+  }
+  __syncwarp();
+  if (p.split_k > 1) cluster_sync_all();  // the other slices have read this CTA's partial
+  else __syncthreads();
+  if (warp == 0) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, TMEM_COLS);
+  }
+  if (threadIdx.x == 0 && *abort_word != 0) atomicExch(p.status, *abort_word);
+}
+
+// K slices per tile: the number whose waves of resident CTAs end first.  A CTA's time is its K blocks
+// and a part that does not shrink (set-up, first loads, the exchange of the partial sums, stores).
+// f32 300 x 2048 x 130 with 1, 2, 4, 8 slices: 69, 39, 24, 17 us; 1024 x 2048 x 1536 74, 81, 76, 121 us.
+static int choose_splits(long long tiles, int k_blocks, int slots, double fixed) {
+  int best = 1;
+  double best_cost = 1e30;
+  for (int s = 1; s <= gemm::MAX_SPLITS && s <= k_blocks; s *= 2) {
+    const long long waves = (tiles * s + slots - 1) / slots;
+    const double cost = static_cast<double>(waves) * (static_cast<double>((k_blocks + s - 1) / s) + fixed);
+    if (cost < best_cost * 0.97) {
+      best_cost = cost;
+      best = s;
+    }
+  }
+  return best;
+}
+
+template <typename T>
+static int32_t launch(Params& p, const Operand& oa, const Operand& ob, double fixed, cudaStream_t stream) {
+  using Tr = Traits<T>;
+  static std::once_flag once[64];
+  int dev = 0;
+  CDL_CUDA(cudaGetDevice(&dev));
+  cudaError_t err = cudaSuccess;
+  std::call_once(once[dev & 63], [&] {
+    err = cudaFuncSetAttribute(gemm_general_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               static_cast<int>(smem_bytes<T>()));
+  });
+  if (err != cudaSuccess) return fail(CDL_ERR_CUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(err));
+  p.split_k = choose_splits(p.num_tiles, p.k_blocks, sm_count(), fixed);
+  CDL_CUDA(launch_pdl_cluster(gemm_general_kernel<T>, dim3(static_cast<unsigned>(p.num_tiles) * p.split_k),
+                              dim3(THREADS), smem_bytes<T>(), p.split_k, stream, p, oa, ob));
+  return CDL_OK;
 }
 
 }  // namespace gemm_general
@@ -104,39 +432,63 @@ int32_t matmul_general_execute(const cdl_tensor* a, const cdl_tensor* b, const c
   using namespace gemm_general;
   const int r = a->rank;
   const long long batch = r == 3 ? a->shape[0] : 1;
+  const long long M = a->shape[r - 2], K = a->shape[r - 1], N = b->shape[r - 1];
+  if (M > 65535LL * 64)
+    return fail(CDL_ERR_UNSUPPORTED, "matmul (general path): more than %d rows", 65535 * 64);
+  auto operand = [&](const cdl_tensor* t, int mn_dim, int k_dim) {
+    Operand o{};
+    o.ptr = t->ptr;
+    o.mn = static_cast<int>(t->shape[mn_dim]);
+    o.s_batch = r == 3 ? t->stride[0] : 0;
+    // an extent of 1 has no meaningful stride
+    o.s_mn = t->shape[mn_dim] > 1 ? t->stride[mn_dim] : 0;
+    o.s_k = t->shape[k_dim] > 1 ? t->stride[k_dim] : 0;
+    o.mn_major = o.s_k != 1 && o.s_mn == 1;
+    const long long inner = o.mn_major ? o.s_mn : o.s_k, outer = o.mn_major ? o.s_k : o.s_mn;
+    o.pairs = inner == 1 && outer % 2 == 0 && o.s_batch % 2 == 0 &&
+              reinterpret_cast<uintptr_t>(t->ptr) % (2 * dtype_size(t->dtype)) == 0;
+    return o;
+  };
+  const Operand oa = operand(a, r - 2, r - 1), ob = operand(b, r - 1, r - 2);
   Params p{};
-  p.a = a->ptr;
-  p.b = b->ptr;
+  p.M = static_cast<int>(M);
+  p.N = static_cast<int>(N);
+  p.K = static_cast<int>(K);
+  p.batch = static_cast<int>(batch);
+  p.num_m_tiles = static_cast<int>((M + TILE - 1) / TILE);
+  p.num_n_tiles = static_cast<int>((N + TILE - 1) / TILE);
+  const long long tiles = batch * p.num_m_tiles * p.num_n_tiles;
+  if (tiles > INT32_MAX / gemm::MAX_SPLITS) return fail(CDL_ERR_UNSUPPORTED, "matmul: too many tiles");
+  p.num_tiles = static_cast<int>(tiles);
+  p.k_blocks = static_cast<int>((K + BK - 1) / BK);
+  p.raster_w = gemm::RASTER_W;
   p.d = d->ptr;
-  p.M = static_cast<int>(a->shape[r - 2]);
-  p.K = static_cast<int>(a->shape[r - 1]);
-  p.N = static_cast<int>(b->shape[r - 1]);
-  p.a_batch = r == 3 ? a->stride[0] : 0;
-  p.a_row = a->stride[r - 2];
-  p.a_col = a->stride[r - 1];
-  p.b_batch = r == 3 ? b->stride[0] : 0;
-  p.b_row = b->stride[r - 2];
-  p.b_col = b->stride[r - 1];
+  p.ldd = M > 1 ? d->stride[r - 2] : N;
   p.d_batch = r == 3 ? d->stride[0] : 0;
-  p.d_row = d->stride[r - 2];
-  p.d_f32 = d->dtype == CDL_F32 ? 1 : 0;
+  p.out_f32 = d->dtype == CDL_F32 ? 1 : 0;
+  auto vec_ok = [](const void* ptr, long long ld, long long bstride, size_t es) {
+    return (reinterpret_cast<uintptr_t>(ptr) & 15) == 0 && (ld * es) % 16 == 0 && (bstride * es) % 16 == 0;
+  };
+  p.d_vec = vec_ok(p.d, p.ldd, p.d_batch, dtype_size(d->dtype));
   if (c != nullptr && beta != 0.0f) {
     p.c = c->ptr;
+    p.ldc = M > 1 ? c->stride[r - 2] : N;
     p.c_batch = r == 3 ? c->stride[0] : 0;
-    p.c_row = c->stride[r - 2];
-    p.c_f32 = c->dtype == CDL_F32 ? 1 : 0;
+    p.c_mode = c->dtype == CDL_F32 ? 2 : 1;
+    p.c_vec = vec_ok(p.c, p.ldc, p.c_batch, dtype_size(c->dtype));
+    p.beta = beta;
   }
   p.alpha = alpha;
-  p.beta = beta;
-  const dim3 grid(static_cast<unsigned>((p.N + TILE - 1) / TILE),
-                  static_cast<unsigned>((p.M + TILE - 1) / TILE), static_cast<unsigned>(batch));
-  if (grid.y > 65535)
-    return fail(CDL_ERR_UNSUPPORTED, "matmul (general path): more than %d rows", 65535 * TILE);
-  ProfileScope ps(PROF_GEMM, 2.0 * batch * p.M * p.N * p.K, stream);
-  if (a->dtype == CDL_F32) gemm_general_kernel<float><<<grid, 256, 0, stream>>>(p);
-  else gemm_general_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(p);
-  CDL_CUDA(cudaGetLastError());
-  return CDL_OK;
+  p.status = device_status_ptr();
+  if (!p.status) return fail(CDL_ERR_CUDA, "cannot resolve the device status word");
+  // A tensor-core accumulator loses about 2^-26 of its value to truncation per step of 16 products
+  // (measured: 6.6e-8 after one K block, 4.7e-7 after eight), a chain of f32 FMAs 3.2e-7 at K = 1500: where
+  // the result is f32 every K block is added to the running sums by itself; a bf16 result, rounded to 2^-9,
+  // takes eight at a time.
+  p.sum_blocks = d->dtype == CDL_F32 || a->dtype == CDL_F32 ? 1 : 8;
+  ProfileScope ps(PROF_GEMM, 2.0 * batch * M * N * K, stream);
+  return a->dtype == CDL_F32 ? launch<float>(p, oa, ob, 4.0, stream)
+                             : launch<__nv_bfloat16>(p, oa, ob, 6.0, stream);
 }
 
 }  // namespace cdl

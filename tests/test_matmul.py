@@ -287,3 +287,64 @@ def test_fused_swiglu_epilogues(cdl, gpu_ok, m, n, k):
     g = gate_in.double()
     assert rel(d_up, g * sig(g) * prod) <= 2.0 ** -6
     assert rel(d_gate, prod * up.double() * (sig(g) + g * sig(g) * (1 - sig(g)))) <= 2.0 ** -6
+
+
+F32_FORMS = ["row", "col", "strided"]
+
+
+def _f32_operand(gen, rows, cols, form):
+    """[rows, cols]: rows contiguous, columns contiguous, or neither (odd strides, odd start)."""
+    if form == "row":
+        return torch.randn(rows, cols + 1, generator=gen)[:, 1:]
+    if form == "col":
+        return torch.randn(cols, rows, generator=gen).T
+    return torch.randn(rows, 3 * cols, generator=gen)[:, 1::3]
+
+
+@pytest.mark.parametrize("m,k,n", [(1, 1, 1), (5, 64, 3), (128, 63, 128), (129, 65, 130), (130, 513, 257), (64, 2048, 70)])
+@pytest.mark.parametrize("fa,fb", [("row", "row"), ("col", "row"), ("row", "col"), ("strided", "strided"), ("col", "strided")])
+def test_f32_products_are_f32(cdl, gpu_ok, m, k, n, fa, fb):
+    """f32 operands of every layout, edges of the 128 x 128 tile and of the 64-wide K block, K shared by
+    1 to 8 CTAs, against f64.  Bound: the dropped products (below 2^-24 each, two of them per term), the
+    truncated sums inside a K block (4 steps of 16 at full size, 2^-23 each) and the rounded additions
+    of at most K / 64 blocks (2^-24 each) are all relative to sum |a b|."""
+    gen = torch.Generator().manual_seed(m + k + n)
+    a, b = _f32_operand(gen, m, k, fa), _f32_operand(gen, k, n, fb)
+
+    def to_dev(t):
+        base = torch.empty(0, dtype=t.dtype).set_(t.untyped_storage())
+        return base.cuda().as_strided(t.shape, t.stride(), t.storage_offset())
+
+    d = cdl.ops.matmul(to_dev(a), to_dev(b), cdl.ops.MatmulOpts(out=torch.float32))
+    expected, bound = a.double() @ b.double(), a.abs().double() @ b.abs().double()
+    tol = (2 * 2.0 ** -24 + 4 * 2.0 ** -23 + (k / 64 + 2) * 2.0 ** -24) * bound + 1e-30
+    assert_all_close("f32 product", d.double().cpu().numpy(), expected.numpy(), tol.numpy())
+
+
+def test_f32_values_without_bf16_pieces(cdl, gpu_ok):
+    """inf, NaN, values at the top of the range and tiny ones give what f32 arithmetic gives."""
+    gen = torch.Generator().manual_seed(31)
+    a, b = torch.randn(200, 300, generator=gen), torch.randn(300, 150, generator=gen)
+    a[3, 7], a[5, 9], a[150, 2] = float("inf"), float("nan"), 3.4e38
+    a[10] *= 1e-36
+    b[:, 149] *= 1e-36
+    b[2] *= 1e-3
+    d = cdl.ops.matmul(a.cuda(), b.cuda(), cdl.ops.MatmulOpts(out=torch.float32)).cpu()
+    expected = (a.double() @ b.double())
+    assert torch.equal(d.isnan(), expected.isnan()) and torch.equal(d.isinf(), expected.isinf())
+    ok = expected.isfinite()
+    bound = (a.abs().double() @ b.abs().double())
+    err = (d.double() - expected).abs()
+    # the products of row 10 and column 149 are below 1e-70: zero in f32
+    assert bool((err[ok] <= 400 * 2.0 ** -24 * bound[ok] + 2.0 ** -126).all())
+
+
+@pytest.mark.parametrize("m,k,n", [(1, 65, 3), (127, 131, 129), (130, 1027, 257)])
+def test_unaligned_bf16_layouts(cdl, gpu_ok, m, k, n):
+    """Odd leading dimensions with K or M / N contiguous in either operand, accumulating into C."""
+    gen = torch.Generator().manual_seed(m)
+    for ta, tb in ((False, False), (True, False), (False, True), (True, True)):
+        a = rand_bf16(gen, k, m + (m + 1) % 2).T[:m] if ta else rand_bf16(gen, m, k)
+        b = rand_bf16(gen, n, k).T if tb else rand_bf16(gen, k, n)
+        run_case(cdl, a, b, torch.bfloat16)
+        run_case(cdl, a, b, torch.float32, c=torch.randn(m, n, generator=gen), alpha=0.5, beta=1.0, in_place=True)
