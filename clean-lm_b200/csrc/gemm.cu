@@ -22,6 +22,7 @@
 #include "ops.h"
 #include "ptx.cuh"
 
+#include <math.h>
 #include <stdlib.h>
 #include <string.h>
 
@@ -838,6 +839,50 @@ static int32_t analyze_operand(const char* name, const cdl_tensor* t, bool contr
   return CDL_OK;
 }
 
+// K slices (1, 2, 4 or 8) of the cluster kernel (gemm_cluster.cu) for a problem, or 0: the 256 x 256
+// tiles of the pair kernel (128 x 256 up to 128 rows).  Both times are estimated, in microseconds, and
+// the shorter one taken.  A cluster CTA costs a launch, an exchange and a store (more with more slices
+// to meet; c8 stands out because a GPC holds few clusters of 8) and 0.23 us per K block, unless all
+// blocks together keep the SMs busy for longer (0.32 us per block and SM); CTAs beyond one per SM add
+// their own launch and store.  A tile pair takes 0.34 us per K block, which no further tile shares until
+// the 74 pairs are used up.  Fitted to 66 shapes (16 to 2048 rows, K 64 to 8192, N 128 to 32768): the
+// choice is 0.3 % from the best on average, 6 % at worst.  In microseconds, pair -> cluster: 64 x 5632 x
+// 2048 36.1 -> 12.0 (4 slices), 256 x 2048 x 2048 15.4 -> 9.2 (4), 256 x 2048 x 6144 15.8 -> 13.4 (1),
+// 512 x 5632 x 2048 31.8 -> 16.9 (2); the other way at 2048 x 2048 x 2048, 17.2 against 19.1.
+static int choose_cluster_splits(long long batch, long long M, long long N, long long K, bool adds_f32,
+                                 bool may_slice) {
+  auto up = [](long long a, long long b) { return (a + b - 1) / b; };
+  const double kb = static_cast<double>(up(K, BK));
+  const double sms = sm_count();
+  const long long pair_tiles = batch * (M <= BM ? 1 : up(M, PAIR_M)) * up(N, BN);
+  const long long pair_slots = M <= BM ? sm_count() : sm_count() / 2;
+  double best = 1e30;
+  for (int s = 1; s <= (may_slice ? 8 : 1) && (s == 1 || s * 8 <= kb); ++s) {
+    const double waves = static_cast<double>(up(pair_tiles * s, pair_slots)), loop = 0.34 * kb / s + 1.9;
+    // An f32 C that is read and added to costs 8 us a tile, which a long main loop hides; slices add with
+    // reductions, 7 us on top of the main loop.
+    const double t = !adds_f32 ? 3.0 + waves * loop
+                     : s == 1  ? 8.0 + waves * sqrt(loop * loop + 64.0)
+                               : 3.0 + waves * (loop + 7.0);
+    if (t < best) best = t;
+  }
+  const long long tiles = batch * up(M, 128) * up(N, CLUSTER_TILE_N);
+  if (tiles > (1 << 20)) return 0;
+  const double per_cta[4] = {4.4, 5.5, 6.7, 10.4};
+  int splits = 0;
+  for (int i = 0; i < 4 && (1 << i) <= kb; ++i) {
+    const double ctas = static_cast<double>(tiles << i);
+    const double deep = 0.23 * kb / (1 << i), wide = (may_slice ? 0.25 : 0.32) * static_cast<double>(tiles) * kb / sms;
+    double t = per_cta[i] + (deep > wide ? deep : wide) + (ctas > sms ? 3.1 * (ctas / sms - 1.0) : 0.0);
+    if (adds_f32) t += (may_slice ? 1.7 : 2.6) * (static_cast<double>(tiles) > sms ? static_cast<double>(tiles) / sms : 1.0);
+    if (t < best) {
+      best = t;
+      splits = 1 << i;
+    }
+  }
+  return splits;
+}
+
 }  // namespace gemm
 
 static int32_t check_epi_operand(const char* name, const cdl_tensor* t, long long M, long long N) {
@@ -914,11 +959,20 @@ int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_t
     CDL_CHECK(rc);
   }
 
-  // Kernel choice: CTA pairs (256 x 256 tiles) whenever the problem has more than one 128-row
-  // slab, unless the caller's options name a variant.
-  const bool use_pair = variant == CDL_GEMM_AUTO ? M > BM : variant == CDL_GEMM_CTA_PAIR;
+  // Kernel choice, unless the caller's options name a variant: clusters that share a tile's K range where
+  // that is estimated to be faster, else CTA pairs (256 x 256 tiles) whenever the problem has more
+  // than one 128-row slab.
+  // The weight-gradient form D = C + A^T B, f32 in place, may add K slices into D with atomics.
+  const bool adds_f32 = use_c && c->dtype == CDL_F32;
+  const bool may_slice = adds_f32 && d->dtype == CDL_F32 && c->ptr == d->ptr && beta == 1.0f &&
+                         !(opts && opts->deterministic != 0);
+  const int cluster_splits =
+      variant == CDL_GEMM_AUTO ? choose_cluster_splits(batch, M, N, K, adds_f32, may_slice) : 0;
+  const bool use_cluster = cluster_splits > 0;
+  const bool use_pair = !use_cluster && (variant == CDL_GEMM_AUTO ? M > BM : variant == CDL_GEMM_CTA_PAIR);
   const int tile_m = use_pair ? PAIR_M : BM;
-  const uint32_t b_box_rows = use_pair ? BN / 2 : BN;
+  const int tile_n = use_cluster ? CLUSTER_TILE_N : BN;
+  const uint32_t b_box_rows = use_pair ? BN / 2 : tile_n;
 
   CUtensorMap tm_a, tm_b;
   {
@@ -949,7 +1003,7 @@ int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_t
   p.K = static_cast<int>(K);
   p.batch = static_cast<int>(batch);
   p.num_m_tiles = static_cast<int>((M + tile_m - 1) / tile_m);
-  p.num_n_tiles = static_cast<int>((N + BN - 1) / BN);
+  p.num_n_tiles = static_cast<int>((N + tile_n - 1) / tile_n);
   const long long tiles = batch * p.num_m_tiles * p.num_n_tiles;
   if (tiles > INT32_MAX) return fail(CDL_ERR_UNSUPPORTED, "matmul: too many tiles");
   p.num_tiles = static_cast<int>(tiles);
@@ -986,7 +1040,7 @@ int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_t
   p.c_vec = use_c ? vec_ok(p.c, p.ldc, p.c_batch, dtype_size(c->dtype)) : 0;
   p.alpha = alpha;
   p.beta = use_c ? beta : 0.0f;
-  p.split_k = 1;
+  p.split_k = use_cluster ? cluster_splits : 1;
   p.sched_counter = nullptr;
   p.atomic_out = 0;
   p.epi_mode = 0;
@@ -1044,6 +1098,18 @@ int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_t
   }
   p.status = device_status_ptr();
   if (!p.status) return fail(CDL_ERR_CUDA, "cannot resolve the device status word");
+
+  if (use_cluster) {
+    // D += A^T B: every element is added to once, by a reduction at the L2, instead of read, added to and
+    // written: 2048 x 5632 x 256 29 us instead of 34, 512 x 1536 x 256 5.6 instead of 7.7.  (In the pair
+    // kernel, where a thread's reductions run along a row, the same costs 42 us instead of 34.)
+    if (may_slice && p.ldc == p.ldd && p.c_batch == p.d_batch && p.d_vec && N % 4 == 0) {
+      p.atomic_out = 1;
+      p.c_mode = 0;
+    }
+    ProfileScope ps(PROF_GEMM, 2.0 * static_cast<double>(batch) * M * N * K, stream);
+    return gemm_cluster_launch(tm_a, tm_b, p, stream);
+  }
 
   static std::once_flag attr_once[64];
   static int max_clusters[64] = {};

@@ -1,0 +1,210 @@
+// BF16 GEMM for problems that leave the 256 x 256 tiles of gemm.cu short of work: few rows (decoding,
+// short sequences, small microbatches) or a small output.  Same operands and epilogues, 128 x 128
+// tiles, and each tile's K range shared by a cluster of 1, 2, 4 or 8 CTAs whose partial sums meet in
+// distributed shared memory (gemm_rows.cuh).
+//
+// What bounds these problems is the weights' way from HBM: a [2048, 5632] matrix is 23 MB, 3.5 us at
+// the copy bandwidth, but only if every SM keeps loads in flight; 64 rows against it are 22 tiles of
+// 128 x 256.  So the split is chosen for the number of SMs that load (choose_cluster_splits in gemm.cu),
+// two CTAs can share an SM (or one has twice the operand stages), and K slices meet on chip: no scratch
+// memory, no atomics, no second launch, a fixed order of the sums.
+#include "gemm_rows.cuh"
+#include "host.h"
+#include "ops.h"
+#include "ptx.cuh"
+
+#include <mutex>
+
+namespace cdl {
+namespace gemm {
+namespace {
+
+constexpr int TILE_M = 128, TILE_N = CLUSTER_TILE_N, BK = 64;
+constexpr int A_BYTES = TILE_M * BK * 2, B_BYTES = TILE_N * BK * 2;
+constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+// Eight warps, all of which drain the accumulator and store; before that one lane of warp 0 issues the
+// loads and one of warp 1 the MMAs.  With two CTAs per SM that leaves 128 registers a thread, which
+// the 16 prefetched rows of an unsplit tile need.
+constexpr int WARPS = 8, THREADS = WARPS * 32;
+constexpr int TMEM_COLS = 128;
+// Operand stages: 3 where two CTAs share an SM, 6 where every CTA has an SM to itself; either way an SM
+// keeps 192 KiB of loads in flight.
+constexpr int SHARED_STAGES = 3, ALONE_STAGES = 6;
+constexpr size_t smem_bytes(int stages) { return 1024 + stages * STAGE_BYTES + 128; }
+static_assert(PART_BYTES <= SHARED_STAGES * STAGE_BYTES, "the partial tile takes the place of the operand stages");
+
+struct Barriers {
+  uint64_t full[ALONE_STAGES];
+  uint64_t empty[ALONE_STAGES];
+  uint64_t acc_full;
+  uint32_t tmem_base;
+  int abort_word;
+};
+static_assert(sizeof(Barriers) <= 128, "barriers fit behind the stages");
+
+template <int S, int STAGES>
+__global__ void __launch_bounds__(THREADS, STAGES == SHARED_STAGES ? 2 : 1)
+    gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
+                        const Params p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                             ~static_cast<uintptr_t>(1023));
+  Barriers* bars = reinterpret_cast<Barriers*>(smem + STAGES * STAGE_BYTES);
+  volatile int* abort_word = &bars->abort_word;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(&bars->full[s], 1);
+      mbar_init(&bars->empty[s], 1);
+    }
+    mbar_init(&bars->acc_full, 1);
+    bars->abort_word = 0;
+    fence_mbar_init();
+    tma_prefetch_desc(&tmap_a);
+    tma_prefetch_desc(&tmap_b);
+  }
+  if (warp == 1) {
+    tmem_alloc(&bars->tmem_base, TMEM_COLS);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = bars->tmem_base;
+  grid_dep_wait();  // the set-up above overlaps the previous kernel's tail
+  grid_dep_launch();
+
+  // One (tile, K slice) per CTA; the slices of a tile are one cluster.
+  const int rank = S > 1 ? static_cast<int>(cluster_ctarank()) : 0;
+  int b, tm, tn;
+  tile_coords(p, static_cast<int>(blockIdx.x) / S, b, tm, tn);
+  const int m0 = tm * TILE_M, n0 = tn * TILE_N;
+  const int kb0 = static_cast<int>(static_cast<long long>(rank) * p.k_blocks / S);
+  const int kb1 = static_cast<int>(static_cast<long long>(rank + 1) * p.k_blocks / S);
+  float* part = reinterpret_cast<float*>(smem);
+  TileOut<S, WARPS> tile_out;
+
+  if (warp == 0) {
+    if (elect_one()) {
+      for (int kb = kb0; kb < kb1; ++kb) {
+        const int it = kb - kb0, s = it % STAGES;
+        if (!mbar_wait(&bars->empty[s], ((it / STAGES) & 1) ^ 1, abort_word, 121)) break;
+        uint8_t* sa = smem + s * STAGE_BYTES;
+        uint8_t* sb = sa + A_BYTES;
+        mbar_arrive_expect_tx(&bars->full[s], STAGE_BYTES);
+        const int k0 = kb * BK;
+        if (p.a_mn) {
+#pragma unroll
+          for (int i = 0; i < TILE_M / 64; ++i)
+            tma_load_3d(sa + i * 8192, &tmap_a, &bars->full[s], m0 + i * 64, k0, b);
+        } else {
+          tma_load_3d(sa, &tmap_a, &bars->full[s], k0, m0, b);
+        }
+        if (p.b_mn) {
+#pragma unroll
+          for (int i = 0; i < TILE_N / 64; ++i)
+            tma_load_3d(sb + i * 8192, &tmap_b, &bars->full[s], n0 + i * 64, k0, b);
+        } else {
+          tma_load_3d(sb, &tmap_b, &bars->full[s], k0, n0, b);
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (elect_one()) {
+      const uint32_t idesc = make_idesc_bf16(TILE_M, TILE_N, p.a_mn, p.b_mn);
+      const uint32_t a_lbo = p.a_mn ? 8192u : 16u, b_lbo = p.b_mn ? 8192u : 16u;
+      const uint32_t a_kstep = p.a_mn ? 2048u : 32u, b_kstep = p.b_mn ? 2048u : 32u;
+      bool ok = true;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        const int it = kb - kb0, s = it % STAGES;
+        if (!mbar_wait(&bars->full[s], (it / STAGES) & 1, abort_word, 221)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t sa = smem_u32(smem + s * STAGE_BYTES), sb = sa + A_BYTES;
+#pragma unroll
+        for (int k = 0; k < BK / 16; ++k)
+          umma_ss(tmem_base, smem_desc_sw128(sa + k * a_kstep, a_lbo, 1024),
+                  smem_desc_sw128(sb + k * b_kstep, b_lbo, 1024), idesc, (it | k) != 0 ? 1u : 0u);
+        umma_commit(&bars->empty[s]);
+      }
+      if (ok) umma_commit(&bars->acc_full);
+    }
+  }
+  __syncwarp();
+  tile_out.prefetch(p, rank, warp, b, m0, n0);
+  {
+    // After this wait every product is done and the operand stages are free: the partial tile goes there.
+    const bool ok = mbar_wait(&bars->acc_full, 0, abort_word, 321);
+    tc_fence_after();
+    const int row = (warp & 3) * 32 + lane, half = warp >> 2;
+    if (ok && m0 + (warp & 3) * 32 < p.M) {
+#pragma unroll
+      for (int c = half * 64; c < half * 64 + 64; c += 16) {
+        uint32_t r[16];
+        tmem_ld16(tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + c, r);
+        tmem_wait_ld();
+        float v[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
+        store_partial(part, row, c, v);
+      }
+    }
+    tc_fence_before();
+  }
+  __syncwarp();
+  if (*abort_word != 0) {
+    // Loads that may still be in flight land before shared memory is used again or released.
+    const unsigned long long t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
+  }
+  if (S > 1) cluster_sync_all();
+  else __syncthreads();
+  tile_out.finish(p, part, rank, warp, b, m0, n0);
+  __syncwarp();
+  if (S > 1) cluster_sync_all();  // the other slices have read this CTA's partial
+  else __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, TMEM_COLS);
+  }
+  if (threadIdx.x == 0 && *abort_word != 0) atomicExch(p.status, *abort_word);
+}
+
+template <int S, int STAGES>
+int32_t launch(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const Params& p, int dev, cudaStream_t stream) {
+  static std::once_flag once[64];
+  cudaError_t err = cudaSuccess;
+  std::call_once(once[dev & 63], [&] {
+    err = cudaFuncSetAttribute(gemm_cluster_kernel<S, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               static_cast<int>(smem_bytes(STAGES)));
+  });
+  if (err != cudaSuccess) return fail(CDL_ERR_CUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(err));
+  CDL_CUDA(launch_pdl_cluster(gemm_cluster_kernel<S, STAGES>, dim3(static_cast<unsigned>(p.num_tiles) * S),
+                              dim3(THREADS), smem_bytes(STAGES), S, stream, tm_a, tm_b, p));
+  return CDL_OK;
+}
+template <int S>
+int32_t launch(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const Params& p, int dev, cudaStream_t stream) {
+  return static_cast<long long>(p.num_tiles) * S <= sm_count() ? launch<S, ALONE_STAGES>(tm_a, tm_b, p, dev, stream)
+                                                               : launch<S, SHARED_STAGES>(tm_a, tm_b, p, dev, stream);
+}
+
+}  // namespace
+
+int32_t gemm_cluster_launch(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const Params& p,
+                            cudaStream_t stream) {
+  int dev = 0;
+  CDL_CUDA(cudaGetDevice(&dev));
+  switch (p.split_k) {
+    case 1: return launch<1>(tm_a, tm_b, p, dev, stream);
+    case 2: return launch<2>(tm_a, tm_b, p, dev, stream);
+    case 4: return launch<4>(tm_a, tm_b, p, dev, stream);
+    default: return launch<8>(tm_a, tm_b, p, dev, stream);
+  }
+}
+
+}  // namespace gemm
+}  // namespace cdl

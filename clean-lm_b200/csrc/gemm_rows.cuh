@@ -1,5 +1,5 @@
 // What the bf16 GEMM kernels share: the problem description and the row-wise epilogue of the kernels
-// whose K slices meet inside a thread-block cluster (gemm_general.cu).
+// whose K slices meet inside a thread-block cluster (gemm_cluster.cu, gemm_general.cu).
 #pragma once
 #include "ptx.cuh"
 
@@ -19,8 +19,8 @@ struct Params {
   long long ldd, ldc, d_batch, c_batch;  // in elements
   int d_vec, c_vec;                      // 1 = rows are 16-byte aligned, vector access allowed
   float alpha, beta;
-  int split_k;     // K slices per tile (pair kernel: accumulate-in-place form only; gemm_general.cu:
-                   // CTAs per cluster); 1 = none
+  int split_k;     // K slices per tile (pair kernel: accumulate-in-place form only; cluster kernels: CTAs
+                   // per cluster); 1 = none
   int sum_blocks;  // gemm_general.cu: K blocks that one tensor-core accumulator sums up
   int atomic_out;  // 1 = add alpha * partial into D with red.global.add (D already holds C)
   // Fused SwiGLU epilogues (bf16 [M, N] operands, 16-byte aligned rows):
@@ -70,6 +70,12 @@ __device__ __forceinline__ float fast_sigmoid(float x) {
   asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(0.5f * x));
   return fmaf(0.5f, t, 0.5f);
 }
+
+// gemm_cluster.cu.  p.split_k = 1, 2, 4 or 8; tensor maps with boxes of 128 rows (K-major operands) or
+// 64 x 64 (MN-major).
+constexpr int CLUSTER_TILE_N = 128;
+int32_t gemm_cluster_launch(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const Params& p,
+                            cudaStream_t stream);
 
 // ------------------------------------------------------------------ K slices that meet in a cluster
 // A cluster of `splits` CTAs holds the partial sums of one 128 x 128 tile, one K slice per CTA.  Every
@@ -178,17 +184,6 @@ struct TileOut {
     const int col = n0 + lane * 4;
     if (!vec(p)) return;
     if (col < p.N) load_extra(p, rank + S * warp, b, m0, col);
-    if (p.c_mode == 2) {
-      // f32 C (the weight-gradient form: as many bytes as the output): the later batches' lines, four to
-      // a row, start their way to L2 as well.
-#pragma unroll
-      for (int i = 0; i < 128 / STEP; i += 8) {
-        const int r = rank + S * (warp + W * (i + (lane >> 2)));
-        if (r < 128 && m0 + r < p.M && n0 + (lane & 3) * 32 < p.N)
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const float*>(p.c) + b * p.c_batch +
-                                                        (m0 + r) * p.ldc + n0 + (lane & 3) * 32));
-      }
-    }
   }
 
   __device__ __forceinline__ void finish(const Params& p, const float* part, int rank, int warp, int b, int m0,
@@ -258,7 +253,15 @@ struct TileOut {
           }
         }
         if (p.epi_mode == 1 || p.epi_mode == 2) store_swiglu(p, v, r0, rows, m0, col);
-        else if (p.out_f32) {
+        else if (p.atomic_out) {
+          float* d = static_cast<float*>(p.d) + b * p.d_batch + m0 * p.ldd + col;
+#pragma unroll
+          for (int i = 0; i < BATCH; ++i)
+            if (r0 + STEP * i < rows)
+              asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(d + (r0 + STEP * i) * p.ldd),
+                           "f"(v[i][0]), "f"(v[i][1]), "f"(v[i][2]), "f"(v[i][3])
+                           : "memory");
+        } else if (p.out_f32) {
           float* d = static_cast<float*>(p.d) + b * p.d_batch + m0 * p.ldd + col;
 #pragma unroll
           for (int i = 0; i < BATCH; ++i)

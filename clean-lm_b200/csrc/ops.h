@@ -10,7 +10,7 @@ namespace cdl {
 int32_t matmul_execute(const cdl_tensor* a, const cdl_tensor* b, const cdl_tensor* c,
                        const cdl_tensor* d, float alpha, float beta, cudaStream_t stream,
                        const cdl_matmul_options* opts = nullptr);
-// gemm_general.cu: any strides, bf16 or f32 inputs, CUDA cores (operands already validated).
+// gemm_general.cu: any strides, bf16 or f32 inputs (operands already validated).
 int32_t matmul_general_execute(const cdl_tensor* a, const cdl_tensor* b, const cdl_tensor* c,
                                const cdl_tensor* d, float alpha, float beta, cudaStream_t stream);
 // Arguments of the RoPE epilogue (epi_mode 3): rotate-half RoPE on the heads (128 columns each)

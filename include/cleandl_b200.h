@@ -81,7 +81,8 @@ int32_t cdl_b200_profile_stop(cdl_profile_record* out, int32_t capacity, int32_t
  * valid choices for a problem, default first.  Nothing in the library reads an environment
  * variable. */
 typedef enum {
-  CDL_GEMM_AUTO = 0,    /* heuristic: CTA pairs whenever M > 128 */
+  CDL_GEMM_AUTO = 0,    /* the faster by estimate of the two below and of 128 x 128 tiles whose K range
+                         * a cluster of 1 to 8 CTAs shares (few rows, small outputs) */
   CDL_GEMM_ONE_CTA = 1, /* 128 x 256 tiles, one CTA per tile */
   CDL_GEMM_CTA_PAIR = 2 /* 256 x 256 tiles, tcgen05.mma.cta_group::2 over a cluster of two CTAs */
 } cdl_gemm_variant;
@@ -111,8 +112,8 @@ typedef struct {
  * dgrad = (A row-major, B transposed view), wgrad = (A transposed view, B row-major, D = C f32,
  * beta 1).  bf16 operands whose base address and non-unit strides are 16-byte aligned take the
  * tensor-core kernels; other layouts (tests/matmul.rs:604-630) and f32 inputs
- * (tests/matmul.rs:243-265; full f32 products, where cuBLASLt uses TF32) take a general
- * CUDA-core kernel that is correct but slow.  K == 0 is an error ("K is zero", matmul.rs tests
+ * (tests/matmul.rs:243-265; full f32 products, where cuBLASLt uses TF32) take a tensor-core
+ * kernel that loads operands of any alignment itself, f32 values as three bf16 pieces.  K == 0 is an error ("K is zero", matmul.rs tests
  * :825-843).  D may alias C. */
 int32_t cdl_b200_matmul(const cdl_tensor* a, const cdl_tensor* b, const cdl_tensor* c,
                         const cdl_tensor* d, float alpha, float beta, void* scratch,
@@ -128,7 +129,8 @@ int32_t cdl_b200_matmul_opt(const cdl_tensor* a, const cdl_tensor* b, const cdl_
                             cdl_stream stream);
 /* Writes the valid choices for this problem to out[0 .. *count), the heuristic default first (the
  * order Executor candidates have, op.rs:301-318); at most `capacity` entries, *count = how many
- * exist.  Problems that take the general CUDA-core kernel have the single candidate AUTO. */
+ * exist.  f32 or unaligned operands have the single candidate AUTO; elsewhere AUTO, whose choice may
+ * be the cluster form, is valid beside the candidates. */
 int32_t cdl_b200_matmul_candidates(const cdl_tensor* a, const cdl_tensor* b, const cdl_tensor* d,
                                    cdl_matmul_options* out, int32_t capacity, int32_t* count);
 /* GEMM with the SwiGLU activation fused into its epilogue, the counterparts of the reference's

@@ -348,3 +348,53 @@ def test_unaligned_bf16_layouts(cdl, gpu_ok, m, k, n):
         b = rand_bf16(gen, n, k).T if tb else rand_bf16(gen, k, n)
         run_case(cdl, a, b, torch.bfloat16)
         run_case(cdl, a, b, torch.float32, c=torch.randn(m, n, generator=gen), alpha=0.5, beta=1.0, in_place=True)
+
+
+@pytest.mark.parametrize("m,k,n", [(1, 64, 8), (16, 576, 1024), (64, 2048, 264), (127, 1032, 136), (129, 4096, 128), (300, 2000, 520)])
+def test_tiles_shared_by_a_cluster(cdl, gpu_ok, m, k, n):
+    """Few rows or a small output: K shared by 1, 2, 4 or 8 CTAs of a cluster, ragged last slices and
+    tiles, every operand layout, C of both types, the accumulating form twice in place (bit-equal with
+    one addition per element), batched, and an output whose rows start off the 16-byte grid."""
+    gen = torch.Generator().manual_seed(m * 7 + n)
+    a, b = rand_bf16(gen, m, k), rand_bf16(gen, k, n)
+    run_case(cdl, a, b, torch.bfloat16)
+    run_case(cdl, rand_bf16(gen, k, (m + 7) // 8 * 8).T[:m], rand_bf16(gen, n, k // 8 * 8 + 8)[:, :k].T, torch.float32)
+    run_case(cdl, a, b, torch.bfloat16, c=rand_bf16(gen, m, n), alpha=0.5, beta=2.0)
+    c = torch.randn(m, n, generator=gen)
+    run_case(cdl, a, b, torch.float32, c=c, alpha=2.0, beta=-1.0)
+    run_case(cdl, a, b, torch.float32, c=c, beta=1.0, in_place=True)
+    run_case(cdl, rand_bf16(gen, 3, m, k), rand_bf16(gen, 3, k, n), torch.bfloat16)
+    run_case(cdl, a, b[:, :n - 3], torch.bfloat16)
+    run_case(cdl, a, b[:, :n - 3], torch.float32, c=c[:, :n - 3], beta=1.0, in_place=True)
+    run_case(cdl, a, b[:, :n - 3], torch.float32, c=c[:, :n - 3].contiguous(), beta=1.0, in_place=True)
+    d1, d2 = (cdl.ops.matmul(a.cuda(), b.cuda(), cdl.ops.MatmulOpts(out=torch.float32)) for _ in range(2))
+    assert torch.equal(d1, d2)
+
+
+@pytest.mark.parametrize("rows,seqlen,heads", [(200, 50, 3), (96, 96, 6)])
+def test_rope_epilogue_of_few_rows(cdl, gpu_ok, rows, seqlen, heads):
+    """The rotation in the cluster kernel's store: q and k heads rotated by their row's position, v heads
+    left alone, dense and ragged, against f64 within bf16's rounding of the result."""
+    L = cdl._lib
+    gen = torch.Generator().manual_seed(rows)
+    a, b = rand_bf16(gen, rows, 256), rand_bf16(gen, 256, heads * 128)
+    ang = torch.arange(seqlen, dtype=torch.float64)[:, None] * 10000.0 ** (-torch.arange(64, dtype=torch.float64) / 64)
+    table = torch.cat([ang.cos(), ang.sin()], 1).float()
+    prod = (a.double() @ b.double()).view(rows, heads, 128)
+    cuts = [0, 17, 18, rows - 30]
+    ragged = torch.zeros(rows, dtype=torch.long)
+    for s, e in zip(cuts, cuts[1:]):
+        ragged[s:e] = torch.arange(e - s).clamp(max=seqlen - 1)
+    for cu, pos in ((None, torch.arange(rows) % seqlen), (torch.tensor(cuts, dtype=torch.int32).cuda(), ragged)):
+        c, s = table[pos, :64].double()[:, None], table[pos, 64:].double()[:, None]
+        want = prod.clone()
+        lo, hi = prod[:, :heads - 1, :64], prod[:, :heads - 1, 64:]
+        want[:, :heads - 1, :64], want[:, :heads - 1, 64:] = lo * c - hi * s, hi * c + lo * s
+        d = torch.empty(rows, heads * 128, dtype=torch.bfloat16, device="cuda")
+        args = [L.tensor_arg(t) for t in (a.cuda(), b.cuda(), table.cuda(), cu, d)]
+        L.check(L.lib.cdl_b200_matmul_rope(L.ref(args[0]), L.ref(args[1]), L.ref(args[2]), heads - 1, seqlen,
+                                           L.ref(args[3]), L.ref(args[4]), None))
+        torch.cuda.synchronize()
+        err = (d.double().cpu().view_as(want) - want).abs()
+        # bf16 rounds to 2^-9 of the value; the f32 sum of 256 products of values below 1 adds little
+        assert bool((err <= 2.0 ** -8 * want.abs() + 1e-4).all())
