@@ -116,10 +116,13 @@ struct Params {
   // CTA order (see cta_coords): number of blocks along the sequence, heads x batch, heads per chunk
   // and (head, batch) pairs of the last chunk
   int kv_blocks, kv_heads_total, kv_chunk, kv_tail;  // dK/dV kernel
+  int kv_split;                                      // CTAs that share an item (split form; else 1)
   int q_blocks, q_heads_total, q_chunk, q_tail;      // dQ kernel
   int variant;  // cdl_attn_variant of the call (read on the host only)
   int* status;
 };
+
+constexpr double KV_SPLIT_FIXED = 6.0;  // see kv_split_of
 
 struct KvBarriers {
   uint64_t kv_full;
@@ -441,11 +444,44 @@ __device__ __forceinline__ void cta_coords(int linear, int blocks, int heads_tot
   hb = first + (r - rank * in_chunk);
 }
 
+// Partial sums of the split form: two [128][PART_LD] f32 tiles over the operand tiles; the four extra
+// floats per row put the rows of a quarter-warp's 128-bit stores on different banks.
+constexpr int PART_LD = 132, PART_FLOATS = 128 * PART_LD;
+static_assert(2 * PART_FLOATS * sizeof(float) <= 6 * TILE_BYTES, "the partial sums take the operand tiles' place");
+// Four columns of one row of both tiles, every slice's; then their sums in slice order.
+__device__ __forceinline__ void load_slices(const float* part, int slices, float4 (&q)[8]) {
+  const uint32_t at = smem_u32(part);
+#pragma unroll
+  for (int s = 0; s < 8; ++s)
+    if (s < slices)
+      asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                   : "=f"(q[s].x), "=f"(q[s].y), "=f"(q[s].z), "=f"(q[s].w)
+                   : "r"(mapa_shared(at, s)));
+}
+__device__ __forceinline__ void sum_slices(const float4 (&q)[8], int slices, float (&v)[4]) {
+  v[0] = v[1] = v[2] = v[3] = 0.f;
+#pragma unroll
+  for (int s = 0; s < 8; ++s)
+    if (s < slices) {
+      v[0] += q[s].x;
+      v[1] += q[s].y;
+      v[2] += q[s].z;
+      v[3] += q[s].w;
+    }
+}
+
 // ROPE: the inverse rotary rotation runs in the store epilogue (p.rope is set).  A template
 // parameter, not a branch on p.rope: with the branch the compiler kept the rotation's registers
 // alive through the main loop of both paths (108 against 28 bytes of spills in the persistent
 // dK/dV kernel, 0.494 against 0.459 ms per call WITHOUT the rotation at B 8, S 2048).
-template <bool ROPE>
+//
+// SPLIT: the item's query blocks are shared by a cluster of p.kv_split CTAs, each of which sums up a
+// slice of them; the partial dV and dK (f32) meet in distributed shared memory, where the operand
+// tiles were, and every CTA adds up and stores its share of the rows in slice order.  For a kv head
+// that many query heads share an item is group x (query blocks) long and there are few of them: 9
+// sequences in 6144 rows, 16 heads on 4, have a longest item of 40 blocks where the work of all
+// items is 16 blocks per SM (see kv_split_of).
+template <bool ROPE, bool SPLIT>
 __global__ void __launch_bounds__(THREADS, 1)
     attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q,
                          const __grid_constant__ CUtensorMap tmap_k,
@@ -459,7 +495,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   // neither is stored.
   Params p = p_in;
   int cta_rank, cta_hb;
-  cta_coords(static_cast<int>(blockIdx.x), p_in.kv_blocks, p_in.kv_heads_total, p_in.kv_chunk, p_in.kv_tail, cta_rank, cta_hb);
+  cta_coords(static_cast<int>(SPLIT ? blockIdx.x / p_in.kv_split : blockIdx.x), p_in.kv_blocks, p_in.kv_heads_total, p_in.kv_chunk, p_in.kv_tail, cta_rank, cta_hb);
   const int cta_b = cta_hb / p_in.Hkv;
   int q_base = 0, k_base = 0, bt = cta_b;
   if (p_in.cu_q != nullptr) {
@@ -477,6 +513,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       p.Sk = min(p.Sk, p_in.Sk);
     }
   }
+  if (SPLIT && cta_rank * BKV >= p.Sk) return;  // a key block beyond its sequence: the whole cluster's
   // Shared memory is used to the last kilobytes, so there is no room for manual alignment slack:
   // the 1024-byte alignment the swizzled tiles need is requested from the compiler and verified.
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -505,7 +542,11 @@ __global__ void __launch_bounds__(THREADS, 1)
   const int m_start = p.causal ? max(0, key0 - shift) / BQ : 0;
   const int m_count = max(0, num_q_blocks - m_start);
   // iteration it -> head kvh * group + it / m_count, query block m_start + it % m_count
-  const int iters = key0 < p.Sk ? m_count * group : 0;  // (a key block beyond a packed sequence)
+  const int all_iters = key0 < p.Sk ? m_count * group : 0;  // (a key block beyond a packed sequence)
+  // This CTA's share of them: iterations it0 .. it0 + iters.
+  const int slice = SPLIT ? static_cast<int>(cluster_ctarank()) : 0;
+  const int it0 = SPLIT ? static_cast<int>(static_cast<long long>(slice) * all_iters / p.kv_split) : 0;
+  const int iters = (SPLIT ? static_cast<int>(static_cast<long long>(slice + 1) * all_iters / p.kv_split) : all_iters) - it0;
 
   if (threadIdx.x == 0) {
     mbar_init(&bars->kv_full, 1);
@@ -554,8 +595,8 @@ __global__ void __launch_bounds__(THREADS, 1)
         tma_load_4d(s_v + dh * PANEL_BYTES, &tmap_v, &bars->kv_full, dh * 64, k_base + key0, kvh, bt);
       }
       for (int it = 0; it < iters; ++it) {
-        const int h = kvh * group + it / m_count;
-        const int q0 = (m_start + it % m_count) * BQ;
+        const int h = kvh * group + (it0 + it) / m_count;
+        const int q0 = (m_start + (it0 + it) % m_count) * BQ;
         const int s = it & 1;
         const uint32_t ph = ((it >> 1) & 1) ^ 1;
         if (!mbar_wait(&bars->q_empty[s], ph, abort_word, 121)) break;
@@ -662,8 +703,8 @@ __global__ void __launch_bounds__(THREADS, 1)
     const int key = key0 + r;
     bool ok = true;
 
-    auto it_head = [&](int it) { return kvh * group + it / m_count; };
-    auto it_q0 = [&](int it) { return (m_start + it % m_count) * BQ; };
+    auto it_head = [&](int it) { return kvh * group + (it0 + it) / m_count; };
+    auto it_q0 = [&](int it) { return (m_start + (it0 + it) % m_count) * BQ; };
     // Row statistics of iteration `it`: threads 0..127 fetch LSE2, 128..255 fetch delta.
     auto fetch_stat = [&](int it) -> float {
       const long long base = (static_cast<long long>(b) * p.H + it_head(it)) * p.Sq_pad + it_q0(it);
@@ -788,13 +829,41 @@ __global__ void __launch_bounds__(THREADS, 1)
     }
 
     // ---- epilogue: dV and dK rows of this key block
+    if (SPLIT) {
+      if (ok && iters > 0) {
+        ok = mbar_wait(&bars->dk_done, 0, abort_word, 326);  // behind every product: all tiles are free
+        tc_fence_after();
+      }
+      if (ok) {
+#pragma unroll
+        for (int which = 0; which < 2; ++which) {
+          float* part = reinterpret_cast<float*>(smem) + which * PART_FLOATS + r * PART_LD + wg * 64;
+          const uint32_t col = (which == 0 ? KV_COL_DV : KV_COL_DK) + wg * 64;
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            uint32_t a[32];
+            if (iters > 0) {
+              tmem_ld32(tmem_base + lane_addr + col + half * 32, a);
+              tmem_wait_ld();
+            } else {
+#pragma unroll
+              for (int i = 0; i < 32; ++i) a[i] = 0u;
+            }
+#pragma unroll
+            for (int g = 0; g < 8; ++g)
+              *reinterpret_cast<uint4*>(part + half * 32 + g * 4) =
+                  make_uint4(a[g * 4], a[g * 4 + 1], a[g * 4 + 2], a[g * 4 + 3]);
+          }
+        }
+      }
+    }
     RopeUnits rope_units;  // the table values of the inverse rotation: on their way while dV is staged
-    if (ROPE) rope_units_load(p.rope, key0, p.rope_rows, ct, rope_units);
-    if (ok && iters > 0) {
+    if (ROPE && !SPLIT) rope_units_load(p.rope, key0, p.rope_rows, ct, rope_units);
+    if (!SPLIT && ok && iters > 0) {
       ok = mbar_wait(&bars->dv_done, 0, abort_word, 325);
       tc_fence_after();
     }
-    if (ok) {
+    if (!SPLIT && ok) {
       // The tiles go out through shared memory and one TMA store per 64-column panel: a thread
       // owns a row, so direct stores would touch 32 rows per instruction.  The staging tiles are
       // operand stages whose readers have completed; the panel layout is the loads' 128-byte swizzle.  A store
@@ -868,6 +937,41 @@ __global__ void __launch_bounds__(THREADS, 1)
     while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
   }
   tc_fence_before();
+  if (SPLIT) {
+    cluster_sync_all();
+    if (warp >= 4) {
+      const float* part = reinterpret_cast<const float*>(smem);
+      __nv_bfloat16* dv = p.dv + bt * p.dv_sb + static_cast<long long>(k_base + key0) * p.dv_ss + kvh * p.dv_sh + lane * 4;
+      __nv_bfloat16* dk = p.dk + bt * p.dk_sb + static_cast<long long>(k_base + key0) * p.dk_ss + kvh * p.dk_sh + lane * 4;
+#pragma unroll 1
+      for (int row = slice + p.kv_split * (warp - 4); row < BKV && key0 + row < p.Sk; row += p.kv_split * 8) {
+        float v[4], x[4];
+        float4 qv[8], qk[8];
+        load_slices(part + row * PART_LD + lane * 4, p.kv_split, qv);
+        load_slices(part + PART_FLOATS + row * PART_LD + lane * 4, p.kv_split, qk);
+        sum_slices(qv, p.kv_split, v);
+        sum_slices(qk, p.kv_split, x);
+        *reinterpret_cast<uint2*>(dv + row * p.dv_ss) = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
+        uint2 q = make_uint2(pack_bf16x2(x[0] * p.scale, x[1] * p.scale), pack_bf16x2(x[2] * p.scale, x[3] * p.scale));
+        if (ROPE) {
+          // as rope_inverse_apply, on the rounded values; column i + 64 of a lane's columns is on lane ^ 16
+          const float* cs = p.rope + static_cast<long long>(min(key0 + row, p.rope_rows - 1)) * 128 + (lane & 15) * 4;
+          const float4 c = __ldg(reinterpret_cast<const float4*>(cs));
+          const float4 sn = __ldg(reinterpret_cast<const float4*>(cs + 64));
+          const float sign = lane < 16 ? 1.f : -1.f;
+          const float own[4] = {bf16_lo(q.x), bf16_hi(q.x), bf16_lo(q.y), bf16_hi(q.y)};
+          float o[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) o[j] = sign * __shfl_xor_sync(0xffffffffu, own[j], 16);
+          q.x = pack_bf16x2(own[0] * c.x + o[0] * sn.x, own[1] * c.y + o[1] * sn.y);
+          q.y = pack_bf16x2(own[2] * c.z + o[2] * sn.z, own[3] * c.w + o[3] * sn.w);
+        }
+        *reinterpret_cast<uint2*>(dk + row * p.dk_ss) = q;
+      }
+    }
+    __syncwarp();
+    cluster_sync_all();  // the other slices have read this CTA's partial sums
+  }
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
@@ -2245,6 +2349,37 @@ __global__ void __launch_bounds__(THREADS, 1)
   if (threadIdx.x == 0 && *abort_word != 0) atomicExch(p.status, *abort_word);
 }
 
+// CTAs per item of the dK/dV kernel.  In block pairs (one takes 1.7 us): the launch cannot end before
+// its longest item, nor before the work of all items spread over the SMs.  A split item costs every one
+// of its CTAs a fixed part (launch, first loads and products, the exchange: 11 us, 6 pairs), and as many
+// clusters run at a time as the GPCs hold, `slots[i]` of 2 << i CTAs.  Packed sequences are on the
+// device: `rows` query rows of evenly long sequences stand in for them, and the bound Sq for the longest.
+// Whole backward, one CTA per item -> chosen split: 16 heads on 4, B 1, S 512 45.9 -> 30.7 us (4), S 1000
+// 79 -> 46 (4), S 2048 145 -> 90 (4), S 4096 301 -> 214 (2); 8 on 2, S 8192 581 -> 383 (2); left alone
+// at 16 on 4, S 8192, 738 against 764.
+static int kv_split_of(const Params& p, long long rows, const int (&slots)[3]) {
+  const double group = static_cast<double>(p.H) / p.Hkv;
+  const double len = p.cu_q ? static_cast<double>(rows) / p.B : p.Sq;
+  const double nq = (len + BQ - 1) / BQ, nk = p.cu_q ? nq : static_cast<double>((p.Sk + BKV - 1) / BKV);
+  const double items = nk * p.Hkv * p.B;
+  const double work = items * group * (p.causal ? (nq + 1) / 2 : nq) / sm_count();
+  const double longest = group * ((p.Sq + BQ - 1) / BQ);
+  int best = 1;
+  double best_cost = longest > work ? longest : work;
+  for (int i = 0; i < 3; ++i) {
+    const int s = 2 << i;
+    if (slots[i] <= 0) continue;
+    const double waves = ceil(items / slots[i]);
+    const double spread = KV_SPLIT_FIXED * waves + 1.1 * work, deep = KV_SPLIT_FIXED + longest / s;
+    const double cost = deep > spread ? deep : spread;
+    if (cost < 0.9 * best_cost) {
+      best = s;
+      best_cost = cost;
+    }
+  }
+  return best;
+}
+
 static long long pad128(long long v) { return (v + 127) / 128 * 128; }
 
 }  // namespace attn_bwd
@@ -2263,6 +2398,7 @@ static int32_t bwd_run(const attn_bwd::Params& p_const, const cdl_tensor* q, con
   attn_bwd::Params p = p_const;  // the CTA-order fields are filled in below
   using namespace attn_bwd;
   static std::once_flag attr_once[64];
+  static int kv_slots[64][3] = {};  // clusters of 2, 4 and 8 CTAs of the split dK/dV kernel the device holds
   int dev = 0;
   CDL_CUDA(cudaGetDevice(&dev));
   cudaError_t attr_err = cudaSuccess;
@@ -2271,14 +2407,31 @@ static int32_t bwd_run(const attn_bwd::Params& p_const, const cdl_tensor* q, con
       if (attr_err == cudaSuccess)
         attr_err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
     };
-    opt_in(reinterpret_cast<const void*>(attn_bwd_dkdv_kernel<false>), KV_SMEM_BYTES);
-    opt_in(reinterpret_cast<const void*>(attn_bwd_dkdv_kernel<true>), KV_SMEM_BYTES);
+    opt_in(reinterpret_cast<const void*>(attn_bwd_dkdv_kernel<false, false>), KV_SMEM_BYTES);
+    opt_in(reinterpret_cast<const void*>(attn_bwd_dkdv_kernel<true, false>), KV_SMEM_BYTES);
+    opt_in(reinterpret_cast<const void*>(attn_bwd_dkdv_kernel<false, true>), KV_SMEM_BYTES);
+    opt_in(reinterpret_cast<const void*>(attn_bwd_dkdv_kernel<true, true>), KV_SMEM_BYTES);
     opt_in(reinterpret_cast<const void*>(attn_bwd_dkdv_persistent_kernel<false>), KVP_SMEM_BYTES);
     opt_in(reinterpret_cast<const void*>(attn_bwd_dkdv_persistent_kernel<true>), KVP_SMEM_BYTES);
     opt_in(reinterpret_cast<const void*>(attn_bwd_dq_kernel<false>), Q_SMEM_BYTES);
     opt_in(reinterpret_cast<const void*>(attn_bwd_dq_kernel<true>), Q_SMEM_BYTES);
     opt_in(reinterpret_cast<const void*>(attn_bwd_dq_persistent_kernel<false>), QP_SMEM_BYTES);
     opt_in(reinterpret_cast<const void*>(attn_bwd_dq_persistent_kernel<true>), QP_SMEM_BYTES);
+    for (int i = 0; i < 3 && attr_err == cudaSuccess; ++i) {
+      cudaLaunchConfig_t cfg = {};
+      cudaLaunchAttribute attr[1];
+      cfg.gridDim = dim3(static_cast<unsigned>(sm_count() & ~15));
+      cfg.blockDim = dim3(THREADS);
+      cfg.dynamicSmemBytes = KV_SMEM_BYTES;
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = 2u << i;
+      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      int n = 0;
+      if (cudaOccupancyMaxActiveClusters(&n, attn_bwd_dkdv_kernel<false, true>, &cfg) == cudaSuccess) kv_slots[dev & 63][i] = n;
+    }
+    (void)cudaGetLastError();
   });
   if (attr_err != cudaSuccess)
     return fail(CDL_ERR_CUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(attr_err));
@@ -2349,7 +2502,12 @@ static int32_t bwd_run(const attn_bwd::Params& p_const, const cdl_tensor* q, con
     // run time from a counter of this stream; without one, a fixed deal).
     const bool persistent = p.variant == CDL_ATTN_PERSISTENT ||
                             (p.variant == CDL_ATTN_AUTO && CDL_ATTN_BWD_PERSISTENT && items > sm_count());
-    if (persistent && items < (1ll << 30)) {
+    p.kv_split = p.variant == CDL_ATTN_AUTO ? kv_split_of(p, q->shape[1], kv_slots[dev & 63]) : 1;
+    if (p.kv_split > 1 && items * p.kv_split < (1ll << 30)) {
+      CDL_CUDA(launch_pdl_cluster(rope ? attn_bwd_dkdv_kernel<true, true> : attn_bwd_dkdv_kernel<false, true>,
+                                  dim3(static_cast<unsigned>(items * p.kv_split)), dim3(THREADS), KV_SMEM_BYTES,
+                                  p.kv_split, stream, tq, tk, tv, tdo, tdk, tdv, p));
+    } else if (persistent && items < (1ll << 30)) {
       const long long ctas = items < sm_count() ? items : sm_count();
       unsigned int* counter = items > ctas ? sched_counter_for(2, dev, stream) : nullptr;
       CDL_CUDA(launch_pdl(rope ? attn_bwd_dkdv_persistent_kernel<true> : attn_bwd_dkdv_persistent_kernel<false>,
@@ -2357,7 +2515,7 @@ static int32_t bwd_run(const attn_bwd::Params& p_const, const cdl_tensor* q, con
                           KVP_SMEM_BYTES, stream, tq, tk, tv, tdo, tdk, tdv, p, counter));
     } else {
       dim3 grid(static_cast<unsigned>(items));
-      CDL_CUDA(launch_pdl(rope ? attn_bwd_dkdv_kernel<true> : attn_bwd_dkdv_kernel<false>, grid, dim3(THREADS), KV_SMEM_BYTES,
+      CDL_CUDA(launch_pdl(rope ? attn_bwd_dkdv_kernel<true, false> : attn_bwd_dkdv_kernel<false, false>, grid, dim3(THREADS), KV_SMEM_BYTES,
                           stream, tq, tk, tv, tdo, tdk, tdv, p));
     }
     CDL_CUDA(cudaGetLastError());

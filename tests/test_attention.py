@@ -476,3 +476,58 @@ def test_packed_rejections(cdl, gpu_ok):
     with pytest.raises(cdl._lib.CdlError, match="i32"):
         cdl.ops.attention_fwd(z(8, 2, 128), z(8, 2, 128), z(8, 2, 128),
                               cdl.ops.AttentionOpts(cu_seqlens_q=cu.float(), cu_seqlens_k=cu))
+
+
+@pytest.mark.parametrize("b,sq,sk,hq,hk,causal", [
+    (1, 640, 640, 8, 1, True),     # one kv head of eight: a few long items
+    (1, 700, 700, 4, 1, True),     # ragged tail; the last key block's items are shorter than the cluster
+    (1, 520, 1300, 8, 1, False),   # no mask, more keys than queries
+    (2, 900, 300, 8, 2, True),     # the first query rows see no key
+    (1, 1700, 1700, 6, 2, True),
+])
+def test_bwd_items_shared_by_a_cluster(cdl, gpu_ok, b, sq, sk, hq, hk, causal):
+    """Few kv heads for many query heads: the query blocks of a dK/dV item are split over a cluster of
+    CTAs whose partial sums meet in distributed shared memory.  Against the oracle, bit-equal in two
+    runs, and with the rotation in the store equal to the separate one up to its rounding."""
+    q, k, v, do = make(b, sq, sk, hq, hk, seed=23)
+    check_bwd(cdl, q, k, v, do, causal)
+    qd, kd, vd, dod = (t.cuda() for t in (q, k, v, do))
+    opts = cdl.ops.AttentionOpts(causal=causal)
+    fwd = cdl.ops.attention_fwd(qd, kd, vd, opts)
+    one = cdl.ops.attention_bwd(qd, kd, vd, fwd.out, dod, fwd.lse, opts)
+    two = cdl.ops.attention_bwd(qd, kd, vd, fwd.out, dod, fwd.lse, opts)
+    assert all(torch.equal(x, y) for x, y in zip(one, two))
+    if sq == sk:
+        L = cdl._lib
+        table = _rope_table(sq).cuda()
+        _, fk, fv = cdl.ops.attention_bwd(qd, kd, vd, fwd.out, dod, fwd.lse, opts, rope_table=table)
+        tx, tt = L.tensor_arg(one[1].view(b * sk, hk, 128)), L.tensor_arg(table)
+        L.check(L.lib.cdl_b200_rope(L.ref(tx), L.ref(tt), hk, sk, 1, None))
+        _assert_same_up_to_one_rounding("dk", fk, one[1])
+        assert torch.equal(fv, two[2])
+
+
+def test_packed_bwd_items_shared_by_a_cluster(cdl, gpu_ok):
+    """The split form on packed sequences of very different lengths (one of them a single row, the
+    bound above the longest) equals the one-CTA form up to the order of its f32 sums."""
+    lens = [700, 1, 129, 380]
+    qd, kd, vd, dod, cu = _packed_inputs(lens, 8, 1)
+    res = []
+    for variant in (cdl._lib.ATTN_AUTO, cdl._lib.ATTN_ONE_SHOT):
+        opts = cdl.ops.AttentionOpts(causal=True, cu_seqlens_q=cu, cu_seqlens_k=cu, max_seqlen_q=900,
+                                     max_seqlen_k=900, variant=variant)
+        fwd = cdl.ops.attention_fwd(qd, kd, vd, opts)
+        res.append(cdl.ops.attention_bwd(qd, kd, vd, fwd.out, dod, fwd.lse, opts))
+    for name, x, y in zip(("dq", "dk", "dv"), *res):
+        x, y = x[:sum(lens)].float(), y[:sum(lens)].float()
+        # one bf16 rounding of each element, either way
+        assert (x - y).abs().max().item() <= 2.0 ** -7 * y.abs().max().item(), name
+
+
+def _packed_inputs(lens, hq, hk):
+    gen = torch.Generator().manual_seed(29)
+    n = sum(lens) + 3
+    q, do = (torch.randn(n, hq, 128, generator=gen).to(torch.bfloat16).cuda() for _ in range(2))
+    k, v = (torch.randn(n, hk, 128, generator=gen).to(torch.bfloat16).cuda() for _ in range(2))
+    cu = torch.tensor([0, *torch.tensor(lens).cumsum(0).tolist()], dtype=torch.int32).cuda()
+    return q, k, v, do, cu
