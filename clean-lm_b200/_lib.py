@@ -2,7 +2,9 @@
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
+import struct
 from pathlib import Path
 
 # The in-tree build; CLEANDL_B200_LIB names another build of the same sources (a variant made by
@@ -225,25 +227,35 @@ def check(status: int) -> None:
         raise CdlError(status, last_error())
 
 
+_TENSOR_BYTES = struct.Struct("Qii4q4q")  # the layout of cdl_tensor
+assert _TENSOR_BYTES.size == ctypes.sizeof(CdlTensor)
+_UNUSED = ((0, 0, 0, 0), (0, 0, 0), (0, 0), (0,), ())  # the dimensions a tensor of rank r leaves over
+
+
 def tensor_arg(t):
-    """Wraps a torch tensor (any strides) as a cdl_tensor; None stays None (a NULL pointer)."""
+    """Wraps a torch tensor (any strides) as a cdl_tensor; None stays None (a NULL pointer).
+
+    Packed in one go: field by field it takes 2.7 us instead of 1.2, and a call of a small operator,
+    which its host time bounds, wraps three to eleven tensors."""
     if t is None:
         return None
-    import torch
-
-    dt = {torch.bfloat16: CDL_BF16, torch.float32: CDL_F32, torch.int32: CDL_I32}.get(t.dtype)
+    dt = _dtype_codes().get(t.dtype)
     if dt is None:
         raise CdlError(-1, f"unsupported element type {t.dtype}: f32 or bf16 expected")
-    if t.dim() > 4:
-        raise CdlError(-1, f"rank {t.dim()} exceeds 4")
-    ct = CdlTensor()
-    ct.ptr = t.data_ptr()
-    ct.dtype = dt
-    ct.rank = t.dim()
-    for i in range(t.dim()):
-        ct.shape[i] = t.shape[i]
-        ct.stride[i] = t.stride(i)
-    return ct
+    shape = t.shape
+    rank = len(shape)
+    if rank > 4:
+        raise CdlError(-1, f"rank {rank} exceeds 4")
+    rest = _UNUSED[rank]
+    return CdlTensor.from_buffer_copy(
+        _TENSOR_BYTES.pack(t.data_ptr(), dt, rank, *shape, *rest, *t.stride(), *rest))
+
+
+@functools.cache
+def _dtype_codes():
+    import torch
+
+    return {torch.bfloat16: CDL_BF16, torch.float32: CDL_F32, torch.int32: CDL_I32}
 
 
 def ref(ct):
