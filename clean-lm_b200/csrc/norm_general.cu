@@ -91,10 +91,10 @@ __global__ void __launch_bounds__(256) norm_general_kernel(const Params p) {
 // Bound by HBM: x is read once and y written once.  V is the widest access that every row's start
 // allows (four f32 where rows are on the 16-byte grid, two or one where they are not: a [8192, 2050]
 // f32 row starts on the 8-byte grid), so a warp's access still covers whole 64- or 128-byte lines.
-// Wide rows take four warps so that a thread's share stays at 32 values: 16 rows are then in flight
-// per SM, where one warp per row would need over 64 registers a thread for the row alone.
-// LayerNorm of f32 [8192, 2050] to f32 (134 MB): 33 us, 4.1 TB/s, 38 us a call; norm_general_kernel, which
-// reads the row three times with scalar accesses, 125 us.
+// Wide rows take four warps so that a thread's share stays at 20 or 32 values: 12 or 9 rows are then in
+// flight per SM, where one warp per row would need over 64 registers a thread for the row alone.
+// LayerNorm of f32 [8192, 2050] to f32 (134 MB): 27 us, 5.0 TB/s; norm_general_kernel, which reads the row
+// three times with scalar accesses, 125 us.
 template <int V>
 __device__ __forceinline__ void load_cols(const float* q, float (&v)[V]) {
   if (V == 4) {
@@ -251,6 +251,8 @@ static cudaError_t launch_rows(const Params& p, cudaStream_t stream) {
   const unsigned rows = static_cast<unsigned>(p.rows), rows8 = (rows + 7) / 8;
   if (p.cols <= 256) return launch_pdl(norm_rows_kernel<V, 8, 1>, dim3(rows8), dim3(256), 0, stream, p);
   if (p.cols <= 1024) return launch_pdl(norm_rows_kernel<V, 32, 1>, dim3(rows8), dim3(256), 0, stream, p);
+  // 20 values leave room for 16 rows per SM; f32 [8192, 2050] 27.1 us, with 32 values 32.8.
+  if (p.cols <= 2560) return launch_pdl(norm_rows_kernel<V, 20, 4>, dim3(rows), dim3(128), 0, stream, p);
   if (p.cols <= 4096) return launch_pdl(norm_rows_kernel<V, 32, 4>, dim3(rows), dim3(128), 0, stream, p);
   return launch_pdl(norm_rows_kernel<V, 64, 4>, dim3(rows), dim3(128), 0, stream, p);
 }

@@ -247,7 +247,7 @@ def test_general_path_shapes(cdl, gpu_ok, norm_type):
 
 
 @pytest.mark.parametrize("norm_type", ["rms", "layer"])
-@pytest.mark.parametrize("cols", [1, 2, 31, 255, 256, 258, 1021, 1024, 1026, 2050, 4095, 4096, 4100, 8190, 8192])
+@pytest.mark.parametrize("cols", [1, 2, 31, 255, 256, 258, 1021, 1024, 1026, 2050, 2560, 2562, 4095, 4096, 4100, 8190, 8192])
 def test_register_rows_column_edges(cdl, gpu_ok, norm_type, cols):
     """Rows kept in registers (norm_rows_kernel): both sides of every capacity, each access width
     (4, 2 and 1 columns), row counts off the CTA's eight, rows with a stride of their own."""
