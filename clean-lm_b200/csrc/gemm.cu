@@ -850,7 +850,7 @@ static int32_t analyze_operand(const char* name, const cdl_tensor* t, bool contr
 // 2048 36.1 -> 12.0 (4 slices), 256 x 2048 x 2048 15.4 -> 9.2 (4), 256 x 2048 x 6144 15.8 -> 13.4 (1),
 // 512 x 5632 x 2048 31.8 -> 16.9 (2); the other way at 2048 x 2048 x 2048, 17.2 against 19.1.
 static int choose_cluster_splits(long long batch, long long M, long long N, long long K, bool adds_f32,
-                                 bool may_slice) {
+                                 bool may_slice, bool reduces) {
   auto up = [](long long a, long long b) { return (a + b - 1) / b; };
   const double kb = static_cast<double>(up(K, BK));
   const double sms = sm_count();
@@ -872,9 +872,11 @@ static int choose_cluster_splits(long long batch, long long M, long long N, long
   int splits = 0;
   for (int i = 0; i < 4 && (1 << i) <= kb; ++i) {
     const double ctas = static_cast<double>(tiles << i);
-    const double deep = 0.23 * kb / (1 << i), wide = (may_slice ? 0.25 : 0.32) * static_cast<double>(tiles) * kb / sms;
+    const double deep = 0.23 * kb / (1 << i), wide = (reduces ? 0.25 : 0.32) * static_cast<double>(tiles) * kb / sms;
     double t = per_cta[i] + (deep > wide ? deep : wide) + (ctas > sms ? 3.1 * (ctas / sms - 1.0) : 0.0);
-    if (adds_f32) t += (may_slice ? 1.7 : 2.6) * (static_cast<double>(tiles) > sms ? static_cast<double>(tiles) / sms : 1.0);
+    if (adds_f32) t += (reduces ? 1.7 : 2.6) * (static_cast<double>(tiles) > sms ? static_cast<double>(tiles) / sms : 1.0);
+    // From two tiles per SM on, unsplit additions into D are walked by one CTA per SM.
+    if (reduces && i == 0 && tiles >= 2 * sm_count()) t = 5.5 + static_cast<double>(tiles) / sms * (3.4 + 0.25 * kb);
     if (t < best) {
       best = t;
       splits = 1 << i;
@@ -966,8 +968,12 @@ int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_t
   const bool adds_f32 = use_c && c->dtype == CDL_F32;
   const bool may_slice = adds_f32 && d->dtype == CDL_F32 && c->ptr == d->ptr && beta == 1.0f &&
                          !(opts && opts->deterministic != 0);
+  // In the cluster kernel it adds every element once, by vector reductions where D's rows allow them.
+  const bool reduces = may_slice && N % 4 == 0 && (reinterpret_cast<uintptr_t>(d->ptr) & 15) == 0 &&
+                       (M == 1 || (d->stride[r - 2] % 4 == 0 && c->stride[r - 2] == d->stride[r - 2])) &&
+                       (r == 2 || (d->stride[0] % 4 == 0 && c->stride[0] == d->stride[0]));
   const int cluster_splits =
-      variant == CDL_GEMM_AUTO ? choose_cluster_splits(batch, M, N, K, adds_f32, may_slice) : 0;
+      variant == CDL_GEMM_AUTO ? choose_cluster_splits(batch, M, N, K, adds_f32, may_slice, reduces) : 0;
   const bool use_cluster = cluster_splits > 0;
   const bool use_pair = !use_cluster && (variant == CDL_GEMM_AUTO ? M > BM : variant == CDL_GEMM_CTA_PAIR);
   const int tile_m = use_pair ? PAIR_M : BM;
@@ -1101,9 +1107,9 @@ int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_t
 
   if (use_cluster) {
     // D += A^T B: every element is added to once, by a reduction at the L2, instead of read, added to and
-    // written: 2048 x 5632 x 256 29 us instead of 34, 512 x 1536 x 256 5.6 instead of 7.7.  (In the pair
+    // written: 2048 x 5632 x 256 29 us instead of 34 (25 as a walk), 512 x 1536 x 256 5.6 instead of 7.7.  (In the pair
     // kernel, where a thread's reductions run along a row, the same costs 42 us instead of 34.)
-    if (may_slice && p.ldc == p.ldd && p.c_batch == p.d_batch && p.d_vec && N % 4 == 0) {
+    if (reduces) {
       p.atomic_out = 1;
       p.c_mode = 0;
     }

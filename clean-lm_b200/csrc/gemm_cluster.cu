@@ -173,6 +173,184 @@ __global__ void __launch_bounds__(THREADS, STAGES == SHARED_STAGES ? 2 : 1)
   if (threadIdx.x == 0 && *abort_word != 0) atomicExch(p.status, *abort_word);
 }
 
+// The unsplit weight-gradient form (D += A^T B, f32): many tiles with few K blocks each, so that launch,
+// set-up, first loads and the store are most of a CTA's life.  One CTA per SM walks the tiles; loads and
+// products of the next tile run under the store of this one (two accumulators, the partial tile in
+// shared memory of its own).  2048 x 5632 with K = 64, 256, 512: 22.7, 25.0, 30.7 us; as one short-lived
+// CTA per tile 25.8, 28.9, 34.1 us.  What is left is the reductions: 92 MB of HBM traffic, 14 us.
+constexpr int WALK_THREADS = 320;  // warp 0 TMA, warp 1 MMA, warps 2-9 drain and store
+constexpr int WALK_TMEM_COLS = 256;
+constexpr size_t WALK_SMEM_BYTES = 1024 + SHARED_STAGES * STAGE_BYTES + PART_BYTES + 128;
+struct WalkBarriers {
+  uint64_t full[SHARED_STAGES];
+  uint64_t empty[SHARED_STAGES];
+  uint64_t acc_full[2];
+  uint64_t acc_empty[2];
+  uint32_t tmem_base;
+  int abort_word;
+};
+static_assert(sizeof(WalkBarriers) <= 128, "barriers fit behind the partial tile");
+__device__ __forceinline__ void store_warps_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+// The same; true in all 256 threads if `flag` is in any.
+__device__ __forceinline__ bool store_warps_any(bool flag) {
+  uint32_t any;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, 1, 256, p;\n\tselp.u32 %0, 1, 0, q;\n\t}\n"
+      : "=r"(any)
+      : "r"(static_cast<uint32_t>(flag))
+      : "memory");
+  return any != 0;
+}
+
+__global__ void __launch_bounds__(WALK_THREADS, 1)
+    gemm_cluster_walk_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
+                             const Params p) {
+  constexpr int STAGES = SHARED_STAGES;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                             ~static_cast<uintptr_t>(1023));
+  float* part = reinterpret_cast<float*>(smem + STAGES * STAGE_BYTES);
+  WalkBarriers* bars = reinterpret_cast<WalkBarriers*>(smem + STAGES * STAGE_BYTES + PART_BYTES);
+  volatile int* abort_word = &bars->abort_word;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(&bars->full[s], 1);
+      mbar_init(&bars->empty[s], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&bars->acc_full[i], 1);
+      mbar_init(&bars->acc_empty[i], WARPS);
+    }
+    bars->abort_word = 0;
+    fence_mbar_init();
+    tma_prefetch_desc(&tmap_a);
+    tma_prefetch_desc(&tmap_b);
+  }
+  if (warp == 1) {
+    tmem_alloc(&bars->tmem_base, WALK_TMEM_COLS);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = bars->tmem_base;
+  grid_dep_wait();
+  grid_dep_launch();
+
+  if (warp == 0) {
+    if (elect_one()) {
+      uint32_t it = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x) {
+        int b, tm, tn;
+        tile_coords(p, tile, b, tm, tn);
+        const int m0 = tm * TILE_M, n0 = tn * TILE_N;
+        for (int kb = 0; kb < p.k_blocks; ++kb, ++it) {
+          const uint32_t s = it % STAGES;
+          if (!mbar_wait(&bars->empty[s], ((it / STAGES) & 1) ^ 1, abort_word, 141)) {
+            ok = false;
+            break;
+          }
+          uint8_t* sa = smem + s * STAGE_BYTES;
+          uint8_t* sb = sa + A_BYTES;
+          mbar_arrive_expect_tx(&bars->full[s], STAGE_BYTES);
+          const int k0 = kb * BK;
+          if (p.a_mn) {
+#pragma unroll
+            for (int i = 0; i < TILE_M / 64; ++i)
+              tma_load_3d(sa + i * 8192, &tmap_a, &bars->full[s], m0 + i * 64, k0, b);
+          } else {
+            tma_load_3d(sa, &tmap_a, &bars->full[s], k0, m0, b);
+          }
+          if (p.b_mn) {
+#pragma unroll
+            for (int i = 0; i < TILE_N / 64; ++i)
+              tma_load_3d(sb + i * 8192, &tmap_b, &bars->full[s], n0 + i * 64, k0, b);
+          } else {
+            tma_load_3d(sb, &tmap_b, &bars->full[s], k0, n0, b);
+          }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (elect_one()) {
+      const uint32_t idesc = make_idesc_bf16(TILE_M, TILE_N, p.a_mn, p.b_mn);
+      const uint32_t a_lbo = p.a_mn ? 8192u : 16u, b_lbo = p.b_mn ? 8192u : 16u;
+      const uint32_t a_kstep = p.a_mn ? 2048u : 32u, b_kstep = p.b_mn ? 2048u : 32u;
+      uint32_t it = 0, t = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x, ++t) {
+        const uint32_t acc = t & 1, d = tmem_base + acc * TILE_N;
+        if (!mbar_wait(&bars->acc_empty[acc], ((t >> 1) & 1) ^ 1, abort_word, 241)) break;
+        tc_fence_after();
+        for (int kb = 0; kb < p.k_blocks; ++kb, ++it) {
+          const uint32_t s = it % STAGES;
+          if (!mbar_wait(&bars->full[s], (it / STAGES) & 1, abort_word, 242)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t sa = smem_u32(smem + s * STAGE_BYTES), sb = sa + A_BYTES;
+#pragma unroll
+          for (int k = 0; k < BK / 16; ++k)
+            umma_ss(d, smem_desc_sw128(sa + k * a_kstep, a_lbo, 1024), smem_desc_sw128(sb + k * b_kstep, b_lbo, 1024),
+                    idesc, (kb | k) != 0 ? 1u : 0u);
+          umma_commit(&bars->empty[s]);
+        }
+        if (ok) umma_commit(&bars->acc_full[acc]);
+      }
+    }
+  } else {
+    const int w = warp - 2, row = (warp & 3) * 32 + lane, half = w >> 2;
+    uint32_t t = 0;
+    for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, ++t) {
+      int b, tm, tn;
+      tile_coords(p, tile, b, tm, tn);
+      const int m0 = tm * TILE_M, n0 = tn * TILE_N;
+      const uint32_t acc = t & 1;
+      const bool ok = mbar_wait(&bars->acc_full[acc], (t >> 1) & 1, abort_word, 341);
+      tc_fence_after();
+      if (ok && m0 + (warp & 3) * 32 < p.M) {
+#pragma unroll
+        for (int c = half * 64; c < half * 64 + 64; c += 16) {
+          uint32_t r[16];
+          tmem_ld16(tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + acc * TILE_N + c, r);
+          tmem_wait_ld();
+          float v[16];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
+          store_partial(part, row, c, v);
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars->acc_empty[acc]);
+      // The whole tile is in shared memory.  A wait that ran out ends the walk of all eight warps here: one
+      // that left alone would keep the others at the barrier.
+      if (store_warps_any(!ok)) break;
+      TileOut<1, WARPS> tile_out;
+      tile_out.finish(p, part, 0, w, b, m0, n0);
+      __syncwarp();
+      store_warps_sync();  // and has been read
+    }
+  }
+  __syncwarp();
+  if (*abort_word != 0) {
+    // Loads that may still be in flight land before shared memory is released.
+    const unsigned long long t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, WALK_TMEM_COLS);
+  }
+  if (threadIdx.x == 0 && *abort_word != 0) atomicExch(p.status, *abort_word);
+}
+
 template <int S, int STAGES>
 int32_t launch(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const Params& p, int dev, cudaStream_t stream) {
   static std::once_flag once[64];
@@ -198,6 +376,19 @@ int32_t gemm_cluster_launch(const CUtensorMap& tm_a, const CUtensorMap& tm_b, co
                             cudaStream_t stream) {
   int dev = 0;
   CDL_CUDA(cudaGetDevice(&dev));
+  // The walk pays where an SM gets two tiles or more.
+  if (p.split_k == 1 && p.atomic_out && p.num_tiles >= 2 * sm_count()) {
+    static std::once_flag once[64];
+    cudaError_t err = cudaSuccess;
+    std::call_once(once[dev & 63], [&] {
+      err = cudaFuncSetAttribute(gemm_cluster_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(WALK_SMEM_BYTES));
+    });
+    if (err != cudaSuccess) return fail(CDL_ERR_CUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(err));
+    CDL_CUDA(launch_pdl(gemm_cluster_walk_kernel, dim3(static_cast<unsigned>(sm_count())), dim3(WALK_THREADS),
+                        WALK_SMEM_BYTES, stream, tm_a, tm_b, p));
+    return CDL_OK;
+  }
   switch (p.split_k) {
     case 1: return launch<1>(tm_a, tm_b, p, dev, stream);
     case 2: return launch<2>(tm_a, tm_b, p, dev, stream);
