@@ -27,6 +27,8 @@
 // are more blocks than SMs) one CTA per SM that walks many blocks handed out at run time, so
 // that launch, allocation, first loads and first products of a block run under the previous
 // block's last products and stores.  Both forms execute the same arithmetic in the same order.
+// The one-CTA-per-block dK/dV kernel also exists in a split form, in which a cluster of CTAs shares a
+// block's queries (few kv heads for many query heads; see SPLIT and kv_split_of).
 // Scratch: LSE2 and delta, f32 [B, H, Sq_pad] each.
 #include "host.h"
 #include "ptx.cuh"

@@ -950,7 +950,7 @@ int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_t
     return fail(CDL_ERR_UNSUPPORTED, "matmul dimension too large");
 
   // f32 inputs, and bf16 operands TMA cannot describe (unaligned pointer or leading dimension):
-  // the general CUDA-core kernel (gemm_general.cu).  Operands without any contiguous dimension
+  // the general kernel (gemm_general.cu).  Operands without any contiguous dimension
   // stay rejected, as in the reference.
   if (f32_inputs) return matmul_general_execute(a, b, c, d, alpha, beta, stream);
   OperandLayout la, lb;

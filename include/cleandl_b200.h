@@ -324,7 +324,9 @@ typedef enum {
   CDL_ATTN_PERSISTENT = 2 /* forward: one CTA per SM walks the 256-row work items, longest first;
                            * part of the exponentials on the FMA pipe; backward: one CTA per SM
                            * walks the key blocks (dK, dV), longest first.  The automatic choice
-                           * of the backward is this form when there are more key blocks than SMs. */
+                           * of the backward is this form when there are more key blocks than SMs, unless
+                           * a few long ones (grouped-query heads) set the time: those are then shared
+                           * by clusters of CTAs, whose f32 sums meet in an order of their own. */
 } cdl_attn_variant;
 typedef struct {
   float softmax_scale; /* <= 0 selects 1/sqrt(D) (exec.rs:198-200) */
