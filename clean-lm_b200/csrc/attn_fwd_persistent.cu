@@ -453,30 +453,19 @@ __global__ void __launch_bounds__(THREADS, 1)
       };
       Tile T0{-1, 0, 0, 0u, 0u, 0u, 0u, 0u, false, false, true};
       Tile T1 = T0;
-      // Moves a tile's cursor to the first block of the next item the tile takes part in.  The
-      // items come from the producer's ring; one that is not published yet is waited for only
-      // when step r needs the answer, i.e. when the tile's next block could be at slot r + 1 or
-      // earlier.  (By then the producer can have published it: all it waits for before that is
-      // the release of slots that steps before r have released.  Waiting earlier could stall the
-      // other tile's products, which the producer may need in order to get there.)
-      auto next_item = [&](Tile& T, const int t, const int r) {
+      // Moves a tile's cursor to the first block of the next item the tile takes part in, as far as
+      // the producer's ring has been filled; where the ring ends before that, the tile stays open.
+      // Nothing is waited for here: the producer may need this lane's other products, or the other
+      // cursor's reads, before it can publish more (a run of items without key blocks fills the ring
+      // while this tile looks for its next block).  The loop over the steps waits.
+      auto next_item = [&](Tile& T, const int t) {
         while (true) {
           const int k = T.k + 1;
-          uint64_t* bar = &bars->item_full[k % ITEM_SLOTS];
-          const uint32_t par = (k / ITEM_SLOTS) & 1;
-          if (!mbar_test(bar, par)) {
-            if (static_cast<int>(T.next_base) > r + 1) {
-              T.open = true;
-              T.n = 0;
-              T.slot = T.next_base;
-              return;
-            }
-            if (!mbar_wait(bar, par, abort_word, 225)) {  // the abort word ends every other wait too
-              T.open = false;
-              T.n = 0;
-              T.slot = T.next_base;
-              return;
-            }
+          if (!mbar_test(&bars->item_full[k % ITEM_SLOTS], (k / ITEM_SLOTS) & 1)) {
+            T.open = true;
+            T.n = 0;
+            T.slot = T.next_base;
+            return;
           }
           T.k = k;
           const int idx = bars->item_ring[k % ITEM_SLOTS];
@@ -500,8 +489,6 @@ __global__ void __launch_bounds__(THREADS, 1)
           }
         }
       };
-      next_item(T0, 0, -1);
-      next_item(T1, 1, -1);
       // Ring slots this lane has seen filled, per stage (slot + 1 of the latest one).
       uint32_t k_seen0 = 0, k_seen1 = 0, v_seen0 = 0, v_seen1 = 0;
       // One tile's part of step r: P V for slot r if the tile has it, then S = Q K^T of the tile's
@@ -509,7 +496,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       // uses) is started only if its operands are there already, so that this step's other
       // products do not wait for it; otherwise it is started in the next step.
       auto turn = [&](Tile& T, const int t, const int r) -> bool {
-        if (T.open && !T.pend) next_item(T, t, r);
+        if (T.open && !T.pend) next_item(T, t);
         if (T.pend && static_cast<int>(T.pend_slot) == r) {
           const uint32_t st = static_cast<uint32_t>(r) % KV_STAGES;
           if (t == 0) CDL_PROBE(r, 6); else CDL_PROBE(r, 7);
@@ -526,7 +513,7 @@ __global__ void __launch_bounds__(THREADS, 1)
           issue_pv(t, st, T.acc, r);
           T.pend = false;
           CDL_PROBE(r, 3 * t + 1);
-          if (T.open) next_item(T, t, r);
+          if (T.open) next_item(T, t);
         }
         if (!T.pend && T.n > 0 && static_cast<int>(T.slot) <= r + 2) {
           const uint32_t s = T.slot;
@@ -555,7 +542,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             T.acc = !first;
             if (T.j + 1 == T.n) {
               umma_commit(&bars->q_empty[t]);  // the last reader of Q_t
-              next_item(T, t, r);
+              next_item(T, t);
             } else {
               ++T.j;
               ++T.slot;
@@ -566,13 +553,25 @@ __global__ void __launch_bounds__(THREADS, 1)
       };
       // r = -1 is the prologue (the first Q K^T of each tile); the loop ends when both tiles have
       // neither a block to start nor a P V due.
-      for (int r = -1; T0.pend || T1.pend || T0.n > 0 || T1.n > 0 || T0.open || T1.open; ++r) {
+      int r = -1;
+      while (T0.pend || T1.pend || T0.n > 0 || T1.n > 0 || T0.open || T1.open) {
         if (!turn(T0, 0, r) || !turn(T1, 1, r)) break;
+        // A tile whose next block could be at slot r + 1 has to know it before the step ends.  It has
+        // read everything published, so no published item reaches beyond slot r and both tiles have
+        // issued all they can: the softmax warps get through every published item, and the producer
+        // can publish the next one.  The step's turns are then taken once more.
+        const bool wait0 = T0.open && static_cast<int>(T0.next_base) <= r + 1;
+        if (wait0 || (T1.open && static_cast<int>(T1.next_base) <= r + 1)) {
+          const int k = (wait0 ? T0.k : T1.k) + 1;
+          if (!mbar_wait(&bars->item_full[k % ITEM_SLOTS], (k / ITEM_SLOTS) & 1, abort_word, 225)) break;
+          continue;
+        }
         // Every P V that reads V of slot r and every Q K^T that reads K of slot r + 1 has been
         // issued (a Q K^T is issued one or two steps before its slot's step).
         if (r >= 0) umma_commit(&bars->v_empty[static_cast<uint32_t>(r) % KV_STAGES]);
         umma_commit(&bars->k_empty[static_cast<uint32_t>(r + 1) % KV_STAGES]);
         if (r >= 0) CDL_PROBE(r, 31);
+        ++r;
       }
     }
     __syncwarp();

@@ -345,6 +345,48 @@ def test_packed_equals_dense_for_equal_lengths(cdl, gpu_ok):
     assert torch.equal(pdv.view(b, s, h, 128), ddv)
 
 
+@pytest.mark.parametrize("n,s,h", [(40, 100, 8), (70, 130, 8), (300, 3, 16)])
+def test_packed_without_a_bound_equals_dense(cdl, gpu_ok, n, s, h):
+    """max_seqlen left at its default, the packed total: nearly all work items of a batch of many short
+    sequences lie beyond their sequence, and every CTA of the forward draws more of them in a row than
+    the item ring has slots."""
+    q, k, v, _ = (t.cuda() for t in make(n, s, s, h, h, seed=6))
+    dense = cdl.ops.attention_fwd(q, k, v)
+    cu = torch.arange(0, (n + 1) * s, s, dtype=torch.int32).cuda()
+    flat = lambda t: t.reshape(n * s, h, 128)
+    packed = cdl.ops.attention_fwd(flat(q), flat(k), flat(v),
+                                   cdl.ops.AttentionOpts(cu_seqlens_q=cu, cu_seqlens_k=cu))
+    assert cdl._lib.device_status() == 0
+    # masked keys weigh at most 2^-126, and up to 127 of them are another sequence's here, zeros there
+    assert (packed.out.view(n, s, h, 128).float() - dense.out.float()).abs().max().item() <= 2.0 ** -112
+    assert torch.equal(packed.lse.view(h, n, s).permute(1, 0, 2), dense.lse)
+
+
+@pytest.mark.parametrize("every", [0, 90])
+def test_many_sequences_without_keys(cdl, gpu_ok, every):
+    """Long runs of items with rows to write and no key block (every 90th sequence has 130 keys, or none
+    has): rows without keys are zero with lse = -inf."""
+    n, h = 700, 8
+    lens_k = [130 if every and i % every == 7 else 0 for i in range(n)]
+    gen = torch.Generator().manual_seed(8)
+    q = torch.randn(n, h, 128, generator=gen).to(torch.bfloat16).cuda()
+    k, v = (torch.randn(max(sum(lens_k), 1), h, 128, generator=gen).to(torch.bfloat16).cuda() for _ in range(2))
+    cu_q = torch.arange(n + 1, dtype=torch.int32).cuda()
+    cu_k = torch.tensor([0, *np.cumsum(lens_k).tolist()], dtype=torch.int32).cuda()
+    out = cdl.ops.attention_fwd(q, k, v, cdl.ops.AttentionOpts(causal=False, cu_seqlens_q=cu_q, cu_seqlens_k=cu_k,
+                                                               max_seqlen_q=1, max_seqlen_k=130))
+    assert cdl._lib.device_status() == 0
+    for i in range(n):
+        k0, k1 = int(cu_k[i]), int(cu_k[i + 1])
+        if k1 == k0:
+            assert float(out.out[i].float().abs().max()) == 0.0 and bool(torch.isneginf(out.lse[:, i]).all())
+            continue
+        ref = oracle.attention(to_f32(q[None, i:i + 1]), to_f32(k[None, k0:k1]), to_f32(v[None, k0:k1]),
+                               to_f32(q[None, i:i + 1]), causal=False)
+        assert_all_close(f"out[{i}]", to_f32(out.out[i:i + 1])[None], ref["out"],
+                         oracle.attention_tolerance(ref["out"], 1e-2, 1e-2))
+
+
 @pytest.mark.parametrize("variant", [1, 2], ids=["one_shot", "persistent"])
 def test_packed_sequence_longer_than_the_bound_is_cut_and_reported(cdl, gpu_ok, variant):
     """max_seqlen_q / max_seqlen_k size the grids and the backward's statistics scratch.  A
