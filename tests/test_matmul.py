@@ -350,7 +350,8 @@ def test_unaligned_bf16_layouts(cdl, gpu_ok, m, k, n):
         run_case(cdl, a, b, torch.float32, c=torch.randn(m, n, generator=gen), alpha=0.5, beta=1.0, in_place=True)
 
 
-@pytest.mark.parametrize("m,k,n", [(1, 64, 8), (16, 576, 1024), (64, 2048, 264), (127, 1032, 136), (129, 4096, 128), (300, 2000, 520)])
+@pytest.mark.parametrize("m,k,n", [(1, 64, 8), (16, 576, 1024), (64, 2048, 264), (127, 1032, 136), (129, 4096, 128), (300, 2000, 520),
+                                   (600, 1024, 1000), (1000, 264, 1528), (200, 4096, 32), (77, 128, 24)])
 def test_tiles_shared_by_a_cluster(cdl, gpu_ok, m, k, n):
     """Few rows or a small output: K shared by 1, 2, 4 or 8 CTAs of a cluster, ragged last slices and
     tiles, every operand layout, C of both types, the accumulating form twice in place (bit-equal with
