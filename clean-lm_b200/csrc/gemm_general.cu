@@ -19,7 +19,9 @@
 // truncates when it adds, so it only ever sums one K block of 64, the small terms first; the blocks
 // are added with round-to-nearest.
 // A value whose pieces leave bf16's range (inf, NaN, the largest and the smallest magnitudes) has no
-// such sum: a CTA that met one computes its part of the tile again with plain FMAs.
+// such sum, and where a product overflows, h.h and h.m or m.h may be infinities of either sign (1e30
+// squared is one): a CTA that met such a value or a sum that is not finite computes its part of the tile
+// again with plain FMAs.
 // Measured error (2-norm, against f64) 1.2e-7 at K = 1024 .. 2048, where a chain of FMAs has 5.7e-7 .. 8.1e-7.
 //
 // What bounds it: the loaders and the shared memory they share with the tensor core (f32: 96 KiB of
@@ -77,7 +79,7 @@ struct Barriers {
   uint64_t acc_empty[2];
   uint32_t tmem_base;
   int abort_word;
-  int outside;  // f32: an element without an exact sum of three bf16 values was met
+  int outside;  // f32: an element without an exact sum of three bf16 values, or a sum that is not finite, was met
 };
 static_assert(sizeof(Barriers) <= 256, "barriers fit behind the stages");
 
@@ -329,6 +331,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     const int quad = warp & 3;
     const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
     const int groups = (blocks + p.sum_blocks - 1) / p.sum_blocks;
+    float zero = 0.f;  // NaN once a sum that is not finite has been met
     for (int g = 0; g < groups; ++g) {
       const int acc = g & 1;
       if (!mbar_wait(&bars->acc_full[acc], (g >> 1) & 1, abort_word, 331)) break;
@@ -350,7 +353,10 @@ __global__ void __launch_bounds__(THREADS, 1)
           // Every product is done and every stage read: the partial tile takes their place.
           float v[32];
 #pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+          for (int j = 0; j < 32; ++j) {
+            v[j] = __uint_as_float(r[j]);
+            if (F32) zero = fmaf(v[j], 0.f, zero);
+          }
           gemm::store_partial(part, quad * 32 + lane, c, v);
         } else {
           tmem_st32(t_row + 2 * TILE + c, r);
@@ -361,6 +367,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars->acc_empty[acc]);
     }
+    if (zero != 0.f) bars->outside = 1;
   }
   __syncwarp();
   if (F32) {

@@ -339,6 +339,27 @@ def test_f32_values_without_bf16_pieces(cdl, gpu_ok):
     assert bool((err[ok] <= 400 * 2.0 ** -24 * bound[ok] + 2.0 ** -126).all())
 
 
+@pytest.mark.parametrize("m,k,n", [(5, 3, 7), (200, 300, 150), (140, 2048, 129)])
+def test_f32_products_that_overflow(cdl, gpu_ok, m, k, n):
+    """Finite values that are exact sums of bf16 pieces, a product of which exceeds the range: the result is
+    the infinity of its sign, as in f32 arithmetic, whatever the signs of the pieces' products; a product
+    that stays below the range while that of its rounded pieces does not is finite."""
+    gen = torch.Generator().manual_seed(37)
+    a, b = torch.randn(m, k, generator=gen), torch.randn(k, n, generator=gen)
+    at = k // 2
+    a[:, at] = 1e30 * (1 + torch.rand(m, generator=gen)) * torch.where(torch.rand(m, generator=gen) < 0.5, -1.0, 1.0)
+    b[at] = 1e30 * (1 + torch.rand(n, generator=gen)) * torch.where(torch.rand(n, generator=gen) < 0.5, -1.0, 1.0)
+    b[at, ::3] = torch.randn(n, generator=gen)[::3]  # every third column stays in range
+    a[m - 1, at] = b[at, 1] = 1.8446742e19  # just below 2^64: the square is below 2^128, the bf16 rounding's is not
+    d = cdl.ops.matmul(a.cuda(), b.cuda(), cdl.ops.MatmulOpts(out=torch.float32)).cpu()
+    expected = (a.double() @ b.double())
+    over = expected.abs() > torch.finfo(torch.float32).max
+    assert not bool(d.isnan().any()) and torch.equal(d.isinf(), over) and not bool(over[m - 1, 1])
+    assert torch.equal(d[over].sign().double(), expected[over].sign())
+    bound = (a.abs().double() @ b.abs().double())
+    assert bool(((d.double() - expected).abs()[~over] <= (k + 1) * 2.0 ** -24 * bound[~over]).all())
+
+
 @pytest.mark.parametrize("m,k,n", [(1, 65, 3), (127, 131, 129), (130, 1027, 257)])
 def test_unaligned_bf16_layouts(cdl, gpu_ok, m, k, n):
     """Odd leading dimensions with K or M / N contiguous in either operand, accumulating into C."""
