@@ -2355,16 +2355,17 @@ __global__ void __launch_bounds__(THREADS, 1)
 // its longest item, nor before the work of all items spread over the SMs.  A split item costs every one
 // of its CTAs a fixed part (launch, first loads and products, the exchange: 11 us, 6 pairs), and as many
 // clusters run at a time as the GPCs hold, `slots[i]` of 2 << i CTAs.  Packed sequences are on the
-// device: `rows` query rows of evenly long sequences stand in for them, and the bound Sq for the longest.
+// device: sequences evenly long, in whole blocks as a dense call has them, stand in for them, and the bound Sq
+// for the longest.
 // Whole backward, one CTA per item -> chosen split: 16 heads on 4, B 1, S 512 45.9 -> 30.7 us (4), S 1000
 // 79 -> 46 (4), S 2048 145 -> 90 (4), S 4096 301 -> 214 (2); 8 on 2, S 8192 581 -> 383 (2); left alone
 // at 16 on 4, S 8192, 738 against 764.
-static int kv_split_of(const Params& p, long long rows, const int (&slots)[3]) {
+static int kv_split_of(const Params& p, long long rows_q, long long rows_k, const int (&slots)[3]) {
+  auto up = [](long long a, long long b) { return (a + b - 1) / b; };
   const double group = static_cast<double>(p.H) / p.Hkv;
-  const double len = p.cu_q ? static_cast<double>(rows) / p.B : p.Sq;
-  const double nq = (len + BQ - 1) / BQ, nk = p.cu_q ? nq : static_cast<double>((p.Sk + BKV - 1) / BKV);
-  const double items = nk * p.Hkv * p.B;
-  const double work = items * group * (p.causal ? (nq + 1) / 2 : nq) / sm_count();
+  const long long nq = up(p.cu_q ? up(rows_q, p.B) : p.Sq, BQ), nk = up(p.cu_q ? up(rows_k, p.B) : p.Sk, BKV);
+  const double items = static_cast<double>(nk * p.Hkv * p.B);
+  const double work = items * group * (p.causal ? (nq + 1) / 2.0 : static_cast<double>(nq)) / sm_count();
   const double longest = group * ((p.Sq + BQ - 1) / BQ);
   int best = 1;
   double best_cost = longest > work ? longest : work;
@@ -2504,7 +2505,7 @@ static int32_t bwd_run(const attn_bwd::Params& p_const, const cdl_tensor* q, con
     // run time from a counter of this stream; without one, a fixed deal).
     const bool persistent = p.variant == CDL_ATTN_PERSISTENT ||
                             (p.variant == CDL_ATTN_AUTO && CDL_ATTN_BWD_PERSISTENT && items > sm_count());
-    p.kv_split = p.variant == CDL_ATTN_AUTO ? kv_split_of(p, q->shape[1], kv_slots[dev & 63]) : 1;
+    p.kv_split = p.variant == CDL_ATTN_AUTO ? kv_split_of(p, q->shape[1], k->shape[1], kv_slots[dev & 63]) : 1;
     if (p.kv_split > 1 && items * p.kv_split < (1ll << 30)) {
       CDL_CUDA(launch_pdl_cluster(rope ? attn_bwd_dkdv_kernel<true, true> : attn_bwd_dkdv_kernel<false, true>,
                                   dim3(static_cast<unsigned>(items * p.kv_split)), dim3(THREADS), KV_SMEM_BYTES,

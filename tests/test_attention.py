@@ -345,6 +345,22 @@ def test_packed_equals_dense_for_equal_lengths(cdl, gpu_ok):
     assert torch.equal(pdv.view(b, s, h, 128), ddv)
 
 
+@pytest.mark.parametrize("b,s,h,hk", [(1, 2048, 16, 4), (2, 640, 8, 2), (5, 300, 8, 1)])
+def test_packed_grouped_query_equals_dense(cdl, gpu_ok, b, s, h, hk):
+    """Grouped-query heads, whose dK/dV items a cluster may share: equal lengths give the same split, and so
+    the same bits, packed and dense."""
+    q, k, v, do = (t.cuda() for t in make(b, s, s, h, hk, seed=15))
+    out = cdl.ops.attention_fwd(q, k, v)
+    dense = cdl.ops.attention_bwd(q, k, v, out.out, do, out.lse)
+    cu = torch.arange(0, (b + 1) * s, s, dtype=torch.int32).cuda()
+    opts = cdl.ops.AttentionOpts(cu_seqlens_q=cu, cu_seqlens_k=cu, max_seqlen_q=s, max_seqlen_k=s)
+    flat = lambda t: t.reshape(b * s, -1, 128)
+    lse = out.lse.permute(1, 0, 2).reshape(h, b * s).contiguous()
+    packed = cdl.ops.attention_bwd(flat(q), flat(k), flat(v), flat(out.out), flat(do), lse, opts)
+    for name, p, d in zip(("dq", "dk", "dv"), packed, dense):
+        assert torch.equal(p.view(d.shape), d), name
+
+
 @pytest.mark.parametrize("n,s,h", [(40, 100, 8), (70, 130, 8), (300, 3, 16)])
 def test_packed_without_a_bound_equals_dense(cdl, gpu_ok, n, s, h):
     """max_seqlen left at its default, the packed total: nearly all work items of a batch of many short
