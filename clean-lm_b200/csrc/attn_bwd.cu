@@ -124,8 +124,6 @@ struct Params {
   int* status;
 };
 
-constexpr double KV_SPLIT_FIXED = 6.0;  // see kv_split_of
-
 struct KvBarriers {
   uint64_t kv_full;
   uint64_t q_full[2], q_empty[2], do_full[2], do_empty[2];
@@ -2353,27 +2351,37 @@ __global__ void __launch_bounds__(THREADS, 1)
 
 // CTAs per item of the dK/dV kernel.  In block pairs (one takes 1.7 us): the launch cannot end before
 // its longest item, nor before the work of all items spread over the SMs.  A split item costs every one
-// of its CTAs a fixed part (launch, first loads and products, the exchange: 11 us, 6 pairs), and as many
-// clusters run at a time as the GPCs hold, `slots[i]` of 2 << i CTAs.  Packed sequences are on the
-// device: sequences evenly long, in whole blocks as a dense call has them, stand in for them, and the bound Sq
-// for the longest.
-// Whole backward, one CTA per item -> chosen split: 16 heads on 4, B 1, S 512 45.9 -> 30.7 us (4), S 1000
-// 79 -> 46 (4), S 2048 145 -> 90 (4), S 4096 301 -> 214 (2); 8 on 2, S 8192 581 -> 383 (2); left alone
-// at 16 on 4, S 8192, 738 against 764.
+// of its CTAs a fixed part (launch, first loads and products, the exchange: 8 us, 5 pairs), as many
+// clusters run at a time as the GPCs hold, `slots[i]` of 2 << i CTAs, and a CTA of a key block beyond its
+// sequence costs its launch (the persistent form draws such an item in a fraction of that).
+// Packed sequences are on the device: sequences evenly long, in whole blocks as a dense call has them,
+// stand in for them, and 1.25 times that for the longest, unless the bound says less.  The bound alone, by
+// default the packed total, says nothing of the lengths.
+// Fitted to 335 shapes (8 to 32 heads, groups of 1, 4 and 8, 1 to 64 sequences, 128 to 8192 rows, bounds tight and
+// loose): 0.4 % from the best choice on average, nowhere more than 2.1 % slower than without a split.
+// Whole backward, one CTA per item -> chosen split: 16 heads on 4, B 1, S 512 46.2 -> 30.5 us (4), S 1000
+// 80 -> 45 (4), S 2048 145 -> 90 (4), S 4096 304 -> 217 (2); 8 on 2, S 4096 264 -> 129 (4); left alone: 16 on
+// 4, 64 sequences of 128 with the bound 8192, 828 against 1380 (4).
+constexpr double KV_SPLIT_FIXED = 5.0, KV_SPLIT_WORK = 1.2, KV_SPLIT_EMPTY = 1.5, KV_SPLIT_LONGEST = 1.25;
 static int kv_split_of(const Params& p, long long rows_q, long long rows_k, const int (&slots)[3]) {
   auto up = [](long long a, long long b) { return (a + b - 1) / b; };
   const double group = static_cast<double>(p.H) / p.Hkv;
-  const long long nq = up(p.cu_q ? up(rows_q, p.B) : p.Sq, BQ), nk = up(p.cu_q ? up(rows_k, p.B) : p.Sk, BKV);
+  const long long len = p.cu_q ? up(rows_q, p.B) : p.Sq;
+  const long long nq = up(len, BQ), nk = up(p.cu_q ? up(rows_k, p.B) : p.Sk, BKV);
+  const long long bound_q = up(p.Sq, BQ), bound_k = up(p.Sk, BKV);
   const double items = static_cast<double>(nk * p.Hkv * p.B);
+  const double empty = bound_k > nk ? static_cast<double>((bound_k - nk) * p.Hkv * p.B) : 0.0;
   const double work = items * group * (p.causal ? (nq + 1) / 2.0 : static_cast<double>(nq)) / sm_count();
-  const double longest = group * ((p.Sq + BQ - 1) / BQ);
+  const long long longest_q = up(static_cast<long long>(KV_SPLIT_LONGEST * len), BQ);
+  const double longest = group * (p.cu_q && longest_q < bound_q ? longest_q : bound_q);
   int best = 1;
   double best_cost = longest > work ? longest : work;
   for (int i = 0; i < 3; ++i) {
     const int s = 2 << i;
     if (slots[i] <= 0) continue;
     const double waves = ceil(items / slots[i]);
-    const double spread = KV_SPLIT_FIXED * waves + 1.1 * work, deep = KV_SPLIT_FIXED + longest / s;
+    const double spread = KV_SPLIT_FIXED * waves + KV_SPLIT_WORK * work + KV_SPLIT_EMPTY * empty * s / sm_count();
+    const double deep = KV_SPLIT_FIXED + longest / s;
     const double cost = deep > spread ? deep : spread;
     if (cost < 0.9 * best_cost) {
       best = s;

@@ -361,6 +361,22 @@ def test_packed_grouped_query_equals_dense(cdl, gpu_ok, b, s, h, hk):
         assert torch.equal(p.view(d.shape), d), name
 
 
+@pytest.mark.parametrize("b,s,h,hk", [(64, 128, 16, 4), (16, 256, 16, 4), (40, 100, 16, 4)])
+def test_short_items_stay_whole_without_a_bound(cdl, gpu_ok, b, s, h, hk):
+    """max_seqlen at its default, the packed total, gives the bits of the true one: a bound that says nothing
+    of the lengths does not make clusters share items that are short."""
+    q, k, v, do = (t[0].cuda() for t in make(1, b * s, b * s, h, hk, seed=16))
+    cu = torch.arange(0, (b + 1) * s, s, dtype=torch.int32).cuda()
+    grads = []
+    for bound in (s, None):
+        opts = cdl.ops.AttentionOpts(cu_seqlens_q=cu, cu_seqlens_k=cu, max_seqlen_q=bound, max_seqlen_k=bound)
+        out = cdl.ops.attention_fwd(q, k, v, opts)
+        grads.append(cdl.ops.attention_bwd(q, k, v, out.out, do, out.lse, opts))
+    assert cdl._lib.device_status() == 0
+    for name, x, y in zip(("dq", "dk", "dv"), *grads):
+        assert torch.equal(x, y), name
+
+
 @pytest.mark.parametrize("n,s,h", [(40, 100, 8), (70, 130, 8), (300, 3, 16)])
 def test_packed_without_a_bound_equals_dense(cdl, gpu_ok, n, s, h):
     """max_seqlen left at its default, the packed total: nearly all work items of a batch of many short
