@@ -21,7 +21,7 @@
 // A value whose pieces leave bf16's range (inf, NaN, the largest and the smallest magnitudes) has no
 // such sum, and where a product overflows, h.h and h.m or m.h may be infinities of either sign (1e30
 // squared is one): a CTA that met such a value or a sum that is not finite computes its part of the tile
-// again with plain FMAs.
+// again with plain FMAs (partial_by_fma).
 // Measured error (2-norm, against f64) 1.2e-7 at K = 1024 .. 2048, where a chain of FMAs has 5.7e-7 .. 8.1e-7.
 //
 // What bounds it: the loaders and the shared memory they share with the tensor core (f32: 96 KiB of
@@ -201,19 +201,136 @@ __device__ __forceinline__ bool store_rows(uint32_t tile, int lane, const PairF3
   return exact;
 }
 
-// The CTA's part of the tile with plain FMAs (see the top of the file).
-__device__ __noinline__ void partial_by_fma(const Params& p, const Operand& oa, const Operand& ob, int b, int m0,
-                                            int n0, int k_begin, int k_end, float* part) {
-  const float* a = static_cast<const float*>(oa.ptr) + b * oa.s_batch;
-  const float* bb = static_cast<const float*>(ob.ptr) + b * ob.s_batch;
-  for (int e = threadIdx.x; e < TILE * TILE; e += blockDim.x) {
-    const int r = e / TILE, c = e % TILE;
-    if (m0 + r >= p.M || n0 + c >= p.N) continue;
-    const float* ar = a + (m0 + r) * oa.s_mn;
-    const float* bc = bb + (n0 + c) * ob.s_mn;
-    float acc = 0.f;
-    for (int k = k_begin; k < k_end; ++k) acc = fmaf(ar[k * oa.s_k], bc[k * ob.s_k], acc);
-    part[r * gemm::PART_LD + c] = acc;
+// ------------------------------------------------------------ plain FMAs
+// A chain of FMAs over K in ascending order, both operands through shared memory FMA_K elements deep
+// ([k][i], two buffers), the next FMA_K on their way in registers meanwhile.
+constexpr int FMA_K = 16;
+template <int N>
+constexpr int fma_tile() { return FMA_K * (N + 4); }
+
+__device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi) {
+  uint64_t v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+  return v;
+}
+__device__ __forceinline__ void unpack_f32x2(uint64_t v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+
+// One operand's N x FMA_K elements, fetched by `THREADS_` threads (lanes walk the contiguous index) and
+// written to shared memory as S.
+template <typename T, typename S, int N, int THREADS_>
+struct FmaSource {
+  static constexpr int PER = N * FMA_K / THREADS_;
+  static_assert(N * FMA_K % THREADS_ == 0 && THREADS_ % N == 0, "a thread's elements are evenly spaced");
+  const T* q;           // this thread's first element of the next FMA_K
+  long long step, adv;  // from element to element, from FMA_K to FMA_K
+  int left_i, left_k;   // elements that exist from the first one on, along M or N and along K
+  int di, dk;           // element to element, along either
+  int at, dat;          // place in shared memory
+  float v[PER];
+  __device__ __forceinline__ void init(const Operand& o, int batch, int mn0, int k0, int k_end) {
+    const int t = threadIdx.x;
+    const int i = o.mn_major ? t % N : t / FMA_K, k = o.mn_major ? t / N : t % FMA_K;
+    di = o.mn_major ? 0 : THREADS_ / FMA_K;
+    dk = o.mn_major ? THREADS_ / N : 0;
+    step = di * o.s_mn + dk * o.s_k;
+    adv = FMA_K * o.s_k;
+    left_i = o.mn - (mn0 + i);
+    left_k = k_end - (k0 + k);
+    at = k * (N + 4) + i;
+    dat = dk * (N + 4) + di;
+    q = static_cast<const T*>(o.ptr) + batch * o.s_batch + (mn0 + i) * o.s_mn + (k0 + k) * o.s_k;
+  }
+  // Zeros outside the operand.
+  __device__ __forceinline__ void fetch() {
+#pragma unroll
+    for (int j = 0; j < PER; ++j) v[j] = j * di < left_i && j * dk < left_k ? as_f32(q[j * step]) : 0.f;
+    q += adv;
+    left_k -= FMA_K;
+  }
+  __device__ __forceinline__ void store(S* tile) const {
+#pragma unroll
+    for (int j = 0; j < PER; ++j) tile[at + j * dat] = static_cast<S>(v[j]);
+  }
+  static __device__ __forceinline__ float as_f32(float x) { return x; }
+  static __device__ __forceinline__ float as_f32(__nv_bfloat16 x) { return __bfloat162float(x); }
+};
+// acc[i][4 c + j] += row ty * 4 + i of A times column tx * 4 + 64 c + j of B over FMA_K elements.  In f32
+// two columns at a time: packed FMAs round as single ones do.
+template <int N, int C>
+__device__ __forceinline__ void fma_block(const float* ta, const float* tb, int tx, int ty, float (&acc)[4][4 * C]) {
+  uint64_t sums[4][2 * C];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 2 * C; ++j) sums[i][j] = pack_f32x2(acc[i][2 * j], acc[i][2 * j + 1]);
+#pragma unroll
+  for (int kk = 0; kk < FMA_K; ++kk) {
+    const float4 av = *reinterpret_cast<const float4*>(ta + kk * (N + 4) + ty * 4);
+    const uint64_t ar[4] = {pack_f32x2(av.x, av.x), pack_f32x2(av.y, av.y), pack_f32x2(av.z, av.z), pack_f32x2(av.w, av.w)};
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      const float4 bv = *reinterpret_cast<const float4*>(tb + kk * (N + 4) + tx * 4 + 64 * c);
+      const uint64_t br[2] = {pack_f32x2(bv.x, bv.y), pack_f32x2(bv.z, bv.w)};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+          asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(sums[i][2 * c + j]) : "l"(ar[i]), "l"(br[j]));
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 2 * C; ++j) unpack_f32x2(sums[i][j], acc[i][2 * j], acc[i][2 * j + 1]);
+}
+
+// The CTA's part of the tile once more (see the top of the file), by the first 512 of its threads, 4 x 8
+// sums each; 12 floats from shared memory for 32 FMAs, which is what bounds it.  1024 x 2048 x 1536 with one
+// value of 1e-35, or only such: 409 us (74 without; 64 x 64 tiles of FMAs alone 457; thread by thread from
+// global memory 5080, B transposed 18080); 2048 x 256 x 2048, all: 118 (33; 142; 1256).  `smem` is the start of the operand stages as an offset into shared memory: a pointer argument
+// would be loaded from as a generic address.  The partial tile goes there, the operands' tiles behind it.
+constexpr int REDO_THREADS = 512, REDO_FLOATS = 2 * fma_tile<TILE>();
+static_assert(gemm::PART_BYTES + 2 * REDO_FLOATS * sizeof(float) <= Traits<float>::STAGES * 6 * PIECE_BYTES,
+              "the FMA tiles fit behind the partial tile");
+__device__ __noinline__ void partial_by_fma(const Operand& oa, const Operand& ob, int b, int m0, int n0, int k_begin,
+                                            int k_end, int smem) {
+  extern __shared__ uint8_t smem_raw[];
+  float* part = reinterpret_cast<float*>(smem_raw + smem);
+  float* tiles = reinterpret_cast<float*>(smem_raw + smem + gemm::PART_BYTES);
+  const bool works = threadIdx.x < REDO_THREADS;
+  const int tx = threadIdx.x & 15, ty = (threadIdx.x >> 4) & 31;
+  FmaSource<float, float, TILE, REDO_THREADS> fa, fb;
+  float acc[4][8] = {};
+  if (works) {
+    fa.init(oa, b, m0, k_begin, k_end);
+    fb.init(ob, b, n0, k_begin, k_end);
+    fa.fetch();
+    fb.fetch();
+  }
+  int buf = 0;
+  for (int k0 = k_begin; k0 < k_end; k0 += FMA_K, buf ^= 1) {
+    float* ta = tiles + buf * REDO_FLOATS;
+    float* tb = ta + fma_tile<TILE>();
+    if (works) {
+      fa.store(ta);
+      fb.store(tb);
+      if (k0 + FMA_K < k_end) {
+        fa.fetch();
+        fb.fetch();
+      }
+    }
+    __syncthreads();  // the other buffer has been read by all who are here
+    if (works) fma_block<TILE, 2>(ta, tb, tx, ty, acc);
+  }
+  if (works) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+        *reinterpret_cast<float4*>(part + (ty * 4 + i) * gemm::PART_LD + tx * 4 + 64 * c) =
+            make_float4(acc[i][4 * c], acc[i][4 * c + 1], acc[i][4 * c + 2], acc[i][4 * c + 3]);
   }
 }
 
@@ -373,7 +490,8 @@ __global__ void __launch_bounds__(THREADS, 1)
   if (F32) {
     __syncthreads();
     if (bars->outside != 0)
-      partial_by_fma(p, oa, ob, b, m0, n0, kb0 * BK, min(kb1 * BK, p.K), part);
+      partial_by_fma(oa, ob, b, m0, n0, kb0 * BK, min(kb1 * BK, p.K),
+                     static_cast<int>(smem - smem_raw));
   }
   if (p.split_k > 1) cluster_sync_all();
   else __syncthreads();

@@ -339,6 +339,33 @@ def test_f32_values_without_bf16_pieces(cdl, gpu_ok):
     assert bool((err[ok] <= 400 * 2.0 ** -24 * bound[ok] + 2.0 ** -126).all())
 
 
+@pytest.mark.parametrize("m,k,n", [(1, 33, 129), (127, 64, 1), (129, 65, 130), (140, 1029, 257), (300, 700, 1500)])
+@pytest.mark.parametrize("fa,fb", [("row", "row"), ("col", "row"), ("row", "col"), ("strided", "strided")])
+def test_f32_tiles_without_bf16_pieces(cdl, gpu_ok, m, k, n, fa, fb):
+    """Tiles with values that have no bf16 pieces (the low bits of 1e-37 lie below bf16's range), edges of the
+    tile, of the K step of 16 and of the K slices: one such value at the end of K, and a row and a column of
+    them.  Bound: a chain of K roundings, 2^-24 of sum |a b| each, and the pieces' of the other tiles; products
+    below 2^-126 lose up to 2^-149 each."""
+    gen = torch.Generator().manual_seed(m + 3 * k + n)
+    for which in ("one", "lines"):
+        a, b = _f32_operand(gen, m, k, fa), _f32_operand(gen, k, n, fb)
+        a[m - 1, k - 1] *= 1e-37
+        if which == "lines":
+            a[m // 2] *= 1e-37
+            b[:, n // 2] *= 1e-37
+            b[:, n // 2] += 1e-30  # products in range, and exact sums beside ones that are not
+
+        def to_dev(t):
+            base = torch.empty(0, dtype=t.dtype).set_(t.untyped_storage())
+            return base.cuda().as_strided(t.shape, t.stride(), t.storage_offset())
+
+        d = cdl.ops.matmul(to_dev(a), to_dev(b), cdl.ops.MatmulOpts(out=torch.float32))
+        expected, bound = a.double() @ b.double(), a.abs().double() @ b.abs().double()
+        tol = (k + 10) * 2.0 ** -24 * bound + k * 2.0 ** -149
+        assert_all_close("f32 product", d.double().cpu().numpy(), expected.numpy(), tol.numpy())
+    assert cdl._lib.device_status() == 0
+
+
 @pytest.mark.parametrize("m,k,n", [(5, 3, 7), (200, 300, 150), (140, 2048, 129)])
 def test_f32_products_that_overflow(cdl, gpu_ok, m, k, n):
     """Finite values that are exact sums of bf16 pieces, a product of which exceeds the range: the result is
