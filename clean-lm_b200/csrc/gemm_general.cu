@@ -4,7 +4,8 @@
 // the reference computes those with TF32 tensor cores, 10 mantissa bits; here the products are full
 // f32, which its tolerance contains).
 //
-// D = alpha * A . B + beta * C, f32 accumulation.  128 x 128 tiles; the K range of a tile is shared by
+// D = alpha * A . B + beta * C, f32 accumulation.  Products of a short K are sums of plain FMAs
+// (gemm_fma_kernel); the others go to the tensor cores.  128 x 128 tiles; the K range of a tile is shared by
 // a cluster of 1, 2, 4 or 8 CTAs whose partial sums meet in distributed shared memory (gemm_rows.cuh).
 //   warp 0       issues the tcgen05.mma (M128 N128 K16)
 //   16 loader warps: a warp takes a row of 64 consecutive elements, a lane two of
@@ -256,10 +257,11 @@ struct FmaSource {
   static __device__ __forceinline__ float as_f32(float x) { return x; }
   static __device__ __forceinline__ float as_f32(__nv_bfloat16 x) { return __bfloat162float(x); }
 };
-// acc[i][4 c + j] += row ty * 4 + i of A times column tx * 4 + 64 c + j of B over FMA_K elements.  In f32
-// two columns at a time: packed FMAs round as single ones do.
+// acc[i][4 c + j] += row ty * 4 + i of A times column tx * 4 + 64 c + j of B over FMA_K elements, of which `left`
+// exist.  In f32 two columns at a time: packed FMAs round as single ones do.
 template <int N, int C>
-__device__ __forceinline__ void fma_block(const float* ta, const float* tb, int tx, int ty, float (&acc)[4][4 * C]) {
+__device__ __forceinline__ void fma_block(const float* ta, const float* tb, int tx, int ty, int left,
+                                          float (&acc)[4][4 * C]) {
   uint64_t sums[4][2 * C];
 #pragma unroll
   for (int i = 0; i < 4; ++i)
@@ -267,6 +269,7 @@ __device__ __forceinline__ void fma_block(const float* ta, const float* tb, int 
     for (int j = 0; j < 2 * C; ++j) sums[i][j] = pack_f32x2(acc[i][2 * j], acc[i][2 * j + 1]);
 #pragma unroll
   for (int kk = 0; kk < FMA_K; ++kk) {
+    if (kk % 4 == 0 && kk >= left) break;
     const float4 av = *reinterpret_cast<const float4*>(ta + kk * (N + 4) + ty * 4);
     const uint64_t ar[4] = {pack_f32x2(av.x, av.x), pack_f32x2(av.y, av.y), pack_f32x2(av.z, av.z), pack_f32x2(av.w, av.w)};
 #pragma unroll
@@ -322,7 +325,7 @@ __device__ __noinline__ void partial_by_fma(const Operand& oa, const Operand& ob
       }
     }
     __syncthreads();  // the other buffer has been read by all who are here
-    if (works) fma_block<TILE, 2>(ta, tb, tx, ty, acc);
+    if (works) fma_block<TILE, 2>(ta, tb, tx, ty, FMA_K, acc);
   }
   if (works) {
 #pragma unroll
@@ -513,6 +516,131 @@ __global__ void __launch_bounds__(THREADS, 1)
   if (threadIdx.x == 0 && *abort_word != 0) atomicExch(p.status, *abort_word);
 }
 
+// The same in f64.
+template <int N, int C>
+__device__ __forceinline__ void fma_block(const double* ta, const double* tb, int tx, int ty, int left,
+                                          double (&acc)[4][4 * C]) {
+  static_assert(C == 1, "");
+#pragma unroll
+  for (int kk = 0; kk < FMA_K; ++kk) {
+    if (kk % 4 == 0 && kk >= left) break;
+    const double2* a2 = reinterpret_cast<const double2*>(ta + kk * (N + 4) + ty * 4);
+    const double2* b2 = reinterpret_cast<const double2*>(tb + kk * (N + 4) + tx * 4);
+    const double ar[4] = {a2[0].x, a2[0].y, a2[1].x, a2[1].y}, br[4] = {b2[0].x, b2[0].y, b2[1].x, b2[1].y};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = fma(ar[i], br[j], acc[i][j]);
+  }
+}
+
+// Products of a short K, one CTA per 64 x 64 tile: 4 x 4 sums a thread, stored as they stand.  Bound by launch,
+// first loads and the store: no tensor memory, no staging of pieces, several CTAs per SM.  f32 products are
+// summed in f64, where they are exact: the result carries one rounding (2.5e-8, 2-norm, against f64), where a
+// chain of f32 FMAs has 4.0e-8 at K = 4 and 7.3e-8 at 16 and the pieces 4.7e-8 and 4.8e-8.  Products of bf16
+// are exact in f32 and a chain of f32 adds has less error than the truncating tensor core (2.2e-8 against 2.5e-8
+// at 16).
+template <typename T> struct FmaSum { using type = float; };
+template <> struct FmaSum<float> { using type = double; };
+constexpr int FMA_TILE = 64, FMA_THREADS = 256, FMA_FLOATS = 2 * fma_tile<FMA_TILE>();
+template <typename T>
+__global__ void __launch_bounds__(FMA_THREADS) gemm_fma_kernel(const Params p, const Operand oa, const Operand ob) {
+  using S = typename FmaSum<T>::type;
+  __shared__ __align__(16) S tiles[2 * FMA_FLOATS];
+  grid_dep_wait();
+  grid_dep_launch();
+  int b, tm, tn;
+  gemm::tile_coords(p, static_cast<int>(blockIdx.x), b, tm, tn);
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int row0 = tm * FMA_TILE + ty * 4, col = tn * FMA_TILE + tx * 4;
+  FmaSource<T, S, FMA_TILE, FMA_THREADS> fa, fb;
+  S acc[4][4] = {};
+  fa.init(oa, b, tm * FMA_TILE, 0, p.K);
+  fb.init(ob, b, tn * FMA_TILE, 0, p.K);
+  fa.fetch();
+  fb.fetch();
+  // C is read ahead of the products: its latency, row after row, is longer than they are.
+  float c[4][4] = {};
+  if (p.c_mode != 0) {
+    const bool vec = p.c_vec && col + 4 <= p.N;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (row0 + i >= p.M) continue;
+      const long long at = b * p.c_batch + (row0 + i) * p.ldc + col;
+      const float* cf = static_cast<const float*>(p.c) + at;
+      const __nv_bfloat16* ch = static_cast<const __nv_bfloat16*>(p.c) + at;
+      if (vec && p.c_mode == 2) {
+        const float4 q = *reinterpret_cast<const float4*>(cf);
+        c[i][0] = q.x; c[i][1] = q.y; c[i][2] = q.z; c[i][3] = q.w;
+      } else if (vec) {
+        const uint2 q = *reinterpret_cast<const uint2*>(ch);
+        c[i][0] = bf16_lo(q.x); c[i][1] = bf16_hi(q.x); c[i][2] = bf16_lo(q.y); c[i][3] = bf16_hi(q.y);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (col + j < p.N) c[i][j] = p.c_mode == 2 ? cf[j] : __bfloat162float(ch[j]);
+      }
+    }
+  }
+  int buf = 0;
+  for (int k0 = 0; k0 < p.K; k0 += FMA_K, buf ^= 1) {
+    S* ta = tiles + buf * FMA_FLOATS;
+    S* tb = ta + fma_tile<FMA_TILE>();
+    fa.store(ta);
+    fb.store(tb);
+    if (k0 + FMA_K < p.K) {
+      fa.fetch();
+      fb.fetch();
+    }
+    __syncthreads();  // the other buffer has been read by all who are here
+    fma_block<FMA_TILE, 1>(ta, tb, tx, ty, p.K - k0, acc);
+  }
+  const bool vec = p.d_vec && col + 4 <= p.N;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if (row0 + i >= p.M) continue;
+    float v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = p.c_mode != 0 ? p.alpha * static_cast<float>(acc[i][j]) + p.beta * c[i][j] : p.alpha * static_cast<float>(acc[i][j]);
+    const long long at = b * p.d_batch + (row0 + i) * p.ldd + col;
+    float* df = static_cast<float*>(p.d) + at;
+    __nv_bfloat16* dh = static_cast<__nv_bfloat16*>(p.d) + at;
+    if (vec && p.out_f32) {
+      *reinterpret_cast<float4*>(df) = make_float4(v[0], v[1], v[2], v[3]);
+    } else if (vec) {
+      *reinterpret_cast<uint2*>(dh) = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (col + j < p.N) {
+          if (p.out_f32) df[j] = v[j];
+          else dh[j] = __float2bfloat16_rn(v[j]);
+        }
+    }
+  }
+}
+
+// Whether the FMAs are done before the tensor-core kernel is: it takes 7.7 to 9 us (bf16 5.6 to 7.5) before K counts,
+// the FMAs 2.7 and, per 16 of K and tile of an SM, 1.3 (bf16 0.7).  In microseconds, tensor cores -> FMAs: f32
+// 1500 x 4 x 1027 10.1 -> 7.1, 2048 x 16 x 2048 19.2 -> 15.6, 4096 x 1 x 4096 64 -> 31, 64 x 48 x 64 8.0 -> 7.6; the
+// other way at 64 x 64 x 8192, 8.7 against 9.3, and 2048 x 24 x 2048, 19.2 against 25.5.  bf16 1500 x 17 x 1027
+// 8.0 -> 7.0, 4096 x 9 x 4097 54.6 -> 32.2, 300 x 49 x 301 7.6 -> 6.5; the other way at 2048 x 25 x 2049, 14.8
+// against 16.7, and 1024 x 33 x 1025, 7.6 against 8.9.
+static bool short_k(const Params& p, bool f32) {
+  const int steps = (p.K + FMA_K - 1) / FMA_K;
+  const long long tiles = static_cast<long long>(p.batch) * ((p.M + FMA_TILE - 1) / FMA_TILE) * ((p.N + FMA_TILE - 1) / FMA_TILE);
+  const long long waves = (tiles + sm_count() - 1) / sm_count();
+  return steps == 1 || steps * waves <= (f32 ? 3 : 4) || (!f32 && steps == 2 && waves <= 4);
+}
+template <typename T>
+static int32_t launch_fma(Params& p, const Operand& oa, const Operand& ob, cudaStream_t stream) {
+  p.num_m_tiles = (p.M + FMA_TILE - 1) / FMA_TILE;
+  p.num_n_tiles = (p.N + FMA_TILE - 1) / FMA_TILE;
+  p.num_tiles = p.batch * p.num_m_tiles * p.num_n_tiles;
+  CDL_CUDA(launch_pdl(gemm_fma_kernel<T>, dim3(static_cast<unsigned>(p.num_tiles)), dim3(FMA_THREADS), 0, stream, p, oa, ob));
+  return CDL_OK;
+}
+
 // K slices per tile: the number whose waves of resident CTAs end first.  A CTA's time is its K blocks
 // and a part that does not shrink (set-up, first loads, the exchange of the partial sums, stores).
 // f32 300 x 2048 x 130 with 1, 2, 4, 8 slices: 69, 39, 24, 17 us; 1024 x 2048 x 1536 74, 81, 76, 121 us.
@@ -612,6 +740,8 @@ int32_t matmul_general_execute(const cdl_tensor* a, const cdl_tensor* b, const c
   // takes eight at a time.
   p.sum_blocks = d->dtype == CDL_F32 || a->dtype == CDL_F32 ? 1 : 8;
   ProfileScope ps(PROF_GEMM, 2.0 * batch * M * N * K, stream);
+  if (short_k(p, a->dtype == CDL_F32))
+    return a->dtype == CDL_F32 ? launch_fma<float>(p, oa, ob, stream) : launch_fma<__nv_bfloat16>(p, oa, ob, stream);
   return a->dtype == CDL_F32 ? launch<float>(p, oa, ob, 4.0, stream)
                              : launch<__nv_bfloat16>(p, oa, ob, 6.0, stream);
 }

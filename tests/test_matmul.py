@@ -339,6 +339,43 @@ def test_f32_values_without_bf16_pieces(cdl, gpu_ok):
     assert bool((err[ok] <= 400 * 2.0 ** -24 * bound[ok] + 2.0 ** -126).all())
 
 
+@pytest.mark.parametrize("m,k,n", [(1, 1, 1), (63, 2, 65), (64, 3, 64), (65, 4, 130), (200, 16, 66), (300, 15, 1000)])
+@pytest.mark.parametrize("fa,fb", [("row", "row"), ("col", "row"), ("row", "col"), ("strided", "strided")])
+def test_f32_products_of_a_short_k_round_once(cdl, gpu_ok, m, k, n, fa, fb):
+    """Up to 16 products are summed exactly but for f64's roundings: the f32 result is the nearest one (half an
+    ulp, and K roundings of 2^-53 of sum |a b| before it)."""
+    gen = torch.Generator().manual_seed(m * 5 + k + n)
+    a, b = _f32_operand(gen, m, k, fa), _f32_operand(gen, k, n, fb)
+
+    def to_dev(t):
+        base = torch.empty(0, dtype=t.dtype).set_(t.untyped_storage())
+        return base.cuda().as_strided(t.shape, t.stride(), t.storage_offset())
+
+    d = cdl.ops.matmul(to_dev(a), to_dev(b), cdl.ops.MatmulOpts(out=torch.float32))
+    expected, bound = a.double() @ b.double(), a.abs().double() @ b.abs().double()
+    tol = 2.0 ** -24 * expected.abs() + k * 2.0 ** -52 * bound + 2.0 ** -149
+    assert_all_close("f32 product", d.double().cpu().numpy(), expected.numpy(), tol.numpy())
+
+
+@pytest.mark.parametrize("m,k,n", [(1, 3, 5), (64, 9, 64), (65, 17, 68), (130, 49, 63), (500, 31, 129), (1100, 33, 1027)])
+def test_short_k_forms(cdl, gpu_ok, m, k, n):
+    """The forms of the general matmul around the rule that sends a short K to plain FMAs: bf16 rows off the
+    grid and f32, C of both types and none, in place, batched, transposed, aligned and unaligned outputs."""
+    gen = torch.Generator().manual_seed(m + 11 * k + n)
+    a, b = rand_bf16(gen, m, k), rand_bf16(gen, k, n)
+    run_case(cdl, a, b, torch.bfloat16)
+    run_case(cdl, a, b, torch.bfloat16, c=rand_bf16(gen, m, n), alpha=0.5, beta=2.0)
+    run_case(cdl, rand_bf16(gen, k, m + (m + 1) % 2).T[:m], rand_bf16(gen, n, k).T, torch.float32,
+             c=torch.randn(m, n, generator=gen), beta=1.0, in_place=True)
+    run_case(cdl, rand_bf16(gen, 3, m, k), rand_bf16(gen, 3, k, n), torch.float32)
+    x, w = torch.randn(2, m, k, generator=gen), torch.randn(2, k, n, generator=gen)
+    c = torch.randn(2, m, n, generator=gen)
+    d = cdl.ops.matmul(x.cuda(), w.cuda(), cdl.ops.MatmulOpts(out=torch.float32, c=c.cuda(), alpha=-1.5, beta=0.5))
+    expected = -1.5 * (x.double() @ w.double()) + 0.5 * c.double()
+    bound = 1.5 * (x.abs().double() @ w.abs().double()) + 0.5 * c.abs().double()
+    assert_all_close("f32", d.double().cpu().numpy(), expected.numpy(), ((k + 4) * 2.0 ** -24 * bound).numpy())
+
+
 @pytest.mark.parametrize("m,k,n", [(1, 33, 129), (127, 64, 1), (129, 65, 130), (140, 1029, 257), (300, 700, 1500)])
 @pytest.mark.parametrize("fa,fb", [("row", "row"), ("col", "row"), ("row", "col"), ("strided", "strided")])
 def test_f32_tiles_without_bf16_pieces(cdl, gpu_ok, m, k, n, fa, fb):
