@@ -12,7 +12,7 @@
 //                them, with plain loads of any alignment, and writes them as bf16 into the
 //                128-byte-swizzled tile the tensor core reads; the loads of the next K block are in
 //                flight meanwhile
-//   4 sum warps  add the tensor core's sums of a few K blocks (Params::sum_blocks) to the running sums
+//   4 sum warps  add the tensor core's sums (of Params::sum_blocks) to the running sums
 //
 // f32 operands.  A f32 value is the exact sum of three bf16 values (8 significant bits each):
 // x = h + m + l.  Of the nine products of two such sums the six of h.h, h.m, m.h, m.m, h.l and l.h are
@@ -34,6 +34,9 @@
 #include "ops.h"
 #include "ptx.cuh"
 
+#include <math.h>
+
+#include <algorithm>
 #include <mutex>
 
 namespace cdl {
@@ -345,7 +348,8 @@ __device__ __forceinline__ void store_out(const Params& p, const float* part, in
   out.finish(p, part, rank, warp, b, m0, n0);
 }
 
-template <typename T>
+// FINE: an accumulator sums up half a K block (see matmul_general_execute).
+template <typename T, bool FINE>
 __global__ void __launch_bounds__(THREADS, 1)
     gemm_general_kernel(const Params p, const Operand oa, const Operand ob) {
   using Tr = Traits<T>;
@@ -397,7 +401,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       const uint32_t idesc = make_idesc_bf16(TILE, TILE, oa.mn_major, ob.mn_major);
       const uint32_t a_lbo = oa.mn_major ? 8192u : 16u, b_lbo = ob.mn_major ? 8192u : 16u;
       const uint32_t a_kstep = oa.mn_major ? 2048u : 32u, b_kstep = ob.mn_major ? 2048u : 32u;
-      for (int it = 0; it < blocks; ++it) {
+      for (int it = 0; !FINE && it < blocks; ++it) {
         const int s = it % STAGES, group = it / p.sum_blocks, acc = group & 1;
         const bool first = it == group * p.sum_blocks, last = it + 1 == blocks || it + 1 == (group + 1) * p.sum_blocks;
         if ((first && !mbar_wait(&bars->acc_empty[acc], ((group >> 1) & 1) ^ 1, abort_word, 231)) ||
@@ -418,6 +422,26 @@ __global__ void __launch_bounds__(THREADS, 1)
                     (!first || (t | k) != 0) ? 1u : 0u);
         umma_commit(&bars->empty[s]);
         if (last) umma_commit(&bars->acc_full[acc]);
+      }
+      if (FINE) {
+        bool ok = true;
+        for (int it = 0; it < blocks && ok; ++it) {
+          const int s = it % STAGES;
+          if (!mbar_wait(&bars->full[s], (it / STAGES) & 1, abort_word, 233)) break;
+          const uint32_t sa = smem_u32(smem + s * stage_bytes<T>()), sb = sa + PIECE_BYTES;
+#pragma unroll
+          for (int acc = 0; acc < 2; ++acc) {
+            ok = mbar_wait(&bars->acc_empty[acc], (it & 1) ^ 1, abort_word, 234);
+            if (!ok) break;
+            tc_fence_after();
+#pragma unroll
+            for (int k = 2 * acc; k < 2 * acc + 2; ++k)
+              umma_ss(tmem_base + acc * TILE, smem_desc_sw128(sa + k * a_kstep, a_lbo, 1024),
+                      smem_desc_sw128(sb + k * b_kstep, b_lbo, 1024), idesc, k & 1);
+            umma_commit(&bars->acc_full[acc]);
+          }
+          if (ok) umma_commit(&bars->empty[s]);
+        }
       }
     }
   } else if (warp <= LOADERS) {
@@ -450,7 +474,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     // in registers would leave the loader warps too few.
     const int quad = warp & 3;
     const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
-    const int groups = (blocks + p.sum_blocks - 1) / p.sum_blocks;
+    const int groups = FINE ? 2 * blocks : (blocks + p.sum_blocks - 1) / p.sum_blocks;
     float zero = 0.f;  // NaN once a sum that is not finite has been met
     for (int g = 0; g < groups; ++g) {
       const int acc = g & 1;
@@ -630,7 +654,7 @@ static bool short_k(const Params& p, bool f32) {
   const int steps = (p.K + FMA_K - 1) / FMA_K;
   const long long tiles = static_cast<long long>(p.batch) * ((p.M + FMA_TILE - 1) / FMA_TILE) * ((p.N + FMA_TILE - 1) / FMA_TILE);
   const long long waves = (tiles + sm_count() - 1) / sm_count();
-  return steps == 1 || steps * waves <= (f32 ? 3 : 4) || (!f32 && steps == 2 && waves <= 4);
+  return steps == 1 || steps * waves <= (f32 ? 3 : 4) || (!f32 && steps == 2 && (waves <= 4 || p.out_f32));
 }
 template <typename T>
 static int32_t launch_fma(Params& p, const Operand& oa, const Operand& ob, cudaStream_t stream) {
@@ -658,7 +682,7 @@ static int choose_splits(long long tiles, int k_blocks, int slots, double fixed)
   return best;
 }
 
-template <typename T>
+template <typename T, bool FINE>
 static int32_t launch(Params& p, const Operand& oa, const Operand& ob, double fixed, cudaStream_t stream) {
   using Tr = Traits<T>;
   static std::once_flag once[64];
@@ -666,12 +690,12 @@ static int32_t launch(Params& p, const Operand& oa, const Operand& ob, double fi
   CDL_CUDA(cudaGetDevice(&dev));
   cudaError_t err = cudaSuccess;
   std::call_once(once[dev & 63], [&] {
-    err = cudaFuncSetAttribute(gemm_general_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    err = cudaFuncSetAttribute(gemm_general_kernel<T, FINE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                static_cast<int>(smem_bytes<T>()));
   });
   if (err != cudaSuccess) return fail(CDL_ERR_CUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(err));
   p.split_k = choose_splits(p.num_tiles, p.k_blocks, sm_count(), fixed);
-  CDL_CUDA(launch_pdl_cluster(gemm_general_kernel<T>, dim3(static_cast<unsigned>(p.num_tiles) * p.split_k),
+  CDL_CUDA(launch_pdl_cluster(gemm_general_kernel<T, FINE>, dim3(static_cast<unsigned>(p.num_tiles) * p.split_k),
                               dim3(THREADS), smem_bytes<T>(), p.split_k, stream, p, oa, ob));
   return CDL_OK;
 }
@@ -734,16 +758,19 @@ int32_t matmul_general_execute(const cdl_tensor* a, const cdl_tensor* b, const c
   p.alpha = alpha;
   p.status = device_status_ptr();
   if (!p.status) return fail(CDL_ERR_CUDA, "cannot resolve the device status word");
-  // A tensor-core accumulator loses about 2^-26 of its value to truncation per step of 16 products
-  // (measured: 6.6e-8 after one K block, 4.7e-7 after eight), a chain of f32 FMAs 3.2e-7 at K = 1500: where
-  // the result is f32 every K block is added to the running sums by itself; a bf16 result, rounded to 2^-9,
-  // takes eight at a time.
-  p.sum_blocks = d->dtype == CDL_F32 || a->dtype == CDL_F32 ? 1 : 8;
+  // A tensor-core accumulator truncates: the sum of n steps of 16 bf16 products lies about 1.6e-8 n below its value
+  // (2-norm, against f64: 3.8e-8 after two steps, 6.5e-8 after four, 4.7e-7 after 32), where a chain of K f32
+  // additions has 7.3e-9 sqrt(K).  So much of K goes into one accumulator that its error stays below the
+  // chain's; accumulators are added with round-to-nearest.  f32 results: half a K block up to K = 100 (4.7e-8 at
+  // K = 64, chain 5.1e-8), else one (1.3e-7 at 2051, chain 3.9e-7).  bf16 results, rounded to 2^-9, take
+  // 0.11 sqrt(K) blocks (2.4e-7 at 2051 before that rounding).
+  const bool f32 = a->dtype == CDL_F32, out_f32 = d->dtype == CDL_F32, fine = !f32 && out_f32 && K <= 100;
+  p.sum_blocks = f32 || out_f32 ? 1 : std::clamp(static_cast<int>(0.11 * sqrt(static_cast<double>(K))), 1, 8);
   ProfileScope ps(PROF_GEMM, 2.0 * batch * M * N * K, stream);
-  if (short_k(p, a->dtype == CDL_F32))
-    return a->dtype == CDL_F32 ? launch_fma<float>(p, oa, ob, stream) : launch_fma<__nv_bfloat16>(p, oa, ob, stream);
-  return a->dtype == CDL_F32 ? launch<float>(p, oa, ob, 4.0, stream)
-                             : launch<__nv_bfloat16>(p, oa, ob, 6.0, stream);
+  if (short_k(p, f32)) return f32 ? launch_fma<float>(p, oa, ob, stream) : launch_fma<__nv_bfloat16>(p, oa, ob, stream);
+  if (f32) return launch<float, false>(p, oa, ob, 4.0, stream);
+  return fine ? launch<__nv_bfloat16, true>(p, oa, ob, 6.0, stream)
+              : launch<__nv_bfloat16, false>(p, oa, ob, 6.0, stream);
 }
 
 }  // namespace cdl

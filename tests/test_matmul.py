@@ -435,6 +435,24 @@ def test_unaligned_bf16_layouts(cdl, gpu_ok, m, k, n):
         run_case(cdl, a, b, torch.float32, c=torch.randn(m, n, generator=gen), alpha=0.5, beta=1.0, in_place=True)
 
 
+@pytest.mark.parametrize("m,k,n,out", [(1500, 64, 1027, torch.float32), (1500, 100, 1027, torch.float32),
+                                       (1500, 513, 1027, torch.bfloat16), (1500, 1027, 1027, torch.bfloat16)])
+def test_unaligned_bf16_sums_lose_no_more_than_a_chain(cdl, gpu_ok, m, k, n, out):
+    """Unaligned bf16 operands: the f32 sums, which a C that cancels them shows where the result is bf16, lie no
+    further from f64 (2-norm) than a chain of f32 additions does; products of bf16 are exact in f32."""
+    gen = torch.Generator().manual_seed(k)
+    a, b = rand_bf16(gen, m, k), rand_bf16(gen, k, n)
+    exact = a.double() @ b.double()
+    chain = torch.zeros(m, n)
+    for i in range(k):
+        chain += a[:, i:i + 1].float() * b[i].float()
+    c = -exact.float() if out == torch.bfloat16 else None
+    d = cdl.ops.matmul(a.cuda(), b.cuda(), cdl.ops.MatmulOpts(
+        out=out, c=c.cuda() if c is not None else None, beta=0.0 if c is None else 1.0)).cpu().double()
+    error = d - exact if c is None else d - (exact + c.double())
+    assert float(error.norm()) <= float((chain.double() - exact).norm())
+
+
 @pytest.mark.parametrize("m,k,n", [(1, 64, 8), (16, 576, 1024), (64, 2048, 264), (127, 1032, 136), (129, 4096, 128), (300, 2000, 520),
                                    (600, 1024, 1000), (1000, 264, 1528), (200, 4096, 32), (77, 128, 24)])
 def test_tiles_shared_by_a_cluster(cdl, gpu_ok, m, k, n):
