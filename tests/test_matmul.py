@@ -475,6 +475,42 @@ def test_tiles_shared_by_a_cluster(cdl, gpu_ok, m, k, n):
     assert torch.equal(d1, d2)
 
 
+@pytest.mark.parametrize("batch,m,k,n", [(1, 2040, 64, 5628), (1, 2048, 72, 5632), (1, 1990, 264, 5640), (1, 2048, 512, 5632),
+                                         (4, 1000, 64, 2400)])
+def test_short_weight_gradients(cdl, gpu_ok, batch, m, k, n):
+    """D += A^T B in f32 with two tiles or more per SM and a short K, which one CTA per SM walks: M, N and K
+    tails, batches, alpha; every element is added to once, so a repetition gives the same bits, and so do
+    launches on several streams at a time.  Bound: truncated sums of K / 16 steps (2^-23 of sum |a b| each), the
+    scaling and the addition into D."""
+    gen = torch.Generator(device="cuda").manual_seed(m + k)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    a = rnd(batch, k, (m + 7) // 8 * 8).to(torch.bfloat16)[:, :, :m].mT
+    b = rnd(batch, n, (k + 7) // 8 * 8).to(torch.bfloat16)[:, :, :k].mT
+    c = rnd(batch, m, n)
+    if batch == 1:
+        a, b, c = a[0], b[0], c[0]
+
+    def run(d):
+        return cdl.ops.matmul(a, b, cdl.ops.MatmulOpts(out=torch.float32, c=d, alpha=-0.5, beta=1.0), out=d)
+
+    first = run(c.clone())
+    expected = c.double() - 0.5 * (a.double() @ b.double())
+    bound = 0.5 * (a.double().abs() @ b.double().abs())
+    tol = (k / 16 + 1) * 2.0 ** -23 * bound + 2.0 ** -24 * expected.abs()
+    assert bool(((first.double() - expected).abs() <= tol).all())
+    assert torch.equal(run(c.clone()), first)
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    copies = [[c.clone() for _ in range(3)] for _ in streams]
+    torch.cuda.synchronize()
+    for i in range(3):
+        for stream, mine in zip(streams, copies):
+            with torch.cuda.stream(stream):
+                run(mine[i])
+    torch.cuda.synchronize()
+    assert all(torch.equal(d, first) for mine in copies for d in mine)
+    assert cdl._lib.device_status() == 0
+
+
 @pytest.mark.parametrize("rows,seqlen,heads", [(200, 50, 3), (96, 96, 6)])
 def test_rope_epilogue_of_few_rows(cdl, gpu_ok, rows, seqlen, heads):
     """The rotation in the cluster kernel's store: q and k heads rotated by their row's position, v heads
