@@ -176,20 +176,29 @@ __global__ void __launch_bounds__(THREADS, STAGES == SHARED_STAGES ? 2 : 1)
 // The unsplit weight-gradient form (D += A^T B, f32): many tiles with few K blocks each, so that launch,
 // set-up, first loads and the store are most of a CTA's life.  One CTA per SM walks the tiles; loads and
 // products of the next tile run under the store of this one (two accumulators, the partial tile in
-// shared memory of its own).  2048 x 5632 with K = 64, 256, 512: 22.7, 25.0, 30.7 us; as one short-lived
+// shared memory of its own).  Two tiles are a CTA's own, every further one is drawn from a counter, so a CTA
+// that finds its SM late (another kernel, e.g. a collective, holds it) takes fewer tiles instead of holding a
+// fixed share back to the end: 2048 x 6144 with K = 128 beside a kernel on 32 SMs 28.0 us, with fixed shares 32.5
+// (alone 18.7 and 18.6; 8192 x 8192, K = 64, alone 106 and 112).  2048 x 5632 with K = 64, 256, 512: 22.7, 25.0, 30.7 us; as one short-lived
 // CTA per tile 25.8, 28.9, 34.1 us.  What is left is the reductions: 92 MB of HBM traffic, 14 us.
 constexpr int WALK_THREADS = 320;  // warp 0 TMA, warp 1 MMA, warps 2-9 drain and store
 constexpr int WALK_TMEM_COLS = 256;
-constexpr size_t WALK_SMEM_BYTES = 1024 + SHARED_STAGES * STAGE_BYTES + PART_BYTES + 128;
+// The producer publishes the tile of step t in slot t % WALK_SLOTS, once the accumulator that step t uses is free.
+// So no CTA holds more than two tiles that it has not begun to store, and the slot has been read by all warps.
+// It also works out the coordinates: the two divisions would stand between a store warp's tiles (0.2 us each).
+constexpr int WALK_SLOTS = 4, WALK_BARRIER_BYTES = 256;
+constexpr size_t WALK_SMEM_BYTES = 1024 + SHARED_STAGES * STAGE_BYTES + PART_BYTES + WALK_BARRIER_BYTES;
 struct WalkBarriers {
   uint64_t full[SHARED_STAGES];
   uint64_t empty[SHARED_STAGES];
   uint64_t acc_full[2];
   uint64_t acc_empty[2];
+  uint64_t tile_full[WALK_SLOTS];
+  int4 tile_ring[WALK_SLOTS];  // batch (-1: no tile is left), first row, first column
   uint32_t tmem_base;
   int abort_word;
 };
-static_assert(sizeof(WalkBarriers) <= 128, "barriers fit behind the partial tile");
+static_assert(sizeof(WalkBarriers) <= WALK_BARRIER_BYTES, "barriers fit behind the partial tile");
 __device__ __forceinline__ void store_warps_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 // The same; true in all 256 threads if `flag` is in any.
 __device__ __forceinline__ bool store_warps_any(bool flag) {
@@ -223,6 +232,7 @@ __global__ void __launch_bounds__(WALK_THREADS, 1)
       mbar_init(&bars->acc_full[i], 1);
       mbar_init(&bars->acc_empty[i], WARPS);
     }
+    for (int i = 0; i < WALK_SLOTS; ++i) mbar_init(&bars->tile_full[i], 1);
     bars->abort_word = 0;
     fence_mbar_init();
     tma_prefetch_desc(&tmap_a);
@@ -243,10 +253,23 @@ __global__ void __launch_bounds__(WALK_THREADS, 1)
     if (elect_one()) {
       uint32_t it = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x) {
-        int b, tm, tn;
-        tile_coords(p, tile, b, tm, tn);
-        const int m0 = tm * TILE_M, n0 = tn * TILE_N;
+      // Every CTA draws after its second tile and each further one, until a draw runs past the last tile; the
+      // launch's last draw, of num_tiles - ctas in all, puts the counter back to zero.  A draw is made as late as
+      // the loads allow: a CTA that held three tiles ahead of its stores would finish after the others.
+      const int ctas = static_cast<int>(gridDim.x);
+      int tile = static_cast<int>(blockIdx.x);
+      for (uint32_t t = 0; ok; ++t) {
+        const bool done = tile >= p.num_tiles;
+        int b = -1, m0 = 0, n0 = 0;
+        if (!done) {
+          int tm, tn;
+          tile_coords(p, tile, b, tm, tn);
+          m0 = tm * TILE_M;
+          n0 = tn * TILE_N;
+        }
+        bars->tile_ring[t % WALK_SLOTS] = make_int4(b, m0, n0, 0);
+        mbar_arrive(&bars->tile_full[t % WALK_SLOTS]);
+        if (done) break;
         for (int kb = 0; kb < p.k_blocks; ++kb, ++it) {
           const uint32_t s = it % STAGES;
           if (!mbar_wait(&bars->empty[s], ((it / STAGES) & 1) ^ 1, abort_word, 141)) {
@@ -272,6 +295,14 @@ __global__ void __launch_bounds__(WALK_THREADS, 1)
             tma_load_3d(sb, &tmap_b, &bars->full[s], k0, n0, b);
           }
         }
+        if (!ok || !mbar_wait(&bars->acc_empty[(t + 1) & 1], (((t + 1) >> 1) & 1) ^ 1, abort_word, 142)) break;
+        if (t == 0 || p.sched_counter == nullptr) {  // (without a counter: fixed shares)
+          tile += ctas;
+        } else {
+          const unsigned drawn = atomicAdd(p.sched_counter, 1u);
+          if (drawn + 1 == static_cast<unsigned>(p.num_tiles - ctas)) atomicExch(p.sched_counter, 0u);
+          tile = 2 * ctas + static_cast<int>(drawn);
+        }
       }
     }
   } else if (warp == 1) {
@@ -279,9 +310,12 @@ __global__ void __launch_bounds__(WALK_THREADS, 1)
       const uint32_t idesc = make_idesc_bf16(TILE_M, TILE_N, p.a_mn, p.b_mn);
       const uint32_t a_lbo = p.a_mn ? 8192u : 16u, b_lbo = p.b_mn ? 8192u : 16u;
       const uint32_t a_kstep = p.a_mn ? 2048u : 32u, b_kstep = p.b_mn ? 2048u : 32u;
-      uint32_t it = 0, t = 0;
+      uint32_t it = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x, ++t) {
+      for (uint32_t t = 0; ok; ++t) {
+        if (!mbar_wait(&bars->tile_full[t % WALK_SLOTS], (t / WALK_SLOTS) & 1, abort_word, 243) ||
+            bars->tile_ring[t % WALK_SLOTS].x < 0)
+          break;
         const uint32_t acc = t & 1, d = tmem_base + acc * TILE_N;
         if (!mbar_wait(&bars->acc_empty[acc], ((t >> 1) & 1) ^ 1, abort_word, 241)) break;
         tc_fence_after();
@@ -304,32 +338,33 @@ __global__ void __launch_bounds__(WALK_THREADS, 1)
     }
   } else {
     const int w = warp - 2, row = (warp & 3) * 32 + lane, half = w >> 2;
-    uint32_t t = 0;
-    for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, ++t) {
-      int b, tm, tn;
-      tile_coords(p, tile, b, tm, tn);
-      const int m0 = tm * TILE_M, n0 = tn * TILE_N;
+    for (uint32_t t = 0;; ++t) {
+      bool ok = mbar_wait(&bars->tile_full[t % WALK_SLOTS], (t / WALK_SLOTS) & 1, abort_word, 342);
+      const int4 tile = ok ? bars->tile_ring[t % WALK_SLOTS] : make_int4(-1, 0, 0, 0);
+      const int b = tile.x, m0 = tile.y, n0 = tile.z;
       const uint32_t acc = t & 1;
-      const bool ok = mbar_wait(&bars->acc_full[acc], (t >> 1) & 1, abort_word, 341);
-      tc_fence_after();
-      if (ok && m0 + (warp & 3) * 32 < p.M) {
+      if (b >= 0) {
+        ok = mbar_wait(&bars->acc_full[acc], (t >> 1) & 1, abort_word, 341);
+        tc_fence_after();
+        if (ok && m0 + (warp & 3) * 32 < p.M) {
 #pragma unroll
-        for (int c = half * 64; c < half * 64 + 64; c += 16) {
-          uint32_t r[16];
-          tmem_ld16(tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + acc * TILE_N + c, r);
-          tmem_wait_ld();
-          float v[16];
+          for (int c = half * 64; c < half * 64 + 64; c += 16) {
+            uint32_t r[16];
+            tmem_ld16(tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + acc * TILE_N + c, r);
+            tmem_wait_ld();
+            float v[16];
 #pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
-          store_partial(part, row, c, v);
+            for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
+            store_partial(part, row, c, v);
+          }
         }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars->acc_empty[acc]);
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bars->acc_empty[acc]);
-      // The whole tile is in shared memory.  A wait that ran out ends the walk of all eight warps here: one
-      // that left alone would keep the others at the barrier.
-      if (store_warps_any(!ok)) break;
+      // The whole tile is in shared memory.  The end of the walk, or a wait that ran out, ends it for all eight
+      // warps here: one that left alone would keep the others at the barrier.
+      if (store_warps_any(!ok || b < 0)) break;
       TileOut<1, WARPS> tile_out;
       tile_out.finish(p, part, 0, w, b, m0, n0);
       __syncwarp();
@@ -385,8 +420,10 @@ int32_t gemm_cluster_launch(const CUtensorMap& tm_a, const CUtensorMap& tm_b, co
                                  static_cast<int>(WALK_SMEM_BYTES));
     });
     if (err != cudaSuccess) return fail(CDL_ERR_CUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(err));
+    Params walk = p;
+    walk.sched_counter = sched_counter_for(0, dev, stream);  // launches of one stream that draw share a counter
     CDL_CUDA(launch_pdl(gemm_cluster_walk_kernel, dim3(static_cast<unsigned>(sm_count())), dim3(WALK_THREADS),
-                        WALK_SMEM_BYTES, stream, tm_a, tm_b, p));
+                        WALK_SMEM_BYTES, stream, tm_a, tm_b, walk));
     return CDL_OK;
   }
   switch (p.split_k) {
