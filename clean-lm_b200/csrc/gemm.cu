@@ -1264,8 +1264,9 @@ int32_t cdl_b200_matmul_candidates(const cdl_tensor* a, const cdl_tensor* b, con
   using namespace cdl;
   if (!a || !b || !d || !count || (capacity > 0 && !out))
     return fail(CDL_ERR_INVALID, "matmul_candidates: a, b, d, count (and out) are required");
-  cdl_matmul_options list[4];
+  cdl_matmul_options list[6];
   int n = 0;
+  list[n++] = {CDL_GEMM_AUTO, 0};  // the heuristic's choice, which may be the cluster form (it has no name of its own)
   const bool tensor_core = a->dtype == CDL_BF16 && b->dtype == CDL_BF16 && a->rank >= 2 &&
                            a->rank == b->rank && [&] {
                              gemm::OperandLayout la, lb;
@@ -1274,11 +1275,10 @@ int32_t cdl_b200_matmul_candidates(const cdl_tensor* a, const cdl_tensor* b, con
                              last_error().clear();
                              return ok;
                            }();
-  if (!tensor_core) {
-    list[n++] = {CDL_GEMM_AUTO, 0};
-  } else {
+  if (tensor_core) {
     const long long M = a->shape[a->rank - 2];
     const bool accumulates = d->dtype == CDL_F32;  // the weight-gradient form may slice K
+    if (accumulates) list[n++] = {CDL_GEMM_AUTO, 1};
     const int first = M > gemm::BM ? CDL_GEMM_CTA_PAIR : CDL_GEMM_ONE_CTA;
     const int second = first == CDL_GEMM_CTA_PAIR ? CDL_GEMM_ONE_CTA : CDL_GEMM_CTA_PAIR;
     list[n++] = {first, 0};

@@ -129,8 +129,8 @@ int32_t cdl_b200_matmul_opt(const cdl_tensor* a, const cdl_tensor* b, const cdl_
                             cdl_stream stream);
 /* Writes the valid choices for this problem to out[0 .. *count), the heuristic default first (the
  * order Executor candidates have, op.rs:301-318); at most `capacity` entries, *count = how many
- * exist.  f32 or unaligned operands have the single candidate AUTO; elsewhere AUTO, whose choice may
- * be the cluster form, is valid beside the candidates. */
+ * exist.  The first is AUTO, whose choice may be the cluster form; f32 or unaligned operands have no
+ * other. */
 int32_t cdl_b200_matmul_candidates(const cdl_tensor* a, const cdl_tensor* b, const cdl_tensor* d,
                                    cdl_matmul_options* out, int32_t capacity, int32_t* count);
 /* GEMM with the SwiGLU activation fused into its epilogue, the counterparts of the reference's

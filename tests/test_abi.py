@@ -73,20 +73,20 @@ def test_candidates_need_no_gpu_and_put_the_heuristic_first(cdl):
     L.check(L.lib.cdl_b200_matmul_candidates(ctypes.byref(a), ctypes.byref(b), ctypes.byref(d), buf, 8,
                                              ctypes.byref(n)))
     assert [(buf[i].variant, buf[i].deterministic) for i in range(n.value)] == [
-        (L.GEMM_CTA_PAIR, 0), (L.GEMM_ONE_CTA, 0)]
-    # the weight-gradient form (f32 output) adds the fixed-order variant of the pair kernel
+        (L.GEMM_AUTO, 0), (L.GEMM_CTA_PAIR, 0), (L.GEMM_ONE_CTA, 0)]
+    # the weight-gradient form (f32 output) adds the fixed-order variants
     a, d = t(4096, 512, 1024, transposed=True), t(1 << 20, 512, 256, dtype=L.CDL_F32)
     b = t(8192, 1024, 256)
     L.check(L.lib.cdl_b200_matmul_candidates(ctypes.byref(a), ctypes.byref(b), ctypes.byref(d), buf, 8,
                                              ctypes.byref(n)))
     assert [(buf[i].variant, buf[i].deterministic) for i in range(n.value)] == [
-        (L.GEMM_CTA_PAIR, 0), (L.GEMM_CTA_PAIR, 1), (L.GEMM_ONE_CTA, 0)]
-    # one 128-row slab: the one-CTA kernel is the default; unaligned operands: the general kernel
+        (L.GEMM_AUTO, 0), (L.GEMM_AUTO, 1), (L.GEMM_CTA_PAIR, 0), (L.GEMM_CTA_PAIR, 1), (L.GEMM_ONE_CTA, 0)]
+    # one 128-row slab: the one-CTA kernel before the pairs; unaligned operands: the general kernel
     a, d = t(4096, 64, 512), t(1 << 20, 64, 256)
     b = t(8192, 512, 256)
     L.check(L.lib.cdl_b200_matmul_candidates(ctypes.byref(a), ctypes.byref(b), ctypes.byref(d), buf, 8,
                                              ctypes.byref(n)))
-    assert buf[0].variant == L.GEMM_ONE_CTA
+    assert [buf[i].variant for i in range(n.value)] == [L.GEMM_AUTO, L.GEMM_ONE_CTA, L.GEMM_CTA_PAIR]
     a = t(4098, 64, 512)
     L.check(L.lib.cdl_b200_matmul_candidates(ctypes.byref(a), ctypes.byref(b), ctypes.byref(d), buf, 8,
                                              ctypes.byref(n)))

@@ -201,7 +201,7 @@ def test_weight_gradient_form_summation_order_option(cdl, gpu_ok):
     assert_all_close("sliced wgrad", to_f32(f1), expected, tol)
     assert (f1 - f2).abs().max().item() <= 1e-5 * float(np.abs(bound).max())
     cands = cdl.ops.matmul_candidates(x.T, dy, w0)
-    assert cands[0] == (cdl._lib.GEMM_CTA_PAIR, False) and len(cands) >= 3
+    assert cands[0] == (cdl._lib.GEMM_AUTO, False) and (cdl._lib.GEMM_CTA_PAIR, True) in cands and len(cands) >= 3
     for variant, det in cands:
         assert_all_close(f"candidate {variant} {det}", to_f32(run(variant=variant, deterministic=det)),
                          expected, tol)
