@@ -91,8 +91,9 @@ __global__ void __launch_bounds__(256) norm_general_kernel(const Params p) {
 // Bound by HBM: x is read once and y written once.  V is the widest access that every row's start
 // allows (four f32 where rows are on the 16-byte grid, two or one where they are not: a [8192, 2050]
 // f32 row starts on the 8-byte grid), so a warp's access still covers whole 64- or 128-byte lines.
-// Wide rows take four warps so that a thread's share stays at 20 or 32 values: 12 or 9 rows are then in
-// flight per SM, where one warp per row would need over 64 registers a thread for the row alone.
+// Wide rows take four warps (single columns up to 16) so that a thread's share stays at 20 or 32 values up to
+// 4096 columns: 12 or 9 rows are then in flight per SM, where one warp per row would need over 64 registers a
+// thread for the row alone.  From there to 8192 a share of 64 leaves 5.
 // LayerNorm of f32 [8192, 2050] to f32 (134 MB): 27 us, 5.0 TB/s; norm_general_kernel, which reads the row
 // three times with scalar accesses, 125 us.
 template <int V>
@@ -246,15 +247,35 @@ static int access_width(const Params& p) {
   return 1;
 }
 
+// One row per CTA (E values a thread, WARPS warps), or one per warp.
+template <int V, int E, int WARPS>
+static cudaError_t launch_as(const Params& p, cudaStream_t stream) {
+  const unsigned rows = static_cast<unsigned>(p.rows);
+  return launch_pdl(norm_rows_kernel<V, E, WARPS>, dim3(WARPS == 1 ? (rows + 7) / 8 : rows),
+                    dim3(WARPS == 1 ? 256 : WARPS * 32), 0, stream, p);
+}
 template <int V>
 static cudaError_t launch_rows(const Params& p, cudaStream_t stream) {
-  const unsigned rows = static_cast<unsigned>(p.rows), rows8 = (rows + 7) / 8;
-  if (p.cols <= 256) return launch_pdl(norm_rows_kernel<V, 8, 1>, dim3(rows8), dim3(256), 0, stream, p);
-  if (p.cols <= 1024) return launch_pdl(norm_rows_kernel<V, 32, 1>, dim3(rows8), dim3(256), 0, stream, p);
-  // 20 values leave room for 16 rows per SM; f32 [8192, 2050] 27.1 us, with 32 values 32.8.
-  if (p.cols <= 2560) return launch_pdl(norm_rows_kernel<V, 20, 4>, dim3(rows), dim3(128), 0, stream, p);
-  if (p.cols <= 4096) return launch_pdl(norm_rows_kernel<V, 32, 4>, dim3(rows), dim3(128), 0, stream, p);
-  return launch_pdl(norm_rows_kernel<V, 64, 4>, dim3(rows), dim3(128), 0, stream, p);
+  if (p.cols <= 256) return launch_as<V, 8, 1>(p, stream);
+  if constexpr (V == 1) {
+    // Single columns: an access moves 64 or 128 bytes, so instructions count, those beyond the row's end too.  A
+    // thread takes few values and capacities lie closer.  LayerNorm of bf16, with the capacities below -> with
+    // these: [40000, 257] 42.2 -> 23.7 us, [1024, 513] 9.4 -> 4.8, [8192, 1025] 26.7 -> 19.4, [8192, 4097] 152 -> 81;
+    // norm_general_kernel takes 37.7, 8.6, 28.9 and 133.
+    if (p.cols <= 384) return launch_as<1, 12, 1>(p, stream);
+    if (p.cols <= 1024) return launch_as<1, 8, 4>(p, stream);
+    if (p.cols <= 1536) return launch_as<1, 12, 4>(p, stream);
+    if (p.cols <= 2560) return launch_as<1, 20, 4>(p, stream);
+    if (p.cols <= 4096) return launch_as<1, 16, 8>(p, stream);
+    if (p.cols <= 5120) return launch_as<1, 20, 8>(p, stream);
+    return launch_as<1, 16, 16>(p, stream);
+  } else {
+    if (p.cols <= 1024) return launch_as<V, 32, 1>(p, stream);
+    // 20 values leave room for 12 rows per SM, 32 for 9; f32 [8192, 2050] 27.1 us, with 32 values 32.8.
+    if (p.cols <= 2560) return launch_as<V, 20, 4>(p, stream);
+    if (p.cols <= 4096) return launch_as<V, 32, 4>(p, stream);
+    return launch_as<V, 64, 4>(p, stream);
+  }
 }
 constexpr int MAX_REGISTER_COLS = 8192;
 

@@ -263,3 +263,21 @@ def test_register_rows_column_edges(cdl, gpu_ok, norm_type, cols):
             y_ref, r_ref = oracle.rmsnorm_fwd(to_f32(x), None, None, 1e-6)
         assert_all_close("y", to_f32(out.y), y_ref, oracle.abs_rel_tolerance(y_ref, 1e-5, 1e-4))
         assert_all_close("r_inv", to_f32(out.r_inv), r_ref, oracle.abs_rel_tolerance(r_ref, 1e-6, 1e-4))
+
+
+@pytest.mark.parametrize("norm_type", ["rms", "layer"])
+@pytest.mark.parametrize("cols", [257, 383, 384, 385, 1023, 1025, 1535, 1537, 2559, 2561, 4097, 5119, 5121, 8191])
+def test_register_rows_single_columns(cdl, gpu_ok, norm_type, cols):
+    """Rows that allow single-column accesses only (an odd width, or an even one at an odd stride): both sides
+    of every capacity, up to 16 warps to a row."""
+    _general_case(cdl, 9, cols, norm_type, F32, F32, F32, F32)
+    _general_case(cdl, 9, cols, norm_type, BF16, BF16, BF16, None)
+    gen = torch.Generator().manual_seed(4)
+    x = torch.randn(7, 8195, generator=gen).cuda()[:, 1:cols + 2]  # cols + 1 columns
+    out = cdl.ops.norm_fwd(x, cdl.ops.NormFwdOpts(save_stats=True, norm_type=norm_type, out=F32))
+    if norm_type == "layer":
+        y_ref, _, r_ref = layernorm_reference(to_f32(x), None, None, 1e-6)
+    else:
+        y_ref, r_ref = oracle.rmsnorm_fwd(to_f32(x), None, None, 1e-6)
+    assert_all_close("y", to_f32(out.y), y_ref, oracle.abs_rel_tolerance(y_ref, 1e-5, 1e-4))
+    assert_all_close("r_inv", to_f32(out.r_inv), r_ref, oracle.abs_rel_tolerance(r_ref, 1e-6, 1e-4))
