@@ -478,9 +478,9 @@ __device__ __forceinline__ void sum_slices(const float4 (&q)[8], int slices, flo
 // SPLIT: the item's query blocks are shared by a cluster of p.kv_split CTAs, each of which sums up a
 // slice of them; the partial dV and dK (f32) meet in distributed shared memory, where the operand
 // tiles were, and every CTA adds up and stores its share of the rows in slice order.  For a kv head
-// that many query heads share an item is group x (query blocks) long and there are few of them: 9
-// sequences in 6144 rows, 16 heads on 4, have a longest item of 40 blocks where the work of all
-// items is 16 blocks per SM (see kv_split_of).
+// that many query heads share an item is group x (query blocks) long and there are few of them: one
+// sequence of 2048, 16 heads on 4, has a longest item of 64 blocks where the work of all items is 15
+// blocks per SM (see kv_split_of).
 template <bool ROPE, bool SPLIT>
 __global__ void __launch_bounds__(THREADS, 1)
     attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q,

@@ -7,7 +7,8 @@
 // the copy bandwidth, but only if every SM keeps loads in flight; 64 rows against it are 22 tiles of
 // 128 x 256.  So the split is chosen for the number of SMs that load (choose_cluster_splits in gemm.cu),
 // two CTAs can share an SM (or one has twice the operand stages), and K slices meet on chip: no scratch
-// memory, no atomics, no second launch, a fixed order of the sums.
+// memory, no second launch, a fixed order of the sums.  The weight-gradient form adds each finished sum to D
+// once, by a reduction at the L2; no other form uses atomics.
 #include "gemm_rows.cuh"
 #include "host.h"
 #include "ops.h"
@@ -23,8 +24,7 @@ constexpr int TILE_M = 128, TILE_N = CLUSTER_TILE_N, BK = 64;
 constexpr int A_BYTES = TILE_M * BK * 2, B_BYTES = TILE_N * BK * 2;
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
 // Eight warps, all of which drain the accumulator and store; before that one lane of warp 0 issues the
-// loads and one of warp 1 the MMAs.  With two CTAs per SM that leaves 128 registers a thread, which
-// the 16 prefetched rows of an unsplit tile need.
+// loads and one of warp 1 the MMAs.  Two CTAs per SM leave 128 registers a thread.
 constexpr int WARPS = 8, THREADS = WARPS * 32;
 constexpr int TMEM_COLS = 128;
 // Operand stages: 3 where two CTAs share an SM, 6 where every CTA has an SM to itself; either way an SM
@@ -179,8 +179,8 @@ __global__ void __launch_bounds__(THREADS, STAGES == SHARED_STAGES ? 2 : 1)
 // shared memory of its own).  Two tiles are a CTA's own, every further one is drawn from a counter, so a CTA
 // that finds its SM late (another kernel, e.g. a collective, holds it) takes fewer tiles instead of holding a
 // fixed share back to the end: 2048 x 6144 with K = 128 beside a kernel on 32 SMs 28.0 us, with fixed shares 32.5
-// (alone 18.7 and 18.6; 8192 x 8192, K = 64, alone 106 and 112).  2048 x 5632 with K = 64, 256, 512: 22.7, 25.0, 30.7 us; as one short-lived
-// CTA per tile 25.8, 28.9, 34.1 us.  What is left is the reductions: 92 MB of HBM traffic, 14 us.
+// (alone 18.7 and 18.6; 8192 x 8192, K = 64, alone 106 and 112).  2048 x 5632 from HBM with K = 64, 256, 512: 22.7,
+// 25.0, 30.7 us; as one short-lived CTA per tile 25.8, 28.9, 34.1 us.  What is left is the reductions: 92 MB of HBM traffic, 14 us.
 constexpr int WALK_THREADS = 320;  // warp 0 TMA, warp 1 MMA, warps 2-9 drain and store
 constexpr int WALK_TMEM_COLS = 256;
 // The producer publishes the tile of step t in slot t % WALK_SLOTS, once the accumulator that step t uses is free.

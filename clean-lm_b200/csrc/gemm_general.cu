@@ -1,8 +1,7 @@
 // Matmul for the operands TMA cannot bring to the tensor cores as they are: bf16 pointers or leading
 // dimensions off the 16-byte grid (the reference hands them to cuBLASLt, tests `unaligned_operands`,
 // crates/cleandl/tests/matmul.rs:604-630) and f32 inputs (`f32_tf32_matmul`, tests/matmul.rs:243-265:
-// the reference computes those with TF32 tensor cores, 10 mantissa bits; here the products are full
-// f32, which its tolerance contains).
+// the reference computes those with TF32 tensor cores, 10 mantissa bits; here they keep f32's 24, see below).
 //
 // D = alpha * A . B + beta * C, f32 accumulation.  Products of a short K are sums of plain FMAs
 // (gemm_fma_kernel); the others go to the tensor cores.  128 x 128 tiles; the K range of a tile is shared by
@@ -14,8 +13,9 @@
 //                flight meanwhile
 //   4 sum warps  add the tensor core's sums (of Params::sum_blocks) to the running sums
 //
-// f32 operands.  A f32 value is the exact sum of three bf16 values (8 significant bits each):
-// x = h + m + l.  Of the nine products of two such sums the six of h.h, h.m, m.h, m.m, h.l and l.h are
+// f32 operands.  A f32 value is the exact sum of three bf16 values (8 significant bits each): x = h + m + l
+// (the splitting of Henry, Tang and Heinecke, "Leveraging the bfloat16 Artificial Intelligence Datatype For
+// Higher-Precision Computations", 2019).  Of the nine products of two such sums the six of h.h, h.m, m.h, m.m, h.l and l.h are
 // taken; the others are below 2^-24 of the product.  bf16 products are exact in f32.  The tensor core
 // truncates when it adds, so it only ever sums one K block of 64, the small terms first; the blocks
 // are added with round-to-nearest.
@@ -23,11 +23,12 @@
 // such sum, and where a product overflows, h.h and h.m or m.h may be infinities of either sign (1e30
 // squared is one): a CTA that met such a value or a sum that is not finite computes its part of the tile
 // again with plain FMAs (partial_by_fma).
-// Measured error (2-norm, against f64) 1.2e-7 at K = 1024 .. 2048, where a chain of FMAs has 5.7e-7 .. 8.1e-7.
+// Measured error (2-norm, against f64) 5.5e-8 at K = 20, 7.8e-8 at 100 and 1.0e-7 to 1.3e-7 at 1024 .. 2048, where a
+// chain of FMAs has 8.2e-8, 1.8e-7 and 5.7e-7 .. 8.1e-7.
 //
 // What bounds it: the loaders and the shared memory they share with the tensor core (f32: 96 KiB of
 // pieces written and 192 KiB read per K block of 64).  1024 x 2048 x 1536 f32 74 us (87 TFLOP/s; 64 x 64
-// tiles of FMAs on the CUDA cores: 460 us, 14 TFLOP/s); 1500 x 1027 x 2051 bf16 with odd rows 52 us
+// tiles of FMAs on the CUDA cores: 460 us, 14 TFLOP/s); 1500 x 1027 x 2051 bf16 with odd rows 51 us
 // (310 us).
 #include "gemm_rows.cuh"
 #include "host.h"

@@ -112,9 +112,11 @@ typedef struct {
  * dgrad = (A row-major, B transposed view), wgrad = (A transposed view, B row-major, D = C f32,
  * beta 1).  bf16 operands whose base address and non-unit strides are 16-byte aligned take the
  * tensor-core kernels; other layouts (tests/matmul.rs:604-630) and f32 inputs
- * (tests/matmul.rs:243-265; full f32 products, where cuBLASLt uses TF32) take a tensor-core
- * kernel that loads operands of any alignment itself, f32 values as three bf16 pieces.  K == 0 is an error ("K is zero", matmul.rs tests
- * :825-843).  D may alias C. */
+ * (tests/matmul.rs:243-265; 24-bit products, where cuBLASLt uses TF32) take a tensor-core
+ * kernel that loads operands of any alignment itself, f32 values as three bf16 pieces of which the six
+ * largest products are summed; a short K takes plain FMAs, f32 products summed in f64.  The error of a
+ * f32 product is at most that of a chain of f32 FMAs.  K == 0 is an error ("K is zero", matmul.rs
+ * tests :825-843).  D may alias C. */
 int32_t cdl_b200_matmul(const cdl_tensor* a, const cdl_tensor* b, const cdl_tensor* c,
                         const cdl_tensor* d, float alpha, float beta, void* scratch,
                         size_t scratch_bytes, cdl_stream stream);
