@@ -842,24 +842,25 @@ static int32_t analyze_operand(const char* name, const cdl_tensor* t, bool contr
 // K slices (1, 2, 4 or 8) of the cluster kernel (gemm_cluster.cu) for a problem, or 0: the 256 x 256
 // tiles of the pair kernel (128 x 256 up to 128 rows).  Both times are estimated, in microseconds, and
 // the cluster kernel taken where it saves 5 %.
-//   wide tiles: launch and set-up; 0.28 us per K block (a quarter more when every pair loads, 0.37 us when
-//     a single wave of tiles brings over 100 MB from HBM); a store that grows with the part of the tile
-//     that exists, four times as dear where an f32 C is added to, and dearer for columns beyond the last
-//     32, above all with a bf16 C; and, for a pair's further tiles, the longer of their products and the
-//     store.
+//   wide tiles: launch and set-up; 0.28 us per K block (a quarter more when every pair loads); a store
+//     that grows with the part of the tile that exists, four times as dear where an f32 C is added to, and
+//     dearer for columns beyond the last 32 and with a bf16 C; and, for a pair's further tiles, the longer of
+//     their products and the store.
 //   cluster: launch, exchange and store (more for more slices, less for fewer rows) and the longest of
 //     one CTA's K blocks (0.23 us), the K blocks of the CTAs that share an SM (0.22 us) and all blocks
-//     over all SMs (0.32 us; 0.25 us where D is reduced into; more for rows of B under 128 bytes); CTAs
-//     beyond one per SM add their own launch and store.  The GPCs hold 14 clusters of 8 and 33 of 4 CTAs
+//     over all SMs (0.28 us; 0.25 us where D is reduced into; more for rows of B under 128 bytes); CTAs
+//     beyond one per SM add their own launch and store.  Tiles that one CTA per SM walks: the products of the
+//     SM that has most of them, and all stores over all SMs.  The GPCs hold 14 clusters of 8 and 33 of 4 CTAs
 //     that have an SM to themselves: more than that run in two turns.
 //   either: the time of its bytes at 6.5 TB/s where they exceed 100 MB.
-// Fitted to 1550 shapes (8 to 2488 rows, N 8 to 32768, K 8 to 16384, batches to 64, C none, bf16 and f32): 1 %
-// from the best choice on average; over 8 % slower than the wide tiles in 8 of them, 22 % at worst.  In
-// microseconds, wide -> cluster: 64 x 5632 x 2048 36.1 -> 12.0 (4 slices), 256 x 2048 x
-// 2048 15.4 -> 9.2 (4), 512 x 5632 x 2048 31.8 -> 16.9 (2); the other way at 2048 x 2048 x 2048, 17.2 against
+// Fitted to 1550 shapes (8 to 2488 rows, N 8 to 32768, K 8 to 16384, batches to 64, C none, bf16 and f32)
+// and corrected on 1067 more (16 to 8192 rows): there 0.5 % from the best choice on average and over 8 % slower
+// than the wide tiles in 2, 10 % at worst.  In microseconds, wide -> cluster: 64 x 5632 x 2048 36.1 -> 12.0 (4
+// slices), 256 x 2048 x 2048 15.4 -> 9.2 (4), 512 x 5632 x 2048 31.8 -> 16.9 (2); the other way at 2048 x 2048 x 2048, 17.2 against
 // 19.1, and for narrow outputs, where a wide tile's loads and store shrink with N: 128 x 32 x 64 3.4
 // against 5.0, 59 x (1024 x 32 x 128) 8.4 against 12.0, D += A^T B 200 x 32 x 4096 7.0 against 10.6; D += A^T B
-// 512 x 5632 x 5632, whose 176 tiles of 128 x 128 leave most SMs waiting for two, 30.6 against 42.6.
+// 512 x 5632 x 5632, whose 176 tiles of 128 x 128 leave most SMs waiting for two, 30.6 against 42.6, and 2048 x 3072 x 5616, 384 tiles
+// to walk in turns of 148, 56 against 91.
 static int choose_cluster_splits(long long batch, long long M, long long N, long long K, bool adds_f32,
                                  bool adds_bf16, bool may_slice, bool reduces) {
   auto up = [](long long a, long long b) { return (a + b - 1) / b; };
@@ -867,8 +868,7 @@ static int choose_cluster_splits(long long batch, long long M, long long N, long
   const double kb = static_cast<double>(up(K, BK));
   const double sms = sm_count();
   const double megabytes = 1e-6 * batch * (2.0 * (M + N) * K + (adds_f32 ? 8.0 : adds_bf16 ? 4.0 : 2.0) * M * N);
-  const bool from_hbm = megabytes > 100.0;
-  const double hbm = from_hbm ? 3.5 + megabytes / 6.5 : 0.0;
+  const double hbm = megabytes > 100.0 ? 3.5 + megabytes / 6.5 : 0.0;
   const bool one_cta = M <= BM;
   const long long wide_tiles = batch * (one_cta ? 1 : up(M, PAIR_M)) * up(N, BN);
   const long long wide_slots = one_cta ? sm_count() : sm_count() / 2;
@@ -878,10 +878,10 @@ static int choose_cluster_splits(long long batch, long long M, long long N, long
   for (int s = 1; s <= (may_slice && !one_cta ? 8 : 1) && (s == 1 || s * 8 <= kb); ++s) {
     const long long units = wide_tiles * s;
     const double busy = units < wide_slots ? static_cast<double>(units) / wide_slots : 1.0;
-    const double loop = (from_hbm && units <= wide_slots ? 0.37 : 0.275) * (1.0 + 0.23 * busy) * kb / s;
+    const double loop = 0.275 * (1.0 + 0.23 * busy) * kb / s;
     double store, step;
     if (!adds_f32) {
-      store = 1.6 * filled + (!adds_bf16 ? ragged : N % 32 == 0 || N < 32 ? 0.6 : N < 128 ? 1.7 : 3.4);
+      store = 1.6 * filled + (!adds_bf16 ? ragged : N % 32 == 0 || N < 32 ? 2.2 : N < 128 ? 3.3 : 5.0);
       step = fmax(fmax(1.2, loop + 0.6), 2.7 * filled);
     } else if (s == 1) {
       store = 0.6 + ragged + (6.2 + 0.7 * busy) * filled;
@@ -896,21 +896,22 @@ static int choose_cluster_splits(long long batch, long long M, long long N, long
   const long long tiles = batch * up(M, 128) * up(N, CLUSTER_TILE_N);
   if (tiles > (1 << 20)) return 0;
   const double rows = part(M, 128), per_sm = static_cast<double>(tiles) / sms;
-  const double fixed[4] = {3.3 + 1.55 * rows, 4.25 + 1.55 * rows, 4.65 + 1.55 * rows, 4.1 + 2.2 * rows};
+  const double fixed[4] = {3.3 + 1.55 * rows, 4.25 + 1.55 * rows, 5.45 + 0.75 * rows, 4.1 + 2.2 * rows};
   const double crowded[4] = {2.1, 3.15, 4.05, 5.55}, short_rows = N < 32 ? 2.0 : N < 64 ? 1.3 : 1.0;
   int splits = 0;
   for (int i = 0; i < 4 && (1 << i) <= kb; ++i) {
     const long long ctas = tiles << i;
     const double per_cta = kb / (1 << i);
     double t = fixed[i] + fmax(fmax(0.23 * per_cta, ctas > sm_count() ? 0.22 * up(ctas, sm_count()) * per_cta : 0.0),
-                               (reduces ? 0.25 : 0.32) * short_rows * per_sm * kb);
+                               (reduces ? 0.25 : 0.28) * short_rows * per_sm * kb);
     if (ctas > sm_count()) t += (crowded[i] + (adds_bf16 ? 0.8 : 0.0)) * (static_cast<double>(ctas) / sms - 1.0);
     else if ((i == 2 && tiles > sm_count() / 4 - 4) || (i == 3 && tiles > sm_count() / 8 - 4)) t *= 2.0;
     if (i == 3) t += 0.13 * static_cast<double>(tiles < 14 ? tiles : 14);
     if (adds_f32) t += reduces ? 0.3 * per_sm : 0.2 + 1.2 * rows;
     if (adds_bf16) t += 0.8 * rows;
     // From two tiles per SM on, unsplit additions into D are walked by one CTA per SM.
-    if (reduces && i == 0 && tiles >= 2 * sm_count()) t = 4.3 + per_sm * (2.2 + 0.24 * kb);
+    if (reduces && i == 0 && tiles >= 2 * sm_count())
+      t = 4.3 + 2.2 * per_sm + 0.24 * kb * static_cast<double>(up(tiles, sm_count()));
     t = fmax(t, hbm);
     if (t < best) {
       best = t;
