@@ -301,7 +301,7 @@ __device__ __forceinline__ void fma_block(const float* ta, const float* tb, int 
 constexpr int REDO_THREADS = 512, REDO_FLOATS = 2 * fma_tile<TILE>();
 static_assert(gemm::PART_BYTES + 2 * REDO_FLOATS * sizeof(float) <= Traits<float>::STAGES * 6 * PIECE_BYTES,
               "the FMA tiles fit behind the partial tile");
-__device__ __noinline__ void partial_by_fma(const Operand& oa, const Operand& ob, int b, int m0, int n0, int k_begin,
+__device__ __noinline__ void partial_by_fma(const Operand oa, const Operand ob, int b, int m0, int n0, int k_begin,
                                             int k_end, int smem) {
   extern __shared__ uint8_t smem_raw[];
   float* part = reinterpret_cast<float*>(smem_raw + smem);
