@@ -14,15 +14,11 @@ from typing import Optional
 import torch
 
 from . import _lib
-from ._lib import CdlMxTensor, check, lib, ref, tensor_arg
+from ._lib import CdlMxTensor, check, current_stream, lib, ref, tensor_arg
 
 MXFP8, NVFP4 = _lib.CDL_MXFP8, _lib.CDL_NVFP4
 ROWWISE, COLWISE = _lib.CDL_MX_ROWWISE, _lib.CDL_MX_COLWISE
 BLOCK = 32  # MXFP8; NVFP4 blocks hold 16 elements
-
-
-def _stream() -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
 def layout_bytes(rows: int, cols: int, dim: int, fmt: int = MXFP8):
@@ -83,14 +79,14 @@ def quantize(x: torch.Tensor, rowwise: bool = True, colwise: bool = False, fmt: 
         yr = MxTensor.empty(rows, cols, ROWWISE, x.device, zero_scales=True, fmt=fmt) if rowwise else None
         yc = MxTensor.empty(rows, cols, COLWISE, x.device, zero_scales=True, fmt=fmt) if colwise else None
     tx, ar, ac = tensor_arg(x), _mx_arg(yr), _mx_arg(yc)
-    check(lib.cdl_b200_mx_quantize(ref(tx), ref(ar), ref(ac), _stream()))
+    check(lib.cdl_b200_mx_quantize(ref(tx), ref(ar), ref(ac), current_stream()))
     return yr, yc
 
 
 def dequantize(t: MxTensor, dtype: torch.dtype = torch.float32) -> torch.Tensor:
     y = torch.empty(t.rows, t.cols, dtype=dtype, device=t.values.device)
     a, ty = t.arg(), tensor_arg(y)
-    check(lib.cdl_b200_mx_dequantize(ref(a), ref(ty), _stream()))
+    check(lib.cdl_b200_mx_dequantize(ref(a), ref(ty), current_stream()))
     return y
 
 
@@ -122,7 +118,7 @@ def norm_fwd_mx(x: torch.Tensor, scale: Optional[torch.Tensor] = None,
     tx, ts, tb, tr = tensor_arg(x), tensor_arg(scale), tensor_arg(bias), tensor_arg(r_inv)
     ar, ac = _mx_arg(yr), _mx_arg(yc)
     check(lib.cdl_b200_rmsnorm_fwd_mx(ref(tx), ref(ts), ref(tb), eps, ref(ar), ref(ac), ref(tr),
-                                      _stream()))
+                                      current_stream()))
     return NormMxOutputs(yr, yc, r_inv)
 
 
@@ -140,9 +136,9 @@ def matmul_mx(a: MxTensor, b: MxTensor, out_dtype: torch.dtype = torch.bfloat16,
         from ._lib import CdlMatmulOptions
         mo = CdlMatmulOptions(int(variant), 0)
         check(lib.cdl_b200_matmul_mx_opt(ref(aa), ref(ab), ref(tc), ref(td), alpha, beta,
-                                         ctypes.byref(mo), _stream()))
+                                         ctypes.byref(mo), current_stream()))
         return out
-    check(lib.cdl_b200_matmul_mx(ref(aa), ref(ab), ref(tc), ref(td), alpha, beta, _stream()))
+    check(lib.cdl_b200_matmul_mx(ref(aa), ref(ab), ref(tc), ref(td), alpha, beta, current_stream()))
     return out
 
 
@@ -152,5 +148,5 @@ def matmul_mx_out(a: MxTensor, b: MxTensor, dim: int = ROWWISE, alpha: float = 1
     if out is None:
         out = MxTensor.empty(a.rows, b.cols, dim, a.values.device, zero_scales=True, fmt=fmt)
     aa, ab, ad = a.arg(), b.arg(), out.arg()
-    check(lib.cdl_b200_matmul_mx_out(ref(aa), ref(ab), ref(ad), alpha, _stream()))
+    check(lib.cdl_b200_matmul_mx_out(ref(aa), ref(ab), ref(ad), alpha, current_stream()))
     return out

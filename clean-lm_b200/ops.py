@@ -19,11 +19,7 @@ from typing import Optional
 import torch
 
 from . import _lib
-from ._lib import CdlAttnDesc, check, lib, ref, tensor_arg
-
-
-def _stream() -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+from ._lib import CdlAttnDesc, check, current_stream, lib, ref, tensor_arg
 
 
 def _require_cuda(*tensors):
@@ -52,22 +48,22 @@ def matmul(a: torch.Tensor, b: torch.Tensor, opts: MatmulOpts | None = None,
     given to write in place (e.g. out = c for accumulating wgrads)."""
     opts = opts or MatmulOpts()
     _require_cuda(a, b, opts.c, out)
-    if a.dim() != b.dim() or a.dim() not in (2, 3):
+    sa, sb = a.shape, b.shape
+    if len(sa) != len(sb) or len(sa) not in (2, 3):
         raise _lib.CdlError(-1, f"matmul operands must both have rank 2 or rank 3 "
-                                f"(got rank {a.dim()} and {b.dim()})")
-    if a.shape[-1] != b.shape[-2]:
-        raise _lib.CdlError(-1, f"matmul contraction dimensions differ: {tuple(a.shape)} x "
-                                f"{tuple(b.shape)}")
+                                f"(got rank {len(sa)} and {len(sb)})")
+    if sa[-1] != sb[-2]:
+        raise _lib.CdlError(-1, f"matmul contraction dimensions differ: {tuple(sa)} x {tuple(sb)}")
     if out is None:
-        out = torch.empty(*a.shape[:-1], b.shape[-1], dtype=opts.out, device=a.device)
+        out = torch.empty(*sa[:-1], sb[-1], dtype=opts.out, device=a.device)
     ta, tb, tc, td = tensor_arg(a), tensor_arg(b), tensor_arg(opts.c), tensor_arg(out)
     if opts.variant == _lib.GEMM_AUTO and not opts.deterministic:
         check(lib.cdl_b200_matmul(ref(ta), ref(tb), ref(tc), ref(td), opts.alpha, opts.beta, None, 0,
-                                  _stream()))
+                                  current_stream()))
     else:
         mo = _lib.CdlMatmulOptions(int(opts.variant), 1 if opts.deterministic else 0)
         check(lib.cdl_b200_matmul_opt(ref(ta), ref(tb), ref(tc), ref(td), opts.alpha, opts.beta,
-                                      ctypes.byref(mo), None, 0, _stream()))
+                                      ctypes.byref(mo), None, 0, current_stream()))
     return out
 
 
@@ -116,16 +112,16 @@ def norm_fwd(x: torch.Tensor, opts: NormFwdOpts | None = None) -> NormFwdOutputs
         mean = torch.empty(x.shape[0], dtype=torch.float32, device=x.device) if opts.save_stats else None
         tm = tensor_arg(mean)
         check(lib.cdl_b200_layernorm_fwd(ref(tx), ref(ts), ref(tb), opts.eps, ref(ty), ref(tm), ref(tr),
-                                         _stream()))
+                                         current_stream()))
         return NormFwdOutputs(y, r_inv, mean)
     if opts.norm_type != "rms":
         raise _lib.CdlError(-1, f"norm_fwd: unknown norm type '{opts.norm_type}'")
     if opts.variant != _lib.NORM_AUTO:
         no = _lib.CdlNormOptions(int(opts.variant))
         check(lib.cdl_b200_rmsnorm_fwd_opt(ref(tx), ref(ts), ref(tb), opts.eps, ref(ty), ref(tr),
-                                           ctypes.byref(no), _stream()))
+                                           ctypes.byref(no), current_stream()))
         return NormFwdOutputs(y, r_inv)
-    check(lib.cdl_b200_rmsnorm_fwd(ref(tx), ref(ts), ref(tb), opts.eps, ref(ty), ref(tr), _stream()))
+    check(lib.cdl_b200_rmsnorm_fwd(ref(tx), ref(ts), ref(tb), opts.eps, ref(ty), ref(tr), current_stream()))
     return NormFwdOutputs(y, r_inv)
 
 
@@ -152,10 +148,10 @@ def norm_bwd(x, dy, scale, r_inv, dscale, residual_dy=None, scratch=None, dx=Non
         no = _lib.CdlNormOptions(int(variant))
         check(lib.cdl_b200_rmsnorm_bwd_opt(*(ref(a) for a in args), ctypes.byref(no),
                                            ctypes.c_void_p(scratch.data_ptr()),
-                                           scratch.numel() * scratch.element_size(), _stream()))
+                                           scratch.numel() * scratch.element_size(), current_stream()))
         return dx
     check(lib.cdl_b200_rmsnorm_bwd(*(ref(a) for a in args), ctypes.c_void_p(scratch.data_ptr()),
-                                   scratch.numel() * scratch.element_size(), _stream()))
+                                   scratch.numel() * scratch.element_size(), current_stream()))
     return dx
 
 
@@ -215,7 +211,7 @@ def attention_fwd(q, k, v, opts: AttentionOpts | None = None, lse: bool = True,
         b = [tensor_arg(t) for t in (out, lse_t)]
         check(lib.cdl_b200_attn_fwd_packed(ctypes.byref(desc), *(ref(x) for x in a),
                                            int(opts.max_seqlen_q or 0), int(opts.max_seqlen_k or 0),
-                                           *(ref(x) for x in b), _stream()))
+                                           *(ref(x) for x in b), current_stream()))
         return AttentionFwdOutputs(out, lse_t)
     if q.dim() != 4:
         raise _lib.CdlError(-1, "attention: q must be [batch, seqlen, heads, head_dim]")
@@ -225,7 +221,7 @@ def attention_fwd(q, k, v, opts: AttentionOpts | None = None, lse: bool = True,
              if lse else None)
     desc = _attn_desc(opts)
     args = [tensor_arg(t) for t in (q, k, v, out, lse_t)]
-    check(lib.cdl_b200_attn_fwd(ctypes.byref(desc), *(ref(a) for a in args), _stream()))
+    check(lib.cdl_b200_attn_fwd(ctypes.byref(desc), *(ref(a) for a in args), current_stream()))
     return AttentionFwdOutputs(out, lse_t)
 
 
@@ -268,7 +264,7 @@ def attention_bwd(q, k, v, out, d_out, lse, opts: AttentionOpts | None = None, s
         fn = lib.cdl_b200_attn_bwd_packed if rope_table is None else lib.cdl_b200_attn_bwd_packed_rope
         check(fn(ctypes.byref(desc), *(ref(x) for x in a), max_q, int(opts.max_seqlen_k or 0),
                  *(ref(x) for x in b), ctypes.c_void_p(scratch.data_ptr()),
-                 scratch.numel() * scratch.element_size(), _stream()))
+                 scratch.numel() * scratch.element_size(), current_stream()))
         return dq, dk, dv
     need = attention_bwd_scratch_bytes(q, k)
     if scratch is None:
@@ -278,5 +274,5 @@ def attention_bwd(q, k, v, out, d_out, lse, opts: AttentionOpts | None = None, s
     args = [tensor_arg(t) for t in tensors]
     fn = lib.cdl_b200_attn_bwd if rope_table is None else lib.cdl_b200_attn_bwd_rope
     check(fn(ctypes.byref(desc), *(ref(a) for a in args), ctypes.c_void_p(scratch.data_ptr()),
-             scratch.numel() * scratch.element_size(), _stream()))
+             scratch.numel() * scratch.element_size(), current_stream()))
     return dq, dk, dv

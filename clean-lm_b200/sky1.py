@@ -14,7 +14,7 @@ from dataclasses import dataclass
 import torch
 
 from . import _lib
-from ._lib import check, lib
+from ._lib import check, current_stream, lib
 
 PARAM_NAMES = _lib._BLOCK_PARAMS
 
@@ -147,9 +147,6 @@ class Sky1Block:
                                         for n in ("qkv", "attn", "lse", "o", "up", "gate", "act")))
         self._x = None
 
-    def _stream(self):
-        return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-
     def forward(self, x: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
         """x: bf16 [tokens, hidden] (or [batch, seqlen, hidden]); keeps a reference for backward."""
         cfg = self.cfg
@@ -160,13 +157,13 @@ class Sky1Block:
             check(lib.cdl_b200_sky1_block_fwd_ragged(
                 ctypes.byref(self._cfg_c), ctypes.byref(self._w_c), x.data_ptr(), self.table.data_ptr(),
                 ctypes.byref(self._rg_c), ctypes.byref(self._s_c), out.data_ptr(),
-                self.workspace.data_ptr(), self.workspace.numel(), self._stream()))
+                self.workspace.data_ptr(), self.workspace.numel(), current_stream()))
             self._x = x
             return out
         check(lib.cdl_b200_sky1_block_fwd(
             ctypes.byref(self._cfg_c), ctypes.byref(self._w_c), x.data_ptr(), self.table.data_ptr(),
             ctypes.byref(self._s_c), out.data_ptr(), self.workspace.data_ptr(),
-            self.workspace.numel(), self._stream()))
+            self.workspace.numel(), current_stream()))
         self._x = x
         return out
 
@@ -197,19 +194,19 @@ class Sky1Block:
                 ctypes.byref(self._cfg_c), ctypes.byref(self._w_c), self._x.data_ptr(),
                 self.table.data_ptr(), ctypes.byref(self._rg_c) if self._rg_c is not None else None,
                 ctypes.byref(self._s_c), dy.data_ptr(), ctypes.byref(self._g_c), dx.data_ptr(),
-                self.workspace.data_ptr(), self.workspace.numel(), ctypes.byref(ev_c), self._stream()))
+                self.workspace.data_ptr(), self.workspace.numel(), ctypes.byref(ev_c), current_stream()))
             return dx
         if self._rg_c is not None:
             check(lib.cdl_b200_sky1_block_bwd_ragged(
                 ctypes.byref(self._cfg_c), ctypes.byref(self._w_c), self._x.data_ptr(),
                 self.table.data_ptr(), ctypes.byref(self._rg_c), ctypes.byref(self._s_c), dy.data_ptr(),
                 ctypes.byref(self._g_c), dx.data_ptr(), self.workspace.data_ptr(),
-                self.workspace.numel(), phase, self._stream()))
+                self.workspace.numel(), phase, current_stream()))
             return dx
         check(lib.cdl_b200_sky1_block_bwd(
             ctypes.byref(self._cfg_c), ctypes.byref(self._w_c), self._x.data_ptr(),
             self.table.data_ptr(), ctypes.byref(self._s_c), dy.data_ptr(), ctypes.byref(self._g_c),
-            dx.data_ptr(), self.workspace.data_ptr(), self.workspace.numel(), phase, self._stream()))
+            dx.data_ptr(), self.workspace.data_ptr(), self.workspace.numel(), phase, current_stream()))
         return dx
 
     def zero_grads(self):
@@ -336,7 +333,7 @@ class Sky1LM:
         from . import ops
 
         L, c = _lib, self.cfg
-        st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        st = current_stream()
         ta = L.tensor_arg
         tok, tgt = ta(tokens), ta(targets)
         emb = ta(self.view("replica", "embedding"))
@@ -391,7 +388,7 @@ class Sky1LM:
         c = self.cfg
         if self.comm is not None:
             torch.cuda.current_stream().wait_stream(self.comm)
-        st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        st = current_stream()
         self.step_count += 1
         sumsq_ptr = None
         if c.max_grad_norm > 0:

@@ -18,19 +18,13 @@ bf16 block; tests hold it to the bf16 block within the format's error.
 """
 from __future__ import annotations
 
-import ctypes
-
 import torch
 
 from . import _lib, mx, ops
-from ._lib import check, lib, ref, tensor_arg
+from ._lib import check, current_stream, lib, ref, tensor_arg
 from .sky1 import Sky1Config, rope_table
 
 WEIGHTS = ("wqkv", "wo", "wup", "wgate", "wdown")
-
-
-def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
 class Sky1BlockMX:
@@ -81,7 +75,7 @@ class Sky1BlockMX:
         cfg = self.cfg
         x3 = x2d.view(cfg.tokens, cfg.heads + 2 * cfg.kv_heads, cfg.head_dim)
         tx, tt = tensor_arg(x3), tensor_arg(self.table)
-        check(lib.cdl_b200_rope(ref(tx), ref(tt), cfg.heads + cfg.kv_heads, cfg.seqlen, backward, _stream()))
+        check(lib.cdl_b200_rope(ref(tx), ref(tt), cfg.heads + cfg.kv_heads, cfg.seqlen, backward, current_stream()))
 
     def _quant(self, name, x):
         mx.quantize(x, rowwise=True, colwise=True, out=self.q[name])
@@ -118,7 +112,7 @@ class Sky1BlockMX:
         self._fwd(n2.y, self.wq["wup"], b["up"])
         self._fwd(n2.y, self.wq["wgate"], b["gate"])
         tg, tu, ta = tensor_arg(b["gate"]), tensor_arg(b["up"]), tensor_arg(b["act"])
-        check(lib.cdl_b200_swiglu_fwd(ref(tg), ref(tu), ref(ta), _stream()))
+        check(lib.cdl_b200_swiglu_fwd(ref(tg), ref(tu), ref(ta), current_stream()))
         qact = self._quant("act", b["act"])
         self._fwd(qact[0], self.wq["wdown"], out, c=b["o"])                # out = act Wdown + o
         return out
@@ -130,7 +124,7 @@ class Sky1BlockMX:
         self._wgrad(self.q["act"][1], qdy[1], g["wdown"])
         self._dgrad(qdy[0], self.wq["wdown"], b["d_act"])
         targs = [tensor_arg(t) for t in (b["d_act"], b["gate"], b["up"], b["d_gate"], b["d_act"])]
-        check(lib.cdl_b200_swiglu_bwd(*(ref(a) for a in targs), _stream()))   # d_up over d_act
+        check(lib.cdl_b200_swiglu_bwd(*(ref(a) for a in targs), current_stream()))   # d_up over d_act
         qdu, qdg = self._quant("d_up", b["d_act"]), self._quant("d_gate", b["d_gate"])
         self._wgrad(self.q["h2"][1], qdu[1], g["wup"])
         self._wgrad(self.q["h2"][1], qdg[1], g["wgate"])
