@@ -372,6 +372,23 @@ __device__ __forceinline__ void store_tile_rows_rope(const Params& p, uint32_t t
   }
 }
 
+// The epilogue of D += alpha * accumulator for the calling warp: rows row0 .. row0 + 31, 128 columns.
+__device__ __forceinline__ void add_tile_rows(const Params& p, const CUtensorMap* tm_d, uint8_t* buf, uint32_t t_row,
+                                              int b, int row0, int col_base, int lane) {
+  if (row0 >= p.M) return;  // warp-uniform; rows past M inside the box are clipped
+#pragma unroll 1
+  for (int ch = 0; ch < BN / 64; ++ch) {
+    const int col0 = col_base + ch * 32;
+    if (col0 >= p.N) break;
+    uint32_t r[32];
+    tmem_ld32(t_row + ch * 32, r);
+    tmem_wait_ld();
+    if (lane == 0) tma_store_wait_read<0>();  // the buffer's last reduction has read it
+    __syncwarp();
+    add_chunk(tm_d, buf, r, p.alpha, lane, col0, row0, b);
+  }
+}
+
 __global__ void __launch_bounds__(THREADS, 1)
     gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
                      const __grid_constant__ CUtensorMap tmap_b, const Params p) {
@@ -535,7 +552,9 @@ __global__ void __launch_bounds__(THREADS, 1)
 constexpr int PAIR_STAGES = 6;
 constexpr int PAIR_STAGE_BYTES = 2 * A_BYTES;  // A 128 x 64 and half of B 128 x 64
 constexpr int PAIR_M = 2 * BM;
-constexpr size_t PAIR_SMEM_BYTES = 1024 + PAIR_STAGES * PAIR_STAGE_BYTES + 256;
+constexpr int PAIR_STAGING = EPI_WARPS * CHUNK_BYTES;  // a buffer per epilogue warp
+constexpr int PAIR_BARRIER_BYTES = 512;
+constexpr size_t PAIR_SMEM_BYTES = 1024 + PAIR_STAGES * PAIR_STAGE_BYTES + PAIR_STAGING + PAIR_BARRIER_BYTES;
 
 // Work units are handed out at run time: a cluster's first unit is its index, every further one
 // comes from a global counter, so a cluster that finds its SMs late (another kernel, e.g. a
@@ -557,14 +576,17 @@ struct PairBarriers {
   uint32_t tmem_base;
   int abort_word;
 };
+static_assert(sizeof(PairBarriers) <= PAIR_BARRIER_BYTES, "barriers fit behind the staging buffers");
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
     gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
-                          const __grid_constant__ CUtensorMap tmap_b, const Params p) {
+                          const __grid_constant__ CUtensorMap tmap_b,
+                          const __grid_constant__ CUtensorMap tmap_d, const Params p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
-  PairBarriers* bars = reinterpret_cast<PairBarriers*>(smem + PAIR_STAGES * PAIR_STAGE_BYTES);
+  uint8_t* staging = smem + PAIR_STAGES * PAIR_STAGE_BYTES;
+  PairBarriers* bars = reinterpret_cast<PairBarriers*>(staging + PAIR_STAGING);
   volatile int* abort_word = &bars->abort_word;
 
   const int warp = threadIdx.x >> 5;
@@ -758,6 +780,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
     // ------------------------------------------------------------ epilogue (warps 2..9, both CTAs)
     const int quad = warp & 3;
     const int half = (warp - 2) >> 2;
+    uint8_t* buf = staging + (warp - 2) * CHUNK_BYTES;
     int t = 0;
     for (;; ++t) {
       const int slot = t % SCHED_SLOTS;
@@ -770,16 +793,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
       tile_coords(p, tile, b, tm, tn);
       const int acc = t & 1;
       const uint32_t acc_ph = (t >> 1) & 1;
+      const int row = tm * PAIR_M + static_cast<int>(rank) * BM + quad * 32 + lane;
+      const int col = tn * BN + half * (BN / 2);
       if (!mbar_wait(&bars->acc_full[acc], acc_ph, abort_word, 311)) break;
       tc_fence_after();
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BN + half * (BN / 2);
-      const int row = tm * PAIR_M + static_cast<int>(rank) * BM + quad * 32 + lane;
-      if (p.epi_mode == 3) store_tile_rows_rope(p, t_row, row, tn * BN + half * (BN / 2));
-      else store_tile_rows(p, t_row, b, row, tn * BN + half * (BN / 2));
+      if (p.tma_add) add_tile_rows(p, &tmap_d, buf, t_row, b, row - lane, col, lane);
+      else if (p.epi_mode == 3) store_tile_rows_rope(p, t_row, row, col);
+      else store_tile_rows(p, t_row, b, row, col);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&bars->acc_empty[acc]), 0));
     }
+    if (p.tma_add && lane == 0) tma_store_wait<0>();
   }
 
   // ------------------------------------------------------------ tear-down
@@ -845,7 +871,8 @@ static int32_t analyze_operand(const char* name, const cdl_tensor* t, bool contr
 //   wide tiles: launch and set-up; 0.28 us per K block (a quarter more when every pair loads); a store
 //     that grows with the part of the tile that exists, four times as dear where an f32 C is added to, and
 //     dearer for columns beyond the last 32 and with a bf16 C; and, for a pair's further tiles, the longer of
-//     their products and the store.
+//     their products and the store.  Where TMA adds into D the store is short, and the time of the additions at
+//     the memory (0.39 us per MB of D) joins as a 2.5-norm (fitted to 160 shapes: 0.6 % from the best on average).
 //   cluster: launch, exchange and store (more for more slices, less for fewer rows) and the longest of
 //     one CTA's K blocks (0.23 us), the K blocks of the CTAs that share an SM (0.22 us) and all blocks
 //     over all SMs (0.28 us; 0.25 us where D is reduced into; more for rows of B under 128 bytes); CTAs
@@ -862,7 +889,7 @@ static int32_t analyze_operand(const char* name, const cdl_tensor* t, bool contr
 // 512 x 5632 x 5632, whose 176 tiles of 128 x 128 leave most SMs waiting for two, 30.6 against 42.6, and 2048 x 3072 x 5616, 384 tiles
 // to walk in turns of 148, 56 against 91.
 static int choose_cluster_splits(long long batch, long long M, long long N, long long K, bool adds_f32,
-                                 bool adds_bf16, bool may_slice, bool reduces) {
+                                 bool adds_bf16, bool may_slice, bool reduces, bool tma_adds) {
   auto up = [](long long a, long long b) { return (a + b - 1) / b; };
   auto part = [](long long n, int tile) { return static_cast<double>(n < tile ? n : tile) / tile; };
   const double kb = static_cast<double>(up(K, BK));
@@ -880,6 +907,13 @@ static int choose_cluster_splits(long long batch, long long M, long long N, long
     const double busy = units < wide_slots ? static_cast<double>(units) / wide_slots : 1.0;
     const double loop = 0.275 * (1.0 + 0.23 * busy) * kb / s;
     double store, step;
+    if (tma_adds) {
+      // the additions' way to memory runs under the products and is felt where it is the longer
+      const double way = 0.39 * 4e-6 * batch * M * N;
+      const double own = 4.3 + loop + 2.8 * filled + static_cast<double>(up(units, wide_slots) - 1) * fmax(1.2, loop + 3.0);
+      best = fmin(best, 0.95 * fmax(pow(pow(own, 2.5) + pow(way, 2.5), 0.4), hbm));
+      continue;
+    }
     if (!adds_f32) {
       store = 1.6 * filled + (!adds_bf16 ? ragged : N % 32 == 0 || N < 32 ? 2.2 : N < 128 ? 3.3 : 5.0);
       step = fmax(fmax(1.2, loop + 0.6), 2.7 * filled);
@@ -1008,8 +1042,14 @@ int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_t
   const bool reduces = may_slice && N % 4 == 0 && (reinterpret_cast<uintptr_t>(d->ptr) & 15) == 0 &&
                        (M == 1 || (d->stride[r - 2] % 4 == 0 && c->stride[r - 2] == d->stride[r - 2])) &&
                        (r == 2 || (d->stride[0] % 4 == 0 && c->stride[0] == d->stride[0]));
+  // In the pair kernel TMA adds, where it can describe D.
+  const bool tma_adds = M > BM && adds_f32 && d->dtype == CDL_F32 && c->ptr == d->ptr && beta == 1.0f &&
+                        (reinterpret_cast<uintptr_t>(d->ptr) & 15) == 0 && d->stride[r - 2] % 4 == 0 &&
+                        d->stride[r - 2] >= N && c->stride[r - 2] == d->stride[r - 2] &&
+                        (r == 2 || batch == 1 ||
+                         (d->stride[0] % 4 == 0 && d->stride[0] > 0 && c->stride[0] == d->stride[0]));
   const int cluster_splits =
-      variant == CDL_GEMM_AUTO ? choose_cluster_splits(batch, M, N, K, adds_f32, use_c && !adds_f32, may_slice, reduces)
+      variant == CDL_GEMM_AUTO ? choose_cluster_splits(batch, M, N, K, adds_f32, use_c && !adds_f32, may_slice, reduces, tma_adds)
                                : 0;
   const bool use_cluster = cluster_splits > 0;
   const bool use_pair = !use_cluster && (variant == CDL_GEMM_AUTO ? M > BM : variant == CDL_GEMM_CTA_PAIR);
@@ -1086,6 +1126,7 @@ int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_t
   p.split_k = use_cluster ? cluster_splits : 1;
   p.sched_counter = nullptr;
   p.atomic_out = 0;
+  p.tma_add = 0;
   p.epi_mode = 0;
   p.aux0 = p.aux1 = nullptr;
   p.out2 = nullptr;
@@ -1142,10 +1183,23 @@ int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_t
   p.status = device_status_ptr();
   if (!p.status) return fail(CDL_ERR_CUDA, "cannot resolve the device status word");
 
+  // D += alpha * A^T B by TMA reductions (every element added to once per K slice).
+  CUtensorMap tm_d = tm_a;  // (a valid map where none is used)
+  const bool adds_in_place = adds_f32 && p.out_f32 && c->ptr == d->ptr && beta == 1.0f && p.ldc == p.ldd &&
+                             p.c_batch == p.d_batch;
+  if (use_pair && tma_adds) {
+    const uint64_t dims[3] = {static_cast<uint64_t>(N), static_cast<uint64_t>(M), static_cast<uint64_t>(batch)};
+    const uint64_t strides[3] = {0, static_cast<uint64_t>(p.ldd) * 4,
+                                 static_cast<uint64_t>(batch > 1 ? p.d_batch : p.ldd * M) * 4};
+    const uint32_t box[3] = {32, 32, 1};
+    CDL_CHECK(encode_tmap(&tm_d, p.d, CDL_F32, 3, dims, strides, box, true));
+    p.tma_add = 1;
+  }
+
   if (use_cluster) {
     // D += A^T B: every element is added to once, by a reduction at the L2, instead of read, added to and
-    // written: 2048 x 5632 x 256 29 us instead of 34 (25 as a walk), 512 x 1536 x 256 5.6 instead of 7.7.  (In the pair
-    // kernel, where a thread's reductions run along a row, the same costs 42 us instead of 34.)
+    // written: 2048 x 5632 x 256 29 us instead of 34 (25 as a walk), 512 x 1536 x 256 5.6 instead of 7.7.  (The pair
+    // kernel's tiles with TMA reductions: 25.9; with a thread's own reductions along its row 42.)
     if (reduces) {
       p.atomic_out = 1;
       p.c_mode = 0;
@@ -1186,8 +1240,7 @@ int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_t
   // whose output is small and whose K is long).  Slices add into D with atomics, which removes
   // the tile-count quantisation (e.g. 192 tiles on 74 CTA pairs = 2.6 waves) at the price of an
   // unordered f32 sum; the caller's `deterministic` option turns it off.
-  if (use_pair && use_c && p.out_f32 && c->dtype == CDL_F32 && c->ptr == d->ptr && beta == 1.0f &&
-      p.ldc == p.ldd && p.c_batch == p.d_batch) {
+  if (use_pair && adds_in_place) {
     if (!(opts && opts->deterministic != 0)) {
       const int nc = max_clusters[dev & 63];
       int best_s = 1;
@@ -1230,7 +1283,7 @@ int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_t
     const int clusters = units < max_clusters[dev & 63] ? static_cast<int>(units) : max_clusters[dev & 63];
     p.sched_counter = units > clusters ? sched_counter_for(0, dev, stream) : nullptr;
     CDL_CUDA(launch_pdl(gemm_bf16_pair_kernel, dim3(2 * clusters), dim3(THREADS), PAIR_SMEM_BYTES, stream,
-                        tm_a, tm_b, p));
+                        tm_a, tm_b, tm_d, p));
   } else {
     const int grid = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
     CDL_CUDA(launch_pdl(gemm_bf16_kernel, dim3(grid), dim3(THREADS), SMEM_BYTES, stream, tm_a, tm_b, p));

@@ -23,6 +23,7 @@ struct Params {
                    // per cluster); 1 = none
   int sum_blocks;  // gemm_general.cu: K blocks that one tensor-core accumulator sums up
   int atomic_out;  // 1 = add alpha * partial into D with red.global.add (D already holds C)
+  int tma_add;     // 1 = the pair kernel adds by TMA reductions (add_chunk)
   // Fused SwiGLU epilogues (bf16 [M, N] operands, 16-byte aligned rows):
   //   1: D = G (the product),           out2 = SiLU(G) * aux0           (aux0 = up projection)
   //   2: D = SiLU(aux0) * R,            out2 = R * aux1 * dSiLU(aux0)   (R = product, aux0 = gate, aux1 = up)
@@ -76,6 +77,30 @@ __device__ __forceinline__ float fast_sigmoid(float x) {
 constexpr int CLUSTER_TILE_N = 128;
 int32_t gemm_cluster_launch(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const Params& p,
                             cudaStream_t stream);
+
+// ------------------------------------------------------------------ D += alpha * accumulator
+// A warp's 32 rows x 32 columns of an f32 accumulator go to D as one TMA reduction from a 4 KiB buffer of shared
+// memory (tensor map of D: [N, M, batch], boxes of 32 x 32, the 128-byte swizzle, under which the rows' 16-byte
+// stores meet no bank twice).  A thread owns a row of the accumulator, so its own accesses to D take 32 lines
+// per instruction and, where C is read first, a round trip to HBM per 32 columns; the reduction is one
+// instruction, nothing waits for it, and the L2 adds whole lines.  Every element is added to once per K slice.
+constexpr int CHUNK_BYTES = 32 * 32 * 4;
+__device__ __forceinline__ void add_chunk(const CUtensorMap* tm_d, uint8_t* buf, const uint32_t (&r)[32], float alpha,
+                                          int lane, int col0, int row0, int b) {
+  const uint32_t row = smem_u32(buf) + lane * 128, x = (lane & 7) << 4;
+#pragma unroll
+  for (int c = 0; c < 8; ++c)
+    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(row + ((c << 4) ^ x)),
+                 "f"(alpha * __uint_as_float(r[4 * c])), "f"(alpha * __uint_as_float(r[4 * c + 1])),
+                 "f"(alpha * __uint_as_float(r[4 * c + 2])), "f"(alpha * __uint_as_float(r[4 * c + 3]))
+                 : "memory");
+  fence_proxy_async_smem();
+  __syncwarp();
+  if (lane == 0) {
+    tma_reduce_add_3d(tm_d, buf, col0, row0, b);
+    tma_store_commit();
+  }
+}
 
 // ------------------------------------------------------------------ K slices that meet in a cluster
 // A cluster of `splits` CTAs holds the partial sums of one 128 x 128 tile, one K slice per CTA.  Every

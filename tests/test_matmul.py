@@ -538,3 +538,36 @@ def test_rope_epilogue_of_few_rows(cdl, gpu_ok, rows, seqlen, heads):
         err = (d.double().cpu().view_as(want) - want).abs()
         # bf16 rounds to 2^-9 of the value; the f32 sum of 256 products of values below 1 adds little
         assert bool((err <= 2.0 ** -8 * want.abs() + 1e-4).all())
+
+
+@pytest.mark.parametrize("batch,m,k,n", [(1, 130, 64, 32), (1, 257, 200, 260), (1, 300, 1024, 33), (3, 160, 512, 72), (1, 2048, 4096, 520)])
+@pytest.mark.parametrize("pad", [0, 4])
+def test_in_place_additions_of_wide_tiles(cdl, gpu_ok, batch, m, k, n, pad):
+    """D += alpha A^T B (f32) by the CTA-pair tiles, whole and in K slices: D a view of a wider buffer, rows and
+    columns that end inside a 32 x 32 chunk, batches.  What lies outside D keeps its values.  Bound as in
+    test_short_weight_gradients, with one more addition per slice."""
+    gen = torch.Generator(device="cuda").manual_seed(m + n)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    a = rnd(batch, k, (m + 7) // 8 * 8).to(torch.bfloat16)[:, :, :m].mT
+    b = rnd(batch, k, (n + 7) // 8 * 8).to(torch.bfloat16)[:, :, :n]
+    buf = rnd(batch, m + 3, (n + 3) // 4 * 4 + pad)
+    if batch == 1:
+        a, b, buf = a[0], b[0], buf[0]
+    view = lambda t: t[..., :m, :n]
+    expected = view(buf).double() - 0.5 * (a.double() @ b.double())
+    bound = 0.5 * (a.double().abs() @ b.double().abs())
+    tol = (k / 16 + 1) * 2.0 ** -23 * bound + 9 * 2.0 ** -24 * (expected.abs() + bound)
+    for deterministic in (False, True):
+        runs = []
+        for _ in range(2):
+            out = buf.clone()
+            d = view(out)
+            cdl.ops.matmul(a, b, cdl.ops.MatmulOpts(out=torch.float32, c=d, alpha=-0.5, beta=1.0, variant=cdl._lib.GEMM_CTA_PAIR,
+                                                    deterministic=deterministic), out=d)
+            assert bool(((d.double() - expected).abs() <= tol).all())
+            outside = torch.ones_like(out, dtype=torch.bool)
+            view(outside)[...] = False
+            assert torch.equal(out[outside], buf[outside])
+            runs.append(out)
+        assert not deterministic or torch.equal(*runs)
+    assert cdl._lib.device_status() == 0
