@@ -372,6 +372,122 @@ __device__ __forceinline__ void store_tile_rows_rope(const Params& p, uint32_t t
   }
 }
 
+// The operands of the fused SwiGLU forms come ahead of their use: a warp's next 32 rows x 32 columns of aux0 (and aux1)
+// by TMA into its 4 KiB buffer (the 64-byte swizzle: a row is 64 bytes, its 16-byte chunk c at c ^ (row / 2 & 3)), the
+// first ones of a tile under its products, the others under the arithmetic and the stores of those before.
+struct SwigluFeed {
+  const CUtensorMap* map0;
+  const CUtensorMap* map1;
+  uint8_t* buf;
+  uint64_t* full;
+  bool two;
+  uint32_t phase;
+  __device__ __forceinline__ void load(int lane, int row0, int col0) {
+    if (lane != 0) return;
+    mbar_arrive_expect_tx(full, two ? 4096 : 2048);
+    tma_load_3d(buf, map0, full, col0, row0, 0);
+    if (two) tma_load_3d(buf + 2048, map1, full, col0, row0, 0);
+  }
+  __device__ __forceinline__ void read(int lane, int which, uint32_t (&w)[16]) const {
+    const uint32_t row = smem_u32(buf) + which * 2048 + lane * 64, x = (lane >> 1 & 3) << 4;
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                   : "=r"(w[4 * c]), "=r"(w[4 * c + 1]), "=r"(w[4 * c + 2]), "=r"(w[4 * c + 3])
+                   : "r"(row + ((c << 4) ^ x))
+                   : "memory");
+  }
+};
+
+// Pairs of f32 in one register pair: one packed operation for two.
+struct F32x2 {
+  uint64_t v;
+  __device__ __forceinline__ F32x2() {}
+  __device__ __forceinline__ F32x2(float lo, float hi) { asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi)); }
+  __device__ __forceinline__ void get(float& lo, float& hi) const { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+};
+__device__ __forceinline__ F32x2 mul2(F32x2 a, F32x2 b) {
+  F32x2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
+  return d;
+}
+__device__ __forceinline__ F32x2 fma2(F32x2 a, F32x2 b, F32x2 c) {
+  F32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return d;
+}
+__device__ __forceinline__ F32x2 tanh2(F32x2 a) {
+  float lo, hi;
+  a.get(lo, hi);
+  asm("tanh.approx.f32 %0, %0;" : "+f"(lo));
+  asm("tanh.approx.f32 %0, %0;" : "+f"(hi));
+  return F32x2(lo, hi);
+}
+__device__ __forceinline__ uint32_t pack2(F32x2 a) {
+  float lo, hi;
+  a.get(lo, hi);
+  return pack_bf16x2(lo, hi);
+}
+
+// The fused SwiGLU epilogues for the calling warp: 32 rows, 128 columns; the first chunk's operands are under way.
+// TWO: mode 2 (d_up, d_gate), else mode 1 (gate, act).  alpha is 1.  Eight warps do this beside the products, so their
+// instructions count: packed pairs take half of what single operations take.
+template <bool TWO>
+__device__ __forceinline__ void store_tile_rows_swiglu(const Params& p, SwigluFeed& feed, uint32_t t_row, int row,
+                                                       int col_base, int lane, volatile int* abort_word) {
+  if (row - lane >= p.M) return;  // warp-uniform
+#pragma unroll 1
+  for (int ch = 0; ch < BN / 64; ++ch) {
+    const int col0 = col_base + ch * 32;
+    if (col0 >= p.N) break;
+    uint32_t r[32], w0[16], w1[16];
+    if (!mbar_wait(feed.full, feed.phase, abort_word, 313)) return;
+    feed.phase ^= 1;
+    feed.read(lane, 0, w0);
+    if (TWO) feed.read(lane, 1, w1);
+    // (load and wait side by side: nothing ties the arithmetic on r to the wait but their order)
+    tmem_ld32(t_row + ch * 32, r);
+    tmem_wait_ld();
+    __syncwarp();  // the buffer has been read
+    if (ch + 1 < BN / 64 && col0 + 32 < p.N) feed.load(lane, row - lane, col0 + 32);
+    uint32_t q1[16], q2[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const F32x2 rr(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+      const F32x2 x0(bf16_lo(w0[j]), bf16_hi(w0[j])), half(0.5f, 0.5f);
+      const F32x2 s = fma2(tanh2(mul2(TWO ? x0 : rr, half)), half, half);  // the sigmoid, as fast_sigmoid
+      if (!TWO) {
+        q1[j] = pack2(rr);
+        q2[j] = pack2(mul2(mul2(rr, s), x0));
+      } else {
+        const F32x2 x1(bf16_lo(w1[j]), bf16_hi(w1[j])), one(1.0f, 1.0f), minus(-1.0f, -1.0f);
+        const F32x2 xs = mul2(x0, s);
+        q1[j] = pack2(mul2(xs, rr));
+        q2[j] = pack2(mul2(mul2(rr, x1), fma2(xs, fma2(s, minus, one), s)));
+      }
+    }
+    if (row < p.M) {
+      __nv_bfloat16* dp = static_cast<__nv_bfloat16*>(p.d) + static_cast<long long>(row) * p.ldd + col0;
+      __nv_bfloat16* op = p.out2 + static_cast<long long>(row) * p.ld_out2 + col0;
+      if (p.wide && col0 + 32 <= p.N) {
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+          st_global_v8(dp + g * 16, reinterpret_cast<const uint32_t(&)[8]>(q1[g * 8]));
+          st_global_v8(op + g * 16, reinterpret_cast<const uint32_t(&)[8]>(q2[g * 8]));
+        }
+      } else {
+#pragma unroll
+        for (int g = 0; g < 4; ++g)
+          if (col0 + g * 8 + 8 <= p.N) {  // N % 8 == 0 is checked on the host
+            *reinterpret_cast<uint4*>(dp + g * 8) = make_uint4(q1[g * 4], q1[g * 4 + 1], q1[g * 4 + 2], q1[g * 4 + 3]);
+            *reinterpret_cast<uint4*>(op + g * 8) = make_uint4(q2[g * 4], q2[g * 4 + 1], q2[g * 4 + 2], q2[g * 4 + 3]);
+          }
+      }
+    }
+    __syncwarp();  // all lanes are at the next chunk's tensor-memory load together
+  }
+}
+
 // The epilogue of D += alpha * accumulator for the calling warp: rows row0 .. row0 + 31, 128 columns.
 __device__ __forceinline__ void add_tile_rows(const Params& p, const CUtensorMap* tm_d, uint8_t* buf, uint32_t t_row,
                                               int b, int row0, int col_base, int lane) {
@@ -572,6 +688,7 @@ struct PairBarriers {
   uint64_t acc_full[2];
   uint64_t acc_empty[2];
   uint64_t sched_full[SCHED_SLOTS];
+  uint64_t extra_full[EPI_WARPS];  // the SwiGLU epilogue's operands, a warp's next chunk
   uint32_t unit_ring[SCHED_SLOTS];
   uint32_t tmem_base;
   int abort_word;
@@ -581,7 +698,8 @@ static_assert(sizeof(PairBarriers) <= PAIR_BARRIER_BYTES, "barriers fit behind t
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
     gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
                           const __grid_constant__ CUtensorMap tmap_b,
-                          const __grid_constant__ CUtensorMap tmap_d, const Params p) {
+                          const __grid_constant__ CUtensorMap tmap_e0,
+                          const __grid_constant__ CUtensorMap tmap_e1, const Params p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -632,6 +750,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
       mbar_init(&bars->acc_empty[i], 2 * EPI_WARPS);  // epilogue warps of both CTAs (leader's copy is used)
     }
     for (int i = 0; i < SCHED_SLOTS; ++i) mbar_init(&bars->sched_full[i], 1);
+    for (int i = 0; i < EPI_WARPS; ++i) mbar_init(&bars->extra_full[i], 1);
     bars->abort_word = 0;
     fence_mbar_init();
     // the peer's slots wait for the leader's 4-byte st.async
@@ -781,6 +900,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
     const int quad = warp & 3;
     const int half = (warp - 2) >> 2;
     uint8_t* buf = staging + (warp - 2) * CHUNK_BYTES;
+    const bool swiglu = p.epi_mode == 1 || p.epi_mode == 2;
+    SwigluFeed feed{&tmap_e0, &tmap_e1, buf, &bars->extra_full[warp - 2], p.epi_mode == 2, 0};
     int t = 0;
     for (;; ++t) {
       const int slot = t % SCHED_SLOTS;
@@ -795,10 +916,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
       const uint32_t acc_ph = (t >> 1) & 1;
       const int row = tm * PAIR_M + static_cast<int>(rank) * BM + quad * 32 + lane;
       const int col = tn * BN + half * (BN / 2);
+      if (swiglu && row - lane < p.M && col < p.N) feed.load(lane, row - lane, col);  // under the products
       if (!mbar_wait(&bars->acc_full[acc], acc_ph, abort_word, 311)) break;
       tc_fence_after();
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BN + half * (BN / 2);
-      if (p.tma_add) add_tile_rows(p, &tmap_d, buf, t_row, b, row - lane, col, lane);
+      if (p.tma_add) add_tile_rows(p, &tmap_e0, buf, t_row, b, row - lane, col, lane);
+      else if (p.epi_mode == 1) store_tile_rows_swiglu<false>(p, feed, t_row, row, col, lane, abort_word);
+      else if (p.epi_mode == 2) store_tile_rows_swiglu<true>(p, feed, t_row, row, col, lane, abort_word);
       else if (p.epi_mode == 3) store_tile_rows_rope(p, t_row, row, col);
       else store_tile_rows(p, t_row, b, row, col);
       tc_fence_before();
@@ -1150,9 +1274,9 @@ int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_t
     p.rope_cols = rope->rot_cols;
     p.rope_nseq = rope->num_seqs;
   } else if (epi_mode != 0) {
-    if (r != 2 || use_c || d->dtype != CDL_BF16 || N % 8 != 0 || !p.d_vec)
+    if (r != 2 || use_c || alpha != 1.0f || d->dtype != CDL_BF16 || N % 8 != 0 || !p.d_vec)
       return fail(CDL_ERR_INVALID,
-                  "matmul (fused SwiGLU): rank 2, no C operand, bf16 output with 16-byte aligned rows "
+                  "matmul (fused SwiGLU): rank 2, alpha 1, no C operand, bf16 output with 16-byte aligned rows "
                   "and N %% 8 == 0 are required");
     CDL_CHECK(check_epi_operand("aux0", aux0, M, N));
     CDL_CHECK(check_epi_operand("out2", out2, M, N));
@@ -1184,7 +1308,7 @@ int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_t
   if (!p.status) return fail(CDL_ERR_CUDA, "cannot resolve the device status word");
 
   // D += alpha * A^T B by TMA reductions (every element added to once per K slice).
-  CUtensorMap tm_d = tm_a;  // (a valid map where none is used)
+  CUtensorMap tm_e0 = tm_a, tm_e1 = tm_a;  // (valid maps where none is used)
   const bool adds_in_place = adds_f32 && p.out_f32 && c->ptr == d->ptr && beta == 1.0f && p.ldc == p.ldd &&
                              p.c_batch == p.d_batch;
   if (use_pair && tma_adds) {
@@ -1192,8 +1316,18 @@ int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_t
     const uint64_t strides[3] = {0, static_cast<uint64_t>(p.ldd) * 4,
                                  static_cast<uint64_t>(batch > 1 ? p.d_batch : p.ldd * M) * 4};
     const uint32_t box[3] = {32, 32, 1};
-    CDL_CHECK(encode_tmap(&tm_d, p.d, CDL_F32, 3, dims, strides, box, true));
+    CDL_CHECK(encode_tmap(&tm_e0, p.d, CDL_F32, 3, dims, strides, box, true));
     p.tma_add = 1;
+  }
+  if (use_pair && (p.epi_mode == 1 || p.epi_mode == 2)) {
+    const cdl_tensor* aux[2] = {aux0, aux1};
+    for (int i = 0; i < p.epi_mode; ++i) {
+      const uint64_t ld = static_cast<uint64_t>(aux[i]->stride[0]) * 2;
+      const uint64_t dims[3] = {static_cast<uint64_t>(N), static_cast<uint64_t>(M), 1};
+      const uint64_t strides[3] = {0, ld, ld * M};
+      const uint32_t box[3] = {32, 32, 1};
+      CDL_CHECK(encode_tmap(i ? &tm_e1 : &tm_e0, aux[i]->ptr, CDL_BF16, 3, dims, strides, box, false, true));
+    }
   }
 
   if (use_cluster) {
@@ -1283,7 +1417,7 @@ int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_t
     const int clusters = units < max_clusters[dev & 63] ? static_cast<int>(units) : max_clusters[dev & 63];
     p.sched_counter = units > clusters ? sched_counter_for(0, dev, stream) : nullptr;
     CDL_CUDA(launch_pdl(gemm_bf16_pair_kernel, dim3(2 * clusters), dim3(THREADS), PAIR_SMEM_BYTES, stream,
-                        tm_a, tm_b, tm_d, p));
+                        tm_a, tm_b, tm_e0, tm_e1, p));
   } else {
     const int grid = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
     CDL_CUDA(launch_pdl(gemm_bf16_kernel, dim3(grid), dim3(THREADS), SMEM_BYTES, stream, tm_a, tm_b, p));

@@ -123,7 +123,7 @@ static EncodeTiledFn encode_fn() {
 
 int32_t encode_tmap(CUtensorMap* out, const void* base, int32_t dtype, int rank,
                     const uint64_t* dims, const uint64_t* strides_bytes, const uint32_t* box,
-                    bool swizzle128) {
+                    bool swizzle128, bool swizzle64) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return fail(CDL_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
   cuuint64_t gdim[5];
@@ -141,7 +141,9 @@ int32_t encode_tmap(CUtensorMap* out, const void* base, int32_t dtype, int rank,
                                                : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
   CUresult r = fn(out, dt, static_cast<cuuint32_t>(rank), const_cast<void*>(base), gdim, gstr, bx,
                   estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                  swizzle128  ? CU_TENSOR_MAP_SWIZZLE_128B
+                  : swizzle64 ? CU_TENSOR_MAP_SWIZZLE_64B
+                              : CU_TENSOR_MAP_SWIZZLE_NONE,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS)
     return fail(CDL_ERR_INVALID,

@@ -50,7 +50,7 @@ constexpr int32_t TMAP_U8 = 100;
 // in BYTES for dims 1.. (the innermost is contiguous).  box is innermost-first.
 int32_t encode_tmap(CUtensorMap* out, const void* base, int32_t dtype, int rank,
                     const uint64_t* dims, const uint64_t* strides_bytes, const uint32_t* box,
-                    bool swizzle128);
+                    bool swizzle128, bool swizzle64 = false);
 
 // Launches `kernel` with the programmatic-serialization attribute (see grid_dep_wait in ptx.cuh):
 // the kernel may begin before the previous kernel of the stream has finished and MUST call

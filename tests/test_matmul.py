@@ -571,3 +571,37 @@ def test_in_place_additions_of_wide_tiles(cdl, gpu_ok, batch, m, k, n, pad):
             runs.append(out)
         assert not deterministic or torch.equal(*runs)
     assert cdl._lib.device_status() == 0
+
+
+@pytest.mark.parametrize("m,n,k,pad", [(4003, 5640, 1024, 0), (2309, 8200, 512, 8), (4096, 5632, 256, 16)])
+def test_fused_swiglu_epilogues_of_wide_tiles(cdl, gpu_ok, m, n, k, pad):
+    """The SwiGLU forms by the CTA-pair tiles, whose epilogue brings its operands in ahead: M and N that end inside a
+    32 x 32 chunk, operands and outputs with padded rows (off the 32-byte grid with 8), padding left alone.  Bound:
+    the bf16 rounding of a result, 2^-8, and of the truncated f32 sums, carried through SiLU (slope below 1.1) and
+    through fast_sigmoid (2^-11 of tanh)."""
+    L = cdl._lib
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    rnd = lambda *s, std=1.0: (torch.randn(*s, generator=gen, device="cuda") * std).to(torch.bfloat16)
+    a, b = rnd(m, k), rnd(k, n, std=k ** -0.5)
+    up, gate, o1, o2 = (rnd(m, n + pad) for _ in range(4))
+    ends = [t[:, n:].clone() for t in (o1, o2)]
+    v = [t[:, :n] for t in (up, gate, o1, o2)]
+    r = a.double() @ b.double()
+    err = (k / 16 + 1) * 2.0 ** -23 * (a.double().abs() @ b.double().abs())
+
+    def close(got, exact, carried):
+        tol = 2.0 ** -8 * exact.abs() + 1.1 * err * carried + 2.0 ** -10 * r.abs() * carried + 1e-30
+        assert bool(((got.double() - exact).abs() <= tol).all())
+
+    for _ in range(3):
+        args = [L.tensor_arg(t) for t in (a, b, v[0], v[2], v[3])]
+        L.check(L.lib.cdl_b200_matmul_swiglu_gate(*(L.ref(t) for t in args), None))
+        close(v[2], r, 1.0)
+        close(v[3], r * torch.sigmoid(r) * v[0].double(), v[0].double().abs())
+        args = [L.tensor_arg(t) for t in (a, b, v[1], v[0], v[2], v[3])]
+        L.check(L.lib.cdl_b200_matmul_swiglu_dgrad(*(L.ref(t) for t in args), None))
+        g, s = v[1].double(), torch.sigmoid(v[1].double())
+        close(v[2], g * s * r, g.abs() + 1)
+        close(v[3], r * v[0].double() * (s + g * s * (1 - s)), v[0].double().abs() * (g.abs() + 1))
+    assert all(torch.equal(t[:, n:], e) for t, e in zip((o1, o2), ends))
+    assert L.device_status() == 0
