@@ -41,10 +41,13 @@ int32_t layernorm_fwd_execute(const cdl_tensor* x, const cdl_tensor* scale, cons
                               float eps, const cdl_tensor* y, const cdl_tensor* mean,
                               const cdl_tensor* r_inv, cudaStream_t stream);
 size_t rmsnorm_bwd_scratch_bytes(long long rows, long long cols);
+// With h (bf16 [rows, cols], cols <= 2048) r_inv is not read: the statistic is taken from x again and h = the norm's
+// forward output is written besides.
 int32_t rmsnorm_bwd_execute(const cdl_tensor* x, const cdl_tensor* dy, const cdl_tensor* res,
                             const cdl_tensor* scale, const cdl_tensor* r_inv, const cdl_tensor* dx,
                             const cdl_tensor* dscale, void* scratch, size_t scratch_bytes,
-                            cudaStream_t stream, const cdl_norm_options* opts = nullptr);
+                            cudaStream_t stream, const cdl_norm_options* opts = nullptr,
+                            const cdl_tensor* h = nullptr, float eps = 0.f);
 int32_t attn_fwd_execute(const cdl_attn_desc* desc, const cdl_tensor* q, const cdl_tensor* k,
                          const cdl_tensor* v, const cdl_tensor* o, const cdl_tensor* lse,
                          cudaStream_t stream);

@@ -21,6 +21,7 @@
 #include <string.h>
 
 #include <mutex>
+#include <type_traits>
 
 namespace cdl {
 namespace norm {
@@ -322,17 +323,29 @@ __global__ void __launch_bounds__(PIPE_THREADS, 1)
   if (threadIdx.x == 0 && *abort_word != 0) atomicExch(status, *abort_word);
 }
 
+// What the backward gives besides, when it takes no r_inv.
+struct Recomputed {
+  __nv_bfloat16* h;
+  long long ldh;
+  float eps;
+};
+
 // Backward.  Every warp walks rows (grid-stride), keeps per-lane partial sums of
 // dscale for its columns in registers when DSCALE is set, and at the end the block folds its
 // warps' partials through shared memory into one row of `partials` [gridDim.x, cols].
-template <int NCH, bool DSCALE>
-__global__ void __launch_bounds__(BWD_THREADS, BWD_BLOCKS_PER_SM)
+//
+// With H the call has no r_inv: the row's statistic is taken again from x, which is in registers anyway, and h, the
+// norm's forward output, is stored beside dx (both the bits of rmsnorm_fwd_kernel: the same sums in the same
+// order).  A training step that does not keep h needs it for the weight gradients; as a kernel of its own it reads x
+// once more and is one more launch.
+template <int NCH, bool DSCALE, bool H>
+__global__ void __launch_bounds__(BWD_THREADS, H && NCH == 8 ? 2 : BWD_BLOCKS_PER_SM)
     rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, long long ldx,
                        const __nv_bfloat16* __restrict__ dy, long long lddy,
                        const __nv_bfloat16* __restrict__ res, long long ldres,
                        const __nv_bfloat16* __restrict__ scale, const float* __restrict__ r_inv,
                        long long r_inv_stride, __nv_bfloat16* __restrict__ dx, long long lddx,
-                       float* __restrict__ partials, int rows, int cols) {
+                       float* __restrict__ partials, int rows, int cols, const Recomputed rec) {
   extern __shared__ float s_part[];  // [cols] when DSCALE
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -358,7 +371,20 @@ __global__ void __launch_bounds__(BWD_THREADS, BWD_BLOCKS_PER_SM)
       vx[c] = in ? ld_nc_v4(xr + col) : make_uint4(0, 0, 0, 0);
       vd[c] = in ? ld_nc_v4(dyr + col) : make_uint4(0, 0, 0, 0);
     }
-    const float r = r_inv[row * r_inv_stride];
+    float r = 0.f;
+    if constexpr (H) {
+      float ss = 0.f;
+#pragma unroll
+      for (int c = 0; c < NCH; ++c) {
+        float f[8];
+        unpack8(vx[c], f);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) ss = fmaf(f[j], f[j], ss);
+      }
+      r = rsqrtf(warp_sum(ss) * inv_cols + rec.eps);
+    } else {
+      r = r_inv[row * r_inv_stride];
+    }
     // g = dy * scale (kept in vd's place as f32 is too large: recompute in the second pass).
     float dot = 0.f;
 #pragma unroll
@@ -396,6 +422,11 @@ __global__ void __launch_bounds__(BWD_THREADS, BWD_BLOCKS_PER_SM)
           for (int j = 0; j < 8; ++j) o[j] += fr[j];
         }
         st_cs_v4(dxr + col, pack8(o));
+        if constexpr (H) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) o[j] = fx[j] * r * fs[j];
+          *reinterpret_cast<uint4*>(rec.h + row * rec.ldh + col) = pack8(o);
+        }
       }
     }
   }
@@ -423,14 +454,15 @@ __global__ void __launch_bounds__(BWD_THREADS, BWD_BLOCKS_PER_SM)
 constexpr int BWD_PIPE_PRODUCERS = 2;
 constexpr int BWD_PIPE_THREADS = (PIPE_CONSUMERS + BWD_PIPE_PRODUCERS) * 32;
 
-template <int NCH>
+template <int NCH, bool H>
 __global__ void __launch_bounds__(BWD_PIPE_THREADS, 1)
     rmsnorm_bwd_pipe_kernel(const __nv_bfloat16* __restrict__ x, long long ldx,
                             const __nv_bfloat16* __restrict__ dy, long long lddy,
                             const __nv_bfloat16* __restrict__ res, long long ldres,
                             const __nv_bfloat16* __restrict__ scale, const float* __restrict__ r_inv,
                             long long r_inv_stride, __nv_bfloat16* __restrict__ dx, long long lddx,
-                            float* __restrict__ partials, int rows, int cols, int stages, int* status) {
+                            float* __restrict__ partials, int rows, int cols, int stages, int* status,
+                            const Recomputed rec) {
   extern __shared__ __align__(128) uint8_t ring[];
   const int row_bytes = cols * 2;
   const int ntens = res != nullptr ? 3 : 2;
@@ -498,7 +530,7 @@ __global__ void __launch_bounds__(BWD_PIPE_THREADS, 1)
       const int s = i % stages;
       const uint32_t ph = (i / stages) & 1;
       const long long row = row_begin + i;
-      const float r = r_inv[row * r_inv_stride];  // on its way while the row's tiles land
+      float r = H ? 0.f : r_inv[row * r_inv_stride];  // on its way while the row's tiles land
       // The consumer warps run independently, so this warp can reach the stage's next use before
       // another warp has taken the previous one (or before that one's copies have landed): a
       // parity wait on `full` would then pass on the phase before last.  The stage's previous
@@ -507,13 +539,30 @@ __global__ void __launch_bounds__(BWD_PIPE_THREADS, 1)
       if (i >= stages && !mbar_wait(&empty[s], ph ^ 1, abort_word, 713)) break;
       if (!mbar_wait(&full[s], ph, abort_word, 712)) break;
       const uint8_t* src = ring + static_cast<size_t>(s) * stage_bytes;
+      // The row is held in registers; with H, where three passes use it, it is read from the ring each time (beside the
+      // dscale sums it would spill).
       uint4 vx[NCH], vd[NCH];
+      auto tile_x = [&](int c, int col) { return H ? ld_shared_v4(src + col * 2) : vx[c]; };
+      auto tile_d = [&](int c, int col) { return H ? ld_shared_v4(src + row_bytes + col * 2) : vd[c]; };
 #pragma unroll
-      for (int c = 0; c < NCH; ++c) {
+      for (int c = 0; c < (H ? 0 : NCH); ++c) {
         const int col = c * 256 + lane * 8;
         const bool in = col < cols;
         vx[c] = in ? *reinterpret_cast<const uint4*>(src + col * 2) : make_uint4(0, 0, 0, 0);
         vd[c] = in ? *reinterpret_cast<const uint4*>(src + row_bytes + col * 2) : make_uint4(0, 0, 0, 0);
+      }
+      if constexpr (H) {
+        float ss = 0.f;
+#pragma unroll
+        for (int c = 0; c < NCH; ++c) {
+          const int col = c * 256 + lane * 8;
+          if (col >= cols) break;
+          float f[8];
+          unpack8(tile_x(c, col), f);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) ss = fmaf(f[j], f[j], ss);
+        }
+        r = rsqrtf(warp_sum(ss) * inv_cols + rec.eps);
       }
       float dot = 0.f;
 #pragma unroll
@@ -521,8 +570,8 @@ __global__ void __launch_bounds__(BWD_PIPE_THREADS, 1)
         const int col = c * 256 + lane * 8;
         if (col < cols) {
           float fx[8], fd[8], fs[8];
-          unpack8(vx[c], fx);
-          unpack8(vd[c], fd);
+          unpack8(tile_x(c, col), fx);
+          unpack8(tile_d(c, col), fd);
           unpack8(*reinterpret_cast<const uint4*>(s_scale + col * 2), fs);
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
@@ -539,8 +588,8 @@ __global__ void __launch_bounds__(BWD_PIPE_THREADS, 1)
         const int col = c * 256 + lane * 8;
         if (col < cols) {
           float fx[8], fd[8], fs[8], o[8];
-          unpack8(vx[c], fx);
-          unpack8(vd[c], fd);
+          unpack8(tile_x(c, col), fx);
+          unpack8(tile_d(c, col), fd);
           unpack8(*reinterpret_cast<const uint4*>(s_scale + col * 2), fs);
 #pragma unroll
           for (int j = 0; j < 8; ++j) o[j] = r * (fd[j] * fs[j] - fx[j] * k);
@@ -551,6 +600,11 @@ __global__ void __launch_bounds__(BWD_PIPE_THREADS, 1)
             for (int j = 0; j < 8; ++j) o[j] += fr[j];
           }
           st_cs_v4(dxr + col, pack8(o));
+          if constexpr (H) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) o[j] = fx[j] * r * fs[j];
+            *reinterpret_cast<uint4*>(rec.h + row * rec.ldh + col) = pack8(o);
+          }
         }
       }
       __syncwarp();
@@ -709,23 +763,24 @@ static void launch_fwd(const cdl_tensor* x, const cdl_tensor* scale, const cdl_t
       eps);
 }
 
-template <int NCH, bool DSCALE>
+template <int NCH, bool DSCALE, bool H>
 static void launch_bwd(const cdl_tensor* x, const cdl_tensor* dy, const cdl_tensor* res,
                        const cdl_tensor* scale, const cdl_tensor* r_inv, const cdl_tensor* dx,
-                       float* partials, int grid, int rows, int cols, cudaStream_t stream) {
+                       float* partials, int grid, int rows, int cols, const Recomputed& rec, cudaStream_t stream) {
   const size_t smem = DSCALE ? static_cast<size_t>(cols) * sizeof(float) : 0;
-  launch_pdl(rmsnorm_bwd_kernel<NCH, DSCALE>, dim3(grid), dim3(BWD_THREADS), smem, stream,
+  launch_pdl(rmsnorm_bwd_kernel<NCH, DSCALE, H>, dim3(grid), dim3(BWD_THREADS), smem, stream,
       static_cast<const __nv_bfloat16*>(x->ptr), x->stride[0],
       static_cast<const __nv_bfloat16*>(dy->ptr), dy->stride[0],
       res ? static_cast<const __nv_bfloat16*>(res->ptr) : nullptr, res ? res->stride[0] : 0,
-      static_cast<const __nv_bfloat16*>(scale->ptr), static_cast<const float*>(r_inv->ptr),
-      r_inv->stride[0], static_cast<__nv_bfloat16*>(dx->ptr), dx->stride[0], partials, rows, cols);
+      static_cast<const __nv_bfloat16*>(scale->ptr), static_cast<const float*>(H ? nullptr : r_inv->ptr),
+      H ? 0 : r_inv->stride[0], static_cast<__nv_bfloat16*>(dx->ptr), dx->stride[0], partials, rows, cols, rec);
 }
 
-template <int NCH>
+template <int NCH, bool H>
 static void launch_bwd_pipe(const cdl_tensor* x, const cdl_tensor* dy, const cdl_tensor* res,
                             const cdl_tensor* scale, const cdl_tensor* r_inv, const cdl_tensor* dx,
-                            float* partials, int rows, int cols, int* status, cudaStream_t stream) {
+                            float* partials, int rows, int cols, int* status, const Recomputed& rec,
+                            cudaStream_t stream) {
   const int row_bytes = cols * 2;
   const int stage_bytes = (res ? 3 : 2) * row_bytes;
   int stages = (160 * 1024) / stage_bytes;
@@ -736,16 +791,32 @@ static void launch_bwd_pipe(const cdl_tensor* x, const cdl_tensor* dy, const cdl
   int dev = 0;
   cudaGetDevice(&dev);
   std::call_once(once[dev & 63], [&] {
-    cudaFuncSetAttribute(rmsnorm_bwd_pipe_kernel<NCH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaFuncSetAttribute(rmsnorm_bwd_pipe_kernel<NCH, H>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          160 * 1024 + 4096 + 2 * 64 * static_cast<int>(sizeof(uint64_t)) + 16);
   });
-  launch_pdl(rmsnorm_bwd_pipe_kernel<NCH>, dim3(sm_count()), dim3(BWD_PIPE_THREADS), smem, stream,
+  launch_pdl(rmsnorm_bwd_pipe_kernel<NCH, H>, dim3(sm_count()), dim3(BWD_PIPE_THREADS), smem, stream,
       static_cast<const __nv_bfloat16*>(x->ptr), x->stride[0],
       static_cast<const __nv_bfloat16*>(dy->ptr), dy->stride[0],
       res ? static_cast<const __nv_bfloat16*>(res->ptr) : nullptr, res ? res->stride[0] : 0,
-      static_cast<const __nv_bfloat16*>(scale->ptr), static_cast<const float*>(r_inv->ptr),
-      r_inv->stride[0], static_cast<__nv_bfloat16*>(dx->ptr), dx->stride[0], partials, rows, cols,
-      stages, status);
+      static_cast<const __nv_bfloat16*>(scale->ptr), static_cast<const float*>(H ? nullptr : r_inv->ptr),
+      H ? 0 : r_inv->stride[0], static_cast<__nv_bfloat16*>(dx->ptr), dx->stride[0], partials, rows, cols,
+      stages, status, rec);
+}
+
+// The backward of rows of up to 2048 columns: the pipelined kernel or, with `grid` CTAs, a warp per row.
+template <bool H>
+static void launch_bwd_rows(bool pipe, const cdl_tensor* x, const cdl_tensor* dy, const cdl_tensor* res,
+                            const cdl_tensor* scale, const cdl_tensor* r_inv, const cdl_tensor* dx, float* partials,
+                            int grid, int r, int c, int* status, const Recomputed& rec, cudaStream_t stream) {
+  auto run = [&](auto nch) {
+    constexpr int NCH = decltype(nch)::value;
+    if (pipe) launch_bwd_pipe<NCH, H>(x, dy, res, scale, r_inv, dx, partials, r, c, status, rec, stream);
+    else launch_bwd<NCH, true, H>(x, dy, res, scale, r_inv, dx, partials, grid, r, c, rec, stream);
+  };
+  if (c <= 256) run(std::integral_constant<int, 1>{});
+  else if (c <= 512) run(std::integral_constant<int, 2>{});
+  else if (c <= 1024) run(std::integral_constant<int, 4>{});
+  else run(std::integral_constant<int, 8>{});
 }
 
 }  // namespace norm
@@ -827,13 +898,13 @@ size_t rmsnorm_bwd_scratch_bytes(long long rows, long long cols) {
 int32_t rmsnorm_bwd_execute(const cdl_tensor* x, const cdl_tensor* dy, const cdl_tensor* res,
                             const cdl_tensor* scale, const cdl_tensor* r_inv, const cdl_tensor* dx,
                             const cdl_tensor* dscale, void* scratch, size_t scratch_bytes,
-                            cudaStream_t stream, const cdl_norm_options* opts) {
+                            cudaStream_t stream, const cdl_norm_options* opts, const cdl_tensor* h, float eps) {
   using namespace norm;
   const char* op = "norm_bwd";
   const int variant = opts ? opts->variant : CDL_NORM_AUTO;
   if (variant < CDL_NORM_AUTO || variant > CDL_NORM_PIPELINED)
     return fail(CDL_ERR_INVALID, "%s: unknown kernel variant %d", op, variant);
-  if (!x || !dy || !scale || !r_inv || !dx || !dscale)
+  if (!x || !dy || !scale || (!r_inv && !h) || !dx || !dscale)
     return fail(CDL_ERR_INVALID, "%s: x, dy, scale, r_inv, dx and dscale are required", op);
   if (x->rank != 2) return fail(CDL_ERR_INVALID, "%s: x must be a 2D tensor", op);
   const long long rows = x->shape[0], cols = x->shape[1];
@@ -845,7 +916,9 @@ int32_t rmsnorm_bwd_execute(const cdl_tensor* x, const cdl_tensor* dy, const cdl
   CDL_CHECK(check_rows(op, "dx", dx, rows, cols));
   if (res) CDL_CHECK(check_rows(op, "residual_dy", res, rows, cols));
   CDL_CHECK(check_vec(op, "scale", scale, cols, CDL_BF16, true));
-  CDL_CHECK(check_vec(op, "r_inv", r_inv, rows, CDL_F32, false));
+  if (h) CDL_CHECK(check_rows(op, "h", h, rows, cols));
+  else CDL_CHECK(check_vec(op, "r_inv", r_inv, rows, CDL_F32, false));
+  if (h && cols > 2048) return fail(CDL_ERR_UNSUPPORTED, "%s: h is given for rows of up to 2048 columns", op);
   CDL_CHECK(check_vec(op, "dscale", dscale, cols, CDL_F32, false));
   if (cols == 0 || rows == 0) return CDL_OK;
   if (rows > INT32_MAX) return fail(CDL_ERR_UNSUPPORTED, "%s: too many rows", op);
@@ -867,22 +940,21 @@ int32_t rmsnorm_bwd_execute(const cdl_tensor* x, const cdl_tensor* dy, const cdl
   // at 65536 rows 139 / 171 us against 147 us for the warp-per-row form without residual.
   const bool pipe = c <= 2048 && r >= 2 * sm_count() &&
                     (variant == CDL_NORM_AUTO || variant == CDL_NORM_PIPELINED);
-  ProfileScope ps(PROF_NORM_BWD, (res ? 8.0 : 6.0) * rows * cols + 6.0 * cols + 4.0 * rows, stream);
-  if (pipe) {
-    num_partials = sm_count();
-    int* status = device_status_ptr();
-    if (!status) return fail(CDL_ERR_CUDA, "cannot resolve the device status word");
-    if (c <= 256) launch_bwd_pipe<1>(x, dy, res, scale, r_inv, dx, partials, r, c, status, stream);
-    else if (c <= 512) launch_bwd_pipe<2>(x, dy, res, scale, r_inv, dx, partials, r, c, status, stream);
-    else if (c <= 1024) launch_bwd_pipe<4>(x, dy, res, scale, r_inv, dx, partials, r, c, status, stream);
-    else launch_bwd_pipe<8>(x, dy, res, scale, r_inv, dx, partials, r, c, status, stream);
-  } else if (c <= 256) launch_bwd<1, true>(x, dy, res, scale, r_inv, dx, partials, grid, r, c, stream);
-  else if (c <= 512) launch_bwd<2, true>(x, dy, res, scale, r_inv, dx, partials, grid, r, c, stream);
-  else if (c <= 1024) launch_bwd<4, true>(x, dy, res, scale, r_inv, dx, partials, grid, r, c, stream);
-  else if (c <= 2048) launch_bwd<8, true>(x, dy, res, scale, r_inv, dx, partials, grid, r, c, stream);
-  else {
-    if (c <= 4096) launch_bwd<16, false>(x, dy, res, scale, r_inv, dx, nullptr, grid, r, c, stream);
-    else launch_bwd<32, false>(x, dy, res, scale, r_inv, dx, nullptr, grid, r, c, stream);
+  ProfileScope ps(PROF_NORM_BWD, ((res ? 8.0 : 6.0) + (h ? 2.0 : 0.0)) * rows * cols + 6.0 * cols + 4.0 * rows, stream);
+  if (c <= 2048) {
+    int* status = nullptr;
+    if (pipe) {
+      num_partials = sm_count();
+      status = device_status_ptr();
+      if (!status) return fail(CDL_ERR_CUDA, "cannot resolve the device status word");
+    }
+    const Recomputed rec{h ? static_cast<__nv_bfloat16*>(h->ptr) : nullptr, h ? h->stride[0] : 0, eps};
+    if (h) launch_bwd_rows<true>(pipe, x, dy, res, scale, r_inv, dx, partials, grid, r, c, status, rec, stream);
+    else launch_bwd_rows<false>(pipe, x, dy, res, scale, r_inv, dx, partials, grid, r, c, status, rec, stream);
+  } else {
+    const Recomputed none{};
+    if (c <= 4096) launch_bwd<16, false, false>(x, dy, res, scale, r_inv, dx, nullptr, grid, r, c, none, stream);
+    else launch_bwd<32, false, false>(x, dy, res, scale, r_inv, dx, nullptr, grid, r, c, none, stream);
     num_partials = r < 256 ? r : 256;
     dim3 g((c + 127) / 128, num_partials);
     launch_pdl(dscale_cols_kernel, g, dim3(128), 0, stream,

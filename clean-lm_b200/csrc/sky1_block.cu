@@ -278,6 +278,7 @@ int32_t sky1_block_bwd(const cdl_sky1_config* cfg, const cdl_sky1_weights* wt, c
   const cdl_tensor wdownT = transposed(wdown), wupT = transposed(wup), wgateT = transposed(wgate);
   const cdl_tensor woT = transposed(wo), wqkvT = transposed(wqkv);
 
+  const bool with_h = d.Hd <= 2048;
   if (phase < 0 || phase > 2) return fail(CDL_ERR_INVALID, "sky1_block_bwd: phase must be 0, 1 or 2");
   // Weight-gradient products: the caller chooses between K slices that meet through f32 atomics
   // (default) and a fixed summation order.
@@ -295,14 +296,16 @@ int32_t sky1_block_bwd(const cdl_sky1_config* cfg, const cdl_sky1_weights* wt, c
   CDL_CHECK(mark(ev ? ev->wdown : nullptr));
   // d_act = dy Wdown^T never reaches memory: the epilogue turns it into d_up and d_gate
   CDL_CHECK(matmul_execute_epi(&tdy, &wdownT, nullptr, &tdact, 1.f, 0.f, 2, &tgate, &tup, &tdgate, st));
-  CDL_CHECK(rmsnorm_fwd_execute(&to, &g2, nullptr, cfg->eps, &th, &tr, st));        // recompute h2, r2
+  // h2 is not kept: the norm's backward gives it again (as a kernel of its own where the rows are too wide for that)
+  // ahead of the weight gradients that need it.
+  CDL_CHECK(matmul_execute(&tdact, &wupT, nullptr, &tdh, 1.f, 0.f, st));            // dh2 = d_up Wup^T
+  CDL_CHECK(matmul_execute(&tdgate, &wgateT, &tdh, &tdh, 1.f, 1.f, st));            // dh2 += d_gate Wgate^T
+  if (!with_h) CDL_CHECK(rmsnorm_fwd_execute(&to, &g2, nullptr, cfg->eps, &th, &tr, st));
+  CDL_CHECK(rmsnorm_bwd_execute(&to, &tdh, &tdy, &g2, &tr, &tdo, &dg2, b.norm_scratch, b.norm_scratch_bytes, st,
+                                nullptr, with_h ? &th : nullptr, cfg->eps));        // d_o (+ dy)
   CDL_CHECK(matmul_execute(&hT, &tdact, &gwup, &gwup, 1.f, 1.f, st, wg));               // dWup += h2^T d_up
   CDL_CHECK(mark(ev ? ev->wup : nullptr));
-  CDL_CHECK(matmul_execute(&tdact, &wupT, nullptr, &tdh, 1.f, 0.f, st));            // dh2 = d_up Wup^T
   CDL_CHECK(matmul_execute(&hT, &tdgate, &gwgate, &gwgate, 1.f, 1.f, st, wg));          // dWgate += h2^T d_gate
-  CDL_CHECK(matmul_execute(&tdgate, &wgateT, &tdh, &tdh, 1.f, 1.f, st));            // dh2 += d_gate Wgate^T
-  CDL_CHECK(rmsnorm_bwd_execute(&to, &tdh, &tdy, &g2, &tr, &tdo, &dg2, b.norm_scratch,
-                                b.norm_scratch_bytes, st));                         // d_o (+ dy)
   CDL_CHECK(mark(ev ? ev->wgate_norm2 : nullptr));
   }
   if (phase == 1) return CDL_OK;
@@ -335,11 +338,11 @@ int32_t sky1_block_bwd(const cdl_sky1_config* cfg, const cdl_sky1_weights* wt, c
     CDL_CHECK(attn_bwd_execute(&ad, &q, &k, &v, &ao, &dao, &lse, &dq, &dk, &dv, b.attn_scratch,
                                b.attn_scratch_bytes, st, &cs));
   }
-  CDL_CHECK(rmsnorm_fwd_execute(&tx, &g1, nullptr, cfg->eps, &th, &tr, st));        // recompute h1, r1
-  CDL_CHECK(matmul_execute(&hT, &tdqkv, &gwqkv, &gwqkv, 1.f, 1.f, st, wg));             // dWqkv += h1^T d_qkv
   CDL_CHECK(matmul_execute(&tdqkv, &wqkvT, nullptr, &tdh, 1.f, 0.f, st));           // dh1 = d_qkv Wqkv^T
-  CDL_CHECK(rmsnorm_bwd_execute(&tx, &tdh, &tdo, &g1, &tr, &tdx, &dg1, b.norm_scratch,
-                                b.norm_scratch_bytes, st));                         // dx (+ d_o)
+  if (!with_h) CDL_CHECK(rmsnorm_fwd_execute(&tx, &g1, nullptr, cfg->eps, &th, &tr, st));
+  CDL_CHECK(rmsnorm_bwd_execute(&tx, &tdh, &tdo, &g1, &tr, &tdx, &dg1, b.norm_scratch, b.norm_scratch_bytes, st,
+                                nullptr, with_h ? &th : nullptr, cfg->eps));        // dx (+ d_o)
+  CDL_CHECK(matmul_execute(&hT, &tdqkv, &gwqkv, &gwqkv, 1.f, 1.f, st, wg));             // dWqkv += h1^T d_qkv
   CDL_CHECK(mark(ev ? ev->wqkv_norm1 : nullptr));
   return CDL_OK;
 }

@@ -330,3 +330,29 @@ def test_rope_ragged_positions(cdl, gpu_ok):
         lo += n_tok
     assert torch.equal(xd[:, 2], x.cuda()[:, 2])      # the third head is not rotated
     assert torch.equal(xd[lo:], x.cuda()[lo:])        # padding rows are untouched
+
+
+@pytest.mark.parametrize("hidden", [264, 520, 1032, 2040, 2056])
+@pytest.mark.parametrize("seqlen", [95, 320])
+def test_block_widths_of_the_norm_backward(cdl, gpu_ok, hidden, seqlen):
+    """The norms' backward gives their forward outputs again for the weight gradients: a warp per row (95 rows) and
+    pipelined (320), rows of 1 to 8 shares of 256 columns, and rows too wide for it.  Against f64 on the device.
+    Weights of variance 1 / hidden keep every product near unit variance, so that the softmax amplifies no rounding: the
+    ten or so bf16 roundings in a chain, 2^-9 of the largest value each, stay below the bound."""
+    sky1 = cdl.sky1
+    cfg = sky1.Sky1Config(batch=1, seqlen=seqlen, hidden=hidden, heads=2, kv_heads=1, head_dim=128, ffn=264)
+    params = sky1.init_params(cfg, seed=hidden, std=hidden ** -0.5)
+    gen = torch.Generator().manual_seed(seqlen)
+    for n in ("norm1", "norm2"):
+        params[n] = (1 + 0.1 * torch.randn(hidden, generator=gen)).to(torch.bfloat16)
+    x, dy = (torch.randn(seqlen, hidden, generator=gen).to(torch.bfloat16).cuda() for _ in range(2))
+    blk = sky1.Sky1Block(cfg, params)
+    blk.forward(x)
+    dx = blk.backward(dy)
+    c = dict(heads=2, kv_heads=1, head_dim=128, eps=cfg.eps)
+    _, dx_ref, g_ref = block_ref.block_forward_backward(
+        x.view(1, seqlen, hidden), {k: v.cuda() for k, v in params.items()}, dy.view(1, seqlen, hidden), c,
+        block_ref.rope_table(seqlen, 128).cuda())
+    for name, got, ref in [("dx", dx, dx_ref.reshape(seqlen, hidden))] + [(n, blk.grads[n], g_ref[n]) for n in sky1.PARAM_NAMES]:
+        assert ((got.double() - ref).abs().max() / ref.abs().max()).item() <= 2e-2, name
+    assert cdl._lib.device_status() == 0
