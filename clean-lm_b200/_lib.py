@@ -154,6 +154,8 @@ SIGNATURES = {
     "cdl_b200_mx_layout": ([ctypes.c_int32, ctypes.c_int32, ctypes.c_int64, ctypes.c_int64,
                             ctypes.POINTER(_sz), ctypes.POINTER(_sz)], ctypes.c_int32),
     "cdl_b200_mx_quantize": ([_T, _MX, _MX, _vp], ctypes.c_int32),
+    "cdl_b200_mx_swiglu_fwd": ([_T, _T, _MX, _MX, _vp], ctypes.c_int32),
+    "cdl_b200_mx_swiglu_bwd": ([_T, _T, _T, _MX, _MX, _MX, _MX, _vp], ctypes.c_int32),
     "cdl_b200_mx_dequantize": ([_MX, _T, _vp], ctypes.c_int32),
     "cdl_b200_rmsnorm_fwd_mx": ([_T, _T, _T, ctypes.c_float, _MX, _MX, _T, _vp], ctypes.c_int32),
     "cdl_b200_matmul_mx": ([_MX, _MX, _T, _T, ctypes.c_float, ctypes.c_float, _vp], ctypes.c_int32),

@@ -75,10 +75,6 @@ __global__ void __launch_bounds__(256)
   *reinterpret_cast<uint4*>(p + half_dim) = pack8(ohi);
 }
 
-__device__ __forceinline__ float sigmoidf_fast(float x) {
-  return __frcp_rn(1.0f + __expf(-x));
-}
-
 // act = SiLU(gate) * up
 __global__ void __launch_bounds__(256)
     swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* __restrict__ up,
@@ -89,7 +85,7 @@ __global__ void __launch_bounds__(256)
   unpack8(ld_nc_v4(gate + idx * 8), g);
   unpack8(ld_nc_v4(up + idx * 8), u);
 #pragma unroll
-  for (int j = 0; j < 8; ++j) a[j] = g[j] * sigmoidf_fast(g[j]) * u[j];
+  for (int j = 0; j < 8; ++j) a[j] = g[j] * sigmoid_exp(g[j]) * u[j];
   *reinterpret_cast<uint4*>(act + idx * 8) = pack8(a);
 }
 
@@ -106,7 +102,7 @@ __global__ void __launch_bounds__(256)
   unpack8(ld_nc_v4(up + idx * 8), u);
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    const float s = sigmoidf_fast(g[j]);
+    const float s = sigmoid_exp(g[j]);
     du[j] = da[j] * g[j] * s;
     dg[j] = da[j] * u[j] * (s + g[j] * s * (1.0f - s));
   }

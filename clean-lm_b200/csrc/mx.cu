@@ -29,13 +29,12 @@
 //   mx_rows_kernel            any shape; with the colwise output 1024 columns at a time through
 //                             shared memory (rows too long for the kernels below, or a bias)
 //   mx_row_cached_kernel      rowwise only, cols <= 8192: the row stays in registers
-//   mx_rowcol_tile_kernel     both outputs, 32 whole rows (or 2048-column panels) in shared memory
+//   mx_rowcol_tile_kernel     the norm's both outputs, 32 whole rows in shared memory
 //   mx_row_full_kernel,       cols % 256 == 0 and no bias: the same two schemes trimmed of every
-//   mx_rowcol_full_kernel     operation the arithmetic does not need (these kernels are bound by
-//                             the ALU pipe, not by HBM)
-//   mx_rowcol_panel_kernel    both outputs by 512- / 1024-column panels, several CTAs per SM; with
-//                             the normalisation the panels of a row are a cluster that shares the
-//                             row sums through distributed shared memory (rows up to 8192)
+//   mx_rowcol_full_kernel     operation the arithmetic does not need
+//   mx_panel_kernel           both outputs by panels of 256 to 1024 columns: of x, of its norm (the panels of a
+//                             row are a cluster that shares the row sums through distributed shared
+//                             memory), of SwiGLU and of its gradients
 //   nvfp4_rows_kernel, nvfp4_row_full_kernel   the NVFP4 rowwise output, general and trimmed
 #include "host.h"
 #include "ops.h"
@@ -67,7 +66,12 @@ struct Params {
   uint8_t* row_sf;
   uint8_t* col_values;  // [cols, rows]; nullable
   uint8_t* col_sf;
-  int panel_cols;  // tile kernel: columns a CTA owns (blockIdx.y selects the panel); cols if one panel
+};
+// Further operands of mx_panel_kernel's SwiGLU sources.
+struct Extra {
+  const __nv_bfloat16* x[2];
+  long long ldx[2];
+  uint8_t *row_values, *row_sf, *col_values, *col_sf;  // the second output
 };
 
 __device__ __forceinline__ long long sf_index(int outer, int block, int blocks) {
@@ -290,6 +294,25 @@ __global__ void __launch_bounds__(256, NCH <= 4 ? 4 : NCH <= 8 ? 2 : 1) mx_row_c
 // CTAs of 256 threads per SM the trimmed rowwise kernels are compiled for: 3 (80 registers, 24
 // warps) measured 0.0253 ms at 16384 x 2048, 2 and 4 (spills at 64 registers) 0.0280 ms.
 constexpr int FULL_MIN_CTAS = 3;
+// Two f32 products with one instruction, then E4M3: the kernels with both outputs are bound by their instructions.
+__device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi) {
+  uint64_t v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+  return v;
+}
+__device__ __forceinline__ uint32_t fp8x2_scaled(float lo, float hi, uint64_t scale2) {
+  uint64_t v;
+  float a, b;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(pack_f32x2(lo, hi)), "l"(scale2));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+  return __nv_cvt_float2_to_fp8x2(make_float2(a, b), __NV_SATFINITE, __NV_E4M3);
+}
+// max(|a|, |b|) per half of packed bf16 pairs, with a sign that means nothing.
+__device__ __forceinline__ uint32_t max_abs_bf16x2(uint32_t a, uint32_t b) {
+  uint32_t m;
+  asm("max.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(m) : "r"(a), "r"(b));
+  return m;
+}
 // Packed bf16 pairs: |a| and max per half (exact: a maximum picks one of its operands).
 __device__ __forceinline__ uint32_t abs_max_bf16x2(uint32_t a, uint32_t b) {
   const __nv_bfloat162 m = __hmax2(__habs2(*reinterpret_cast<const __nv_bfloat162*>(&a)),
@@ -322,15 +345,16 @@ __device__ __forceinline__ void norm_packed8(const uint4& xq, float r, const flo
 // Rowwise quantisation of a lane's 8 packed bf16 values, a quarter of a 32-element block (all
 // four lanes of a block call): returns the 8 E4M3 bytes, e = the block's scale exponent.
 __device__ __forceinline__ uint2 quantize_packed8(const uint32_t (&q)[4], uint32_t& e) {
-  uint32_t m = max_bf16x2(abs_max_bf16x2(q[0], q[1]), abs_max_bf16x2(q[2], q[3]));
-  m = max_bf16x2(m, __shfl_xor_sync(0xffffffffu, m, 1));
-  m = max_bf16x2(m, __shfl_xor_sync(0xffffffffu, m, 2));
-  m = max_bf16x2(m, __byte_perm(m, 0, 0x1032));  // both halves: the block's amax
-  e = scale_exponent(__uint_as_float(m & 0xFFFF0000u));
+  uint32_t m = max_abs_bf16x2(max_abs_bf16x2(q[0], q[1]), max_abs_bf16x2(q[2], q[3]));
+  m = max_abs_bf16x2(m, __shfl_xor_sync(0xffffffffu, m, 1));
+  m = max_abs_bf16x2(m, __shfl_xor_sync(0xffffffffu, m, 2));
+  m = max_abs_bf16x2(m, __byte_perm(m, 0, 0x1032));  // both halves: the block's amax
+  e = scale_exponent(__uint_as_float(m & 0x7FFF0000u));
   const float ds = descale_of(e);
+  const uint64_t ds2 = pack_f32x2(ds, ds);
   uint2 o;
-  o.x = fp8x4(bf16_lo(q[0]) * ds, bf16_hi(q[0]) * ds, bf16_lo(q[1]) * ds, bf16_hi(q[1]) * ds);
-  o.y = fp8x4(bf16_lo(q[2]) * ds, bf16_hi(q[2]) * ds, bf16_lo(q[3]) * ds, bf16_hi(q[3]) * ds);
+  o.x = fp8x2_scaled(bf16_lo(q[0]), bf16_hi(q[0]), ds2) | (fp8x2_scaled(bf16_lo(q[1]), bf16_hi(q[1]), ds2) << 16);
+  o.y = fp8x2_scaled(bf16_lo(q[2]), bf16_hi(q[2]), ds2) | (fp8x2_scaled(bf16_lo(q[3]), bf16_hi(q[3]), ds2) << 16);
   return o;
 }
 // The scale vector as f32 in shared memory (all threads of the CTA call; ends with a barrier;
@@ -402,20 +426,16 @@ __global__ void __launch_bounds__(256, NCH <= 8 ? FULL_MIN_CTAS : 1) mx_row_full
   }
 }
 
-// Rowwise and colwise outputs, rows short enough for 32 of them to sit in shared memory
+// Rowwise and colwise outputs of the norm, rows short enough for 32 of them to sit in shared memory
 // (TILE [32][cols + 8] bf16): a CTA of 32 warps owns 32 rows.  A warp loads its row into the
 // tile while it sums the squares, replaces it by the bf16 result (writing the rowwise output on
 // the way), and after one barrier every thread quantises whole 32-row blocks of its columns.
-// x is read once; the colwise stores are one 32-byte sector per thread.
-template <bool NORM>
+// x is read once; the colwise stores are one 32-byte sector per thread.  For what mx_panel_kernel does not
+// take: a bias, or rows that no eight panels make up.
 __global__ void __launch_bounds__(1024, 1) mx_rowcol_tile_kernel(const Params p) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   __nv_bfloat16* tile = reinterpret_cast<__nv_bfloat16*>(smem_raw);
-  // Without the normalisation nothing couples the columns of a row, so wide matrices are cut
-  // into panels of panel_cols columns (blockIdx.y); with it there is one panel, the whole row.
-  const int pc0 = blockIdx.y * p.panel_cols;
-  const int pcols = min(p.panel_cols, p.cols - pc0);
-  const int ld = p.panel_cols + 8;
+  const int ld = p.cols + 8;
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int row_blocks = p.cols / BLOCK;
@@ -424,45 +444,38 @@ __global__ void __launch_bounds__(1024, 1) mx_rowcol_tile_kernel(const Params p)
   for (long long row0 = static_cast<long long>(blockIdx.x) * 32; row0 < p.rows;
        row0 += static_cast<long long>(gridDim.x) * 32) {
     const long long row = row0 + warp;  // rows % 32 == 0: always a real row
-    const __nv_bfloat16* xr = p.x + row * p.ldx + pc0;
+    const __nv_bfloat16* xr = p.x + row * p.ldx;
     __nv_bfloat16* trow = tile + warp * ld;
     float ss = 0.f;
-    for (int c = lane * 8; c < pcols; c += 256) {
+    for (int c = lane * 8; c < p.cols; c += 256) {
       const uint4 q = ld_nc_v4(xr + c);
       *reinterpret_cast<uint4*>(trow + c) = q;
-      if (NORM) {
-        float f[8];
-        unpack8(q, f);
+      float f[8];
+      unpack8(q, f);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) ss = fmaf(f[j], f[j], ss);
-      }
+      for (int j = 0; j < 8; ++j) ss = fmaf(f[j], f[j], ss);
     }
-    float r = 1.0f;
-    if (NORM) {
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-      r = rsqrtf(ss * inv_cols + p.eps);
-      if (lane == 0 && p.r_inv != nullptr) p.r_inv[row * p.r_inv_stride] = r;
-    }
-    for (int c0 = 0; c0 < pcols; c0 += 256) {  // warp-uniform
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    const float r = rsqrtf(ss * inv_cols + p.eps);
+    if (lane == 0 && p.r_inv != nullptr) p.r_inv[row * p.r_inv_stride] = r;
+    for (int c0 = 0; c0 < p.cols; c0 += 256) {  // warp-uniform
       const int c = c0 + lane * 8;
-      const bool active = c < pcols;
+      const bool active = c < p.cols;
       float f[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) f[j] = 0.f;
       if (active) {
-        apply_norm8<NORM>(p, *reinterpret_cast<const uint4*>(trow + c), pc0 + c, r, f);
-        if (NORM) {
-          uint4 q;
-          q.x = pack_rounded(f[0], f[1]); q.y = pack_rounded(f[2], f[3]);
-          q.z = pack_rounded(f[4], f[5]); q.w = pack_rounded(f[6], f[7]);
-          *reinterpret_cast<uint4*>(trow + c) = q;
-        }
+        apply_norm8<true>(p, *reinterpret_cast<const uint4*>(trow + c), c, r, f);
+        uint4 q;
+        q.x = pack_rounded(f[0], f[1]); q.y = pack_rounded(f[2], f[3]);
+        q.z = pack_rounded(f[4], f[5]); q.w = pack_rounded(f[6], f[7]);
+        *reinterpret_cast<uint4*>(trow + c) = q;
       }
-      if (p.row_values != nullptr) quantize_row8(p, f, active, row, pc0 + c, lane, row_blocks);
+      if (p.row_values != nullptr) quantize_row8(p, f, active, row, c, lane, row_blocks);
     }
     __syncthreads();
-    for (int c = threadIdx.x; c < pcols; c += 1024) {
+    for (int c = threadIdx.x; c < p.cols; c += 1024) {
       float v[32];
       float amax = 0.f;
 #pragma unroll
@@ -476,8 +489,8 @@ __global__ void __launch_bounds__(1024, 1) mx_rowcol_tile_kernel(const Params p)
 #pragma unroll
       for (int j = 0; j < 8; ++j)
         w[j] = fp8x4(v[4 * j] * ds, v[4 * j + 1] * ds, v[4 * j + 2] * ds, v[4 * j + 3] * ds);
-      st_global_v8(p.col_values + static_cast<long long>(pc0 + c) * p.rows + row0, w);
-      p.col_sf[sf_index(pc0 + c, static_cast<int>(row0 / BLOCK), col_blocks)] = static_cast<uint8_t>(e);
+      st_global_v8(p.col_values + static_cast<long long>(c) * p.rows + row0, w);
+      p.col_sf[sf_index(c, static_cast<int>(row0 / BLOCK), col_blocks)] = static_cast<uint8_t>(e);
     }
     __syncthreads();
   }
@@ -486,107 +499,91 @@ __global__ void __launch_bounds__(1024, 1) mx_rowcol_tile_kernel(const Params p)
 // Colwise quantisation of columns pc0 + 2 c2 and pc0 + 2 c2 + 1 of a staged tile of 32 rows
 // (ld bf16 per row): one 32-bit load brings a pair, the maximum over the rows runs on the pairs,
 // and each column leaves as one 32-byte sector of the transposed output.
-__device__ __forceinline__ void quantize_column_pair(const Params& p, const __nv_bfloat16* tile, int ld,
-                                                     int c2, int pc0, long long row0, int col_blocks) {
+__device__ __forceinline__ void quantize_column_pair(uint8_t* values, uint8_t* sf, int rows, const __nv_bfloat16* tile,
+                                                     int ld, int c2, int pc0, long long row0) {
   const uint32_t* tp = reinterpret_cast<const uint32_t*>(tile) + c2;
   const int ldw = ld >> 1;
   uint32_t w[32];
 #pragma unroll
   for (int j = 0; j < 32; ++j) w[j] = tp[j * ldw];
-  uint32_t m = abs_max_bf16x2(w[0], w[1]);
+  uint32_t m = max_abs_bf16x2(w[0], w[1]);
 #pragma unroll
-  for (int j = 2; j < 32; j += 2) m = max_bf16x2(m, abs_max_bf16x2(w[j], w[j + 1]));
-  const uint32_t e_lo = scale_exponent(__uint_as_float(m << 16));
-  const uint32_t e_hi = scale_exponent(__uint_as_float(m & 0xFFFF0000u));
+  for (int j = 2; j < 32; j += 2) m = max_abs_bf16x2(m, max_abs_bf16x2(w[j], w[j + 1]));
+  const uint32_t e_lo = scale_exponent(__uint_as_float((m << 16) & 0x7FFF0000u));
+  const uint32_t e_hi = scale_exponent(__uint_as_float(m & 0x7FFF0000u));
   const float ds_lo = descale_of(e_lo), ds_hi = descale_of(e_hi);
+  const uint64_t lo2 = pack_f32x2(ds_lo, ds_lo), hi2 = pack_f32x2(ds_hi, ds_hi);
   uint32_t o_lo[8], o_hi[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    o_lo[j] = fp8x4(bf16_lo(w[4 * j]) * ds_lo, bf16_lo(w[4 * j + 1]) * ds_lo,
-                    bf16_lo(w[4 * j + 2]) * ds_lo, bf16_lo(w[4 * j + 3]) * ds_lo);
-    o_hi[j] = fp8x4(bf16_hi(w[4 * j]) * ds_hi, bf16_hi(w[4 * j + 1]) * ds_hi,
-                    bf16_hi(w[4 * j + 2]) * ds_hi, bf16_hi(w[4 * j + 3]) * ds_hi);
+    o_lo[j] = fp8x2_scaled(bf16_lo(w[4 * j]), bf16_lo(w[4 * j + 1]), lo2) |
+              (fp8x2_scaled(bf16_lo(w[4 * j + 2]), bf16_lo(w[4 * j + 3]), lo2) << 16);
+    o_hi[j] = fp8x2_scaled(bf16_hi(w[4 * j]), bf16_hi(w[4 * j + 1]), hi2) |
+              (fp8x2_scaled(bf16_hi(w[4 * j + 2]), bf16_hi(w[4 * j + 3]), hi2) << 16);
   }
   const int col = pc0 + 2 * c2;
-  uint8_t* dst = p.col_values + static_cast<long long>(col) * p.rows + row0;
+  uint8_t* dst = values + static_cast<long long>(col) * rows + row0;
   st_global_v8(dst, o_lo);
-  st_global_v8(dst + p.rows, o_hi);
+  st_global_v8(dst + rows, o_hi);
   // col is even: the next column's scale sits 16 bytes on (same 128-column tile)
-  uint8_t* csf = p.col_sf + sf_index(col, static_cast<int>(row0 / BLOCK), col_blocks);
+  uint8_t* csf = sf + sf_index(col, static_cast<int>(row0 / BLOCK), rows / BLOCK);
   csf[0] = static_cast<uint8_t>(e_lo);
   csf[16] = static_cast<uint8_t>(e_hi);
 }
 
-// mx_rowcol_tile_kernel for panels whose width is a multiple of 256 and no bias, trimmed like
-// mx_row_full_kernel (packed block maxima, f32 scale vector in shared memory behind the tile, no
-// idle lanes, index arithmetic hoisted out of the stripes).  The colwise phase takes two columns
-// per thread: one 32-bit shared-memory load brings a bf16 pair, the maximum over the 32 rows runs
-// on the pairs, and each column still leaves as one 32-byte sector.
-template <bool NORM>
+// mx_rowcol_tile_kernel for cols % 256 == 0 and no bias, trimmed like mx_row_full_kernel (packed block maxima, f32 scale
+// vector in shared memory behind the tile, no idle lanes, index arithmetic hoisted out of the stripes).
 __global__ void __launch_bounds__(1024, 1) mx_rowcol_full_kernel(const Params p) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   __nv_bfloat16* tile = reinterpret_cast<__nv_bfloat16*>(smem_raw);
-  const int ld = p.panel_cols + 8;
+  const int ld = p.cols + 8;
   float4* s_gamma = reinterpret_cast<float4*>(smem_raw + static_cast<size_t>(64) * ld);
-  const int pc0 = blockIdx.y * p.panel_cols;
-  const int pcols = min(p.panel_cols, p.cols - pc0);
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int row_tiles = (p.cols / BLOCK + 3) >> 2;
-  const int col_blocks = p.rows / BLOCK;
   const float inv_cols = 1.0f / static_cast<float>(p.cols);
-  const bool has_gamma = NORM && p.gamma != nullptr;
-  if (has_gamma) stage_gamma(p.gamma, p.cols, s_gamma);  // with NORM the panel is the whole row
-  // Block of (stripe at column c0, lane): b = (pc0 + c0) / 32 + lane / 4, the first term a multiple of 8.
+  const bool has_gamma = p.gamma != nullptr;
+  if (has_gamma) stage_gamma(p.gamma, p.cols, s_gamma);
+  // Block of (stripe at column c0, lane): b = c0 / 32 + lane / 4, the first term a multiple of 8.
   const int sf_lane = (lane >> 4) * 512 + ((lane >> 2) & 3);
   const bool rowwise = p.row_values != nullptr;
   for (long long row0 = static_cast<long long>(blockIdx.x) * 32; row0 < p.rows;
        row0 += static_cast<long long>(gridDim.x) * 32) {
     const long long row = row0 + warp;  // rows % 32 == 0: always a real row
-    const __nv_bfloat16* xr = p.x + row * p.ldx + pc0;
+    const __nv_bfloat16* xr = p.x + row * p.ldx;
     __nv_bfloat16* trow = tile + warp * ld;
     float ss = 0.f;
-    for (int c = lane * 8; c < pcols; c += 256) {
+    for (int c = lane * 8; c < p.cols; c += 256) {
       const uint4 q = ld_nc_v4(xr + c);
       *reinterpret_cast<uint4*>(trow + c) = q;
-      if (NORM) {
-        float f[8];
-        unpack8(q, f);
+      float f[8];
+      unpack8(q, f);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) ss = fmaf(f[j], f[j], ss);
-      }
+      for (int j = 0; j < 8; ++j) ss = fmaf(f[j], f[j], ss);
     }
-    float r = 1.0f;
-    if (NORM) {
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-      r = rsqrtf(ss * inv_cols + p.eps);
-      if (lane == 0 && p.r_inv != nullptr) p.r_inv[row * p.r_inv_stride] = r;
-    }
-    if (NORM || rowwise) {
-      uint8_t* out = rowwise ? p.row_values + row * p.cols + pc0 + lane * 8 : nullptr;
-      uint8_t* sf = rowwise ? p.row_sf + ((row >> 7) * row_tiles + (pc0 >> 7)) * 512 +
-                                  (row & 31) * 16 + ((row & 127) >> 5) * 4 + sf_lane
-                            : nullptr;
-      for (int c0 = 0; c0 < pcols; c0 += 256) {
-        const int c = c0 + lane * 8;
-        const uint4 xq = *reinterpret_cast<const uint4*>(trow + c);
-        uint32_t q[4] = {xq.x, xq.y, xq.z, xq.w};
-        if (NORM) {
-          norm_packed8(xq, r, has_gamma ? s_gamma + (c0 >> 2) + lane : nullptr, q);
-          *reinterpret_cast<uint4*>(trow + c) = make_uint4(q[0], q[1], q[2], q[3]);
-        }
-        if (rowwise) {  // CTA-uniform: the shuffles see whole warps
-          uint32_t e;
-          const uint2 o = quantize_packed8(q, e);
-          *reinterpret_cast<uint2*>(out + c0) = o;
-          if ((lane & 3) == 0) sf[(c0 >> 7) * 512] = static_cast<uint8_t>(e);
-        }
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    const float r = rsqrtf(ss * inv_cols + p.eps);
+    if (lane == 0 && p.r_inv != nullptr) p.r_inv[row * p.r_inv_stride] = r;
+    uint8_t* out = rowwise ? p.row_values + row * p.cols + lane * 8 : nullptr;
+    uint8_t* sf = rowwise ? p.row_sf + (row >> 7) * row_tiles * 512 + (row & 31) * 16 + ((row & 127) >> 5) * 4 + sf_lane
+                          : nullptr;
+    for (int c0 = 0; c0 < p.cols; c0 += 256) {
+      const int c = c0 + lane * 8;
+      const uint4 xq = *reinterpret_cast<const uint4*>(trow + c);
+      uint32_t q[4];
+      norm_packed8(xq, r, has_gamma ? s_gamma + (c0 >> 2) + lane : nullptr, q);
+      *reinterpret_cast<uint4*>(trow + c) = make_uint4(q[0], q[1], q[2], q[3]);
+      if (rowwise) {  // CTA-uniform: the shuffles see whole warps
+        uint32_t e;
+        const uint2 o = quantize_packed8(q, e);
+        *reinterpret_cast<uint2*>(out + c0) = o;
+        if ((lane & 3) == 0) sf[(c0 >> 7) * 512] = static_cast<uint8_t>(e);
       }
     }
     __syncthreads();
-    for (int c2 = threadIdx.x; c2 < pcols / 2; c2 += 1024)
-      quantize_column_pair(p, tile, ld, c2, pc0, row0, col_blocks);
+    for (int c2 = threadIdx.x; c2 < p.cols / 2; c2 += 1024)
+      quantize_column_pair(p.col_values, p.col_sf, p.rows, tile, ld, c2, 0, row0);
     __syncthreads();
   }
 }
@@ -595,97 +592,192 @@ __device__ __forceinline__ void st_shared_cluster_f32(uint32_t cluster_addr, flo
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(cluster_addr), "f"(v) : "memory");
 }
 
-// Rowwise and colwise outputs by panels of W = panel_cols columns (512 or 1024, cols % W == 0,
-// no bias): CTA (blockIdx.x, blockIdx.y) owns rows [32 y, +32) x columns [W x, +W) with W / 2
-// threads, so that several CTAs share an SM and one's loads run under another's arithmetic (the
-// whole-row kernels above hold one CTA per SM and leave half of the issue slots idle), and the
-// last wave of CTAs is short.  With NORM the CTAs of a row of panels form a cluster (at most 8):
-// each sums the squares of its part of the 32 rows, writes the 32 partial sums into every
-// member's shared memory, and after one cluster barrier all of them add the parts in rank order,
-// so that every member normalises with the same bits.
-template <bool NORM>
-__global__ void __launch_bounds__(512, 2) mx_rowcol_panel_kernel(const Params p) {
+// Rowwise and colwise outputs by panels: a CTA of W / 2 threads owns 32 rows x W columns, a lane 8 neighbouring
+// columns of 8 (row, 256-column chunk) units.  What is quantised is
+//   PLAIN       x
+//   NORM        x r gamma; the panels of a row (at most 8) are a cluster: each sums the squares of its part
+//               of the 32 rows, writes the 32 partial sums into every member's shared memory, and after a cluster
+//               barrier all add the parts in rank order, so that every member normalises with the same bits
+//   SWIGLU      bf16(SiLU(gate) up)                                    x = gate, extra.x = {up}
+//   SWIGLU_BWD  the two gradients of that, d_up and d_gate, in bf16    x = gate, extra.x = {up, d_act}
+// (the values that the stand-alone kernels of elem.cu store: the SwiGLU tensors never exist in HBM).
+// Bound by the issue of instructions (17 per element at 2.2 per clock and SM for PLAIN), at 0.8 of the copy rate: panels rather
+// than whole rows let two CTAs share an SM, so that one loads while the other quantises.  Both ways, us before
+// (32 whole rows per CTA) -> panels: [16384, 5632] 91.9 -> 69.0 (5.35 TB/s), [16384, 2048] 33.0 -> 26.8;
+// SwiGLU [16384, 5632] with its quantisations, as separate kernels -> here: forward 188 -> 130, backward 329 -> 240.
+enum Source { PLAIN, NORM, SWIGLU, SWIGLU_BWD };
+constexpr int panel_outputs(int src) { return src == SWIGLU_BWD ? 2 : 1; }
+constexpr int panel_inputs(int src) { return src == SWIGLU_BWD ? 3 : src == SWIGLU ? 2 : 1; }
+constexpr size_t panel_smem(int w, int src) {
+  return static_cast<size_t>(panel_outputs(src)) * 64 * (w + 8) + (src == NORM ? 8 * 32 * 4 : 0);
+}
+constexpr int panel_ctas(int w, int src) { return (src == SWIGLU_BWD || src == NORM ? 3 : 4) * 512 / w; }
+
+template <int W, int SRC>
+__global__ void __launch_bounds__(W / 2, panel_ctas(W, SRC)) mx_panel_kernel(const Params p, const Extra x) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
-  const int W = p.panel_cols;
-  const int ld = W + 8;
-  __nv_bfloat16* tile = reinterpret_cast<__nv_bfloat16*>(smem_raw);
-  float4* s_gamma = reinterpret_cast<float4*>(smem_raw + static_cast<size_t>(64) * ld);  // [W] f32
-  float* s_ss = reinterpret_cast<float*>(s_gamma + W / 4);                               // [8][32]
-  const int pc0 = blockIdx.x * W;
-  const long long row0 = static_cast<long long>(blockIdx.y) * 32;
-  const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
-  const int warps = blockDim.x >> 5;
+  constexpr int LD = W + 8, CHUNKS = W / 256, WARPS = W / 64, UNITS = 8;
+  constexpr int IN = panel_inputs(SRC), OUT = panel_outputs(SRC);
+  constexpr int BATCH = SRC == SWIGLU_BWD ? 2 : SRC == SWIGLU ? 4 : 8;  // units whose loads are in flight together
+  __nv_bfloat16* tile = reinterpret_cast<__nv_bfloat16*>(smem_raw);    // [OUT][32][LD]
+  float* s_ss = reinterpret_cast<float*>(smem_raw + OUT * 64 * LD);    // NORM: [8][32]
+  const int panels = (p.cols + W - 1) / W;
+  const int panel = static_cast<int>(blockIdx.x) % panels;
+  const long long row0 = static_cast<long long>(static_cast<int>(blockIdx.x) / panels) * 32;
+  const int pc0 = panel * W;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int row_tiles = (p.cols / BLOCK + 3) >> 2;
-  const int col_blocks = p.rows / BLOCK;
-  const bool has_gamma = NORM && p.gamma != nullptr;
-  const bool rowwise = p.row_values != nullptr;
-  const uint32_t rank = NORM ? cluster_ctarank() : 0;
-  const uint32_t members = NORM ? gridDim.x : 1;
-  if (has_gamma) stage_gamma(p.gamma + pc0, W, s_gamma);
-  // A member's shared memory may be written only once that member runs: every CTA of the cluster
-  // passes this barrier before the first remote store.
-  if (NORM) cluster_sync_all();
+  grid_dep_wait();
+  grid_dep_launch();
 
-  for (int rr = warp; rr < 32; rr += warps) {
-    const __nv_bfloat16* xr = p.x + (row0 + rr) * p.ldx + pc0;
-    __nv_bfloat16* trow = tile + rr * ld;
-    float ss = 0.f;
-    for (int c = lane * 8; c < W; c += 256) {
-      const uint4 q = ld_nc_v4(xr + c);
-      *reinterpret_cast<uint4*>(trow + c) = q;
-      if (NORM) {
-        float f[8];
-        unpack8(q, f);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) ss = fmaf(f[j], f[j], ss);
+  // This lane's place in the outputs of the tile's first row and chunk.  Blocks of (chunk at column c0, lane):
+  // (pc0 + c0) / 32 + lane / 4, the first term a multiple of 8; the tile's 32 rows are one group of a scale tile.
+  const long long to_values = row0 * p.cols + pc0 + lane * 8;
+  const long long to_sf = ((row0 >> 7) * row_tiles + (pc0 >> 7) + (lane >> 4)) * 512 + ((row0 & 127) >> 5) * 4 + ((lane >> 2) & 3);
+  __nv_bfloat16* const to_tile = tile + lane * 8;
+  // A lane's 8 columns of one unit: bf16 results q of output o to the tile, and the rowwise output.
+  auto emit = [&](int o, int rr, int c0, const uint32_t (&q)[4]) {
+    *reinterpret_cast<uint4*>(to_tile + (o * 32 + rr) * LD + c0) = make_uint4(q[0], q[1], q[2], q[3]);
+    uint8_t* values = o ? x.row_values : p.row_values;
+    if (values != nullptr) {  // uniform: the shuffles see whole warps; cols % 32 == 0, so the lanes of a block agree
+      uint32_t e;
+      const uint2 v = quantize_packed8(q, e);
+      if (pc0 + c0 + lane * 8 < p.cols) {
+        *reinterpret_cast<uint2*>(values + to_values + (rr * p.cols + c0)) = v;
+        if ((lane & 3) == 0) ((o ? x.row_sf : p.row_sf) + to_sf)[rr * 16 + c0 * 4] = static_cast<uint8_t>(e);
       }
     }
-    if (NORM) {
+  };
+  auto unit_row = [&](int u) { return warp + WARPS * (u / CHUNKS); };
+  auto unit_col = [&](int u) { return (u % CHUNKS) * 256; };
+  const __nv_bfloat16* src[IN];  // this lane's place in the inputs of the tile's first row and chunk
+  long long ld[IN];
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-      if (lane < members)
-        st_shared_cluster_f32(mapa_shared(smem_u32(s_ss + rank * 32 + rr), lane), ss);
-    }
+  for (int k = 0; k < IN; ++k) {
+    ld[k] = k == 0 ? p.ldx : x.ldx[k > 0 ? k - 1 : 0];
+    src[k] = (k == 0 ? p.x : x.x[k > 0 ? k - 1 : 0]) + row0 * ld[k] + pc0 + lane * 8;
   }
-  if (NORM) cluster_sync_all();  // every member's partial sums have landed; nothing remote after this
 
-  const int sf_lane = (lane >> 4) * 512 + ((lane >> 2) & 3);
-  if (NORM || rowwise) {
-    for (int rr = warp; rr < 32; rr += warps) {
-      const long long row = row0 + rr;
-      __nv_bfloat16* trow = tile + rr * ld;
-      float r = 1.0f;
-      if (NORM) {
+#pragma unroll
+  for (int u0 = 0; u0 < UNITS; u0 += BATCH) {
+    uint4 v[BATCH][IN];
+#pragma unroll
+    for (int i = 0; i < BATCH; ++i) {
+      const int col = pc0 + unit_col(u0 + i) + lane * 8;
+#pragma unroll
+      for (int k = 0; k < IN; ++k)
+        v[i][k] = col < p.cols ? ld_nc_v4(src[k] + unit_row(u0 + i) * ld[k] + unit_col(u0 + i)) : make_uint4(0, 0, 0, 0);
+    }
+    if constexpr (SRC == NORM) {
+      // A member's shared memory may be written only once that member runs.
+      cluster_sync_all();
+      const uint32_t rank = cluster_ctarank();
+#pragma unroll
+      for (int rw = 0; rw < UNITS / CHUNKS; ++rw) {
         float ss = 0.f;
-        for (uint32_t k = 0; k < members; ++k) ss += s_ss[k * 32 + rr];
-        r = rsqrtf(ss * (1.0f / static_cast<float>(p.cols)) + p.eps);
-        if (rank == 0 && lane == 0 && p.r_inv != nullptr) p.r_inv[row * p.r_inv_stride] = r;
-      }
-      uint8_t* out = rowwise ? p.row_values + row * p.cols + pc0 + lane * 8 : nullptr;
-      uint8_t* sf = rowwise ? p.row_sf + ((row >> 7) * row_tiles + (pc0 >> 7)) * 512 +
-                                  (row & 31) * 16 + ((row & 127) >> 5) * 4 + sf_lane
-                            : nullptr;
-      for (int c0 = 0; c0 < W; c0 += 256) {
-        const int c = c0 + lane * 8;
-        const uint4 xq = *reinterpret_cast<const uint4*>(trow + c);
-        uint32_t q[4] = {xq.x, xq.y, xq.z, xq.w};
-        if (NORM) {
-          norm_packed8(xq, r, has_gamma ? s_gamma + (c0 >> 2) + lane : nullptr, q);
-          *reinterpret_cast<uint4*>(trow + c) = make_uint4(q[0], q[1], q[2], q[3]);
+#pragma unroll
+        for (int c = 0; c < CHUNKS; ++c) {
+          float f[8];
+          unpack8(v[rw * CHUNKS + c][0], f);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) ss = fmaf(f[j], f[j], ss);
         }
-        if (rowwise) {  // CTA-uniform: the shuffles see whole warps
-          uint32_t e;
-          const uint2 o = quantize_packed8(q, e);
-          *reinterpret_cast<uint2*>(out + c0) = o;
-          if ((lane & 3) == 0) sf[(c0 >> 7) * 512] = static_cast<uint8_t>(e);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        if (lane < panels)
+          st_shared_cluster_f32(mapa_shared(smem_u32(s_ss + rank * 32 + warp + WARPS * rw), lane), ss);
+      }
+      cluster_sync_all();  // every member's partial sums have landed; nothing remote after this
+      uint4 gamma[CHUNKS];
+#pragma unroll
+      for (int c = 0; c < CHUNKS; ++c)
+        if (p.gamma != nullptr) gamma[c] = ld_nc_v4(p.gamma + pc0 + c * 256 + lane * 8);
+#pragma unroll
+      for (int rw = 0; rw < UNITS / CHUNKS; ++rw) {
+        const int rr = warp + WARPS * rw;
+        float ss = 0.f;
+        for (int k = 0; k < panels; ++k) ss += s_ss[k * 32 + rr];
+        const float r = rsqrtf(ss * (1.0f / static_cast<float>(p.cols)) + p.eps);
+        if (panel == 0 && lane == 0 && p.r_inv != nullptr) p.r_inv[(row0 + rr) * p.r_inv_stride] = r;
+#pragma unroll
+        for (int c = 0; c < CHUNKS; ++c) {
+          float f[8], g[8];
+          unpack8(v[rw * CHUNKS + c][0], f);
+          if (p.gamma != nullptr) unpack8(gamma[c], g);
+          uint32_t q[4];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) f[j] = p.gamma != nullptr ? f[j] * r * g[j] : f[j] * r;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) q[j] = pack_bf16x2(f[2 * j], f[2 * j + 1]);
+          emit(0, rr, c * 256, q);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < BATCH; ++i) {
+        const int rr = unit_row(u0 + i), c0 = unit_col(u0 + i);
+        if constexpr (SRC == PLAIN) {
+          const uint32_t q[4] = {v[i][0].x, v[i][0].y, v[i][0].z, v[i][0].w};
+          emit(0, rr, c0, q);
+        } else {
+          float g[8], up[8], o0[8];
+          uint32_t q[4];
+          unpack8(v[i][0], g);
+          unpack8(v[i][1], up);
+          if constexpr (SRC == SWIGLU) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) o0[j] = g[j] * sigmoid_exp(g[j]) * up[j];
+          } else {
+            float da[8], o1[8];
+            unpack8(v[i][2], da);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const float sg = sigmoid_exp(g[j]);
+              o0[j] = da[j] * g[j] * sg;
+              o1[j] = da[j] * up[j] * (sg + g[j] * sg * (1.0f - sg));
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) q[j] = pack_bf16x2(o1[2 * j], o1[2 * j + 1]);
+            emit(1, rr, c0, q);
+          }
+#pragma unroll
+          for (int j = 0; j < 4; ++j) q[j] = pack_bf16x2(o0[2 * j], o0[2 * j + 1]);
+          emit(0, rr, c0, q);
         }
       }
     }
   }
   __syncthreads();
-  for (int c2 = threadIdx.x; c2 < W / 2; c2 += blockDim.x)
-    quantize_column_pair(p, tile, ld, c2, pc0, row0, col_blocks);
+  const int c2 = threadIdx.x;
+  if (pc0 + 2 * c2 < p.cols) {
+#pragma unroll
+    for (int o = 0; o < OUT; ++o)
+      quantize_column_pair(o ? x.col_values : p.col_values, o ? x.col_sf : p.col_sf, p.rows, tile + o * 32 * LD, LD, c2, pc0,
+                           row0);
+  }
+}
+
+template <int W, int SRC>
+static int32_t launch_panels(const Params& p, const Extra& x, cudaStream_t stream) {
+  static std::once_flag once[64];
+  int dev = 0;
+  CDL_CUDA(cudaGetDevice(&dev));
+  cudaError_t err = cudaSuccess;
+  std::call_once(once[dev & 63], [&] {
+    err = cudaFuncSetAttribute(mx_panel_kernel<W, SRC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               static_cast<int>(panel_smem(W, SRC)));
+  });
+  if (err != cudaSuccess) return fail(CDL_ERR_CUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(err));
+  const int panels = (p.cols + W - 1) / W;
+  CDL_CUDA(launch_pdl_cluster(mx_panel_kernel<W, SRC>, dim3(static_cast<unsigned>(p.rows / 32) * panels), dim3(W / 2),
+                              panel_smem(W, SRC), SRC == NORM ? panels : 1, stream, p, x));
+  return CDL_OK;
+}
+// Panels of 512 columns unless they leave a part of the last one idle that 256 columns would not, or SMs without work.
+template <int SRC>
+static int32_t launch_panels(const Params& p, const Extra& x, cudaStream_t stream) {
+  const bool narrow = (p.cols + 255) / 256 % 2 != 0 || static_cast<long long>(p.rows / 32) * (p.cols / 512) < 2 * sm_count();
+  return narrow ? launch_panels<256, SRC>(p, x, stream) : launch_panels<512, SRC>(p, x, stream);
 }
 
 // NVFP4 rowwise output (NormOutput::Nvfp4Rowwise, no global scale): blocks of 16 elements, scale
@@ -976,72 +1068,36 @@ static int32_t mx_rows_run(const char* op, const cdl_tensor* x, const cdl_tensor
     else nvfp4_rows_kernel<false><<<grid, 256, 0, stream>>>(p);
 #undef CDL_FP4_FULL
   } else if (y_col) {
+    if (!norm) return launch_panels<PLAIN>(p, Extra{}, stream);
+    // The norm: whole rows, where 32 of them fit a CTA's shared memory and there is work for two SMs in three (4096 x 2048
+    // 13 us, by panels 18); else panels that make up the row in a cluster of at most 8 (1024 x 2048 7.7 us, whole
+    // rows 11.6).
+    const size_t tile_bytes = 32 * static_cast<size_t>(cols + 8) * 2, gamma_bytes = scale ? static_cast<size_t>(cols) * 4 : 0;
+    const bool full = cols % 256 == 0 && !bias && tile_bytes + gamma_bytes <= 227 * 1024;
+    if (!bias && !(full && rows / 32 * 3 >= 2 * sm_count())) {
+      if (cols % 256 == 0 && cols <= 2048 && (cols % 512 != 0 || rows / 32 * (cols / 512) < 2 * sm_count()))
+        return launch_panels<256, NORM>(p, Extra{}, stream);
+      if (cols % 512 == 0 && cols <= 4096) return launch_panels<512, NORM>(p, Extra{}, stream);
+      if (cols % 1024 == 0 && cols <= 8192) return launch_panels<1024, NORM>(p, Extra{}, stream);
+    }
     int dev = 0;
     CDL_CUDA(cudaGetDevice(&dev));
-    const size_t tile_bytes = 32 * static_cast<size_t>(cols + 8) * 2;
-    const size_t gamma_bytes = norm && scale ? static_cast<size_t>(cols) * 4 : 0;
-    const bool whole_rows = tile_bytes <= 227 * 1024;
-    // panels a multiple of 256 columns wide and no bias: the trimmed kernel
-    const bool full = cols % 256 == 0 && !(norm && bias) &&
-                      (!whole_rows || tile_bytes + gamma_bytes <= 227 * 1024);
     static std::once_flag once[64];
     cudaError_t err = cudaSuccess;
     std::call_once(once[dev & 63], [&] {
-      const void* fns[8] = {reinterpret_cast<const void*>(&mx_rows_kernel<true, true>),
-                            reinterpret_cast<const void*>(&mx_rows_kernel<false, true>),
-                            reinterpret_cast<const void*>(&mx_rowcol_tile_kernel<true>),
-                            reinterpret_cast<const void*>(&mx_rowcol_tile_kernel<false>),
-                            reinterpret_cast<const void*>(&mx_rowcol_full_kernel<true>),
-                            reinterpret_cast<const void*>(&mx_rowcol_full_kernel<false>),
-                            reinterpret_cast<const void*>(&mx_rowcol_panel_kernel<true>),
-                            reinterpret_cast<const void*>(&mx_rowcol_panel_kernel<false>)};
-      for (int i = 0; i < 8 && err == cudaSuccess; ++i)
-        err = cudaFuncSetAttribute(fns[i], cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   i < 2 ? static_cast<int>(COL_SMEM_BYTES) : 227 * 1024);
+      err = cudaFuncSetAttribute(mx_rows_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(COL_SMEM_BYTES));
+      if (err == cudaSuccess)
+        err = cudaFuncSetAttribute(mx_rowcol_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+      if (err == cudaSuccess)
+        err = cudaFuncSetAttribute(mx_rowcol_full_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     });
     if (err != cudaSuccess)
       return fail(CDL_ERR_CUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(err));
     const unsigned grid = static_cast<unsigned>(rows / 32);
-    // Panels of 1024 (else 512) columns when they tile the row: every plain quantisation, and the
-    // normalisation of rows too long for 32 of them to sit in one CTA's shared memory (the panels
-    // of a row then form a cluster, which holds at most 8 CTAs; rows that fit measured the same
-    // either way and stay with the whole-row kernel).
-    const int panel = cols % 1024 == 0 ? 1024 : cols % 512 == 0 ? 512 : 0;
-    const bool use_panels = panel != 0 && rows / 32 <= 65535 &&
-                            (!norm || (!bias && cols / panel <= 8 && !(whole_rows && full)));
-    if (use_panels) {
-      p.panel_cols = panel;
-      const size_t smem = 64 * static_cast<size_t>(panel + 8) + static_cast<size_t>(panel) * 4 + 8 * 32 * 4;
-      cudaLaunchConfig_t cfg{};
-      cfg.gridDim = dim3(static_cast<unsigned>(cols / panel), grid);
-      cfg.blockDim = dim3(static_cast<unsigned>(panel / 2));
-      cfg.dynamicSmemBytes = smem;
-      cfg.stream = stream;
-      cudaLaunchAttribute attr{};
-      attr.id = cudaLaunchAttributeClusterDimension;
-      attr.val.clusterDim.x = norm ? static_cast<unsigned>(cols / panel) : 1;
-      attr.val.clusterDim.y = 1;
-      attr.val.clusterDim.z = 1;
-      cfg.attrs = &attr;
-      cfg.numAttrs = 1;
-      if (norm) CDL_CUDA(cudaLaunchKernelEx(&cfg, mx_rowcol_panel_kernel<true>, p));
-      else CDL_CUDA(cudaLaunchKernelEx(&cfg, mx_rowcol_panel_kernel<false>, p));
-    } else if (whole_rows) {
-      p.panel_cols = static_cast<int>(cols);
-      if (full && norm) mx_rowcol_full_kernel<true><<<grid, 1024, tile_bytes + gamma_bytes, stream>>>(p);
-      else if (full) mx_rowcol_full_kernel<false><<<grid, 1024, tile_bytes, stream>>>(p);
-      else if (norm) mx_rowcol_tile_kernel<true><<<grid, 1024, tile_bytes, stream>>>(p);
-      else mx_rowcol_tile_kernel<false><<<grid, 1024, tile_bytes, stream>>>(p);
-    } else if (!norm) {
-      // plain quantisation of wide rows: panels of 2048 columns (a multiple of the 256-column stripe)
-      p.panel_cols = 2048;
-      const dim3 g2(grid, static_cast<unsigned>((cols + 2047) / 2048));
-      if (full) mx_rowcol_full_kernel<false><<<g2, 1024, 32 * (2048 + 8) * 2, stream>>>(p);
-      else mx_rowcol_tile_kernel<false><<<g2, 1024, 32 * (2048 + 8) * 2, stream>>>(p);
-    } else {
-      if (norm) mx_rows_kernel<true, true><<<grid, 1024, COL_SMEM_BYTES, stream>>>(p);
-      else mx_rows_kernel<false, true><<<grid, 1024, COL_SMEM_BYTES, stream>>>(p);
-    }
+    if (full) mx_rowcol_full_kernel<<<grid, 1024, tile_bytes + gamma_bytes, stream>>>(p);
+    else if (tile_bytes <= 227 * 1024) mx_rowcol_tile_kernel<<<grid, 1024, tile_bytes, stream>>>(p);
+    else mx_rows_kernel<true, true><<<grid, 1024, COL_SMEM_BYTES, stream>>>(p);
   } else {
     const long long want = (rows + 7) / 8;
     const unsigned grid = static_cast<unsigned>(want < 16LL * sm_count() ? want : 16LL * sm_count());
@@ -1098,6 +1154,56 @@ int32_t mx_quantize_execute(const cdl_tensor* x, const cdl_mx_tensor* y_row,
   return mx_rows_run("mx_quantize", x, nullptr, nullptr, 0.f, false, y_row, y_col, nullptr, stream);
 }
 
+// SwiGLU and the two-way quantisation of its results in one pass (mx_panel_kernel); d_act null: the forward.
+static int32_t mx_swiglu_run(const char* op, const cdl_tensor* d_act, const cdl_tensor* gate, const cdl_tensor* up,
+                             const cdl_mx_tensor* y0_row, const cdl_mx_tensor* y0_col, const cdl_mx_tensor* y1_row,
+                             const cdl_mx_tensor* y1_col, cudaStream_t stream) {
+  using namespace mx;
+  const bool bwd = d_act != nullptr;
+  if (!gate || !up) return fail(CDL_ERR_INVALID, "%s: gate and up are required", op);
+  if (gate->rank != 2) return fail(CDL_ERR_INVALID, "%s: gate must be a 2D tensor", op);
+  const long long rows = gate->shape[0], cols = gate->shape[1];
+  for (const cdl_tensor* t : {gate, up, d_act}) {
+    if (!t) continue;
+    if (t->rank != 2 || t->shape[0] != rows || t->shape[1] != cols || t->dtype != CDL_BF16)
+      return fail(CDL_ERR_INVALID, "%s: the inputs must be bf16 [%lld, %lld]", op, rows, cols);
+    if ((cols > 1 && t->stride[1] != 1) || (reinterpret_cast<uintptr_t>(t->ptr) & 15) != 0 ||
+        (rows > 1 && t->stride[0] % 8 != 0))
+      return fail(CDL_ERR_UNSUPPORTED, "%s: the inputs must have packed, 16-byte aligned rows", op);
+  }
+  const cdl_mx_tensor* outs[4] = {y0_row, y0_col, y1_row, y1_col};
+  for (int i = 0; i < (bwd ? 4 : 2); ++i) {
+    if (!outs[i]) return fail(CDL_ERR_INVALID, "%s: all outputs are required", op);
+    if (outs[i]->format != CDL_MXFP8) return fail(CDL_ERR_UNSUPPORTED, "%s: the outputs must be MXFP8", op);
+    CDL_CHECK(mx_check(op, "output", outs[i], i % 2 ? CDL_MX_COLWISE : CDL_MX_ROWWISE, rows, cols));
+  }
+  if (rows == 0 || cols == 0) return CDL_OK;
+  if (rows > INT32_MAX / 2 || cols > 65536)
+    return fail(CDL_ERR_UNSUPPORTED, "%s: shape [%lld, %lld] is too large", op, rows, cols);
+  Params p{};
+  p.x = static_cast<const __nv_bfloat16*>(gate->ptr);
+  p.ldx = gate->stride[0];
+  p.rows = static_cast<int>(rows);
+  p.cols = static_cast<int>(cols);
+  p.row_values = static_cast<uint8_t*>(y0_row->values);
+  p.row_sf = static_cast<uint8_t*>(y0_row->scale_factors);
+  p.col_values = static_cast<uint8_t*>(y0_col->values);
+  p.col_sf = static_cast<uint8_t*>(y0_col->scale_factors);
+  Extra x{};
+  x.x[0] = static_cast<const __nv_bfloat16*>(up->ptr);
+  x.ldx[0] = up->stride[0];
+  if (bwd) {
+    x.x[1] = static_cast<const __nv_bfloat16*>(d_act->ptr);
+    x.ldx[1] = d_act->stride[0];
+    x.row_values = static_cast<uint8_t*>(y1_row->values);
+    x.row_sf = static_cast<uint8_t*>(y1_row->scale_factors);
+    x.col_values = static_cast<uint8_t*>(y1_col->values);
+    x.col_sf = static_cast<uint8_t*>(y1_col->scale_factors);
+  }
+  ProfileScope ps(PROF_ELEMENTWISE, static_cast<double>(rows) * cols * (bwd ? 6.0 + 4.125 : 4.0 + 2.0625), stream);
+  return bwd ? launch_panels<SWIGLU_BWD>(p, x, stream) : launch_panels<SWIGLU>(p, x, stream);
+}
+
 int32_t mx_dequantize_execute(const cdl_mx_tensor* x, const cdl_tensor* y, cudaStream_t stream) {
   const char* op = "mx_dequantize";
   if (!x || !y) return fail(CDL_ERR_INVALID, "%s: x and y are required", op);
@@ -1133,6 +1239,21 @@ int32_t cdl_b200_mx_layout(int32_t format, int32_t dim, int64_t rows, int64_t co
 int32_t cdl_b200_mx_quantize(const cdl_tensor* x, const cdl_mx_tensor* y_rowwise,
                              const cdl_mx_tensor* y_colwise, cdl_stream stream) {
   return cdl::mx_quantize_execute(x, y_rowwise, y_colwise, static_cast<cudaStream_t>(stream));
+}
+
+int32_t cdl_b200_mx_swiglu_fwd(const cdl_tensor* gate, const cdl_tensor* up, const cdl_mx_tensor* act_rowwise,
+                               const cdl_mx_tensor* act_colwise, cdl_stream stream) {
+  return cdl::mx_swiglu_run("mx_swiglu_fwd", nullptr, gate, up, act_rowwise, act_colwise, nullptr, nullptr,
+                            static_cast<cudaStream_t>(stream));
+}
+
+int32_t cdl_b200_mx_swiglu_bwd(const cdl_tensor* d_act, const cdl_tensor* gate, const cdl_tensor* up,
+                               const cdl_mx_tensor* d_gate_rowwise, const cdl_mx_tensor* d_gate_colwise,
+                               const cdl_mx_tensor* d_up_rowwise, const cdl_mx_tensor* d_up_colwise,
+                               cdl_stream stream) {
+  if (!d_act) return cdl::fail(CDL_ERR_INVALID, "mx_swiglu_bwd: d_act is required");
+  return cdl::mx_swiglu_run("mx_swiglu_bwd", d_act, gate, up, d_up_rowwise, d_up_colwise, d_gate_rowwise,
+                            d_gate_colwise, static_cast<cudaStream_t>(stream));
 }
 
 int32_t cdl_b200_mx_dequantize(const cdl_mx_tensor* x, const cdl_tensor* y, cdl_stream stream) {

@@ -528,6 +528,8 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
 __device__ __forceinline__ float bf16_lo(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t v) { return __uint_as_float(v & 0xFFFF0000u); }
 
+__device__ __forceinline__ float sigmoid_exp(float x) { return __frcp_rn(1.0f + __expf(-x)); }
+
 // 256-bit global accesses (sm_100): one full 32-byte sector per thread per instruction.  The
 // address must be 32-byte aligned.
 __device__ __forceinline__ void ld_global_v8(const void* p, uint32_t (&r)[8]) {

@@ -83,6 +83,19 @@ def quantize(x: torch.Tensor, rowwise: bool = True, colwise: bool = False, fmt: 
     return yr, yc
 
 
+def swiglu_fwd(gate: torch.Tensor, up: torch.Tensor, out) -> None:
+    """MXFP8 (rowwise, colwise) `out` = SiLU(gate) * up, rounded to bf16 in between."""
+    tg, tu, ar, ac = tensor_arg(gate), tensor_arg(up), out[0].arg(), out[1].arg()
+    check(lib.cdl_b200_mx_swiglu_fwd(ref(tg), ref(tu), ref(ar), ref(ac), current_stream()))
+
+
+def swiglu_bwd(d_act: torch.Tensor, gate: torch.Tensor, up: torch.Tensor, d_gate, d_up) -> None:
+    """The gradients of SwiGLU in the same form: `d_gate` and `d_up` are (rowwise, colwise) pairs."""
+    ts = [tensor_arg(t) for t in (d_act, gate, up)]
+    outs = [t.arg() for t in (*d_gate, *d_up)]
+    check(lib.cdl_b200_mx_swiglu_bwd(*(ref(t) for t in ts), *(ref(t) for t in outs), current_stream()))
+
+
 def dequantize(t: MxTensor, dtype: torch.dtype = torch.float32) -> torch.Tensor:
     y = torch.empty(t.rows, t.cols, dtype=dtype, device=t.values.device)
     a, ty = t.arg(), tensor_arg(y)

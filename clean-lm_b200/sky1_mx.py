@@ -13,8 +13,9 @@ Which quantisation a product needs (blocks run along its contraction dimension):
   dgrad     dX[T,K] = dY[T,N] . W^T[N,K]      dY rowwise,           W^T colwise = W rowwise, transposed view
   wgrad     dW[K,N] = X^T[K,T] . dY[T,N]      X^T rowwise = X colwise, transposed view;  dY colwise
 Weights are quantised both ways once per optimizer step (`requantize_weights`), activations and
-gradients once where they are produced.  Experimental: numerics are those of MXFP8, not of the
-bf16 block; tests hold it to the bf16 block within the format's error.
+gradients once where they are produced (SwiGLU and its gradients leave as MXFP8 only).
+Experimental: numerics are those of MXFP8, not of the bf16 block; tests hold it to the bf16 block
+within the format's error.
 """
 from __future__ import annotations
 
@@ -40,8 +41,8 @@ class Sky1BlockMX:
         bf = dict(dtype=torch.bfloat16, device=device)
         self.buf = {
             "qkv": torch.empty(t, q, **bf), "attn": torch.empty(t, hd, **bf), "o": torch.empty(t, h, **bf),
-            "up": torch.empty(t, f, **bf), "gate": torch.empty(t, f, **bf), "act": torch.empty(t, f, **bf),
-            "d_act": torch.empty(t, f, **bf), "d_gate": torch.empty(t, f, **bf), "dh": torch.empty(t, h, **bf),
+            "up": torch.empty(t, f, **bf), "gate": torch.empty(t, f, **bf),
+            "d_act": torch.empty(t, f, **bf), "dh": torch.empty(t, h, **bf),
             "d_o": torch.empty(t, h, **bf), "d_attn": torch.empty(t, hd, **bf), "d_qkv": torch.empty(t, q, **bf),
         }
         self.r_inv = {1: torch.empty(t, dtype=torch.float32, device=device),
@@ -111,9 +112,8 @@ class Sky1BlockMX:
                             out=mx.NormMxOutputs(*self.q["h2"], self.r_inv[2]))
         self._fwd(n2.y, self.wq["wup"], b["up"])
         self._fwd(n2.y, self.wq["wgate"], b["gate"])
-        tg, tu, ta = tensor_arg(b["gate"]), tensor_arg(b["up"]), tensor_arg(b["act"])
-        check(lib.cdl_b200_swiglu_fwd(ref(tg), ref(tu), ref(ta), current_stream()))
-        qact = self._quant("act", b["act"])
+        qact = self.q["act"]
+        mx.swiglu_fwd(b["gate"], b["up"], qact)
         self._fwd(qact[0], self.wq["wdown"], out, c=b["o"])                # out = act Wdown + o
         return out
 
@@ -123,9 +123,8 @@ class Sky1BlockMX:
         qdy = self._quant("dy", dy)
         self._wgrad(self.q["act"][1], qdy[1], g["wdown"])
         self._dgrad(qdy[0], self.wq["wdown"], b["d_act"])
-        targs = [tensor_arg(t) for t in (b["d_act"], b["gate"], b["up"], b["d_gate"], b["d_act"])]
-        check(lib.cdl_b200_swiglu_bwd(*(ref(a) for a in targs), current_stream()))   # d_up over d_act
-        qdu, qdg = self._quant("d_up", b["d_act"]), self._quant("d_gate", b["d_gate"])
+        qdu, qdg = self.q["d_up"], self.q["d_gate"]
+        mx.swiglu_bwd(b["d_act"], b["gate"], b["up"], qdg, qdu)
         self._wgrad(self.q["h2"][1], qdu[1], g["wup"])
         self._wgrad(self.q["h2"][1], qdg[1], g["wgate"])
         self._dgrad(qdu[0], self.wq["wup"], b["dh"])

@@ -273,6 +273,16 @@ int32_t cdl_b200_mx_layout(int32_t format, int32_t dim, int64_t rows, int64_t co
  * to even, saturating; zeros when the scale rounds to zero (block_scale.rs:28-31, 55-66). */
 int32_t cdl_b200_mx_quantize(const cdl_tensor* x, const cdl_mx_tensor* y_rowwise,
                              const cdl_mx_tensor* y_colwise, cdl_stream stream);
+/* SwiGLU with block-scaled results, the elementwise step between a block's MXFP8 products: the bf16 values that
+ * cdl_b200_swiglu_fwd / _bwd store, quantised both ways as by cdl_b200_mx_quantize, without the tensors in
+ * between.  gate, up, d_act: bf16 [rows, cols] with packed, 16-byte aligned rows; outputs MXFP8
+ * (rows % 32 == 0, cols % 32 == 0), all required. */
+int32_t cdl_b200_mx_swiglu_fwd(const cdl_tensor* gate, const cdl_tensor* up, const cdl_mx_tensor* act_rowwise,
+                               const cdl_mx_tensor* act_colwise, cdl_stream stream);
+int32_t cdl_b200_mx_swiglu_bwd(const cdl_tensor* d_act, const cdl_tensor* gate, const cdl_tensor* up,
+                               const cdl_mx_tensor* d_gate_rowwise, const cdl_mx_tensor* d_gate_colwise,
+                               const cdl_mx_tensor* d_up_rowwise, const cdl_mx_tensor* d_up_colwise,
+                               cdl_stream stream);
 
 /* y (bf16 or f32 [rows, cols], packed rows) = values * scale.  A test and debugging aid. */
 int32_t cdl_b200_mx_dequantize(const cdl_mx_tensor* x, const cdl_tensor* y, cdl_stream stream);

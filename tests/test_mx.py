@@ -535,3 +535,30 @@ def test_matmul_mx_with_c(cdl, gpu_ok, fmt):
     expected = acc.double().numpy() + 2.0 * prod
     assert_all_close("in place", to_f32(d), expected,
                      oracle.matmul_tolerance(expected, 2.0 * bound + np.abs(acc.double().numpy()), False))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,cols", [(32, 32), (64, 96), (128, 256), (96, 288), (160, 544), (64, 2816), (2048, 5632)])
+def test_swiglu_with_quantised_results(cdl, gpu_ok, rows, cols):
+    """SwiGLU and its gradients as MXFP8, both ways, in one pass: the bits of the stand-alone kernels followed by the
+    quantiser.  Inputs include rows of a wider buffer, large and infinite values."""
+    L = cdl._lib
+    gen = torch.Generator(device="cuda").manual_seed(rows + cols)
+    d_act, gate, up = (torch.randn(rows, cols + 8, generator=gen, device="cuda").to(torch.bfloat16)[:, :cols] for _ in range(3))
+    gate[3, 5], up[7, 9], d_act[1, 2], gate[2] = 1e30, float("inf"), -1e38, -200.0
+    packed = [t.contiguous() for t in (d_act, gate, up)]
+    act, d_gate, d_up = (torch.empty_like(packed[0]) for _ in range(3))
+    args = [L.tensor_arg(t) for t in (*packed, act, d_gate, d_up)]
+    L.check(L.lib.cdl_b200_swiglu_fwd(L.ref(args[1]), L.ref(args[2]), L.ref(args[3]), None))
+    L.check(L.lib.cdl_b200_swiglu_bwd(*(L.ref(args[i]) for i in (0, 1, 2, 4, 5)), None))
+
+    def pair():
+        return tuple(cdl.mx.MxTensor.empty(rows, cols, dim, zero_scales=True) for dim in (cdl.mx.ROWWISE, cdl.mx.COLWISE))
+
+    got_act, got_gate, got_up = pair(), pair(), pair()
+    cdl.mx.swiglu_fwd(gate, up, got_act)
+    cdl.mx.swiglu_bwd(d_act, gate, up, got_gate, got_up)
+    for got, plain in ((got_act, act), (got_gate, d_gate), (got_up, d_up)):
+        for g, e in zip(got, cdl.mx.quantize(plain, rowwise=True, colwise=True)):
+            assert torch.equal(g.values, e.values) and torch.equal(g.scale_factors, e.scale_factors)
+    assert L.device_status() == 0
