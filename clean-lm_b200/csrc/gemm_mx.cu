@@ -25,6 +25,7 @@
 // [496,508)).  The epilogue of a tile drains the 16 shared columns first and signals; the first
 // MMA of the next tile waits for that signal only, so the rest of the epilogue still overlaps
 // the next tile's main loop.
+#include "gemm_rows.cuh"
 #include "host.h"
 #include "ops.h"
 #include "ptx.cuh"
@@ -312,6 +313,8 @@ __global__ void __launch_bounds__(THREADS, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
+  grid_dep_wait();  // set-up above overlaps the previous kernel's tail; global memory from here on
+  grid_dep_launch();
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
@@ -497,16 +500,18 @@ __global__ void __launch_bounds__(THREADS, 1)
 // barrier; tcgen05.cp.cta_group::2 then moves them into both CTAs' tensor memory, each from its
 // own shared memory.  The rest is the protocol of the bf16 pair kernel: the leader issues every
 // MMA and commits to both CTAs' barriers, the peer's epilogue warps arrive remotely.
-template <int FP4>
+// ADD: D += alpha * accumulator in f32 by TMA reductions (add_chunk), whose buffers take a stage's room.
+template <int FP4, bool ADD>
 struct PairCfg {
   static constexpr int SFT = Cfg<FP4>::SFT;
   static constexpr int HALF_B_BYTES = B_BYTES / 2;
   static constexpr int SF_OFF = A_BYTES + HALF_B_BYTES;
   static constexpr int SF_BYTES = 3 * SFT * SF_TILE;
   static constexpr int STAGE_BYTES = SF_OFF + (FP4 ? 6 : 2) * 1024;  // 34 / 38 KiB, 1024-aligned
-  static constexpr int STAGES = FP4 ? 5 : 6;
+  static constexpr int STAGES = FP4 || ADD ? 5 : 6;
+  static constexpr int STAGING = ADD ? EPI_WARPS * gemm::CHUNK_BYTES : 0;
   static constexpr int TX_BYTES = A_BYTES + HALF_B_BYTES + SF_BYTES;  // per CTA and stage
-  static constexpr size_t SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + 256;
+  static constexpr size_t SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + STAGING + 256;
   static_assert(SF_OFF + SF_BYTES <= STAGE_BYTES, "stage layout");
   static_assert(SMEM_BYTES <= 232448, "exceeds the 227 KiB of shared memory a CTA can opt in to");
 };
@@ -521,21 +526,23 @@ struct PairBarriers {
   int abort_word;
 };
 
-template <int FP4>
+template <int FP4, bool ADD>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
     gemm_mx_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
                         const __grid_constant__ CUtensorMap tmap_b,
                         const __grid_constant__ CUtensorMap tmap_sfa,
-                        const __grid_constant__ CUtensorMap tmap_sfb, const Params p) {
+                        const __grid_constant__ CUtensorMap tmap_sfb,
+                        const __grid_constant__ CUtensorMap tmap_d, const Params p) {
   using C = Cfg<FP4>;
-  using PC = PairCfg<FP4>;
+  using PC = PairCfg<FP4, ADD>;
   constexpr int STAGE_BYTES = PC::STAGE_BYTES;
   constexpr int NSTAGES = PC::STAGES;
   constexpr int SFT = C::SFT;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
-  PairBarriers* bars = reinterpret_cast<PairBarriers*>(smem + NSTAGES * STAGE_BYTES);
+  uint8_t* staging = smem + NSTAGES * STAGE_BYTES;
+  PairBarriers* bars = reinterpret_cast<PairBarriers*>(staging + PC::STAGING);
   volatile int* abort_word = &bars->abort_word;
 
   const int warp = threadIdx.x >> 5;
@@ -572,6 +579,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
   cluster_sync_all();  // both CTAs' barriers exist before anything signals across the pair
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
+  grid_dep_wait();  // set-up above overlaps the previous kernel's tail; global memory from here on
+  grid_dep_launch();
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer (both CTAs)
@@ -691,7 +700,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
       const bool backwards = owner && acc == 0;
       auto emit = [&](const uint32_t (&r)[32], int ch) {
         const int col0 = col_base + ch * 32;
-        if (p.out_mx == 0) {
+        if (ADD) {
+          if (row - lane >= p.M || col0 >= p.N) return;  // warp-uniform; what lies outside D in a box is clipped
+          uint8_t* buf = staging + (warp - 2) * gemm::CHUNK_BYTES;
+          if (lane == 0) tma_store_wait_read<0>();  // the buffer's last reduction has read it
+          __syncwarp();
+          gemm::add_chunk(&tmap_d, buf, r, p.alpha, lane, col0, row - lane, 0);
+        } else if (p.out_mx == 0) {
           if (row < p.M && col0 < p.N) store32(p, r, row, col0);
         } else if (col0 < p.N) {
           if (p.out_mx == 2) store32_nvfp4(p, r, row, col0);
@@ -724,6 +739,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&bars->acc_empty[acc]), 0));
     }
+    if (ADD && lane == 0) tma_store_wait<0>();
   }
 
   // ------------------------------------------------------------ tear-down
@@ -817,14 +833,14 @@ static int32_t matmul_mx_run(const char* op, const cdl_mx_tensor* a, const cdl_m
     if (attr_err == cudaSuccess)
       attr_err = cudaFuncSetAttribute(gemm_mx_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       static_cast<int>(Cfg<1>::SMEM_BYTES));
-    if (attr_err == cudaSuccess)
-      attr_err = cudaFuncSetAttribute(gemm_mx_pair_kernel<0>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(PairCfg<0>::SMEM_BYTES));
-    if (attr_err == cudaSuccess)
-      attr_err = cudaFuncSetAttribute(gemm_mx_pair_kernel<1>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(PairCfg<1>::SMEM_BYTES));
+    auto pair = [&](auto kernel, size_t bytes) {
+      if (attr_err == cudaSuccess)
+        attr_err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+    };
+    pair(gemm_mx_pair_kernel<0, false>, PairCfg<0, false>::SMEM_BYTES);
+    pair(gemm_mx_pair_kernel<1, false>, PairCfg<1, false>::SMEM_BYTES);
+    pair(gemm_mx_pair_kernel<0, true>, PairCfg<0, true>::SMEM_BYTES);
+    pair(gemm_mx_pair_kernel<1, true>, PairCfg<1, true>::SMEM_BYTES);
   });
   if (attr_err != cudaSuccess)
     return fail(CDL_ERR_CUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(attr_err));
@@ -903,14 +919,27 @@ static int32_t matmul_mx_run(const char* op, const cdl_mx_tensor* a, const cdl_m
     CDL_CHECK(sf_map(&tsb, b->scale_factors, N));
     int grid = 2 * p.num_tiles < sm_count() ? 2 * p.num_tiles : sm_count();
     grid &= ~1;
-    if (fp4)
-      gemm_mx_pair_kernel<1><<<grid, THREADS, PairCfg<1>::SMEM_BYTES, stream>>>(ta, tbh, tsa, tsb, p);
-    else
-      gemm_mx_pair_kernel<0><<<grid, THREADS, PairCfg<0>::SMEM_BYTES, stream>>>(ta, tbh, tsa, tsb, p);
+    // D += alpha * A . B by TMA reductions, where they can describe D: every element is added to once.
+    CUtensorMap td = ta;  // (a valid map where none is used)
+    const bool add = p.c_mode == 2 && p.out_f32 && p.c == p.d && beta == 1.f && p.ldc == p.ldd &&
+                     (reinterpret_cast<uintptr_t>(p.d) & 15) == 0 && p.ldd % 4 == 0 && p.ldd >= N;
+    if (add) {
+      const uint64_t dims[3] = {static_cast<uint64_t>(N), static_cast<uint64_t>(M), 1};
+      const uint64_t strides[3] = {0, static_cast<uint64_t>(p.ldd) * 4, static_cast<uint64_t>(p.ldd) * 4 * M};
+      const uint32_t box[3] = {32, 32, 1};
+      CDL_CHECK(encode_tmap(&td, p.d, CDL_F32, 3, dims, strides, box, true));
+    }
+    auto launch = [&](auto kernel, size_t smem) {
+      return launch_pdl(kernel, dim3(static_cast<unsigned>(grid)), dim3(THREADS), smem, stream, ta, tbh, tsa, tsb, td, p);
+    };
+    if (fp4) CDL_CUDA(add ? launch(gemm_mx_pair_kernel<1, true>, PairCfg<1, true>::SMEM_BYTES)
+                          : launch(gemm_mx_pair_kernel<1, false>, PairCfg<1, false>::SMEM_BYTES));
+    else CDL_CUDA(add ? launch(gemm_mx_pair_kernel<0, true>, PairCfg<0, true>::SMEM_BYTES)
+                      : launch(gemm_mx_pair_kernel<0, false>, PairCfg<0, false>::SMEM_BYTES));
   } else {
-    const int grid = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
-    if (fp4) gemm_mx_kernel<1><<<grid, THREADS, Cfg<1>::SMEM_BYTES, stream>>>(ta, tb, p);
-    else gemm_mx_kernel<0><<<grid, THREADS, Cfg<0>::SMEM_BYTES, stream>>>(ta, tb, p);
+    const unsigned grid = static_cast<unsigned>(p.num_tiles < sm_count() ? p.num_tiles : sm_count());
+    if (fp4) CDL_CUDA(launch_pdl(gemm_mx_kernel<1>, dim3(grid), dim3(THREADS), Cfg<1>::SMEM_BYTES, stream, ta, tb, p));
+    else CDL_CUDA(launch_pdl(gemm_mx_kernel<0>, dim3(grid), dim3(THREADS), Cfg<0>::SMEM_BYTES, stream, ta, tb, p));
   }
   CDL_CUDA(cudaGetLastError());
   return CDL_OK;

@@ -139,8 +139,8 @@ class Sky1BlockMX:
         ops.attention_bwd(self._q, self._k, self._v, b["attn"].view(cfg.batch, cfg.seqlen, h, cfg.head_dim),
                           b["d_attn"].view(cfg.batch, cfg.seqlen, h, cfg.head_dim), self.lse,
                           ops.AttentionOpts(causal=True), scratch=self.attn_scratch,
-                          dq=dqv[:, :, :h], dk=dqv[:, :, h:h + kv], dv=dqv[:, :, h + kv:])
-        self._rope(b["d_qkv"], 1)
+                          dq=dqv[:, :, :h], dk=dqv[:, :, h:h + kv], dv=dqv[:, :, h + kv:],
+                          rope_table=self.table)  # d_q and d_k leave rotated back
         qdq = self._quant("d_qkv", b["d_qkv"])
         self._wgrad(self.q["h1"][1], qdq[1], g["wqkv"])
         self._dgrad(qdq[0], self.wq["wqkv"], b["dh"])

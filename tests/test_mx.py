@@ -562,3 +562,26 @@ def test_swiglu_with_quantised_results(cdl, gpu_ok, rows, cols):
         for g, e in zip(got, cdl.mx.quantize(plain, rowwise=True, colwise=True)):
             assert torch.equal(g.values, e.values) and torch.equal(g.scale_factors, e.scale_factors)
     assert L.device_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fmt", ["mxfp8", "nvfp4"])
+@pytest.mark.parametrize("m,k,n,pad", [(130, 64, 36, 0), (257, 128, 264, 4), (512, 192, 2100, 0), (2048, 4096, 1030, 6)])
+def test_matmul_mx_adds_in_place(cdl, gpu_ok, fmt, m, k, n, pad):
+    """D += alpha A . B in f32 by the pair kernel: rows and columns that end inside a 32 x 32 chunk, D a view of a wider
+    buffer (pad 6: off the 16-byte grid, the other way of adding), against the same product without C, whose addition is
+    rounded once.  What lies outside D keeps its values, a repetition gives the same bits."""
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    f = cdl.mx.NVFP4 if fmt == "nvfp4" else cdl.mx.MXFP8
+    a, b = (torch.randn(r, k, generator=gen, device="cuda").to(torch.bfloat16) for r in (m, n))
+    qa, qb = (cdl.mx.quantize(t, rowwise=True, fmt=f)[0] for t in (a, b))
+    qb = qb.transposed()
+    buf = torch.randn(m + 2, (n + 3) // 4 * 4 + pad, generator=gen, device="cuda")
+    prod = cdl.mx.matmul_mx(qa, qb, out_dtype=torch.float32, alpha=-0.5)
+    expected = buf.clone()
+    expected[:m, :n] += prod
+    for _ in range(2):
+        out = buf.clone()
+        cdl.mx.matmul_mx(qa, qb, out=out[:m, :n], c=out[:m, :n], alpha=-0.5, beta=1.0)
+        assert torch.equal(out, expected)
+    assert cdl._lib.device_status() == 0
