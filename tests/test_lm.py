@@ -203,3 +203,33 @@ def test_lm_config5_full_size_loss_curve_10_steps(cdl, gpu_ok):
     assert np.isfinite(losses).all()
     assert (np.abs(losses - ref) / ref).max() <= 1e-2, (losses, ref)
     assert np.abs(losses - ref).max() <= 0.03, (losses, ref)
+
+
+@pytest.mark.parametrize("vocab", [8, 4104, 8192, 8200, 16384, 16392, 32768])
+def test_cross_entropy_row_forms(cdl, gpu_ok, vocab):
+    """Rows held in registers (up to 16384) and read twice, edges of a thread's share, rows of a wider buffer, masked
+    (-inf) and lowest finite logits, ignored targets.  Bounds: f32 sums of the exponentials, the bf16 gradient."""
+    L = cdl._lib
+    gen = torch.Generator(device="cuda").manual_seed(vocab)
+    rows = 37
+    buf = (torch.randn(rows, vocab + 16, generator=gen, device="cuda") * 4).to(torch.bfloat16)
+    logits = buf[:, :vocab]
+    if vocab <= 32768:
+        logits[3, 1:] = float("-inf")
+        logits[4, ::2] = torch.finfo(torch.bfloat16).min
+        logits[5, 0] = 1e4
+    targets = torch.randint(0, vocab, (rows,), generator=gen, device="cuda", dtype=torch.int32)
+    targets[0], targets[1], targets[2], targets[3], targets[4] = -1, vocab, vocab - 1, 0, 1
+    x = logits.double()
+    tail, loss = buf[:, vocab:].clone(), torch.empty(rows, device="cuda")
+    args = [L.tensor_arg(t) for t in (logits, targets, loss)]
+    L.check(L.lib.cdl_b200_cross_entropy(*(L.ref(a) for a in args), 0.5, None))
+    counts = (targets >= 0) & (targets < vocab)
+    picked = targets.clamp(0, vocab - 1).long()[:, None]
+    lse = x.logsumexp(1)
+    expected = torch.where(counts, lse - x.gather(1, picked)[:, 0], 0.0)
+    assert bool(((loss.double() - expected).abs() <= 1e-5 * (1 + lse.abs() + expected.abs())).all())
+    grad = (x.softmax(1) - torch.zeros_like(x).scatter_(1, picked, 1.0)) * 0.5 * counts[:, None]
+    # the f32 lse carries 2^-24 |lse| into every probability, __expf 2^-21 and more for large arguments
+    assert bool(((logits.double() - grad).abs() <= (2.0 ** -8 + 1e-4) * grad.abs() + 2.0 ** -22 * (1 + lse.abs())[:, None]).all())
+    assert torch.equal(buf[:, vocab:], tail)
