@@ -1091,14 +1091,16 @@ static int32_t check_epi_operand(const char* name, const cdl_tensor* t, long lon
 
 int32_t matmul_execute(const cdl_tensor* a, const cdl_tensor* b, const cdl_tensor* c,
                        const cdl_tensor* d, float alpha, float beta, cudaStream_t stream,
-                       const cdl_matmul_options* opts) {
-  return matmul_execute_epi(a, b, c, d, alpha, beta, 0, nullptr, nullptr, nullptr, stream, opts, nullptr);
+                       const cdl_matmul_options* opts, void* scratch, size_t scratch_bytes) {
+  return matmul_execute_epi(a, b, c, d, alpha, beta, 0, nullptr, nullptr, nullptr, stream, opts, nullptr, scratch,
+                            scratch_bytes);
 }
 
 int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_tensor* c,
                            const cdl_tensor* d, float alpha, float beta, int epi_mode,
                            const cdl_tensor* aux0, const cdl_tensor* aux1, const cdl_tensor* out2,
-                           cudaStream_t stream, const cdl_matmul_options* opts, const RopeEpilogue* rope) {
+                           cudaStream_t stream, const cdl_matmul_options* opts, const RopeEpilogue* rope,
+                           void* scratch, size_t scratch_bytes) {
   using namespace gemm;
   const int variant = opts ? opts->variant : CDL_GEMM_AUTO;
   if (variant < CDL_GEMM_AUTO || variant > CDL_GEMM_CTA_PAIR)
@@ -1146,12 +1148,12 @@ int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_t
   // f32 inputs, and bf16 operands TMA cannot describe (unaligned pointer or leading dimension):
   // the general kernel (gemm_general.cu).  Operands without any contiguous dimension
   // stay rejected, as in the reference.
-  if (f32_inputs) return matmul_general_execute(a, b, c, d, alpha, beta, stream);
+  if (f32_inputs) return matmul_general_execute(a, b, c, d, alpha, beta, scratch, scratch_bytes, stream);
   OperandLayout la, lb;
   for (int which = 0; which < 2; ++which) {
     const int32_t rc = which == 0 ? analyze_operand("a", a, true, &la) : analyze_operand("b", b, false, &lb);
     if (rc == CDL_ERR_UNSUPPORTED && epi_mode == 0)
-      return matmul_general_execute(a, b, c, d, alpha, beta, stream);
+      return matmul_general_execute(a, b, c, d, alpha, beta, scratch, scratch_bytes, stream);
     CDL_CHECK(rc);
   }
 
@@ -1433,18 +1435,16 @@ extern "C" {
 int32_t cdl_b200_matmul(const cdl_tensor* a, const cdl_tensor* b, const cdl_tensor* c,
                         const cdl_tensor* d, float alpha, float beta, void* scratch,
                         size_t scratch_bytes, cdl_stream stream) {
-  (void)scratch;
-  (void)scratch_bytes;
-  return cdl::matmul_execute(a, b, c, d, alpha, beta, static_cast<cudaStream_t>(stream));
+  return cdl::matmul_execute(a, b, c, d, alpha, beta, static_cast<cudaStream_t>(stream), nullptr, scratch,
+                             scratch_bytes);
 }
 
 int32_t cdl_b200_matmul_opt(const cdl_tensor* a, const cdl_tensor* b, const cdl_tensor* c,
                             const cdl_tensor* d, float alpha, float beta,
                             const cdl_matmul_options* options, void* scratch, size_t scratch_bytes,
                             cdl_stream stream) {
-  (void)scratch;
-  (void)scratch_bytes;
-  return cdl::matmul_execute(a, b, c, d, alpha, beta, static_cast<cudaStream_t>(stream), options);
+  return cdl::matmul_execute(a, b, c, d, alpha, beta, static_cast<cudaStream_t>(stream), options, scratch,
+                             scratch_bytes);
 }
 
 int32_t cdl_b200_matmul_candidates(const cdl_tensor* a, const cdl_tensor* b, const cdl_tensor* d,
@@ -1514,10 +1514,18 @@ int32_t cdl_b200_matmul_swiglu_dgrad(const cdl_tensor* a, const cdl_tensor* b, c
 
 int32_t cdl_b200_matmul_scratch_bytes(const cdl_tensor* a, const cdl_tensor* b,
                                       const cdl_tensor* d, size_t* bytes_out) {
-  (void)a;
-  (void)b;
-  (void)d;
+  using namespace cdl;
   if (bytes_out) *bytes_out = 0;
+  if (!a || !b || !d || !bytes_out || (a->rank != 2 && a->rank != 3) || b->rank != a->rank || d->rank != a->rank ||
+      a->dtype != b->dtype || (a->dtype != CDL_F32 && a->dtype != CDL_BF16) || a->shape[a->rank - 1] != b->shape[a->rank - 2])
+    return CDL_OK;  // (the call itself says what is wrong)
+  if (a->dtype == CDL_BF16) {
+    gemm::OperandLayout la, lb;
+    const int32_t ra = gemm::analyze_operand("a", a, true, &la), rb = gemm::analyze_operand("b", b, false, &lb);
+    last_error().clear();
+    if (ra == CDL_ERR_INVALID || rb == CDL_ERR_INVALID || (ra == CDL_OK && rb == CDL_OK)) return CDL_OK;
+  }
+  *bytes_out = matmul_general_scratch_bytes(a, b, d);
   return CDL_OK;
 }
 

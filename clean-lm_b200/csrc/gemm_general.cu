@@ -27,9 +27,10 @@
 // chain of FMAs has 8.2e-8, 1.8e-7 and 5.7e-7 .. 8.1e-7.
 //
 // What bounds it: the loaders and the shared memory they share with the tensor core (f32: 96 KiB of
-// pieces written and 192 KiB read per K block of 64).  1024 x 2048 x 1536 f32 74 us (87 TFLOP/s; 64 x 64
-// tiles of FMAs on the CUDA cores: 460 us, 14 TFLOP/s); 1500 x 1027 x 2051 bf16 with odd rows 51 us
-// (310 us).
+// pieces written and 192 KiB read per K block of 64), and every operand is converted again for each tile that uses it.
+// With scratch for the pieces lay_out_kernel converts each operand once and gemm_pieces_kernel multiplies them by TMA;
+// worth_laying_out chooses.  us without -> with scratch (FMAs on the CUDA cores): 1024 x 2048 x 1536 f32 69 -> 45
+// (460), 1500 x 1027 x 2051 bf16 with odd rows 51 -> 25 (310).
 #include "gemm_rows.cuh"
 #include "host.h"
 #include "ops.h"
@@ -39,6 +40,7 @@
 
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 namespace cdl {
 namespace gemm_general {
@@ -186,19 +188,23 @@ __device__ __forceinline__ bool store_rows(uint32_t tile, int lane, const PairBf
                  : "memory");
   return true;
 }
+// The pieces of two neighbours: x = h + m + l.  Returns false where that does not hold (NaN and infinities leave one).
+__device__ __forceinline__ bool split_pair(float x, float y, uint32_t& h, uint32_t& m, uint32_t& l) {
+  h = pack_bf16x2(x, y);
+  const float rx = x - bf16_lo(h), ry = y - bf16_hi(h);
+  m = pack_bf16x2(rx, ry);
+  const float tx = rx - bf16_lo(m), ty = ry - bf16_hi(m);
+  l = pack_bf16x2(tx, ty);
+  return bf16_lo(l) == tx && bf16_hi(l) == ty;
+}
 __device__ __forceinline__ bool store_rows(uint32_t tile, int lane, const PairF32 (&v)[ROWS]) {
   const uint32_t chunk = (lane >> 2) << 4, in = (lane & 3) << 2;
   bool exact = true;
 #pragma unroll
   for (int i = 0; i < ROWS; ++i) {
     const uint32_t at = tile + i * 128 + (chunk ^ ((i & 7) << 4)) + in;
-    const float x = __uint_as_float(v[i].x), y = __uint_as_float(v[i].y);
-    const uint32_t h = pack_bf16x2(x, y);
-    const float rx = x - bf16_lo(h), ry = y - bf16_hi(h);
-    const uint32_t m = pack_bf16x2(rx, ry);
-    const float tx = rx - bf16_lo(m), ty = ry - bf16_hi(m);
-    const uint32_t l = pack_bf16x2(tx, ty);
-    exact = exact && bf16_lo(l) == tx && bf16_hi(l) == ty;  // false for NaN (inf leaves one)
+    uint32_t h, m, l;
+    exact = split_pair(__uint_as_float(v[i].x), __uint_as_float(v[i].y), h, m, l) && exact;
     asm volatile("st.shared.b32 [%0], %1;" ::"r"(at), "r"(h) : "memory");
     asm volatile("st.shared.b32 [%0], %1;" ::"r"(at + PIECE_BYTES), "r"(m) : "memory");
     asm volatile("st.shared.b32 [%0], %1;" ::"r"(at + 2 * PIECE_BYTES), "r"(l) : "memory");
@@ -341,10 +347,10 @@ __device__ __noinline__ void partial_by_fma(const Operand oa, const Operand ob, 
   }
 }
 
-template <int S, int W>
+template <int S, int W, bool PAIR = false>
 __device__ __forceinline__ void store_out(const Params& p, const float* part, int rank, int warp, int b, int m0,
                                           int n0) {
-  gemm::TileOut<S, W> out;
+  gemm::TileOut<S, W, PAIR> out;
   out.prefetch(p, rank, warp, b, m0, n0);
   out.finish(p, part, rank, warp, b, m0, n0);
 }
@@ -541,6 +547,339 @@ __global__ void __launch_bounds__(THREADS, 1)
   if (threadIdx.x == 0 && *abort_word != 0) atomicExch(p.status, *abort_word);
 }
 
+// ------------------------------------------------------------ operands laid out first
+// The loaders above bring an operand's row in once for every tile that uses it, two elements a lane, and split
+// f32 values as often.  With scratch lent by the caller each operand is read once instead: lay_out_kernel
+// writes it as bf16 pieces with rows on the 16-byte grid (an aligned bf16 operand stays where it is),
+// and gemm_pieces_kernel loads the pieces by TMA.  Same pieces, same products, same sums.
+struct Layout {
+  const void* src;  // element (o, i) of a batch at src + batch * s_batch + o * s_outer + i * s_inner
+  long long s_batch, s_outer, s_inner;
+  __nv_bfloat16* dst;  // [piece][batch][outer][pitch]
+  long long piece;     // elements per piece
+  int outer, inner, pitch;
+  int mn_major;  // 1: `inner` runs along M or N
+  int mn_tiles, k_blocks;
+  int* outside;  // f32: [batch][mn tile][k block], 1 where a value is not the sum of its pieces
+};
+
+// One CTA per 128 (M or N) x 64 (K) block: 128 row segments of 64 elements, a lane two neighbours.  Bound by launch
+// and latency.
+constexpr int LAY_THREADS = 256, LAY_ROWS = 128 / (LAY_THREADS / 32);
+template <typename T>
+__global__ void __launch_bounds__(LAY_THREADS) lay_out_kernel(const Layout la, const Layout lb, int blocks_a) {
+  grid_dep_wait();
+  grid_dep_launch();
+  const bool second = static_cast<int>(blockIdx.x) >= blocks_a;
+  const Layout l = second ? lb : la;
+  int r = static_cast<int>(blockIdx.x) - (second ? blocks_a : 0);
+  const int kb = r % l.k_blocks;
+  r /= l.k_blocks;
+  const int tile = r % l.mn_tiles, b = r / l.mn_tiles;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int seg = warp * LAY_ROWS;  // this warp's first row segment
+  const int o0 = l.mn_major ? kb * BK + (seg & 63) : tile * TILE + seg;
+  const int i0 = (l.mn_major ? tile * TILE + (seg & 64) : kb * BK) + 2 * lane;
+  const T* src = static_cast<const T*>(l.src) + b * l.s_batch + o0 * l.s_outer + i0 * l.s_inner;
+  __nv_bfloat16* dst = l.dst + (static_cast<long long>(b) * l.outer + o0) * l.pitch + i0;
+  const int rows = l.outer - o0, first = i0 < l.inner ? rows : 0, second_e = i0 + 1 < l.inner ? rows : 0;
+  typename PairOf<T>::type v[LAY_ROWS];
+#pragma unroll
+  for (int i = 0; i < LAY_ROWS; ++i, src += l.s_outer) {
+    v[i].x = load_one_if(src, first - i);
+    v[i].y = load_one_if(src + l.s_inner, second_e - i);
+  }
+  bool exact = true;
+#pragma unroll
+  for (int i = 0; i < LAY_ROWS; ++i, dst += l.pitch) {
+    if (i >= first) break;
+    if constexpr (Traits<T>::PIECES == 1) {
+      *reinterpret_cast<uint32_t*>(dst) = v[i].x | (v[i].y << 16);
+    } else {
+      uint32_t h, m, lo;
+      exact = split_pair(__uint_as_float(v[i].x), __uint_as_float(v[i].y), h, m, lo) && exact;
+      *reinterpret_cast<uint32_t*>(dst) = h;
+      *reinterpret_cast<uint32_t*>(dst + l.piece) = m;
+      *reinterpret_cast<uint32_t*>(dst + 2 * l.piece) = lo;
+    }
+  }
+  if (Traits<T>::PIECES > 1) {
+    const int any = __syncthreads_or(!exact);
+    if (threadIdx.x == 0) l.outside[(static_cast<long long>(b) * l.mn_tiles + tile) * l.k_blocks + kb] = any != 0;
+  }
+}
+
+// One CTA takes a 128 x 128 tile (M128 N128), a pair of CTAs 256 x 128 (cta_group::2, M256 N128: each its own 128 rows of
+// A and half of B's 128 columns).  Products whose operands both come from shared memory run at 107 clk per M128
+// N128 K16 in one CTA and at 64 in a pair; one CTA is for up to 128 rows.  A K block arrives in slots, a piece of A and
+// the same piece of B each, the last pieces first: they are released first.  bf16: two CTAs share an SM where there
+// are more than one per SM; the running sums live in registers, so the two accumulators take half of the tensor memory.
+template <typename T>
+struct PieceTraits;
+template <>
+struct PieceTraits<float> {
+  static constexpr int SUM_WARPS = 16;
+};
+template <>
+struct PieceTraits<__nv_bfloat16> {
+  static constexpr int SUM_WARPS = 8;
+};
+constexpr int slot_bytes(bool pair) { return PIECE_BYTES + (pair ? PIECE_BYTES / 2 : PIECE_BYTES); }
+constexpr int shared_slots(bool pair) { return pair ? 4 : 3; }  // 96 KiB
+constexpr int alone_slots(bool pair) { return pair ? 9 : 6; }
+constexpr int MAX_SLOTS = 9;
+struct PieceBarriers {
+  uint64_t full[MAX_SLOTS];
+  uint64_t empty[MAX_SLOTS];
+  uint64_t acc_full[2];
+  uint64_t acc_empty[2];
+  uint32_t tmem_base;
+  int abort_word;
+  int outside;
+};
+static_assert(sizeof(PieceBarriers) <= 256, "barriers fit behind the slots");
+constexpr size_t piece_smem_bytes(int slots, bool pair) { return 1024 + slots * slot_bytes(pair) + 256; }
+static_assert(gemm::PART_BYTES <= shared_slots(true) * slot_bytes(true), "the partial tile takes the slots' place");
+template <typename T>
+constexpr int piece_threads() { return (2 + PieceTraits<T>::SUM_WARPS) * 32; }
+
+// warp 0 loads, warp 1 issues the products (of a pair: the first CTA's), the others add the accumulators up; all store.
+template <typename T, int SLOTS, bool PAIR>
+__global__ void __launch_bounds__(piece_threads<T>(), SLOTS == shared_slots(PAIR) ? 2 : 1)
+    gemm_pieces_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
+                       const Params p, const Operand oa, const Operand ob, const int* __restrict__ outside_a,
+                       const int* __restrict__ outside_b) {
+  constexpr int PIECES = Traits<T>::PIECES, SUM_WARPS = PieceTraits<T>::SUM_WARPS;
+  constexpr bool F32 = PIECES == 3;
+  constexpr int COLS = TILE * 4 / SUM_WARPS, W = SUM_WARPS + 2, CTAS = PAIR ? 2 : 1, SLOT = slot_bytes(PAIR);
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                             ~static_cast<uintptr_t>(1023));
+  PieceBarriers* bars = reinterpret_cast<PieceBarriers*>(smem + SLOTS * SLOT);
+  volatile int* abort_word = &bars->abort_word;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool clustered = PAIR || p.split_k > 1;
+  const int ctarank = clustered ? static_cast<int>(cluster_ctarank()) : 0;
+  const int half = PAIR ? ctarank & 1 : 0, rank = ctarank / CTAS;  // CTA of the pair, K slice
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < SLOTS; ++s) {
+      mbar_init(&bars->full[s], 1);
+      mbar_init(&bars->empty[s], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&bars->acc_full[i], 1);
+      mbar_init(&bars->acc_empty[i], CTAS * SUM_WARPS);  // (of a pair: the first CTA's is used)
+    }
+    bars->abort_word = 0;
+    bars->outside = 0;
+    fence_mbar_init();
+    tma_prefetch_desc(&tmap_a);
+    tma_prefetch_desc(&tmap_b);
+  }
+  if (warp == 1) {
+    if (PAIR) {
+      tmem_alloc_pair(&bars->tmem_base, 2 * TILE);
+      tmem_relinquish_pair();
+    } else {
+      tmem_alloc(&bars->tmem_base, 2 * TILE);
+      tmem_relinquish();
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (PAIR) cluster_sync_all();  // both CTAs' barriers exist before anything signals across the pair
+  tc_fence_after();
+  const uint32_t tmem_base = bars->tmem_base;
+  grid_dep_wait();
+  grid_dep_launch();
+
+  int b, tm, tn;
+  gemm::tile_coords(p, static_cast<int>(blockIdx.x) / (p.split_k * CTAS), b, tm, tn);
+  const int m0 = tm * TILE * CTAS + half * TILE, n0 = tn * TILE;
+  const int kb0 = static_cast<int>(static_cast<long long>(rank) * p.k_blocks / p.split_k);
+  const int kb1 = static_cast<int>(static_cast<long long>(rank + 1) * p.k_blocks / p.split_k);
+  const int blocks = kb1 - kb0;  // at least 1: the host never takes more slices than K blocks
+  float* part = reinterpret_cast<float*>(smem);
+  // a barrier of the pair's first CTA, of its second
+  auto in_first = [&](uint64_t* bar) { return mapa_shared(smem_u32(bar), ctarank & ~1); };
+  auto in_second = [&](uint64_t* bar) { return mapa_shared(smem_u32(bar), ctarank | 1); };
+
+  if (warp == 0) {
+    if (elect_one()) {
+      uint32_t n = 0;
+      bool ok = true;
+      for (int kb = kb0; kb < kb1 && ok; ++kb)
+        for (int piece = PIECES - 1; piece >= 0; --piece, ++n) {
+          const uint32_t s = n % SLOTS;
+          ok = mbar_wait(&bars->empty[s], ((n / SLOTS) & 1) ^ 1, abort_word, 151);
+          if (!ok) break;
+          uint8_t* sa = smem + s * SLOT;
+          uint8_t* sb = sa + PIECE_BYTES;
+          const int k0 = kb * BK;
+          if constexpr (PAIR) {
+            // the bytes of both CTAs land on the first one's barrier
+            if (half == 0) mbar_arrive_expect_tx(&bars->full[s], 2 * SLOT);
+            const uint32_t full = in_first(&bars->full[s]);
+            if (p.a_mn) {
+              tma_load_4d_pair(sa, &tmap_a, full, m0, k0, b, piece);
+              tma_load_4d_pair(sa + 8192, &tmap_a, full, m0 + 64, k0, b, piece);
+            } else {
+              tma_load_4d_pair(sa, &tmap_a, full, k0, m0, b, piece);
+            }
+            if (p.b_mn) tma_load_4d_pair(sb, &tmap_b, full, n0 + half * 64, k0, b, piece);
+            else tma_load_4d_pair(sb, &tmap_b, full, k0, n0 + half * 64, b, piece);
+          } else {
+            mbar_arrive_expect_tx(&bars->full[s], SLOT);
+            if (p.a_mn) {
+              tma_load_4d(sa, &tmap_a, &bars->full[s], m0, k0, b, piece);
+              tma_load_4d(sa + 8192, &tmap_a, &bars->full[s], m0 + 64, k0, b, piece);
+            } else {
+              tma_load_4d(sa, &tmap_a, &bars->full[s], k0, m0, b, piece);
+            }
+            if (p.b_mn) {
+              tma_load_4d(sb, &tmap_b, &bars->full[s], n0, k0, b, piece);
+              tma_load_4d(sb + 8192, &tmap_b, &bars->full[s], n0 + 64, k0, b, piece);
+            } else {
+              tma_load_4d(sb, &tmap_b, &bars->full[s], k0, n0, b, piece);
+            }
+          }
+        }
+    }
+  } else if (warp == 1) {
+    if (half == 0 && elect_one()) {
+      const uint32_t idesc = make_idesc_bf16(TILE * CTAS, TILE, p.a_mn, p.b_mn);
+      const uint32_t a_lbo = p.a_mn ? 8192u : 16u, b_lbo = p.b_mn ? 8192u : 16u;
+      const uint32_t a_kstep = p.a_mn ? 2048u : 32u, b_kstep = p.b_mn ? 2048u : 32u;
+      const uint32_t base = smem_u32(smem);
+      auto commit = [&](uint64_t* bar) {
+        if (PAIR) {
+          umma_commit_pair(in_first(bar));
+          umma_commit_pair(in_second(bar));
+        } else {
+          umma_commit(bar);
+        }
+      };
+      uint32_t n = 0;  // slots of a K block: n (the last pieces), n + 1, ...
+      bool ok = true;
+      for (int it = 0; it < blocks && ok; ++it, n += PIECES) {
+        const int group = it / p.sum_blocks, acc = group & 1;
+        const bool first = it == group * p.sum_blocks, last = it + 1 == blocks || it + 1 == (group + 1) * p.sum_blocks;
+        if (first) ok = mbar_wait(&bars->acc_empty[acc], ((group >> 1) & 1) ^ 1, abort_word, 251);
+        uint32_t at[PIECES];  // by piece
+#pragma unroll
+        for (int i = 0; i < PIECES; ++i) {
+          const uint32_t s = (n + i) % SLOTS;
+          at[PIECES - 1 - i] = base + s * SLOT;
+          ok = ok && mbar_wait(&bars->full[s], ((n + i) / SLOTS) & 1, abort_word, 252);
+        }
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t d = tmem_base + acc * TILE;
+        auto product = [&](int pa, int pb, bool fresh) {
+          const uint32_t sa = at[pa], sb = at[pb] + PIECE_BYTES;
+#pragma unroll
+          for (int k = 0; k < BK / 16; ++k) {
+            const uint64_t da = smem_desc_sw128(sa + k * a_kstep, a_lbo, 1024), db = smem_desc_sw128(sb + k * b_kstep, b_lbo, 1024);
+            if (PAIR) umma_ss_pair(d, da, db, idesc, fresh && k == 0 ? 0u : 1u);
+            else umma_ss(d, da, db, idesc, fresh && k == 0 ? 0u : 1u);
+          }
+        };
+        auto release = [&](int piece) { commit(&bars->empty[(n + PIECES - 1 - piece) % SLOTS]); };
+        if constexpr (F32) {  // the smallest products first
+          product(2, 0, first);
+          product(0, 2, false);
+          release(2);
+          product(1, 1, false);
+          product(1, 0, false);
+          product(0, 1, false);
+          release(1);
+          product(0, 0, false);
+          release(0);
+        } else {
+          product(0, 0, first);
+          release(0);
+        }
+        if (last) commit(&bars->acc_full[acc]);
+      }
+    }
+  } else {
+    const int quad = warp & 3, col0 = ((warp - 2) >> 2) * COLS;
+    if (F32 && m0 < p.M) {
+      int any = 0;
+      const long long fa = (static_cast<long long>(b) * ((p.M + TILE - 1) / TILE) + m0 / TILE) * p.k_blocks;
+      const long long fb = (static_cast<long long>(b) * p.num_n_tiles + tn) * p.k_blocks;
+      for (int i = kb0 + static_cast<int>(threadIdx.x) - 64; i < kb1; i += SUM_WARPS * 32)
+        any |= outside_a[fa + i] | outside_b[fb + i];
+      if (any) bars->outside = 1;
+    }
+    const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + col0;
+    const int groups = (blocks + p.sum_blocks - 1) / p.sum_blocks;
+    float sum[COLS];
+#pragma unroll
+    for (int j = 0; j < COLS; ++j) sum[j] = 0.f;
+    bool ok = true;
+    for (int g = 0; g < groups; ++g) {
+      const int acc = g & 1;
+      ok = mbar_wait(&bars->acc_full[acc], (g >> 1) & 1, abort_word, 351);
+      if (!ok) break;
+      tc_fence_after();
+#pragma unroll
+      for (int c = 0; c < COLS; c += 16) {
+        uint32_t r[16];
+        tmem_ld16(t_row + acc * TILE + c, r);
+        tmem_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 16; ++j) sum[c + j] = g == 0 ? __uint_as_float(r[j]) : sum[c + j] + __uint_as_float(r[j]);
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        if (PAIR) mbar_arrive_cluster(in_first(&bars->acc_empty[acc]));
+        else mbar_arrive(&bars->acc_empty[acc]);
+      }
+    }
+    // The last accumulator is complete: every slot has been read, the partial tile takes their place.
+    if (ok) gemm::store_partial(part, quad * 32 + lane, col0, sum);
+    if (F32) {
+      float zero = 0.f;  // NaN once a sum that is not finite has been met
+#pragma unroll
+      for (int j = 0; j < COLS; ++j) zero = fmaf(sum[j], 0.f, zero);
+      if (zero != 0.f) bars->outside = 1;
+    }
+  }
+  __syncwarp();
+  if (*abort_word != 0) {
+    // Loads that may still be in flight land before shared memory is used again or released.
+    const unsigned long long t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
+  }
+  if (F32) {
+    __syncthreads();
+    if (bars->outside != 0)
+      partial_by_fma(oa, ob, b, m0, n0, kb0 * BK, min(kb1 * BK, p.K), static_cast<int>(smem - smem_raw));
+  }
+  if (clustered) cluster_sync_all();
+  else __syncthreads();
+  if (m0 < p.M) {
+    switch (p.split_k) {
+      case 1: store_out<1, W, PAIR>(p, part, rank, warp, b, m0, n0); break;
+      case 2: store_out<2, W, PAIR>(p, part, rank, warp, b, m0, n0); break;
+      case 4: store_out<4, W, PAIR>(p, part, rank, warp, b, m0, n0); break;
+      default: store_out<PAIR ? 4 : 8, W, PAIR>(p, part, rank, warp, b, m0, n0); break;
+    }
+  }
+  __syncwarp();
+  if (clustered) cluster_sync_all();  // the other slices have read this CTA's partial; the pair is done
+  else __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    if (PAIR) tmem_dealloc_pair(tmem_base, 2 * TILE);
+    else tmem_dealloc(tmem_base, 2 * TILE);
+  }
+  if (threadIdx.x == 0 && *abort_word != 0) atomicExch(p.status, *abort_word);
+}
+
 // The same in f64.
 template <int N, int C>
 __device__ __forceinline__ void fma_block(const double* ta, const double* tb, int tx, int ty, int left,
@@ -683,6 +1022,43 @@ static int choose_splits(long long tiles, int k_blocks, int slots, double fixed)
   return best;
 }
 
+// The two tensor-core paths in microseconds, fitted to 200 products (M 16 .. 4100, K 64 .. 4099, odd and even rows, forward and
+// weight-gradient layouts) timed on both and with every K slicing: a wave's cost is a CTA's set-up and stores, its K
+// blocks and the exchange of the slices' sums.  The root mean square of what the fits miss is 8 to 16 %.
+// Waves are counted in clusters: with one CTA per SM 74 clusters of two fit on 148 SMs, 33 of four and 14 of
+// eight (an SM of a group that cannot take a whole one stays empty).
+static long long cluster_slots(int ctas) {
+  const long long sms = sm_count();
+  return std::max(1LL, ctas == 1 ? sms : ctas == 2 ? sms / 2 : ctas == 4 ? sms * 33 / 148 : sms * 14 / 148);
+}
+static double general_us(bool f32, long long batch, long long M, long long N, int k_blocks, int odd_operands) {
+  const long long tiles = batch * ((M + TILE - 1) / TILE) * ((N + TILE - 1) / TILE);
+  const int s = choose_splits(tiles, k_blocks, sm_count(), f32 ? 4.0 : 6.0);
+  const long long waves = (tiles + cluster_slots(s) - 1) / cluster_slots(s);
+  const double blocks = (k_blocks + s - 1) / s;
+  // (the loaders bring in only the rows and columns that exist)
+  const double fill = static_cast<double>(std::min<long long>(M, TILE) * std::min<long long>(N, TILE)) / (TILE * TILE);
+  return f32 ? 2.5 + waves * (5.4 + (s > 1 ? 1.2 : 0.0) + (s > 2 ? 3.4 : 0.0) + blocks * (0.40 + 1.45 * fill + 0.18 * odd_operands))
+             : 1.7 + waves * (5.5 + (s > 1 ? 0.7 : 0.0) + (s > 2 ? 3.1 : 0.0) + blocks * (0.95 * fill + 0.12 * odd_operands));
+}
+static double pieces_us(bool f32, bool pair, long long tiles, int k_blocks, int s, double laid_elements) {
+  const int ctas = s * (pair ? 2 : 1);
+  const long long slots = cluster_slots(ctas);
+  const double waves = (tiles + slots - 1) / slots, blocks = waves * ((k_blocks + s - 1) / s);
+  const double lay = laid_elements * 1e-6, split = s > 1, four = s > 1 && ctas >= 4, eight = ctas >= 8;
+  if (f32) return 2.4 + 1.81 * lay + blocks * (pair ? 0.81 : 1.08) + waves * (8.5 - 0.2 * split + 1.2 * four + 1.7 * eight);
+  // two CTAs fit on an SM: they share the tensor core, not the set-up
+  const long long two = tiles * ctas > sm_count() ? 2 * slots : slots;
+  const double sets = (tiles + two - 1) / two;
+  return 1.3 + 0.87 * lay + blocks * (pair ? 0.29 : 0.19) + sets * (8.2 - 1.1 * split + 1.2 * four + 0.3 * eight);
+}
+static int choose_piece_splits(bool f32, bool pair, long long tiles, int k_blocks) {
+  int best = 1;
+  for (int s = 2; s * (pair ? 2 : 1) <= gemm::MAX_SPLITS && s <= k_blocks; s *= 2)
+    if (pieces_us(f32, pair, tiles, k_blocks, s, 0) < pieces_us(f32, pair, tiles, k_blocks, best, 0)) best = s;
+  return best;
+}
+
 template <typename T, bool FINE>
 static int32_t launch(Params& p, const Operand& oa, const Operand& ob, double fixed, cudaStream_t stream) {
   using Tr = Traits<T>;
@@ -701,33 +1077,184 @@ static int32_t launch(Params& p, const Operand& oa, const Operand& ob, double fi
   return CDL_OK;
 }
 
+// What gemm_pieces_kernel needs in scratch, in this order: the pieces of A, of B (f32 always, bf16 where TMA cannot read
+// the operand where it is), and for f32 the two lists of blocks with values that have no pieces.
+struct PiecePlan {
+  bool lay_a, lay_b;
+  int pitch_a, pitch_b;
+  long long piece_a, piece_b;  // elements of one piece
+  size_t off_b, off_flags_a, off_flags_b, bytes;
+};
+static bool tma_can_read(const Operand& o, long long batch, int outer, int inner) {
+  const long long s_in = o.mn_major ? o.s_mn : o.s_k, s_out = o.mn_major ? o.s_k : o.s_mn;
+  return (inner == 1 || s_in == 1) && (outer == 1 || (s_out % 8 == 0 && s_out >= inner)) &&
+         (batch == 1 || (o.s_batch > 0 && o.s_batch % 8 == 0)) && reinterpret_cast<uintptr_t>(o.ptr) % 16 == 0;
+}
+static PiecePlan plan_pieces(const Operand& oa, const Operand& ob, long long batch, int K, bool f32) {
+  PiecePlan q{};
+  auto up = [](long long a, long long b) { return (a + b - 1) / b * b; };
+  const int pieces = f32 ? 3 : 1;
+  size_t at = 0;
+  for (int i = 0; i < 2; ++i) {
+    const Operand& o = i ? ob : oa;
+    const int outer = o.mn_major ? K : o.mn, inner = o.mn_major ? o.mn : K;
+    const bool lay = f32 || !tma_can_read(o, batch, outer, inner);
+    const long long pitch = up(inner, 8), piece = batch * outer * pitch;
+    (i ? q.lay_b : q.lay_a) = lay;
+    (i ? q.pitch_b : q.pitch_a) = static_cast<int>(pitch);
+    (i ? q.piece_b : q.piece_a) = piece;
+    if (i) q.off_b = at;
+    if (lay) at += up(2 * pieces * piece, 256);
+  }
+  if (f32) {
+    const long long kb = (K + BK - 1) / BK;
+    q.off_flags_a = at;
+    at += up(4 * batch * ((oa.mn + TILE - 1) / TILE) * kb, 256);
+    q.off_flags_b = at;
+    at += up(4 * batch * ((ob.mn + TILE - 1) / TILE) * kb, 256);
+  }
+  q.bytes = at;
+  return q;
+}
+
+template <typename T, int SLOTS, bool PAIR>
+static int32_t launch_pieces_kernel(const Params& p, const CUtensorMap& ta, const CUtensorMap& tb, const Operand& oa,
+                                    const Operand& ob, const int* fa, const int* fb, cudaStream_t stream) {
+  static std::once_flag once[64];
+  int dev = 0;
+  CDL_CUDA(cudaGetDevice(&dev));
+  cudaError_t err = cudaSuccess;
+  std::call_once(once[dev & 63], [&] {
+    err = cudaFuncSetAttribute(gemm_pieces_kernel<T, SLOTS, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               static_cast<int>(piece_smem_bytes(SLOTS, PAIR)));
+  });
+  if (err != cudaSuccess) return fail(CDL_ERR_CUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(err));
+  const int cluster = p.split_k * (PAIR ? 2 : 1);
+  CDL_CUDA(launch_pdl_cluster(gemm_pieces_kernel<T, SLOTS, PAIR>, dim3(static_cast<unsigned>(p.num_tiles) * cluster),
+                              dim3(piece_threads<T>()), piece_smem_bytes(SLOTS, PAIR), cluster, stream, ta, tb, p, oa, ob,
+                              fa, fb));
+  return CDL_OK;
+}
+
+template <typename T>
+static int32_t launch_pieces(Params& p, const Operand& oa, const Operand& ob, const PiecePlan& q, char* scratch,
+                             cudaStream_t stream) {
+  constexpr bool F32 = Traits<T>::PIECES == 3;
+  const bool pair = p.M > TILE;
+  CUtensorMap maps[2];
+  Layout lay[2] = {};
+  int blocks[2] = {0, 0};
+  for (int i = 0; i < 2; ++i) {
+    const Operand& o = i ? ob : oa;
+    const int outer = o.mn_major ? p.K : o.mn, inner = o.mn_major ? o.mn : p.K;
+    const bool laid = i ? q.lay_b : q.lay_a;
+    const long long s_in = o.mn_major ? o.s_mn : o.s_k, s_out = o.mn_major ? o.s_k : o.s_mn;
+    const int pitch = i ? q.pitch_b : q.pitch_a;
+    const long long piece = i ? q.piece_b : q.piece_a;
+    const void* base = laid ? scratch + (i ? q.off_b : 0) : o.ptr;
+    const long long ld = laid ? pitch : outer > 1 ? s_out : pitch, sb = laid || p.batch == 1 ? outer * ld : o.s_batch;
+    const uint64_t dims[4] = {static_cast<uint64_t>(inner), static_cast<uint64_t>(outer), static_cast<uint64_t>(p.batch),
+                              F32 ? 3u : 1u};
+    const uint64_t strides[4] = {0, 2 * static_cast<uint64_t>(ld), 2 * static_cast<uint64_t>(sb),
+                                 2 * static_cast<uint64_t>(laid ? piece : sb * p.batch)};
+    const uint32_t box[4] = {64, static_cast<uint32_t>(o.mn_major || (i == 1 && pair) ? 64 : TILE), 1, 1};
+    CDL_CHECK(encode_tmap(&maps[i], base, CDL_BF16, 4, dims, strides, box, true));
+    if (laid) {
+      Layout& l = lay[i];
+      l = {o.ptr, o.s_batch, s_out, s_in, static_cast<__nv_bfloat16*>(const_cast<void*>(base)), piece, outer, inner, pitch,
+           o.mn_major, (o.mn + TILE - 1) / TILE, p.k_blocks,
+           reinterpret_cast<int*>(scratch + (i ? q.off_flags_b : q.off_flags_a))};
+      blocks[i] = p.batch * l.mn_tiles * l.k_blocks;
+    }
+  }
+  p.a_mn = oa.mn_major;
+  p.b_mn = ob.mn_major;
+  if (blocks[0] + blocks[1] > 0)
+    CDL_CUDA(launch_pdl(lay_out_kernel<T>, dim3(static_cast<unsigned>(blocks[0] + blocks[1])), dim3(LAY_THREADS), 0,
+                        stream, lay[0], lay[1], blocks[0]));
+  const int* fa = reinterpret_cast<const int*>(scratch + q.off_flags_a);
+  const int* fb = reinterpret_cast<const int*>(scratch + q.off_flags_b);
+  auto run = [&](auto is_pair) {
+    constexpr bool PAIR = decltype(is_pair)::value;
+    constexpr int CTAS = PAIR ? 2 : 1;
+    p.num_m_tiles = (p.M + TILE * CTAS - 1) / (TILE * CTAS);
+    p.num_tiles = p.batch * p.num_m_tiles * p.num_n_tiles;
+    p.split_k = choose_piece_splits(F32, PAIR, p.num_tiles, p.k_blocks);
+    if (!F32 && static_cast<long long>(p.num_tiles) * p.split_k * CTAS > sm_count())
+      return launch_pieces_kernel<__nv_bfloat16, shared_slots(PAIR), PAIR>(p, maps[0], maps[1], oa, ob, fa, fb, stream);
+    return launch_pieces_kernel<T, alone_slots(PAIR), PAIR>(p, maps[0], maps[1], oa, ob, fa, fb, stream);
+  };
+  return pair ? run(std::true_type{}) : run(std::false_type{});
+}
+
+// Whether the operands are laid out first: where that is estimated to be faster by a tenth, about what the estimates
+// miss.  Of 90 random shapes (M 8 .. 8192, K and N 64 .. 4096) it is taken for two thirds, f32 1.30 and bf16 1.44 times as
+// fast on average (general kernel -> laid out first, us; f32: 16 x 1027 x 2051 29.9 -> 21.1, 512 x 2051 x 1027 62 -> 32,
+// 2047 x 2047 x 2047 152 -> 92; the other way 2049 x 64 x 2049 19.8 and 30.5, 512 x 1027 x 2051 29.0 and 30.4,
+// 16 x 515 x 515 13.0 and 13.5.  bf16: 64 x 2049 x 2049 33.9 -> 15.2, 2047 x 2047 x 4095 167 -> 53; the other way
+// 1500 x 300 x 900 11.6 and 11.7, 250 x 129 x 131 9.7 and 9.9).
+static bool worth_laying_out(const Operand& oa, const Operand& ob, const PiecePlan& plan, long long batch, long long K, bool f32,
+                             bool fine) {
+  const long long M = oa.mn, N = ob.mn, kb = (K + BK - 1) / BK;
+  const long long blocks = batch * ((M + TILE - 1) / TILE + (N + TILE - 1) / TILE) * kb;
+  if (fine || blocks > INT32_MAX) return false;
+  const bool pair = M > TILE;
+  const long long m_tile = pair ? 2 * TILE : TILE, tiles = batch * ((M + m_tile - 1) / m_tile) * ((N + TILE - 1) / TILE);
+  const int s = choose_piece_splits(f32, pair, tiles, static_cast<int>(kb));
+  const double laid = (plan.lay_a ? 1.0 * M : 0.0) + (plan.lay_b ? 1.0 * N : 0.0);
+  return pieces_us(f32, pair, tiles, static_cast<int>(kb), s, laid * K * batch) <
+         0.9 * general_us(f32, batch, M, N, static_cast<int>(kb), !oa.pairs + !ob.pairs);
+}
+
 }  // namespace gemm_general
+
+static gemm_general::Operand general_operand(const cdl_tensor* t, int mn_dim, int k_dim) {
+  gemm_general::Operand o{};
+  o.ptr = t->ptr;
+  o.mn = static_cast<int>(t->shape[mn_dim]);
+  o.s_batch = t->rank == 3 ? t->stride[0] : 0;
+  // an extent of 1 has no meaningful stride
+  o.s_mn = t->shape[mn_dim] > 1 ? t->stride[mn_dim] : 0;
+  o.s_k = t->shape[k_dim] > 1 ? t->stride[k_dim] : 0;
+  o.mn_major = o.s_k != 1 && o.s_mn == 1;
+  const long long inner = o.mn_major ? o.s_mn : o.s_k, outer = o.mn_major ? o.s_k : o.s_mn;
+  o.pairs = inner == 1 && outer % 2 == 0 && o.s_batch % 2 == 0 &&
+            reinterpret_cast<uintptr_t>(t->ptr) % (2 * dtype_size(t->dtype)) == 0;
+  return o;
+}
+
+size_t matmul_general_scratch_bytes(const cdl_tensor* a, const cdl_tensor* b, const cdl_tensor* d) {
+  using namespace gemm_general;
+  const int r = a->rank;
+  const long long batch = r == 3 ? a->shape[0] : 1;
+  const long long M = a->shape[r - 2], K = a->shape[r - 1], N = b->shape[r - 1];
+  const bool f32 = a->dtype == CDL_F32;
+  if (batch <= 0 || M <= 0 || N <= 0 || K <= 0 || batch > 65535 || M > INT32_MAX || N > INT32_MAX || K > INT32_MAX)
+    return 0;
+  Params p{};
+  p.M = static_cast<int>(M);
+  p.N = static_cast<int>(N);
+  p.K = static_cast<int>(K);
+  p.batch = static_cast<int>(batch);
+  p.out_f32 = d->dtype == CDL_F32;
+  if (short_k(p, f32)) return 0;
+  const Operand oa = general_operand(a, r - 2, r - 1), ob = general_operand(b, r - 1, r - 2);
+  const PiecePlan plan = plan_pieces(oa, ob, batch, p.K, f32);
+  return worth_laying_out(oa, ob, plan, batch, K, f32, !f32 && p.out_f32 && K <= 100) ? plan.bytes : 0;
+}
 
 // Operands as validated by matmul_execute_epi (ranks, shapes, dtypes of one kind, contiguous last
 // dimension of C and D); nothing here depends on alignment.
 int32_t matmul_general_execute(const cdl_tensor* a, const cdl_tensor* b, const cdl_tensor* c,
-                               const cdl_tensor* d, float alpha, float beta, cudaStream_t stream) {
+                               const cdl_tensor* d, float alpha, float beta, void* scratch, size_t scratch_bytes,
+                               cudaStream_t stream) {
   using namespace gemm_general;
   const int r = a->rank;
   const long long batch = r == 3 ? a->shape[0] : 1;
   const long long M = a->shape[r - 2], K = a->shape[r - 1], N = b->shape[r - 1];
   if (M > 65535LL * 64)
     return fail(CDL_ERR_UNSUPPORTED, "matmul (general path): more than %d rows", 65535 * 64);
-  auto operand = [&](const cdl_tensor* t, int mn_dim, int k_dim) {
-    Operand o{};
-    o.ptr = t->ptr;
-    o.mn = static_cast<int>(t->shape[mn_dim]);
-    o.s_batch = r == 3 ? t->stride[0] : 0;
-    // an extent of 1 has no meaningful stride
-    o.s_mn = t->shape[mn_dim] > 1 ? t->stride[mn_dim] : 0;
-    o.s_k = t->shape[k_dim] > 1 ? t->stride[k_dim] : 0;
-    o.mn_major = o.s_k != 1 && o.s_mn == 1;
-    const long long inner = o.mn_major ? o.s_mn : o.s_k, outer = o.mn_major ? o.s_k : o.s_mn;
-    o.pairs = inner == 1 && outer % 2 == 0 && o.s_batch % 2 == 0 &&
-              reinterpret_cast<uintptr_t>(t->ptr) % (2 * dtype_size(t->dtype)) == 0;
-    return o;
-  };
-  const Operand oa = operand(a, r - 2, r - 1), ob = operand(b, r - 1, r - 2);
+  const Operand oa = general_operand(a, r - 2, r - 1), ob = general_operand(b, r - 1, r - 2);
   Params p{};
   p.M = static_cast<int>(M);
   p.N = static_cast<int>(N);
@@ -769,6 +1296,12 @@ int32_t matmul_general_execute(const cdl_tensor* a, const cdl_tensor* b, const c
   p.sum_blocks = f32 || out_f32 ? 1 : std::clamp(static_cast<int>(0.11 * sqrt(static_cast<double>(K))), 1, 8);
   ProfileScope ps(PROF_GEMM, 2.0 * batch * M * N * K, stream);
   if (short_k(p, f32)) return f32 ? launch_fma<float>(p, oa, ob, stream) : launch_fma<__nv_bfloat16>(p, oa, ob, stream);
+  if (scratch != nullptr && reinterpret_cast<uintptr_t>(scratch) % 16 == 0) {
+    const PiecePlan plan = plan_pieces(oa, ob, batch, p.K, f32);
+    if (scratch_bytes >= plan.bytes && worth_laying_out(oa, ob, plan, batch, K, f32, fine))
+      return f32 ? launch_pieces<float>(p, oa, ob, plan, static_cast<char*>(scratch), stream)
+                 : launch_pieces<__nv_bfloat16>(p, oa, ob, plan, static_cast<char*>(scratch), stream);
+  }
   if (f32) return launch<float, false>(p, oa, ob, 4.0, stream);
   return fine ? launch<__nv_bfloat16, true>(p, oa, ob, 6.0, stream)
               : launch<__nv_bfloat16, false>(p, oa, ob, 6.0, stream);

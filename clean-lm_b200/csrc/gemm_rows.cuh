@@ -162,8 +162,13 @@ __device__ __forceinline__ int rope_position(const Params& p, int row) {
 // executed here is executed once or twice per launch, from a cold instruction cache.  Unrolled over
 // 16 rows with all forms in the row's body, a row cost 2000 clk and the store of a tile 34000; like this
 // the tile takes a tenth of it.
-template <int S, int W>
+//
+// PAIR: the cluster holds S pairs of CTAs; slice s of this CTA's 128 rows lies in CTA 2 s + (its rank & 1).
+template <int S, int W, bool PAIR = false>
 struct TileOut {
+  static __device__ __forceinline__ uint32_t part_of(uint32_t at, int s) {
+    return S == 1 ? at : mapa_shared(at, PAIR ? 2 * s + (cluster_ctarank() & 1) : s);
+  }
   static constexpr int STEP = S * W;
   static constexpr int BATCH = S == 8 ? 2 : 4;
   uint4 pre[BATCH];
@@ -230,7 +235,7 @@ struct TileOut {
         const uint32_t at = base + min(r0 + STEP * i, 127) * (PART_LD * 4) + lane * 16;
         float4 q[S];
 #pragma unroll
-        for (int s = 0; s < S; ++s) q[s] = ld_part_f4<S>(S == 1 ? at : mapa_shared(at, s));
+        for (int s = 0; s < S; ++s) q[s] = ld_part_f4<S>(part_of(at, s));
         v[i][0] = q[0].x; v[i][1] = q[0].y; v[i][2] = q[0].z; v[i][3] = q[0].w;
 #pragma unroll
         for (int s = 1; s < S; ++s) {
@@ -329,40 +334,52 @@ struct TileOut {
   }
 
   // Rows off the 16-byte grid or a column count that is no multiple of 4 (never a fused form): lane l
-  // takes columns l, l + 32, l + 64 and l + 96, so that every access of the warp is contiguous.
+  // takes columns l, l + 32, l + 64 and l + 96, so that every access of the warp is contiguous; four rows at a time,
+  // whose loads of C are in flight together.
   static __device__ __forceinline__ void finish_scalar(const Params& p, uint32_t base, int rank, int warp, int b,
                                                        int m0, int n0) {
+    constexpr int ROWS = 4;
     const int lane = threadIdx.x & 31;
     const int rows = min(128, p.M - m0);
+    const long long at_c = b * p.c_batch + m0 * p.ldc + n0 + lane, at_d = b * p.d_batch + m0 * p.ldd + n0 + lane;
 #pragma unroll 1
-    for (int r = rank + S * warp; r < rows; r += STEP) {
-      const long long row = m0 + r;
-      float v[4] = {0.f, 0.f, 0.f, 0.f}, c[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int r0 = rank + S * warp; r0 < rows; r0 += STEP * ROWS) {
+      float v[ROWS][4], c[ROWS][4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int col = n0 + lane + 32 * j;
-        if (p.c_mode != 0 && col < p.N)
-          c[j] = p.c_mode == 2 ? static_cast<const float*>(p.c)[b * p.c_batch + row * p.ldc + col]
-                               : __bfloat162float(static_cast<const __nv_bfloat16*>(p.c)[b * p.c_batch + row * p.ldc + col]);
-      }
+      for (int i = 0; i < ROWS; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const uint32_t at = base + (r * PART_LD + lane + 32 * j) * 4;
-        float q[S];
-#pragma unroll
-        for (int s = 0; s < S; ++s) q[s] = ld_part_f1<S>(S == 1 ? at : mapa_shared(at, s));
-#pragma unroll
-        for (int s = 0; s < S; ++s) v[j] += q[s];
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int col = n0 + lane + 32 * j;
-        if (col < p.N) {
-          const float x = p.c_mode != 0 ? p.alpha * v[j] + p.beta * c[j] : p.alpha * v[j];
-          if (p.out_f32) static_cast<float*>(p.d)[b * p.d_batch + row * p.ldd + col] = x;
-          else static_cast<__nv_bfloat16*>(p.d)[b * p.d_batch + row * p.ldd + col] = __float2bfloat16_rn(x);
+        for (int j = 0; j < 4; ++j) {
+          const int r = r0 + STEP * i;
+          const long long at = at_c + r * p.ldc + 32 * j;
+          c[i][j] = 0.f;
+          if (p.c_mode != 0 && r < rows && n0 + lane + 32 * j < p.N)
+            c[i][j] = p.c_mode == 2 ? static_cast<const float*>(p.c)[at]
+                                    : __bfloat162float(static_cast<const __nv_bfloat16*>(p.c)[at]);
         }
-      }
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const uint32_t at = base + (min(r0 + STEP * i, 127) * PART_LD + lane + 32 * j) * 4;
+          float q[S];
+#pragma unroll
+          for (int s = 0; s < S; ++s) q[s] = ld_part_f1<S>(part_of(at, s));
+          v[i][j] = q[0];
+#pragma unroll
+          for (int s = 1; s < S; ++s) v[i][j] += q[s];
+        }
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int r = r0 + STEP * i;
+          if (r < rows && n0 + lane + 32 * j < p.N) {
+            const long long at = at_d + r * p.ldd + 32 * j;
+            const float x = p.c_mode != 0 ? p.alpha * v[i][j] + p.beta * c[i][j] : p.alpha * v[i][j];
+            if (p.out_f32) static_cast<float*>(p.d)[at] = x;
+            else static_cast<__nv_bfloat16*>(p.d)[at] = __float2bfloat16_rn(x);
+          }
+        }
     }
   }
 };

@@ -57,14 +57,26 @@ def matmul(a: torch.Tensor, b: torch.Tensor, opts: MatmulOpts | None = None,
     if out is None:
         out = torch.empty(*sa[:-1], sb[-1], dtype=opts.out, device=a.device)
     ta, tb, tc, td = tensor_arg(a), tensor_arg(b), tensor_arg(opts.c), tensor_arg(out)
+    scratch, scratch_bytes = None, 0
+    if not (_on_grid(a) and _on_grid(b)):
+        n = ctypes.c_size_t(0)
+        check(lib.cdl_b200_matmul_scratch_bytes(ta, tb, td, ctypes.byref(n)))
+        if n.value:
+            block = torch.empty(n.value, dtype=torch.uint8, device=out.device)
+            scratch, scratch_bytes = block.data_ptr(), n.value
     if opts.variant == _lib.GEMM_AUTO and not opts.deterministic:
-        check(lib.cdl_b200_matmul(ref(ta), ref(tb), ref(tc), ref(td), opts.alpha, opts.beta, None, 0,
-                                  current_stream()))
+        check(lib.cdl_b200_matmul(ta, tb, tc, td, opts.alpha, opts.beta, scratch, scratch_bytes, current_stream()))
     else:
         mo = _lib.CdlMatmulOptions(int(opts.variant), 1 if opts.deterministic else 0)
-        check(lib.cdl_b200_matmul_opt(ref(ta), ref(tb), ref(tc), ref(td), opts.alpha, opts.beta,
-                                      ctypes.byref(mo), None, 0, current_stream()))
+        check(lib.cdl_b200_matmul_opt(ta, tb, tc, td, opts.alpha, opts.beta, ctypes.byref(mo), scratch, scratch_bytes,
+                                      current_stream()))
     return out
+
+
+def _on_grid(t: torch.Tensor) -> bool:
+    """Whether a bf16 operand's rows start on the 16-byte grid: the product needs no scratch then."""
+    return (t.dtype is torch.bfloat16 and t.data_ptr() & 15 == 0
+            and all(s == 1 or s & 7 == 0 for s in t.stride()))
 
 
 def matmul_candidates(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor) -> list:

@@ -115,7 +115,9 @@ typedef struct {
  * (tests/matmul.rs:243-265; 24-bit products, where cuBLASLt uses TF32) take a tensor-core
  * kernel that loads operands of any alignment itself, f32 values as three bf16 pieces of which the six
  * largest products are summed; a short K takes plain FMAs, f32 products summed in f64.  The error of a
- * f32 product is at most that of a chain of f32 FMAs.  K == 0 is an error ("K is zero", matmul.rs
+ * f32 product is at most that of a chain of f32 FMAs.  scratch (nullable; 16-byte aligned, as many bytes as
+ * cdl_b200_matmul_scratch_bytes says, 0 for many products) lets the operands of such a product be converted
+ * once instead of in every tile; without it, or with less, the result comes from the other kernel.  K == 0 is an error ("K is zero", matmul.rs
  * tests :825-843).  D may alias C. */
 int32_t cdl_b200_matmul(const cdl_tensor* a, const cdl_tensor* b, const cdl_tensor* c,
                         const cdl_tensor* d, float alpha, float beta, void* scratch,

@@ -7,6 +7,8 @@ K = 0 (:825-843), rejection messages (:355-468), with the
 tolerance of :199-202.  The acceptance bound of this build (max relative error 2e-2 against an
 f32-accumulated reference) is checked as well.
 """
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -604,4 +606,39 @@ def test_fused_swiglu_epilogues_of_wide_tiles(cdl, gpu_ok, m, n, k, pad):
         close(v[2], g * s * r, g.abs() + 1)
         close(v[3], r * v[0].double() * (s + g * s * (1 - s)), v[0].double().abs() * (g.abs() + 1))
     assert all(torch.equal(t[:, n:], e) for t, e in zip((o1, o2), ends))
+    assert L.device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("batch,m,k,n", [(1, 1, 64, 1), (1, 127, 129, 130), (3, 129, 200, 65), (1, 1000, 1027, 700), (1, 70, 4099, 33),
+                                         (1, 400, 4099, 129), (16, 128, 515, 128), (1, 64, 2049, 2049),
+                                         (3, 385, 1540, 641)])
+@pytest.mark.parametrize("ta,tb", [(False, False), (True, False), (False, True)])
+def test_operands_laid_out_in_scratch(cdl, gpu_ok, dtype, batch, m, k, n, ta, tb):
+    """Operands that TMA cannot read in place (one of them or both off the 16-byte grid, f32): with scratch for their
+    pieces, with too little and with none, against f64.  Bounds as in test_f32_products_are_f32; bf16 products are
+    exact, their sums truncate over at most 8 K blocks of 4 steps at a time."""
+    L = cdl._lib
+    gen = torch.Generator(device="cuda").manual_seed(m + k)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda").to(dtype)
+    a = rnd(batch, k, m + 1)[:, :, 1:].mT if ta else rnd(batch, m, k + 3)[:, :, 3:]
+    b = rnd(batch, n, (k + 7) // 8 * 8)[:, :, :k].mT if tb else rnd(batch, k, n)  # (tb: aligned rows)
+    c = torch.randn(batch, m, n, generator=gen, device="cuda")
+    if batch == 1:
+        a, b, c = a[0], b[0], c[0]
+    expected = c.double() + 0.5 * (a.double() @ b.double())
+    bound = 0.5 * (a.double().abs() @ b.double().abs())
+    steps = 4 if dtype == torch.float32 else 32
+    tol = (2 * 2.0 ** -24 + steps * 2.0 ** -23 + (k / 64 + 2) * 2.0 ** -24) * bound + 2.0 ** -23 * expected.abs() + 1e-30
+    need = ctypes.c_size_t(0)
+    args = [L.tensor_arg(t) for t in (a, b, c)]
+    L.check(L.lib.cdl_b200_matmul_scratch_bytes(*(L.ref(t) for t in args), ctypes.byref(need)))
+    for size in sorted({need.value, max(need.value - 1, 0), 0}):
+        scratch = torch.full((need.value + 16,), 0xff, dtype=torch.uint8, device="cuda")  # (NaN patterns)
+        d = c.clone()
+        td = L.tensor_arg(d)
+        L.check(L.lib.cdl_b200_matmul(L.ref(args[0]), L.ref(args[1]), L.ref(td), L.ref(td), 0.5, 1.0,
+                                      scratch.data_ptr() if size else None, size, None))
+        assert bool(((d.double() - expected).abs() <= tol).all()), size
+        assert bool((scratch[size:] == 0xff).all())
     assert L.device_status() == 0
