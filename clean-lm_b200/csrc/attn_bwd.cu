@@ -98,6 +98,11 @@ struct Params {
   int B, H, Hkv, Sq, Sk, Sq_pad;
   int causal;
   float scale, scale_log2;
+  // 1: the dQ kernel does not wait for the dK/dV kernel ahead of it, whose results it does not read: its CTAs start on
+  // SMs that have no dK/dV item left.  What they read is complete: they are launched once every dK/dV CTA has passed
+  // its own wait for the kernels before (the preprocess among them; the statistics are read from the L2).  They wait
+  // at their end instead, so that whoever waits for the dQ kernel has waited for both.
+  int dq_early;
   const float* lse2;   // [B, H, Sq_pad]  LSE * log2(e), +inf for rows that contribute nothing
   const float* delta;  // [B, H, Sq_pad]
   __nv_bfloat16* dq;
@@ -1576,7 +1581,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   const int cta_b = cta_hb / p_in.H;
   int q_base = 0, k_base = 0, bt = cta_b;
   if (p_in.cu_q != nullptr) {
-    grid_dep_wait();  // the sequence offsets may come from the previous kernel of the stream
+    if (!p_in.dq_early) grid_dep_wait();  // the sequence offsets may come from the previous kernel of the stream
     q_base = p_in.cu_q[cta_b];
     p.Sq = p_in.cu_q[cta_b + 1] - q_base;
     k_base = p_in.cu_k[cta_b];
@@ -1590,6 +1595,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   }
   if ((smem_u32(smem) & 1023u) != 0) {
     if (threadIdx.x == 0) atomicExch(p.status, 902);
+    if (p.dq_early) grid_dep_wait();
     return;
   }
   uint8_t* s_q = smem;
@@ -1639,7 +1645,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
-  grid_dep_wait();  // the set-up above overlaps the previous kernel's tail; global memory from here on
+  if (!p.dq_early) grid_dep_wait();  // the set-up above overlaps the previous kernel's tail; global memory from here on
   grid_dep_launch();
 
   if (warp == 0) {
@@ -1751,8 +1757,8 @@ __global__ void __launch_bounds__(THREADS, 1)
     const int row = q0 + r;
     const int shift = p.Sk - p.Sq;
     const long long stat_idx = (static_cast<long long>(b) * p.H + h) * p.Sq_pad + row;
-    const float lse2 = p.lse2[stat_idx];   // +inf for rows that contribute nothing (and padding)
-    const float delta = p.delta[stat_idx];
+    const float lse2 = __ldcg(p.lse2 + stat_idx);   // +inf for rows that contribute nothing (and padding)
+    const float delta = __ldcg(p.delta + stat_idx);
     const int key_limit = p.causal ? min(p.Sk - 1, row + shift) : p.Sk - 1;
     const int warp_limit = p.causal ? min(p.Sk - 1, q0 + quad * 32 + shift) : p.Sk - 1;
     bool ok = true;
@@ -1880,6 +1886,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     tmem_dealloc(tmem_base, TMEM_COLS);
   }
   if (threadIdx.x == 0 && *abort_word != 0) atomicExch(p.status, *abort_word);
+  if (p.dq_early) grid_dep_wait();  // see Params::dq_early
 }
 
 // ---------------------------------------------------------------- dQ kernel, persistent form
@@ -2007,7 +2014,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
-  grid_dep_wait();  // the set-up above overlaps the previous kernel's tail; global memory from here on
+  if (!p.dq_early) grid_dep_wait();  // the set-up above overlaps the previous kernel's tail; global memory from here on
   grid_dep_launch();
 
   if (warp == 0) {
@@ -2190,8 +2197,8 @@ __global__ void __launch_bounds__(THREADS, 1)
     if (idx >= 0) {
       v = q_item_of(p, idx);
       if (v.n_kv > 0) {
-        lse2 = p.lse2[stat_index(v)];
-        delta = p.delta[stat_index(v)];
+        lse2 = __ldcg(p.lse2 + stat_index(v));
+        delta = __ldcg(p.delta + stat_index(v));
       }
     }
     for (int k = 0; idx >= 0 && ok; ++k) {
@@ -2264,8 +2271,8 @@ __global__ void __launch_bounds__(THREADS, 1)
       if (idx_next >= 0) {
         vn = q_item_of(p, idx_next);
         if (vn.n_kv > 0) {
-          lse2_next = p.lse2[stat_index(vn)];
-          delta_next = p.delta[stat_index(vn)];
+          lse2_next = __ldcg(p.lse2 + stat_index(vn));
+          delta_next = __ldcg(p.delta + stat_index(vn));
         }
       }
 
@@ -2347,6 +2354,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     tmem_dealloc(tmem_base, TMEM_COLS);
   }
   if (threadIdx.x == 0 && *abort_word != 0) atomicExch(p.status, *abort_word);
+  if (p.dq_early) grid_dep_wait();  // see Params::dq_early
 }
 
 // CTAs per item of the dK/dV kernel.  In block pairs (one takes 1.7 us): the launch cannot end before
@@ -2499,6 +2507,16 @@ static int32_t bwd_run(const attn_bwd::Params& p_const, const cdl_tensor* q, con
     while (tail < heads_total && tail * blocks < static_cast<long long>(CDL_ATTN_BWD_TAIL_X) * sm_count()) tail += chunk;
     return static_cast<int>(tail < heads_total ? tail : heads_total);
   };
+  // dQ may lie where the dK/dV kernel still reads (dq given the memory of q or d_out): then it waits.
+  auto apart = [](const cdl_tensor* a, const cdl_tensor* b) {
+    auto end = [](const cdl_tensor* t) {
+      long long last = 0;
+      for (int i = 0; i < t->rank; ++i) last += (t->shape[i] - 1) * t->stride[i];
+      return reinterpret_cast<uintptr_t>(t->ptr) + 2 * static_cast<uintptr_t>(last + 1);
+    };
+    return end(a) <= reinterpret_cast<uintptr_t>(b->ptr) || end(b) <= reinterpret_cast<uintptr_t>(a->ptr);
+  };
+  p.dq_early = have_q && have_k && apart(dq, q) && apart(dq, k) && apart(dq, v) && apart(dq, d_o) ? 1 : 0;
   p.kv_blocks = static_cast<int>((Sk + BKV - 1) / BKV);
   p.kv_heads_total = static_cast<int>(Hkv * B);
   p.kv_chunk = chunk_of(Hkv * B);

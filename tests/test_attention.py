@@ -516,6 +516,27 @@ def test_packed_bwd_with_rope_equals_bwd_then_inverse_rope(cdl, gpu_ok, variant)
         cdl.ops.attention_bwd(qd, kd, vd, fwd.out, dod, fwd.lse, opts, rope_table=table[:100].contiguous())
 
 
+@pytest.mark.parametrize("b,s,hq,hk", [(1, 300, 4, 4), (2, 1024, 8, 2), (4, 2048, 16, 16)])
+@pytest.mark.parametrize("variant", [1, 2], ids=["one_shot", "persistent"])
+@pytest.mark.parametrize("target", ["q", "d_out"])
+def test_dq_may_take_the_place_of_an_input(cdl, gpu_ok, b, s, hq, hk, variant, target):
+    """dQ written over Q or over dOut: the bits of a call with a buffer of its own (the dK/dV kernel reads both), also
+    where many calls follow one another on the stream."""
+    gen = torch.Generator(device="cuda").manual_seed(s)
+    rnd = lambda h: torch.randn(b, s, h, 128, generator=gen, device="cuda").to(torch.bfloat16)
+    q, k, v, d_out = rnd(hq), rnd(hk), rnd(hk), rnd(hq)
+    opts = cdl.ops.AttentionOpts(causal=True, variant=variant)
+    fwd = cdl.ops.attention_fwd(q, k, v)
+    own = cdl.ops.attention_bwd(q, k, v, fwd.out, d_out, fwd.lse, opts)
+    for _ in range(10):
+        x = {"q": q.clone(), "d_out": d_out.clone()}
+        got = cdl.ops.attention_bwd(x["q"], k, v, fwd.out, x["d_out"], fwd.lse, opts, dq=x[target])
+        again = cdl.ops.attention_bwd(q, k, v, fwd.out, d_out, fwd.lse, opts)
+        for name, g, a, o in zip(("dq", "dk", "dv"), got, again, own):
+            assert torch.equal(g, o) and torch.equal(a, o), name
+    assert cdl._lib.device_status() == 0
+
+
 def test_forward_on_several_streams_at_once(cdl, gpu_ok):
     """The persistent forward hands its work items out through a counter that belongs to the
     launching stream.  Calls with many more items than SMs, enqueued on three streams so that they
