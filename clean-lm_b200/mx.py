@@ -155,6 +155,14 @@ def matmul_mx(a: MxTensor, b: MxTensor, out_dtype: torch.dtype = torch.bfloat16,
     return out
 
 
+def matmul_mx_rope(a: MxTensor, b: MxTensor, table: torch.Tensor, rot_heads: int, seqlen: int,
+                   out: torch.Tensor) -> torch.Tensor:
+    """bf16 `out` = A . B with the rotary embedding applied to its first `rot_heads` heads of 128 columns."""
+    aa, ab, tt, td = a.arg(), b.arg(), tensor_arg(table), tensor_arg(out)
+    check(lib.cdl_b200_matmul_mx_rope(ref(aa), ref(ab), ref(tt), rot_heads, seqlen, ref(td), current_stream()))
+    return out
+
+
 def matmul_mx_out(a: MxTensor, b: MxTensor, dim: int = ROWWISE, alpha: float = 1.0,
                   out: Optional[MxTensor] = None, fmt: int = MXFP8) -> MxTensor:
     """The same product with `MatmulOutput::BlockScaled { format, dim }`: a block-scaled [M, N] result."""

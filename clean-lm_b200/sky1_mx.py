@@ -21,8 +21,7 @@ from __future__ import annotations
 
 import torch
 
-from . import _lib, mx, ops
-from ._lib import check, current_stream, lib, ref, tensor_arg
+from . import mx, ops
 from .sky1 import Sky1Config, rope_table
 
 WEIGHTS = ("wqkv", "wo", "wup", "wgate", "wdown")
@@ -72,12 +71,6 @@ class Sky1BlockMX:
         for n in WEIGHTS:
             mx.quantize(self.params[n], rowwise=True, colwise=True, out=self.wq[n])
 
-    def _rope(self, x2d, backward: int):
-        cfg = self.cfg
-        x3 = x2d.view(cfg.tokens, cfg.heads + 2 * cfg.kv_heads, cfg.head_dim)
-        tx, tt = tensor_arg(x3), tensor_arg(self.table)
-        check(lib.cdl_b200_rope(ref(tx), ref(tt), cfg.heads + cfg.kv_heads, cfg.seqlen, backward, current_stream()))
-
     def _quant(self, name, x):
         mx.quantize(x, rowwise=True, colwise=True, out=self.q[name])
         return self.q[name]
@@ -101,8 +94,7 @@ class Sky1BlockMX:
         self._x = x
         n1 = mx.norm_fwd_mx(x, p["norm1"], eps=cfg.eps, colwise=True, save_stats=True,
                             out=mx.NormMxOutputs(*self.q["h1"], self.r_inv[1]))
-        self._fwd(n1.y, self.wq["wqkv"], b["qkv"])
-        self._rope(b["qkv"], 0)
+        mx.matmul_mx_rope(n1.y, self.wq["wqkv"][1], self.table, cfg.heads + cfg.kv_heads, cfg.seqlen, b["qkv"])
         att = ops.attention_fwd(self._q, self._k, self._v, ops.AttentionOpts(causal=True),
                                 out=b["attn"].view(cfg.batch, cfg.seqlen, cfg.heads, cfg.head_dim))
         self.lse = att.lse

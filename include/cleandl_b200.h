@@ -314,6 +314,11 @@ int32_t cdl_b200_matmul_mx(const cdl_mx_tensor* a, const cdl_mx_tensor* b, const
 int32_t cdl_b200_matmul_mx_opt(const cdl_mx_tensor* a, const cdl_mx_tensor* b, const cdl_tensor* c,
                                const cdl_tensor* d, float alpha, float beta,
                                const cdl_matmul_options* options, cdl_stream stream);
+/* D = RoPE(A . B) with MXFP8 operands: as cdl_b200_matmul_rope on dense sequences (bf16 [M, N], N % 128 == 0, 16-byte
+ * aligned rows; heads [0, rot_heads) rotated by position row % seqlen); the same values as cdl_b200_matmul_mx and
+ * cdl_b200_rope after it. */
+int32_t cdl_b200_matmul_mx_rope(const cdl_mx_tensor* a, const cdl_mx_tensor* b, const cdl_tensor* cos_sin,
+                                int32_t rot_heads, int32_t seqlen, const cdl_tensor* d, cdl_stream stream);
 
 /* The same product with a block-scaled output: MatmulOutput::BlockScaled { Mxfp8, dim }
  * (crates/cleandl/src/execgraph/ops/matmul.rs:826-834; test crates/cleandl/tests/matmul.rs:

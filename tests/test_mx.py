@@ -585,3 +585,27 @@ def test_matmul_mx_adds_in_place(cdl, gpu_ok, fmt, m, k, n, pad):
         cdl.mx.matmul_mx(qa, qb, out=out[:m, :n], c=out[:m, :n], alpha=-0.5, beta=1.0)
         assert torch.equal(out, expected)
     assert cdl._lib.device_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,k,heads,rot,seqlen", [(64, 64, 1, 1, 64), (300, 128, 3, 2, 150), (1000, 256, 6, 0, 1000), (2304, 512, 10, 8, 768)])
+def test_matmul_mx_rope(cdl, gpu_ok, m, k, heads, rot, seqlen):
+    """The rotation in the store of the MXFP8 product: the plain product's bf16 values, rotated (f64, within the one bf16
+    rounding and the f32 ones of the two terms); heads beyond the rotated ones are the plain product's bits."""
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    a, b = torch.randn(m, k, generator=gen, device="cuda").to(torch.bfloat16), torch.randn(heads * 128, k, generator=gen, device="cuda").to(torch.bfloat16)
+    qa, qb = cdl.mx.quantize(a, rowwise=True)[0], cdl.mx.quantize(b, rowwise=True)[0].transposed()
+    table = cdl.sky1.rope_table(seqlen, 128)
+    buf = torch.full((m + 1, heads * 128 + 8), 7.0, device="cuda", dtype=torch.bfloat16)
+    out = buf[:m, :heads * 128]
+    cdl.mx.matmul_mx_rope(qa, qb, table, rot, seqlen, out)
+    prod = cdl.mx.matmul_mx(qa, qb)
+    x = prod.double().view(m, heads, 2, 64)[:, :rot]
+    t = table.double()[torch.arange(m, device="cuda") % seqlen].view(m, 1, 2, 64)
+    lo, hi, c, s = x[:, :, 0], x[:, :, 1], t[:, :, 0], t[:, :, 1]
+    exact = torch.stack([lo * c - hi * s, hi * c + lo * s], 2).reshape(m, rot * 128)
+    size = (x.abs().sum(2, keepdim=True)).expand(-1, -1, 2, -1).reshape(m, rot * 128)
+    assert bool(((out[:, :rot * 128].double() - exact).abs() <= 2.0 ** -8 * exact.abs() + 2.0 ** -22 * size).all())
+    assert torch.equal(out[:, rot * 128:], prod[:, rot * 128:])
+    assert bool((buf[m:] == 7).all()) and bool((buf[:, heads * 128:] == 7).all())
+    assert cdl._lib.device_status() == 0
