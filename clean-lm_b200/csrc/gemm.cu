@@ -770,7 +770,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
   cluster_sync_all();  // both CTAs' barriers exist before anything signals across the pair
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
-  grid_dep_wait();  // set-up above overlaps the previous kernel's tail; global memory from here on
+  if (!p.early) grid_dep_wait();  // set-up above overlaps the previous kernel's tail; global memory from here on
   grid_dep_launch();
 
   if (warp == 0) {
@@ -946,6 +946,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
     tmem_dealloc_pair(tmem_base, TMEM_COLS);
   }
   if (threadIdx.x == 0 && *abort_word != 0) atomicExch(p.status, *abort_word);
+  if (p.early) grid_dep_wait();
 }
 
 // Splits a [rows, cols] (or batched) bf16 view into major-ness and leading dimension.
@@ -1091,16 +1092,16 @@ static int32_t check_epi_operand(const char* name, const cdl_tensor* t, long lon
 
 int32_t matmul_execute(const cdl_tensor* a, const cdl_tensor* b, const cdl_tensor* c,
                        const cdl_tensor* d, float alpha, float beta, cudaStream_t stream,
-                       const cdl_matmul_options* opts, void* scratch, size_t scratch_bytes) {
+                       const cdl_matmul_options* opts, void* scratch, size_t scratch_bytes, int early) {
   return matmul_execute_epi(a, b, c, d, alpha, beta, 0, nullptr, nullptr, nullptr, stream, opts, nullptr, scratch,
-                            scratch_bytes);
+                            scratch_bytes, early);
 }
 
 int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_tensor* c,
                            const cdl_tensor* d, float alpha, float beta, int epi_mode,
                            const cdl_tensor* aux0, const cdl_tensor* aux1, const cdl_tensor* out2,
                            cudaStream_t stream, const cdl_matmul_options* opts, const RopeEpilogue* rope,
-                           void* scratch, size_t scratch_bytes) {
+                           void* scratch, size_t scratch_bytes, int early) {
   using namespace gemm;
   const int variant = opts ? opts->variant : CDL_GEMM_AUTO;
   if (variant < CDL_GEMM_AUTO || variant > CDL_GEMM_CTA_PAIR)
@@ -1253,6 +1254,7 @@ int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_t
   p.sched_counter = nullptr;
   p.atomic_out = 0;
   p.tma_add = 0;
+  p.early = early;
   p.epi_mode = 0;
   p.aux0 = p.aux1 = nullptr;
   p.out2 = nullptr;
@@ -1417,10 +1419,10 @@ int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_t
   if (use_pair) {
     const long long units = static_cast<long long>(p.num_tiles) * p.split_k;
     const int clusters = units < max_clusters[dev & 63] ? static_cast<int>(units) : max_clusters[dev & 63];
-    p.sched_counter = units > clusters ? sched_counter_for(0, dev, stream) : nullptr;
+    p.sched_counter = units > clusters ? sched_counter_for(gemm_counter_kind(early), dev, stream) : nullptr;
     CDL_CUDA(launch_pdl(gemm_bf16_pair_kernel, dim3(2 * clusters), dim3(THREADS), PAIR_SMEM_BYTES, stream,
                         tm_a, tm_b, tm_e0, tm_e1, p));
-  } else {
+  } else {  // (this one always waits at its start)
     const int grid = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
     CDL_CUDA(launch_pdl(gemm_bf16_kernel, dim3(grid), dim3(THREADS), SMEM_BYTES, stream, tm_a, tm_b, p));
   }

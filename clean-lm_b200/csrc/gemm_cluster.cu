@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(THREADS, STAGES == SHARED_STAGES ? 2 : 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
-  grid_dep_wait();  // the set-up above overlaps the previous kernel's tail
+  if (!p.early) grid_dep_wait();  // the set-up above overlaps the previous kernel's tail
   grid_dep_launch();
 
   // One (tile, K slice) per CTA; the slices of a tile are one cluster.
@@ -171,6 +171,7 @@ __global__ void __launch_bounds__(THREADS, STAGES == SHARED_STAGES ? 2 : 1)
     tmem_dealloc(tmem_base, TMEM_COLS);
   }
   if (threadIdx.x == 0 && *abort_word != 0) atomicExch(p.status, *abort_word);
+  if (p.early) grid_dep_wait();
 }
 
 // The unsplit weight-gradient form (D += A^T B, f32): many tiles with few K blocks each, so that launch,
@@ -246,7 +247,7 @@ __global__ void __launch_bounds__(WALK_THREADS, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
-  grid_dep_wait();
+  if (!p.early) grid_dep_wait();
   grid_dep_launch();
 
   if (warp == 0) {
@@ -384,6 +385,7 @@ __global__ void __launch_bounds__(WALK_THREADS, 1)
     tmem_dealloc(tmem_base, WALK_TMEM_COLS);
   }
   if (threadIdx.x == 0 && *abort_word != 0) atomicExch(p.status, *abort_word);
+  if (p.early) grid_dep_wait();
 }
 
 template <int S, int STAGES>
@@ -421,7 +423,7 @@ int32_t gemm_cluster_launch(const CUtensorMap& tm_a, const CUtensorMap& tm_b, co
     });
     if (err != cudaSuccess) return fail(CDL_ERR_CUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(err));
     Params walk = p;
-    walk.sched_counter = sched_counter_for(0, dev, stream);  // launches of one stream that draw share a counter
+    walk.sched_counter = sched_counter_for(gemm_counter_kind(p.early), dev, stream);  // launches of one stream that draw share a counter
     CDL_CUDA(launch_pdl(gemm_cluster_walk_kernel, dim3(static_cast<unsigned>(sm_count())), dim3(WALK_THREADS),
                         WALK_SMEM_BYTES, stream, tm_a, tm_b, walk));
     return CDL_OK;

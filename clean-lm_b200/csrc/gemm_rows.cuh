@@ -45,6 +45,7 @@ struct Params {
   // between launches; one counter per device and stream).
   unsigned int* sched_counter;
   int* status;
+  int early;  // 1 = starts before the kernel ahead of it has finished (see grid_dep_wait)
 };
 
 __device__ __forceinline__ void tile_coords(const Params& p, int tile, int& b, int& m, int& n) {

@@ -7,9 +7,12 @@
 
 namespace cdl {
 
+// early > 0: the product may start before the kernel enqueued ahead of it has finished (the conditions are at
+// grid_dep_wait in ptx.cuh); the products of a chain have different numbers, 1 to 4.
 int32_t matmul_execute(const cdl_tensor* a, const cdl_tensor* b, const cdl_tensor* c,
                        const cdl_tensor* d, float alpha, float beta, cudaStream_t stream,
-                       const cdl_matmul_options* opts = nullptr, void* scratch = nullptr, size_t scratch_bytes = 0);
+                       const cdl_matmul_options* opts = nullptr, void* scratch = nullptr, size_t scratch_bytes = 0,
+                       int early = 0);
 // gemm_general.cu: any strides, bf16 or f32 inputs (operands already validated).  With enough scratch, 16-byte
 // aligned, the operands are laid out in it first; the bytes are 0 where that would not pay.
 int32_t matmul_general_execute(const cdl_tensor* a, const cdl_tensor* b, const cdl_tensor* c,
@@ -32,7 +35,8 @@ int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_t
                            const cdl_tensor* d, float alpha, float beta, int epi_mode,
                            const cdl_tensor* aux0, const cdl_tensor* aux1, const cdl_tensor* out2,
                            cudaStream_t stream, const cdl_matmul_options* opts = nullptr,
-                           const RopeEpilogue* rope = nullptr, void* scratch = nullptr, size_t scratch_bytes = 0);
+                           const RopeEpilogue* rope = nullptr, void* scratch = nullptr, size_t scratch_bytes = 0,
+                           int early = 0);
 // norm_general.cu: any float types, strides and column counts (layer = 0 RmsNorm, 1 LayerNorm).
 int32_t norm_general_execute(int layer, const cdl_tensor* x, const cdl_tensor* scale,
                              const cdl_tensor* bias, float eps, const cdl_tensor* y,

@@ -32,6 +32,14 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
 // prefetch) overlaps the predecessor's tail; grid_dep_wait() returns once the predecessor grid has
 // completed and its writes are visible.  grid_dep_launch() lets the successor's CTAs be scheduled
 // as soon as this grid's CTAs free their SMs.  Both are no-ops for a normal launch.
+//
+// A kernel that neither reads nor overwrites anything its predecessor writes, nor writes what it reads, may start early:
+// it leaves out the wait at its start, so that its CTAs fill the SMs that the predecessor's last wave leaves idle,
+// and waits at its end instead, so that whoever waits for it has waited for both.  What it reads is
+// complete all the same, if every kernel calls grid_dep_launch() after its own wait: the CTAs of an early kernel are
+// launched once all CTAs of its predecessor have passed theirs (or, where that one is early too, have been
+// launched under the same condition), and operands come from the L2 (TMA).  A chain of early kernels must be
+// independent of one another down to the kernel that waits, and draw their work from counters of their own.
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -279,6 +279,20 @@ int32_t sky1_block_bwd(const cdl_sky1_config* cfg, const cdl_sky1_weights* wt, c
   const cdl_tensor woT = transposed(wo), wqkvT = transposed(wqkv);
 
   const bool with_h = d.Hd <= 2048;
+  // Products that depend on nothing that runs since the last wait start early (the number: see matmul_execute): the gate and
+  // up gradients beside the weight gradient of the down projection; after the norm's backward (its closing
+  // kernel only adds up d_gain) the weight gradients of up, gate and wo and d_attn, one behind the other; dWqkv.
+  // The last waves of 176 tiles on 74 CTA pairs then run into one another.  Gradients that shared memory would
+  // race: those wait.
+  auto apart = [](const void* x, long long nx, const void* y, long long ny) {
+    const char *a = static_cast<const char*>(x), *b = static_cast<const char*>(y);
+    return a + 4 * nx <= b || b + 4 * ny <= a;
+  };
+  const long long ffn = d.Hd * d.F, wo_size = HD * d.Hd;
+  const int chain = apart(gr->wup, ffn, gr->wgate, ffn) && apart(gr->wup, ffn, gr->wo, wo_size) &&
+                    apart(gr->wgate, ffn, gr->wo, wo_size) && apart(gr->norm2, d.Hd, gr->wup, ffn) &&
+                    apart(gr->norm2, d.Hd, gr->wgate, ffn) && apart(gr->norm2, d.Hd, gr->wo, wo_size) ? 1 : 0;
+  const int qkv_early = apart(gr->norm1, d.Hd, gr->wqkv, d.Hd * d.QKV) ? 1 : 0;
   if (phase < 0 || phase > 2) return fail(CDL_ERR_INVALID, "sky1_block_bwd: phase must be 0, 1 or 2");
   // Weight-gradient products: the caller chooses between K slices that meet through f32 atomics
   // (default) and a fixed summation order.
@@ -295,7 +309,8 @@ int32_t sky1_block_bwd(const cdl_sky1_config* cfg, const cdl_sky1_weights* wt, c
   CDL_CHECK(matmul_execute(&actT, &tdy, &gwdown, &gwdown, 1.f, 1.f, st, wg));          // dWdown += act^T dy
   CDL_CHECK(mark(ev ? ev->wdown : nullptr));
   // d_act = dy Wdown^T never reaches memory: the epilogue turns it into d_up and d_gate
-  CDL_CHECK(matmul_execute_epi(&tdy, &wdownT, nullptr, &tdact, 1.f, 0.f, 2, &tgate, &tup, &tdgate, st));
+  CDL_CHECK(matmul_execute_epi(&tdy, &wdownT, nullptr, &tdact, 1.f, 0.f, 2, &tgate, &tup, &tdgate, st, nullptr, nullptr,
+                               nullptr, 0, 1));
   // h2 is not kept: the norm's backward gives it again (as a kernel of its own where the rows are too wide for that)
   // ahead of the weight gradients that need it.
   CDL_CHECK(matmul_execute(&tdact, &wupT, nullptr, &tdh, 1.f, 0.f, st));            // dh2 = d_up Wup^T
@@ -303,16 +318,17 @@ int32_t sky1_block_bwd(const cdl_sky1_config* cfg, const cdl_sky1_weights* wt, c
   if (!with_h) CDL_CHECK(rmsnorm_fwd_execute(&to, &g2, nullptr, cfg->eps, &th, &tr, st));
   CDL_CHECK(rmsnorm_bwd_execute(&to, &tdh, &tdy, &g2, &tr, &tdo, &dg2, b.norm_scratch, b.norm_scratch_bytes, st,
                                 nullptr, with_h ? &th : nullptr, cfg->eps));        // d_o (+ dy)
-  CDL_CHECK(matmul_execute(&hT, &tdact, &gwup, &gwup, 1.f, 1.f, st, wg));               // dWup += h2^T d_up
+  CDL_CHECK(matmul_execute(&hT, &tdact, &gwup, &gwup, 1.f, 1.f, st, wg, nullptr, 0, chain));     // dWup += h2^T d_up
   CDL_CHECK(mark(ev ? ev->wup : nullptr));
-  CDL_CHECK(matmul_execute(&hT, &tdgate, &gwgate, &gwgate, 1.f, 1.f, st, wg));          // dWgate += h2^T d_gate
+  CDL_CHECK(matmul_execute(&hT, &tdgate, &gwgate, &gwgate, 1.f, 1.f, st, wg, nullptr, 0, 2 * chain));  // dWgate += h2^T d_gate
   CDL_CHECK(mark(ev ? ev->wgate_norm2 : nullptr));
   }
   if (phase == 1) return CDL_OK;
   // attention
-  CDL_CHECK(matmul_execute(&attnT, &tdo, &gwo, &gwo, 1.f, 1.f, st, wg));                // dWo += attn^T d_o
+  // (in a call of its own this half does not know what is ahead of it)
+  CDL_CHECK(matmul_execute(&attnT, &tdo, &gwo, &gwo, 1.f, 1.f, st, wg, nullptr, 0, phase == 0 ? 3 * chain : 0));  // dWo += attn^T d_o
   CDL_CHECK(mark(ev ? ev->wo : nullptr));
-  CDL_CHECK(matmul_execute(&tdo, &woT, nullptr, &tdattn, 1.f, 0.f, st));            // d_attn = d_o Wo^T
+  CDL_CHECK(matmul_execute(&tdo, &woT, nullptr, &tdattn, 1.f, 0.f, st, nullptr, nullptr, 0, 4));  // d_attn = d_o Wo^T
   // d_q and d_k leave the attention backward already rotated back (the transpose of the rotary
   // embedding runs in its store epilogues)
   if (d.rg) {
@@ -342,7 +358,7 @@ int32_t sky1_block_bwd(const cdl_sky1_config* cfg, const cdl_sky1_weights* wt, c
   if (!with_h) CDL_CHECK(rmsnorm_fwd_execute(&tx, &g1, nullptr, cfg->eps, &th, &tr, st));
   CDL_CHECK(rmsnorm_bwd_execute(&tx, &tdh, &tdo, &g1, &tr, &tdx, &dg1, b.norm_scratch, b.norm_scratch_bytes, st,
                                 nullptr, with_h ? &th : nullptr, cfg->eps));        // dx (+ d_o)
-  CDL_CHECK(matmul_execute(&hT, &tdqkv, &gwqkv, &gwqkv, 1.f, 1.f, st, wg));             // dWqkv += h1^T d_qkv
+  CDL_CHECK(matmul_execute(&hT, &tdqkv, &gwqkv, &gwqkv, 1.f, 1.f, st, wg, nullptr, 0, qkv_early));  // dWqkv += h1^T d_qkv
   CDL_CHECK(mark(ev ? ev->wqkv_norm1 : nullptr));
   return CDL_OK;
 }

@@ -356,3 +356,47 @@ def test_block_widths_of_the_norm_backward(cdl, gpu_ok, hidden, seqlen):
     for name, got, ref in [("dx", dx, dx_ref.reshape(seqlen, hidden))] + [(n, blk.grads[n], g_ref[n]) for n in sky1.PARAM_NAMES]:
         assert ((got.double() - ref).abs().max() / ref.abs().max()).item() <= 2e-2, name
     assert cdl._lib.device_status() == 0
+
+
+@pytest.mark.parametrize("dims", [dict(batch=1, seqlen=129, hidden=256, heads=2, kv_heads=1, head_dim=128, ffn=384),
+                                  dict(batch=2, seqlen=640, hidden=1024, heads=8, kv_heads=4, head_dim=128, ffn=2816),
+                                  dict(batch=1, seqlen=1024, hidden=2056, heads=4, kv_heads=4, head_dim=128, ffn=1024)])
+def test_block_backward_products_that_overlap(cdl, gpu_ok, dims):
+    """The backward's products that start beside one another: many passes in a row give the same bits, those of the two
+    halves with a synchronisation between them; gradients of two weights in one buffer give the sum of both (f32
+    sums of the same addends in another order: 2^-23 of the two magnitudes each time one is added)."""
+    sky1 = cdl.sky1
+    cfg = sky1.Sky1Config(deterministic=True, **dims)
+    params = sky1.init_params(cfg, seed=3, std=cfg.hidden ** -0.5)
+    x, dy = (torch.randn(cfg.tokens, cfg.hidden, generator=torch.Generator().manual_seed(i)).to(torch.bfloat16).cuda() for i in (4, 5))
+
+    def passes(n, halves=False, **grads):
+        blk = sky1.Sky1Block(cfg, params, **grads)
+        blk.zero_grads()
+        for _ in range(n):
+            blk.forward(x)
+            dx = torch.empty_like(x)
+            if halves:
+                blk.backward(dy, dx, phase=1)
+                torch.cuda.synchronize()
+                blk.backward(dy, dx, phase=2)
+            else:
+                blk.backward(dy, dx)
+        torch.cuda.synchronize()
+        return dx, blk.grads
+
+    ref_dx, ref = passes(10, halves=True)
+    for _ in range(3):
+        dx, grads = passes(10)
+        assert torch.equal(dx, ref_dx)
+        for name in sky1.PARAM_NAMES:
+            assert torch.equal(grads[name], ref[name]), name
+    one_dx, one = passes(1)
+    shared = {name: torch.zeros_like(g) for name, g in one.items()}
+    shared["wup"] = shared["wgate"]
+    dx, grads = passes(1, grads=shared)
+    assert torch.equal(dx, one_dx)
+    total = one["wup"].double() + one["wgate"].double()
+    slack = 2.0 ** -22 * (one["wup"].double().abs() + one["wgate"].double().abs()) + 2.0 ** -23 * 8 * total.abs().max()
+    assert bool(((grads["wgate"].double() - total).abs() <= slack).all())
+    assert cdl._lib.device_status() == 0
