@@ -64,6 +64,27 @@ __global__ void __launch_bounds__(THREADS, STAGES == SHARED_STAGES ? 2 : 1)
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
   }
+  // One (tile, K slice) per CTA; the slices of a tile are one cluster.
+  const int rank = S > 1 ? static_cast<int>(cluster_ctarank()) : 0;
+  int b, tm, tn;
+  tile_coords(p, static_cast<int>(blockIdx.x) / S, b, tm, tn);
+  const int m0 = tm * TILE_M, n0 = tn * TILE_N;
+  const int kb0 = static_cast<int>(static_cast<long long>(rank) * p.k_blocks / S);
+  const int kb1 = static_cast<int>(static_cast<long long>(rank + 1) * p.k_blocks / S);
+  // B is the weights: on their way from HBM to the L2 while the kernel ahead still runs.
+  if (warp == 2 && tm == 0 && !p.atomic_out) {
+    if (elect_one()) {
+      for (int kb = kb0; kb < kb1 && kb < kb0 + STAGES; ++kb) {
+        if (p.b_mn) {
+#pragma unroll
+          for (int i = 0; i < TILE_N / 64; ++i) tma_prefetch_3d(&tmap_b, n0 + i * 64, kb * BK, b);
+        } else {
+          tma_prefetch_3d(&tmap_b, kb * BK, n0, b);
+        }
+      }
+    }
+    __syncwarp();
+  }
   if (warp == 1) {
     tmem_alloc(&bars->tmem_base, TMEM_COLS);
     tmem_relinquish();
@@ -75,13 +96,6 @@ __global__ void __launch_bounds__(THREADS, STAGES == SHARED_STAGES ? 2 : 1)
   if (!p.early) grid_dep_wait();  // the set-up above overlaps the previous kernel's tail
   grid_dep_launch();
 
-  // One (tile, K slice) per CTA; the slices of a tile are one cluster.
-  const int rank = S > 1 ? static_cast<int>(cluster_ctarank()) : 0;
-  int b, tm, tn;
-  tile_coords(p, static_cast<int>(blockIdx.x) / S, b, tm, tn);
-  const int m0 = tm * TILE_M, n0 = tn * TILE_N;
-  const int kb0 = static_cast<int>(static_cast<long long>(rank) * p.k_blocks / S);
-  const int kb1 = static_cast<int>(static_cast<long long>(rank + 1) * p.k_blocks / S);
   float* part = reinterpret_cast<float*>(smem);
   TileOut<S, WARPS> tile_out;
 
