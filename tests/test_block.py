@@ -400,3 +400,34 @@ def test_block_backward_products_that_overlap(cdl, gpu_ok, dims):
     slack = 2.0 ** -22 * (one["wup"].double().abs() + one["wgate"].double().abs()) + 2.0 ** -23 * 8 * total.abs().max()
     assert bool(((grads["wgate"].double() - total).abs() <= slack).all())
     assert cdl._lib.device_status() == 0
+
+
+@pytest.mark.parametrize("dims", [dict(batch=1, seqlen=100, hidden=256, heads=2, kv_heads=2, head_dim=128, ffn=320),
+                                  dict(batch=2, seqlen=300, hidden=512, heads=4, kv_heads=2, head_dim=128, ffn=1408),
+                                  dict(batch=4, seqlen=600, hidden=1024, heads=8, kv_heads=8, head_dim=128, ffn=2816)])
+def test_block_backward_weights_in_any_order(cdl, gpu_ok, dims):
+    """d_up Wup^T + d_gate Wgate^T is one product whose operands are read through one tensor map: the same bits for Wgate behind
+    Wup, ahead of it or in a buffer of its own."""
+    sky1 = cdl.sky1
+    cfg = sky1.Sky1Config(deterministic=True, **dims)
+    params = sky1.init_params(cfg, seed=3, std=cfg.hidden ** -0.5)
+    x, dy = (torch.randn(cfg.tokens, cfg.hidden, generator=torch.Generator().manual_seed(i)).to(torch.bfloat16).cuda() for i in (4, 5))
+    n = params["wup"].numel()
+    got = []
+    for up, gate in ((0, n + 64), (n + 64, 0), (0, None)):
+        blk = sky1.Sky1Block(cfg, params)
+        blk.zero_grads()
+        buf = torch.empty(2 * n + 64, dtype=torch.bfloat16, device="cuda")
+        buf[up:up + n].copy_(params["wup"].flatten())
+        if gate is not None:
+            buf[gate:gate + n].copy_(params["wgate"].flatten())
+            blk._w_c.wgate = buf.data_ptr() + 2 * gate
+        blk._w_c.wup = buf.data_ptr() + 2 * up
+        blk.forward(x)
+        got.append((blk.backward(dy), dict(blk.grads)))
+        torch.cuda.synchronize()
+    for dx, grads in got[1:]:
+        assert torch.equal(dx, got[0][0])
+        for name in sky1.PARAM_NAMES:
+            assert torch.equal(grads[name], got[0][1][name]), name
+    assert cdl._lib.device_status() == 0
