@@ -159,6 +159,7 @@ SIGNATURES = {
     "cdl_b200_mx_dequantize": ([_MX, _T, _vp], ctypes.c_int32),
     "cdl_b200_rmsnorm_fwd_mx": ([_T, _T, _T, ctypes.c_float, _MX, _MX, _T, _vp], ctypes.c_int32),
     "cdl_b200_matmul_mx": ([_MX, _MX, _T, _T, ctypes.c_float, ctypes.c_float, _vp], ctypes.c_int32),
+    "cdl_b200_matmul_mx_early": ([_MX, _MX, _T, _T, ctypes.c_float, ctypes.c_float, _vp], ctypes.c_int32),
     "cdl_b200_matmul_mx_rope": ([_MX, _MX, _T, ctypes.c_int32, ctypes.c_int32, _T, _vp], ctypes.c_int32),
     "cdl_b200_matmul_mx_opt": ([_MX, _MX, _T, _T, ctypes.c_float, ctypes.c_float, _MO, _vp],
                                ctypes.c_int32),

@@ -100,6 +100,7 @@ struct Params {
   const float* rope_table;
   int rope_seqlen, rope_cols;
   int* status;
+  int early;  // 1 = starts before the kernel ahead of it has finished (see grid_dep_wait)
 };
 
 struct Barriers {
@@ -620,7 +621,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
   cluster_sync_all();  // both CTAs' barriers exist before anything signals across the pair
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
-  grid_dep_wait();  // set-up above overlaps the previous kernel's tail; global memory from here on
+  if (!p.early) grid_dep_wait();  // set-up above overlaps the previous kernel's tail; global memory from here on
   grid_dep_launch();
 
   if (warp == 0) {
@@ -819,6 +820,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
     tmem_dealloc_pair(tmem_base, TMEM_COLS);
   }
   if (threadIdx.x == 0 && *abort_word != 0) atomicExch(p.status, *abort_word);
+  if (p.early) grid_dep_wait();
 }
 
 }  // namespace gemm_mx
@@ -826,7 +828,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 static int32_t matmul_mx_run(const char* op, const cdl_mx_tensor* a, const cdl_mx_tensor* b,
                              const cdl_tensor* c, const cdl_tensor* d, const cdl_mx_tensor* d_mx,
                              float alpha, float beta, cudaStream_t stream,
-                             const cdl_matmul_options* opts = nullptr, const RopeEpilogue* rope = nullptr) {
+                             const cdl_matmul_options* opts = nullptr, const RopeEpilogue* rope = nullptr,
+                             bool early = false) {
   using namespace gemm_mx;
   if (!a || !b || (!d && !d_mx)) return fail(CDL_ERR_INVALID, "%s: a, b and d are required", op);
   const int variant = opts ? opts->variant : CDL_GEMM_AUTO;
@@ -992,6 +995,7 @@ static int32_t matmul_mx_run(const char* op, const cdl_mx_tensor* a, const cdl_m
     CDL_CHECK(sf_map(&tsb, b->scale_factors, N));
     int grid = 2 * p.num_tiles < sm_count() ? 2 * p.num_tiles : sm_count();
     grid &= ~1;
+    p.early = early;  // (the one-CTA kernel always waits at its start)
     // D += alpha * A . B by TMA reductions, where they can describe D: every element is added to once.
     CUtensorMap td = ta;  // (a valid map where none is used)
     const bool add = p.c_mode == 2 && p.out_f32 && p.c == p.d && beta == 1.f && p.ldc == p.ldd &&
@@ -1053,6 +1057,12 @@ extern "C" {
 int32_t cdl_b200_matmul_mx(const cdl_mx_tensor* a, const cdl_mx_tensor* b, const cdl_tensor* c,
                            const cdl_tensor* d, float alpha, float beta, cdl_stream stream) {
   return cdl::matmul_mx_execute(a, b, c, d, alpha, beta, static_cast<cudaStream_t>(stream));
+}
+
+int32_t cdl_b200_matmul_mx_early(const cdl_mx_tensor* a, const cdl_mx_tensor* b, const cdl_tensor* c,
+                                 const cdl_tensor* d, float alpha, float beta, cdl_stream stream) {
+  return cdl::matmul_mx_run("matmul (block-scaled operands)", a, b, c, d, nullptr, alpha, beta,
+                            static_cast<cudaStream_t>(stream), nullptr, nullptr, true);
 }
 
 int32_t cdl_b200_matmul_mx_opt(const cdl_mx_tensor* a, const cdl_mx_tensor* b, const cdl_tensor* c,

@@ -155,6 +155,14 @@ def matmul_mx(a: MxTensor, b: MxTensor, out_dtype: torch.dtype = torch.bfloat16,
     return out
 
 
+def matmul_mx_early(a: MxTensor, b: MxTensor, out: torch.Tensor, c: Optional[torch.Tensor] = None,
+                    beta: float = 0.0) -> torch.Tensor:
+    """`out` = A . B + beta * C beside the product enqueued just before on this stream, of which it is independent."""
+    aa, ab, tc, td = a.arg(), b.arg(), tensor_arg(c), tensor_arg(out)
+    check(lib.cdl_b200_matmul_mx_early(ref(aa), ref(ab), ref(tc), ref(td), 1.0, beta, current_stream()))
+    return out
+
+
 def matmul_mx_rope(a: MxTensor, b: MxTensor, table: torch.Tensor, rot_heads: int, seqlen: int,
                    out: torch.Tensor) -> torch.Tensor:
     """bf16 `out` = A . B with the rotary embedding applied to its first `rot_heads` heads of 128 columns."""

@@ -314,6 +314,11 @@ int32_t cdl_b200_matmul_mx(const cdl_mx_tensor* a, const cdl_mx_tensor* b, const
 int32_t cdl_b200_matmul_mx_opt(const cdl_mx_tensor* a, const cdl_mx_tensor* b, const cdl_tensor* c,
                                const cdl_tensor* d, float alpha, float beta,
                                const cdl_matmul_options* options, cdl_stream stream);
+/* cdl_b200_matmul_mx that may run beside the product enqueued just before it on the stream (cdl_b200_matmul_mx or another of
+ * these): the caller states that neither reads or writes what the other, or one of these ahead of it, writes.  Whatever is
+ * enqueued next waits for both. */
+int32_t cdl_b200_matmul_mx_early(const cdl_mx_tensor* a, const cdl_mx_tensor* b, const cdl_tensor* c,
+                                 const cdl_tensor* d, float alpha, float beta, cdl_stream stream);
 /* D = RoPE(A . B) with MXFP8 operands: as cdl_b200_matmul_rope on dense sequences (bf16 [M, N], N % 128 == 0, 16-byte
  * aligned rows; heads [0, rot_heads) rotated by position row % seqlen); the same values as cdl_b200_matmul_mx and
  * cdl_b200_rope after it. */

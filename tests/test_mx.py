@@ -609,3 +609,30 @@ def test_matmul_mx_rope(cdl, gpu_ok, m, k, heads, rot, seqlen):
     assert torch.equal(out[:, rot * 128:], prod[:, rot * 128:])
     assert bool((buf[m:] == 7).all()) and bool((buf[:, heads * 128:] == 7).all())
     assert cdl._lib.device_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,k,n", [(64, 64, 96), (256, 128, 256), (700, 1024, 520), (2048, 2048, 5632)])
+def test_matmul_mx_early_beside_the_product_ahead(cdl, gpu_ok, m, k, n):
+    """Chains of products that start beside one another, and the ordinary product that reads what they wrote: the bits of the
+    ordinary calls, many times in a row; one row of tiles, several per CTA pair, the one-CTA kernel (up to 128 rows)."""
+    gen = torch.Generator(device="cuda").manual_seed(m + n)
+    r = lambda *s: torch.randn(*s, generator=gen, device="cuda").to(torch.bfloat16)
+    q = lambda t: cdl.mx.quantize(t, rowwise=True)[0]
+    a, b = [q(r(m, k)) for _ in range(3)], [q(r(n, k)).transposed() for _ in range(3)]
+    plain = [cdl.mx.matmul_mx(x, y) for x, y in zip(a, b)]
+    total = cdl.mx.matmul_mx(a[0], b[0], c=plain[2], beta=1.0)
+    grad = torch.randn(m, n, generator=gen, device="cuda")
+    ref = grad.clone()
+    cdl.mx.matmul_mx(a[1], b[1], out=ref, c=ref, beta=1.0)
+    for _ in range(20):
+        out = [torch.full_like(plain[0], float("nan")) for _ in range(3)]
+        got = grad.clone()
+        cdl.mx.matmul_mx(a[0], b[0], out=out[0])
+        cdl.mx.matmul_mx_early(a[1], b[1], got, c=got, beta=1.0)
+        cdl.mx.matmul_mx_early(a[1], b[1], out[1])
+        cdl.mx.matmul_mx_early(a[2], b[2], out[2])
+        last = cdl.mx.matmul_mx(a[0], b[0], c=out[2], beta=1.0)
+        assert all(torch.equal(o, p) for o, p in zip(out, plain))
+        assert torch.equal(got, ref) and torch.equal(last, total)
+    assert cdl._lib.device_status() == 0
