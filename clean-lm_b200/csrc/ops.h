@@ -18,6 +18,10 @@ int32_t matmul_execute(const cdl_tensor* a, const cdl_tensor* b, const cdl_tenso
 int32_t matmul_general_execute(const cdl_tensor* a, const cdl_tensor* b, const cdl_tensor* c,
                                const cdl_tensor* d, float alpha, float beta, void* scratch, size_t scratch_bytes,
                                cudaStream_t stream);
+// Zeros in the rows of a packed [rows] tensor that no sequence covers (of one longer than max_seqlen: its rest), beside the
+// kernel enqueued ahead, which must not touch them, and ahead of whatever comes next.
+int32_t clear_rest_execute(void* x, long long row_bytes, long long rows, const int32_t* cu_seqlens, int32_t num_seqs,
+                           int32_t max_seqlen, cudaStream_t stream);
 size_t matmul_general_scratch_bytes(const cdl_tensor* a, const cdl_tensor* b, const cdl_tensor* d);
 // Arguments of the RoPE epilogue (epi_mode 3): rotate-half RoPE on the heads (128 columns each)
 // below rot_cols of the product; position = row % seqlen, or the row's offset inside its sequence

@@ -219,7 +219,7 @@ int32_t sky1_block_fwd(const cdl_sky1_config* cfg, const cdl_sky1_weights* wt, c
     const cdl_tensor ao = attn_view_packed(sv->attn, d), lse = lse_view_packed(sv->lse, d);
     // Rows after the last sequence are not written by the attention kernel; they are read by the
     // output projection and, in the backward, by dWo += attn^T d_o, so they must not hold NaNs.
-    CDL_CUDA(cudaMemsetAsync(sv->attn, 0, static_cast<size_t>(d.T) * d.H * d.D * 2, st));
+    CDL_CHECK(clear_rest_execute(sv->attn, d.H * d.D * 2, d.T, d.rg->cu_seqlens, d.rg->num_seqs, d.rg->max_seqlen, st));
     CDL_CHECK(attn_fwd_packed_execute(&ad, &q, &k, &v, &cu, &cu, d.rg->max_seqlen, d.rg->max_seqlen,
                                       &ao, &lse, st));
   } else {
@@ -334,7 +334,7 @@ int32_t sky1_block_bwd(const cdl_sky1_config* cfg, const cdl_sky1_weights* wt, c
     const cdl_tensor cu = cu_view(d);
     // Rows after the last sequence get no gradient from the attention kernels: clear the buffer
     // so that the GEMMs that read all T rows of d_qkv see zeros there.
-    CDL_CUDA(cudaMemsetAsync(b.dqkv, 0, static_cast<size_t>(d.T) * d.QKV * 2, st));
+    CDL_CHECK(clear_rest_execute(b.dqkv, d.QKV * 2, d.T, d.rg->cu_seqlens, d.rg->num_seqs, d.rg->max_seqlen, st));
     const cdl_tensor q = head_view_packed(sv->qkv, d, 0, d.H), k = head_view_packed(sv->qkv, d, d.H, d.Hkv),
                      v = head_view_packed(sv->qkv, d, d.H + d.Hkv, d.Hkv);
     const cdl_tensor dq = head_view_packed(b.dqkv, d, 0, d.H), dk = head_view_packed(b.dqkv, d, d.H, d.Hkv),

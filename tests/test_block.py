@@ -431,3 +431,33 @@ def test_block_backward_weights_in_any_order(cdl, gpu_ok, dims):
         for name in sky1.PARAM_NAMES:
             assert torch.equal(grads[name], got[0][1][name]), name
     assert cdl._lib.device_status() == 0
+
+
+@pytest.mark.parametrize("lens,pad,bound", [((150, 37, 260), 6, 260), ((1,), 0, 1), ((5, 0, 300, 0, 64), 700, 300), ((130, 250), 3, 200)])
+def test_ragged_block_clears_rows_that_no_sequence_covers(cdl, gpu_ok, lens, pad, bound):
+    """Rows after the last sequence, and those of a sequence beyond the bound: results do not depend on what the attention's
+    buffers held there."""
+    sky1 = cdl.sky1
+    total = sum(lens) + pad
+    cfg = sky1.Sky1Config(batch=1, seqlen=total, hidden=256, heads=2, kv_heads=1, head_dim=128, ffn=384, deterministic=True)
+    params = sky1.init_params(cfg, seed=5, std=0.05)
+    x, dy = (torch.randn(total, cfg.hidden, generator=torch.Generator().manual_seed(i)).to(torch.bfloat16).cuda() for i in (6, 7))
+    cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32)
+    rest = [r for b, n in enumerate(lens) for r in range(int(cu[b]) + bound, int(cu[b + 1]))] + list(range(total - pad, total))
+    dy[rest] = 0
+    results = []
+    for fill in (0.0, float("nan")):
+        blk = sky1.Sky1Block(cfg, params, cu_seqlens=cu.cuda(), max_seqlen=bound)
+        blk.zero_grads()
+        blk.saved["attn"].fill_(fill)
+        blk.workspace.fill_(0 if fill == 0.0 else 0xff)
+        out = blk.forward(x)
+        attn = blk.saved["attn"].view(total, -1).clone()
+        blk.workspace.fill_(0 if fill == 0.0 else 0xff)
+        dx = blk.backward(dy)
+        torch.cuda.synchronize()
+        assert not attn[total - pad:].any()
+        results.append((out, dx, blk.grads["wqkv"], blk.grads["wo"]))
+        assert cdl._lib.device_status() == (0 if bound >= max(lens) else 921)  # (a sequence that is cut is reported)
+    for a, b in zip(*results):
+        assert torch.isfinite(b.float()).all() and torch.equal(a, b)
