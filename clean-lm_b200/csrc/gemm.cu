@@ -902,6 +902,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
     uint8_t* buf = staging + (warp - 2) * CHUNK_BYTES;
     const bool swiglu = p.epi_mode == 1 || p.epi_mode == 2;
     SwigluFeed feed{&tmap_e0, &tmap_e1, buf, &bars->extra_full[warp - 2], p.epi_mode == 2, 0};
+    if (p.early == 2) grid_dep_wait();
     int t = 0;
     for (;; ++t) {
       const int slot = t % SCHED_SLOTS;
@@ -1283,7 +1284,7 @@ int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_t
   p.sched_counter = nullptr;
   p.atomic_out = 0;
   p.tma_add = 0;
-  p.early = early;
+  p.early = (early & EARLY_PRODUCTS) ? (use_pair ? 2 : 0) : early > 0 ? 1 : 0;
   p.fold = second ? static_cast<int>(K1 / BK) : INT32_MAX;
   p.first_a = second && second->a < 0;
   p.first_b = second && second->b < 0;
@@ -1375,7 +1376,7 @@ int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_t
       p.c_mode = 0;
     }
     ProfileScope ps(PROF_GEMM, 2.0 * static_cast<double>(batch) * M * N * K, stream);
-    return gemm_cluster_launch(tm_a, tm_b, p, stream);
+    return gemm_cluster_launch(tm_a, tm_b, p, early, stream);
   }
 
   static std::once_flag attr_once[64];

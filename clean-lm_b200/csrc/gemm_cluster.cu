@@ -425,7 +425,7 @@ int32_t launch(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const Params& p
 }  // namespace
 
 int32_t gemm_cluster_launch(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const Params& p,
-                            cudaStream_t stream) {
+                            int early, cudaStream_t stream) {
   int dev = 0;
   CDL_CUDA(cudaGetDevice(&dev));
   // The walk pays where an SM gets two tiles or more.
@@ -438,7 +438,7 @@ int32_t gemm_cluster_launch(const CUtensorMap& tm_a, const CUtensorMap& tm_b, co
     });
     if (err != cudaSuccess) return fail(CDL_ERR_CUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(err));
     Params walk = p;
-    walk.sched_counter = sched_counter_for(gemm_counter_kind(p.early), dev, stream);  // launches of one stream that draw share a counter
+    walk.sched_counter = sched_counter_for(gemm_counter_kind(early), dev, stream);  // launches of one stream that draw share a counter
     CDL_CUDA(launch_pdl(gemm_cluster_walk_kernel, dim3(static_cast<unsigned>(sm_count())), dim3(WALK_THREADS),
                         WALK_SMEM_BYTES, stream, tm_a, tm_b, walk));
     return CDL_OK;

@@ -45,7 +45,9 @@ struct Params {
   // between launches; one counter per device and stream).
   unsigned int* sched_counter;
   int* status;
-  int early;  // 1 = starts before the kernel ahead of it has finished (see grid_dep_wait)
+  // 1 = starts before the kernel ahead of it has finished (see grid_dep_wait); 2 (CTA pairs) = the same, but what the
+  // epilogue reads comes from that kernel: the epilogue waits for it.
+  int early;
   // The sum of two products in one accumulator: K blocks from `fold` on are those of the second one.  Its operands are the
   // other matrix of their tensor maps' third dimension; which of the two lies first in memory is first_a, first_b.
   // fold is out of reach for others.
@@ -84,7 +86,7 @@ __device__ __forceinline__ float fast_sigmoid(float x) {
 // 64 x 64 (MN-major).
 constexpr int CLUSTER_TILE_N = 128;
 int32_t gemm_cluster_launch(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const Params& p,
-                            cudaStream_t stream);
+                            int early, cudaStream_t stream);
 
 // ------------------------------------------------------------------ D += alpha * accumulator
 // A warp's 32 rows x 32 columns of an f32 accumulator go to D as one TMA reduction from a 4 KiB buffer of shared

@@ -97,7 +97,7 @@ inline cudaError_t launch_pdl_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 
 // Device counter for a kernel that hands out its work at run time (see host.cu); nullptr: none.
 unsigned int* sched_counter_for(int kind, int dev, cudaStream_t stream);
 // The kind of a GEMM's counter; those that start early (1 to 4) may overlap and have one each.
-inline int gemm_counter_kind(int early) { return early > 0 ? 3 + early : 0; }
+inline int gemm_counter_kind(int early) { return (early & 7) > 0 ? 3 + (early & 7) : 0; }
 
 // Opt-in per-launch timing (cdl_b200_profile_start / _stop).  When enabled, a launcher brackets
 // its kernel with two pre-created CUDA events on the launching stream; when disabled the scope

@@ -232,7 +232,9 @@ int32_t sky1_block_fwd(const cdl_sky1_config* cfg, const cdl_sky1_weights* wt, c
   CDL_CHECK(rmsnorm_fwd_execute(&to, &g2, nullptr, cfg->eps, &th, nullptr, st));
   CDL_CHECK(matmul_execute(&th, &wup, nullptr, &tup, 1.f, 0.f, st));
   // gate = h2 Wgate and act = SiLU(gate) * up in one kernel (fused epilogue)
-  CDL_CHECK(matmul_execute_epi(&th, &wgate, nullptr, &tgate, 1.f, 0.f, 1, &tup, nullptr, &tact, st));
+  // (its products run beside the last tiles of the up projection, which only its epilogue reads)
+  CDL_CHECK(matmul_execute_epi(&th, &wgate, nullptr, &tgate, 1.f, 0.f, 1, &tup, nullptr, &tact, st, nullptr, nullptr,
+                               nullptr, 0, EARLY_PRODUCTS | 1));
   CDL_CHECK(matmul_execute(&tact, &wdown, &to, &tout, 1.f, 1.f, st));  // out = act Wdown + o
   return CDL_OK;
 }
