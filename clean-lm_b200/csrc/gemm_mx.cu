@@ -100,7 +100,7 @@ struct Params {
   const float* rope_table;
   int rope_seqlen, rope_cols;
   int* status;
-  int early;  // 1 = starts before the kernel ahead of it has finished (see grid_dep_wait)
+  int early;  // 1 = starts before the kernel ahead of it has finished (see grid_dep_wait): block of 8 x 2048 3975 -> 3917 us
 };
 
 struct Barriers {

