@@ -1188,11 +1188,13 @@ static int32_t launch_pieces(Params& p, const Operand& oa, const Operand& ob, co
 }
 
 // Whether the operands are laid out first: where that is estimated to be faster by a tenth, about what the estimates
-// miss.  Of 90 random shapes (M 8 .. 8192, K and N 64 .. 4096) it is taken for two thirds, f32 1.30 and bf16 1.44 times as
-// fast on average (general kernel -> laid out first, us; f32: 16 x 1027 x 2051 29.9 -> 21.1, 512 x 2051 x 1027 62 -> 32,
-// 2047 x 2047 x 2047 152 -> 92; the other way 2049 x 64 x 2049 19.8 and 30.5, 512 x 1027 x 2051 29.0 and 30.4,
-// 16 x 515 x 515 13.0 and 13.5.  bf16: 64 x 2049 x 2049 33.9 -> 15.2, 2047 x 2047 x 4095 167 -> 53; the other way
-// 1500 x 300 x 900 11.6 and 11.7, 250 x 129 x 131 9.7 and 9.9).
+// miss, and the other kernel takes long enough to hide the host's part: asking for the scratch, allocating it, a second
+// launch and two tensor maps cost an eager caller 7 us on top of the 11 of a call (three products of 529 x 2049 x 451, none
+// above 22 us: 51 us, all laid out 55).  General kernel -> laid out first, us; f32: 16 x 1027 x 2051 29.9 -> 21.1,
+// 512 x 2051 x 1027 62 -> 32, 2047 x 2047 x 2047 152 -> 92; the other way 2049 x 64 x 2049 19.8 and 30.5,
+// 512 x 1027 x 2051 29.0 and 30.4, 16 x 515 x 515 13.0 and 13.5.  bf16: 64 x 2049 x 2049 33.9 -> 15.2, 2047 x 2047 x 4095
+// 167 -> 53; the other way 1500 x 300 x 900 11.6 and 11.7, 250 x 129 x 131 9.7 and 9.9.  Of 90 random shapes (M 8 .. 8192, K and
+// N 64 .. 4096) those that it takes run f32 1.3 and bf16 1.8 times as fast on average.
 static bool worth_laying_out(const Operand& oa, const Operand& ob, const PiecePlan& plan, long long batch, long long K, bool f32,
                              bool fine) {
   const long long M = oa.mn, N = ob.mn, kb = (K + BK - 1) / BK;
@@ -1202,8 +1204,8 @@ static bool worth_laying_out(const Operand& oa, const Operand& ob, const PiecePl
   const long long m_tile = pair ? 2 * TILE : TILE, tiles = batch * ((M + m_tile - 1) / m_tile) * ((N + TILE - 1) / TILE);
   const int s = choose_piece_splits(f32, pair, tiles, static_cast<int>(kb));
   const double laid = (plan.lay_a ? 1.0 * M : 0.0) + (plan.lay_b ? 1.0 * N : 0.0);
-  return pieces_us(f32, pair, tiles, static_cast<int>(kb), s, laid * K * batch) <
-         0.9 * general_us(f32, batch, M, N, static_cast<int>(kb), !oa.pairs + !ob.pairs);
+  const double other = general_us(f32, batch, M, N, static_cast<int>(kb), !oa.pairs + !ob.pairs);
+  return other > 18.0 && pieces_us(f32, pair, tiles, static_cast<int>(kb), s, laid * K * batch) < 0.9 * other;
 }
 
 }  // namespace gemm_general

@@ -612,7 +612,8 @@ def test_fused_swiglu_epilogues_of_wide_tiles(cdl, gpu_ok, m, n, k, pad):
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("batch,m,k,n", [(1, 1, 64, 1), (1, 127, 129, 130), (3, 129, 200, 65), (1, 1000, 1027, 700), (1, 70, 4099, 33),
                                          (1, 400, 4099, 129), (16, 128, 515, 128), (1, 64, 2049, 2049),
-                                         (3, 385, 1540, 641)])
+                                         (3, 385, 1540, 641),
+                                         (1, 257, 4099, 193), (2, 130, 6000, 131), (1, 1025, 1027, 705)])
 @pytest.mark.parametrize("ta,tb", [(False, False), (True, False), (False, True)])
 def test_operands_laid_out_in_scratch(cdl, gpu_ok, dtype, batch, m, k, n, ta, tb):
     """Operands that TMA cannot read in place (one of them or both off the 16-byte grid, f32): with scratch for their
