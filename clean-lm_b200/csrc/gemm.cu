@@ -565,20 +565,20 @@ __global__ void __launch_bounds__(THREADS, 1)
           uint8_t* sa = smem + s * STAGE_BYTES;
           uint8_t* sb = sa + A_BYTES;
           mbar_arrive_expect_tx(&bars->full[s], STAGE_BYTES);
-          const int k0 = fold_k(p, kb), za = fold_z(p, kb, b, p.first_a), zb = fold_z(p, kb, b, p.first_b);
+          const int k0 = kb * BK;
           if (p.a_mn) {
 #pragma unroll
             for (int i = 0; i < BM / 64; ++i)
-              tma_load_3d(sa + i * 8192, &tmap_a, &bars->full[s], m0 + i * 64, k0, za);
+              tma_load_3d(sa + i * 8192, &tmap_a, &bars->full[s], m0 + i * 64, k0, b);
           } else {
-            tma_load_3d(sa, &tmap_a, &bars->full[s], k0, m0, za);
+            tma_load_3d(sa, &tmap_a, &bars->full[s], k0, m0, b);
           }
           if (p.b_mn) {
 #pragma unroll
             for (int i = 0; i < BN / 64; ++i)
-              tma_load_3d(sb + i * 8192, &tmap_b, &bars->full[s], n0 + i * 64, k0, zb);
+              tma_load_3d(sb + i * 8192, &tmap_b, &bars->full[s], n0 + i * 64, k0, b);
           } else {
-            tma_load_3d(sb, &tmap_b, &bars->full[s], k0, n0, zb);
+            tma_load_3d(sb, &tmap_b, &bars->full[s], k0, n0, b);
           }
         }
       }
@@ -828,20 +828,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
           // Bytes of both CTAs land on the leader's barrier.
           if (rank == 0) mbar_arrive_expect_tx(&bars->full[s], 2 * PAIR_STAGE_BYTES);
           const uint32_t full_leader = mapa_shared(smem_u32(&bars->full[s]), 0);
-          const int k0 = fold_k(p, kb), za = fold_z(p, kb, b, p.first_a), zb = fold_z(p, kb, b, p.first_b);
+          const int k0 = kb * BK;
           if (p.a_mn) {
 #pragma unroll
             for (int i = 0; i < BM / 64; ++i)
-              tma_load_3d_pair(sa + i * 8192, &tmap_a, full_leader, m0 + i * 64, k0, za);
+              tma_load_3d_pair(sa + i * 8192, &tmap_a, full_leader, m0 + i * 64, k0, b);
           } else {
-            tma_load_3d_pair(sa, &tmap_a, full_leader, k0, m0, za);
+            tma_load_3d_pair(sa, &tmap_a, full_leader, k0, m0, b);
           }
           if (p.b_mn) {
 #pragma unroll
             for (int i = 0; i < BN / 128; ++i)
-              tma_load_3d_pair(sb + i * 8192, &tmap_b, full_leader, n0 + i * 64, k0, zb);
+              tma_load_3d_pair(sb + i * 8192, &tmap_b, full_leader, n0 + i * 64, k0, b);
           } else {
-            tma_load_3d_pair(sb, &tmap_b, full_leader, k0, n0, zb);
+            tma_load_3d_pair(sb, &tmap_b, full_leader, k0, n0, b);
           }
         }
       }
@@ -1098,36 +1098,11 @@ int32_t matmul_execute(const cdl_tensor* a, const cdl_tensor* b, const cdl_tenso
                             scratch_bytes, early);
 }
 
-int32_t matmul_sum_execute(const cdl_tensor* a0, const cdl_tensor* b0, const cdl_tensor* a1, const cdl_tensor* b1,
-                           const cdl_tensor* d, cudaStream_t stream) {
-  // One tensor map reaches both matrices of an operand if they are laid out alike and a multiple of 16 bytes apart.
-  auto apart = [](const cdl_tensor* s, const cdl_tensor* t) {
-    return (reinterpret_cast<intptr_t>(t->ptr) - reinterpret_cast<intptr_t>(s->ptr)) / 2;
-  };
-  auto alike = [](const cdl_tensor* s, const cdl_tensor* t) {
-    return s->dtype == CDL_BF16 && t->dtype == CDL_BF16 && s->rank == 2 && t->rank == 2 && s->shape[0] == t->shape[0] &&
-           s->shape[1] == t->shape[1] && s->stride[0] == t->stride[0] && s->stride[1] == t->stride[1] &&
-           reinterpret_cast<uintptr_t>(s->ptr) % 16 == 0 && reinterpret_cast<uintptr_t>(t->ptr) % 16 == 0;
-  };
-  const long long da = apart(a0, a1), db = apart(b0, b1), most = 1LL << 38;
-  gemm::OperandLayout la, lb;
-  const bool one = alike(a0, a1) && alike(b0, b1) && a0->shape[1] % gemm::BK == 0 && a0->shape[1] <= INT32_MAX / 2 &&
-                   da != 0 && db != 0 && llabs(da) < most && llabs(db) < most &&
-                   gemm::analyze_operand("a", a0, true, &la) == CDL_OK && gemm::analyze_operand("b", b0, false, &lb) == CDL_OK;
-  if (!one) {
-    CDL_CHECK(matmul_execute(a0, b0, nullptr, d, 1.f, 0.f, stream));
-    return matmul_execute(a1, b1, d, d, 1.f, 1.f, stream);
-  }
-  const SecondProduct second{da, db};
-  return matmul_execute_epi(a0, b0, nullptr, d, 1.f, 0.f, 0, nullptr, nullptr, nullptr, stream,
-                            nullptr, nullptr, nullptr, 0, 0, &second);
-}
-
 int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_tensor* c,
                            const cdl_tensor* d, float alpha, float beta, int epi_mode,
                            const cdl_tensor* aux0, const cdl_tensor* aux1, const cdl_tensor* out2,
                            cudaStream_t stream, const cdl_matmul_options* opts, const RopeEpilogue* rope,
-                           void* scratch, size_t scratch_bytes, int early, const SecondProduct* second) {
+                           void* scratch, size_t scratch_bytes, int early) {
   using namespace gemm;
   const int variant = opts ? opts->variant : CDL_GEMM_AUTO;
   if (variant < CDL_GEMM_AUTO || variant > CDL_GEMM_CTA_PAIR)
@@ -1147,11 +1122,10 @@ int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_t
     return fail(CDL_ERR_INVALID, "matmul output must be f32 or bf16");
   const int r = a->rank;
   const long long batch = r == 3 ? a->shape[0] : 1;
-  const long long M = a->shape[r - 2], K1 = a->shape[r - 1], N = b->shape[r - 1];
-  const long long K = second ? 2 * K1 : K1;  // (of the two products, K1 % 64 == 0)
-  if (b->shape[r - 2] != K1)
+  const long long M = a->shape[r - 2], K = a->shape[r - 1], N = b->shape[r - 1];
+  if (b->shape[r - 2] != K)
     return fail(CDL_ERR_INVALID, "matmul contraction dimensions differ: a is [.., %lld, %lld], b is [.., %lld, %lld]",
-                M, K1, (long long)b->shape[r - 2], N);
+                M, K, (long long)b->shape[r - 2], N);
   if (r == 3 && (b->shape[0] != batch || d->shape[0] != batch))
     return fail(CDL_ERR_INVALID, "matmul batch dimensions differ");
   if (d->shape[r - 2] != M || d->shape[r - 1] != N)
@@ -1214,27 +1188,24 @@ int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_t
   CUtensorMap tm_a, tm_b;
   {
     // Innermost-first dims: K-major operand = [K, M|N, batch]; MN-major = [M|N, K, batch].
-    const uint64_t bs_a = static_cast<uint64_t>(second ? llabs(second->a) : batch > 1 ? la.batch : la.ld * (la.mn_major ? K : M)) * 2;
-    const uint64_t bs_b = static_cast<uint64_t>(second ? llabs(second->b) : batch > 1 ? lb.batch : lb.ld * (lb.mn_major ? K : N)) * 2;
+    const uint64_t bs_a = static_cast<uint64_t>(batch > 1 ? la.batch : la.ld * (la.mn_major ? K : M)) * 2;
+    const uint64_t bs_b = static_cast<uint64_t>(batch > 1 ? lb.batch : lb.ld * (lb.mn_major ? K : N)) * 2;
     uint64_t da[3], sa[3], db[3], sb[3];
     uint32_t ba[3], bb[3];
     if (la.mn_major) {
-      da[0] = M; da[1] = K1; ba[0] = 64; ba[1] = 64;
+      da[0] = M; da[1] = K; ba[0] = 64; ba[1] = 64;
     } else {
-      da[0] = K1; da[1] = M; ba[0] = 64; ba[1] = BM;
+      da[0] = K; da[1] = M; ba[0] = 64; ba[1] = BM;
     }
-    da[2] = second ? 2 : batch; ba[2] = 1; sa[0] = 0; sa[1] = la.ld * 2; sa[2] = bs_a;
+    da[2] = batch; ba[2] = 1; sa[0] = 0; sa[1] = la.ld * 2; sa[2] = bs_a;
     if (lb.mn_major) {
-      db[0] = N; db[1] = K1; bb[0] = 64; bb[1] = 64;
+      db[0] = N; db[1] = K; bb[0] = 64; bb[1] = 64;
     } else {
-      db[0] = K1; db[1] = N; bb[0] = 64; bb[1] = b_box_rows;
+      db[0] = K; db[1] = N; bb[0] = 64; bb[1] = b_box_rows;
     }
-    db[2] = second ? 2 : batch; bb[2] = 1; sb[0] = 0; sb[1] = lb.ld * 2; sb[2] = bs_b;
-    auto lower = [](const cdl_tensor* t, long long to_second) {
-      return static_cast<const __nv_bfloat16*>(t->ptr) + (to_second < 0 ? to_second : 0);
-    };
-    CDL_CHECK(encode_tmap(&tm_a, second ? lower(a, second->a) : a->ptr, CDL_BF16, 3, da, sa, ba, true));
-    CDL_CHECK(encode_tmap(&tm_b, second ? lower(b, second->b) : b->ptr, CDL_BF16, 3, db, sb, bb, true));
+    db[2] = batch; bb[2] = 1; sb[0] = 0; sb[1] = lb.ld * 2; sb[2] = bs_b;
+    CDL_CHECK(encode_tmap(&tm_a, a->ptr, CDL_BF16, 3, da, sa, ba, true));
+    CDL_CHECK(encode_tmap(&tm_b, b->ptr, CDL_BF16, 3, db, sb, bb, true));
   }
 
   Params p;
@@ -1285,9 +1256,6 @@ int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_t
   p.atomic_out = 0;
   p.tma_add = 0;
   p.early = (early & EARLY_PRODUCTS) ? (use_pair ? 2 : 0) : early > 0 ? 1 : 0;
-  p.fold = second ? static_cast<int>(K1 / BK) : INT32_MAX;
-  p.first_a = second && second->a < 0;
-  p.first_b = second && second->b < 0;
   p.epi_mode = 0;
   p.aux0 = p.aux1 = nullptr;
   p.out2 = nullptr;

@@ -76,12 +76,11 @@ __global__ void __launch_bounds__(THREADS, STAGES == SHARED_STAGES ? 2 : 1)
   if (warp == 2 && tm == 0 && !p.atomic_out) {
     if (elect_one()) {
       for (int kb = kb0; kb < kb1 && kb < kb0 + STAGES; ++kb) {
-        const int k0 = fold_k(p, kb), zb = fold_z(p, kb, b, p.first_b);
         if (p.b_mn) {
 #pragma unroll
-          for (int i = 0; i < TILE_N / 64; ++i) tma_prefetch_3d(&tmap_b, n0 + i * 64, k0, zb);
+          for (int i = 0; i < TILE_N / 64; ++i) tma_prefetch_3d(&tmap_b, n0 + i * 64, kb * BK, b);
         } else {
-          tma_prefetch_3d(&tmap_b, k0, n0, zb);
+          tma_prefetch_3d(&tmap_b, kb * BK, n0, b);
         }
       }
     }
@@ -109,20 +108,20 @@ __global__ void __launch_bounds__(THREADS, STAGES == SHARED_STAGES ? 2 : 1)
         uint8_t* sa = smem + s * STAGE_BYTES;
         uint8_t* sb = sa + A_BYTES;
         mbar_arrive_expect_tx(&bars->full[s], STAGE_BYTES);
-        const int k0 = fold_k(p, kb), za = fold_z(p, kb, b, p.first_a), zb = fold_z(p, kb, b, p.first_b);
+        const int k0 = kb * BK;
         if (p.a_mn) {
 #pragma unroll
           for (int i = 0; i < TILE_M / 64; ++i)
-            tma_load_3d(sa + i * 8192, &tmap_a, &bars->full[s], m0 + i * 64, k0, za);
+            tma_load_3d(sa + i * 8192, &tmap_a, &bars->full[s], m0 + i * 64, k0, b);
         } else {
-          tma_load_3d(sa, &tmap_a, &bars->full[s], k0, m0, za);
+          tma_load_3d(sa, &tmap_a, &bars->full[s], k0, m0, b);
         }
         if (p.b_mn) {
 #pragma unroll
           for (int i = 0; i < TILE_N / 64; ++i)
-            tma_load_3d(sb + i * 8192, &tmap_b, &bars->full[s], n0 + i * 64, k0, zb);
+            tma_load_3d(sb + i * 8192, &tmap_b, &bars->full[s], n0 + i * 64, k0, b);
         } else {
-          tma_load_3d(sb, &tmap_b, &bars->full[s], k0, n0, zb);
+          tma_load_3d(sb, &tmap_b, &bars->full[s], k0, n0, b);
         }
       }
     }

@@ -48,14 +48,7 @@ struct Params {
   // 1 = starts before the kernel ahead of it has finished (see grid_dep_wait); 2 (CTA pairs) = the same, but what the
   // epilogue reads comes from that kernel: the epilogue waits for it.
   int early;
-  // The sum of two products in one accumulator: K blocks from `fold` on are those of the second one.  Its operands are the
-  // other matrix of their tensor maps' third dimension; which of the two lies first in memory is first_a, first_b.
-  // fold is out of reach for others.
-  int fold, first_a, first_b;
 };
-// Coordinates of K block kb: along K, and of the matrix.
-__device__ __forceinline__ int fold_k(const Params& p, int kb) { return (kb < p.fold ? kb : kb - p.fold) * 64; }
-__device__ __forceinline__ int fold_z(const Params& p, int kb, int b, int first) { return kb < p.fold ? b + first : 1 - first; }
 
 __device__ __forceinline__ void tile_coords(const Params& p, int tile, int& b, int& m, int& n) {
   const int per_batch = p.num_m_tiles * p.num_n_tiles;

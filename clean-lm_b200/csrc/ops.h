@@ -36,10 +36,6 @@ struct RopeEpilogue {
   const int* cu_seqlens;
   int num_seqs;
 };
-// A second product of the same shape and layout added to the first: how far (elements) its operands lie from the first's.
-struct SecondProduct {
-  long long a, b;
-};
 // epi_mode 1: d = product, out2 = SiLU(product) * aux0.  epi_mode 2: d = SiLU(aux0) * product,
 // out2 = product * aux1 * dSiLU(aux0).  epi_mode 3: d = RoPE(product), see RopeEpilogue.
 int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_tensor* c,
@@ -47,11 +43,7 @@ int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_t
                            const cdl_tensor* aux0, const cdl_tensor* aux1, const cdl_tensor* out2,
                            cudaStream_t stream, const cdl_matmul_options* opts = nullptr,
                            const RopeEpilogue* rope = nullptr, void* scratch = nullptr, size_t scratch_bytes = 0,
-                           int early = 0, const SecondProduct* second = nullptr);
-// D = A0 . B0 + A1 . B1 (bf16, rank 2), as one product where one tensor map reaches both matrices of an operand: D is
-// rounded once and not read again (block of 1 x 256 tokens, 5632 wide: 307.8 -> 303.9 us).
-int32_t matmul_sum_execute(const cdl_tensor* a0, const cdl_tensor* b0, const cdl_tensor* a1, const cdl_tensor* b1,
-                           const cdl_tensor* d, cudaStream_t stream);
+                           int early = 0);
 // norm_general.cu: any float types, strides and column counts (layer = 0 RmsNorm, 1 LayerNorm).
 int32_t norm_general_execute(int layer, const cdl_tensor* x, const cdl_tensor* scale,
                              const cdl_tensor* bias, float eps, const cdl_tensor* y,

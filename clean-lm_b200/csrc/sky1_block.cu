@@ -315,7 +315,8 @@ int32_t sky1_block_bwd(const cdl_sky1_config* cfg, const cdl_sky1_weights* wt, c
                                nullptr, 0, 1));
   // h2 is not kept: the norm's backward gives it again (as a kernel of its own where the rows are too wide for that)
   // ahead of the weight gradients that need it.
-  CDL_CHECK(matmul_sum_execute(&tdact, &wupT, &tdgate, &wgateT, &tdh, st));         // dh2 = d_up Wup^T + d_gate Wgate^T
+  CDL_CHECK(matmul_execute(&tdact, &wupT, nullptr, &tdh, 1.f, 0.f, st));            // dh2 = d_up Wup^T
+  CDL_CHECK(matmul_execute(&tdgate, &wgateT, &tdh, &tdh, 1.f, 1.f, st));            // dh2 += d_gate Wgate^T
   if (!with_h) CDL_CHECK(rmsnorm_fwd_execute(&to, &g2, nullptr, cfg->eps, &th, &tr, st));
   CDL_CHECK(rmsnorm_bwd_execute(&to, &tdh, &tdy, &g2, &tr, &tdo, &dg2, b.norm_scratch, b.norm_scratch_bytes, st,
                                 nullptr, with_h ? &th : nullptr, cfg->eps));        // d_o (+ dy)

@@ -461,3 +461,33 @@ def test_ragged_block_clears_rows_that_no_sequence_covers(cdl, gpu_ok, lens, pad
         assert cdl._lib.device_status() == (0 if bound >= max(lens) else 921)  # (a sequence that is cut is reported)
     for a, b in zip(*results):
         assert torch.isfinite(b.float()).all() and torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dims", [dict(batch=1, seqlen=200, hidden=256, heads=2, kv_heads=2, head_dim=128, ffn=320),
+                                  dict(batch=2, seqlen=640, hidden=1024, heads=8, kv_heads=4, head_dim=128, ffn=2816),
+                                  dict(batch=1, seqlen=300, hidden=512, heads=4, kv_heads=4, head_dim=128, ffn=1400)])
+def test_block_backward_has_the_bits_of_its_operators(cdl, gpu_ok, dims):
+    """The feed-forward half of the backward, call by call through the operators: the same bits, dh2 among them, which is
+    the bf16 sum of two products."""
+    sky1, ops, L = cdl.sky1, cdl.ops, cdl._lib
+    cfg = sky1.Sky1Config(deterministic=True, **dims)
+    params = sky1.init_params(cfg, seed=3, std=cfg.hidden ** -0.5)
+    x, dy = (torch.randn(cfg.tokens, cfg.hidden, generator=torch.Generator().manual_seed(i)).to(torch.bfloat16).cuda() for i in (4, 5))
+    blk = sky1.Sky1Block(cfg, params)
+    blk.zero_grads()
+    blk.forward(x)
+    blk.backward(dy)
+    w, s = blk.params, blk.saved
+    d_up, d_gate = torch.empty_like(s["up"]), torch.empty_like(s["gate"])
+    args = [L.tensor_arg(t) for t in (dy, w["wdown"].T, s["gate"], s["up"], d_up, d_gate)]
+    L.check(L.lib.cdl_b200_matmul_swiglu_dgrad(*(L.ref(t) for t in args), None))
+    dh = ops.matmul(d_up, w["wup"].T)
+    ops.matmul(d_gate, w["wgate"].T, ops.MatmulOpts(c=dh, beta=1.0), out=dh)
+    h = ops.norm_fwd(s["o"], ops.NormFwdOpts(scale=w["norm2"], eps=cfg.eps, save_stats=True))
+    g = {n: torch.zeros_like(blk.grads[n]) for n in ("norm2", "wup", "wgate", "wo")}
+    d_o = ops.norm_bwd(s["o"], dh, w["norm2"], h.r_inv, g["norm2"], residual_dy=dy)
+    for name, left, right in (("wup", h.y, d_up), ("wgate", h.y, d_gate), ("wo", s["attn"], d_o)):
+        ops.matmul(left.T, right, ops.MatmulOpts(out=torch.float32, c=g[name], beta=1.0, deterministic=True), out=g[name])
+    for name, t in g.items():
+        assert torch.equal(blk.grads[name], t), name
+    assert L.device_status() == 0
