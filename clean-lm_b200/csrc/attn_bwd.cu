@@ -733,7 +733,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         uint32_t sr[2][32];
         tmem_ld32(tmem_base + lane_addr + KV_COL_S + wg * 64, sr[0]);
         tmem_ld32(tmem_base + lane_addr + KV_COL_S + wg * 64 + 32, sr[1]);
-        tmem_wait_ld();
+        tmem_wait_ld(sr[0], sr[1]);
         float x[64];
         const uint64_t scale2 = pk2(p.scale_log2, p.scale_log2);
 #pragma unroll
@@ -792,7 +792,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         uint32_t dr[2][32];
         tmem_ld32(tmem_base + lane_addr + KV_COL_DP + wg * 64, dr[0]);
         tmem_ld32(tmem_base + lane_addr + KV_COL_DP + wg * 64 + 32, dr[1]);
-        tmem_wait_ld();
+        tmem_wait_ld(dr[0], dr[1]);
         uint32_t pk[32];
 #pragma unroll
         for (int ch = 0; ch < 8; ++ch) {
@@ -850,7 +850,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             uint32_t a[32];
             if (iters > 0) {
               tmem_ld32(tmem_base + lane_addr + col + half * 32, a);
-              tmem_wait_ld();
+              tmem_wait_ld(a);
             } else {
 #pragma unroll
               for (int i = 0; i < 32; ++i) a[i] = 0u;
@@ -897,7 +897,7 @@ __global__ void __launch_bounds__(THREADS, 1)
           uint32_t a[32];
           if (iters > 0) {
             tmem_ld32(tmem_base + lane_addr + col + half * 32, a);
-            tmem_wait_ld();
+            tmem_wait_ld(a);
           } else {
 #pragma unroll
             for (int i = 0; i < 32; ++i) a[i] = 0u;
@@ -1343,7 +1343,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         uint32_t sr[2][32];
         tmem_ld32(tmem_base + lane_addr + KV_COL_S + wg * 64, sr[0]);
         tmem_ld32(tmem_base + lane_addr + KV_COL_S + wg * 64 + 32, sr[1]);
-        tmem_wait_ld();
+        tmem_wait_ld(sr[0], sr[1]);
         float x[64];
         const uint64_t scale2 = pk2(p.scale_log2, p.scale_log2);
 #pragma unroll
@@ -1410,7 +1410,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             uint32_t dr[2][32];
             tmem_ld32(tmem_base + lane_addr + KV_COL_DP + wg * 64, dr[0]);
             tmem_ld32(tmem_base + lane_addr + KV_COL_DP + wg * 64 + 32, dr[1]);
-            tmem_wait_ld();
+            tmem_wait_ld(dr[0], dr[1]);
             uint32_t pk[32];
 #pragma unroll
             for (int ch = 0; ch < 8; ++ch) {
@@ -1496,7 +1496,7 @@ __global__ void __launch_bounds__(THREADS, 1)
           for (int half = 0; half < 2; ++half) {
             uint32_t a[32];
             tmem_ld32(tmem_base + lane_addr + col + half * 32, a);
-            tmem_wait_ld();
+            tmem_wait_ld(a);
             const float sc = which == 0 ? 1.0f : p.scale;  // dS^T was accumulated without the scale
 #pragma unroll
             for (int gq = 0; gq < 4; ++gq) {
@@ -1774,7 +1774,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         uint32_t sr[2][32];
         tmem_ld32(tmem_base + lane_addr + Q_COL_S + s * 128 + wg * 64, sr[0]);
         tmem_ld32(tmem_base + lane_addr + Q_COL_S + s * 128 + wg * 64 + 32, sr[1]);
-        tmem_wait_ld();
+        tmem_wait_ld(sr[0], sr[1]);
         float x[64];
         const uint64_t scale2 = pk2(p.scale_log2, p.scale_log2), neg_lse2 = pk2(-lse2, -lse2);
 #pragma unroll
@@ -1795,7 +1795,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         uint32_t dr[2][32];
         tmem_ld32(tmem_base + lane_addr + Q_COL_DP + wg * 64, dr[0]);
         tmem_ld32(tmem_base + lane_addr + Q_COL_DP + wg * 64 + 32, dr[1]);
-        tmem_wait_ld();
+        tmem_wait_ld(dr[0], dr[1]);
         const uint64_t delta2 = pk2(delta, delta);
 #pragma unroll
         for (int c = 0; c < 32; ++c) {
@@ -1837,7 +1837,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         uint32_t a[32];
         if (n_kv > 0) {
           tmem_ld32(tmem_base + lane_addr + Q_COL_DQ + wg * 64 + half * 32, a);
-          tmem_wait_ld();
+          tmem_wait_ld(a);
         } else {
 #pragma unroll
           for (int i = 0; i < 32; ++i) a[i] = 0u;
@@ -2220,7 +2220,7 @@ __global__ void __launch_bounds__(THREADS, 1)
           uint32_t sr[2][32];
           tmem_ld32(tmem_base + lane_addr + Q_COL_S + s * 128 + wg * 64, sr[0]);
           tmem_ld32(tmem_base + lane_addr + Q_COL_S + s * 128 + wg * 64 + 32, sr[1]);
-          tmem_wait_ld();
+          tmem_wait_ld(sr[0], sr[1]);
           float x[64];
           const uint64_t scale2 = pk2(p.scale_log2, p.scale_log2), neg_lse2 = pk2(-lse2, -lse2);
 #pragma unroll
@@ -2241,7 +2241,7 @@ __global__ void __launch_bounds__(THREADS, 1)
           uint32_t dr[2][32];
           tmem_ld32(tmem_base + lane_addr + Q_COL_DP + wg * 64, dr[0]);
           tmem_ld32(tmem_base + lane_addr + Q_COL_DP + wg * 64 + 32, dr[1]);
-          tmem_wait_ld();
+          tmem_wait_ld(dr[0], dr[1]);
           const uint64_t delta2 = pk2(delta, delta);
 #pragma unroll
           for (int c = 0; c < 32; ++c) {
@@ -2300,7 +2300,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         for (int half = 0; half < 2; ++half) {
           uint32_t a[32];
           tmem_ld32(tmem_base + lane_addr + Q_COL_DQ + wg * 64 + half * 32, a);
-          tmem_wait_ld();
+          tmem_wait_ld(a);
           const float sc = p.scale;
 #pragma unroll
           for (int gq = 0; gq < 4; ++gq) {

@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       uint32_t sr[4][32];
 #pragma unroll
       for (int c = 0; c < 4; ++c) tmem_ld32(t_s + c * 32, sr[c]);
-      tmem_wait_ld();
+      tmem_wait_ld(sr[0], sr[1], sr[2], sr[3]);
       const int key0 = j * BKV;
       // Warp-uniform: does any row of this warp see a masked key in this block?
       const int warp_first_row = m0 + t * BQ + quad * 32;
@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         for (int c = 0; c < 4; ++c) {
           uint32_t orow[32];
           tmem_ld32(t_o + c * 32, orow);
-          tmem_wait_ld();
+          tmem_wait_ld(orow);
 #pragma unroll
           for (int i = 0; i < 32; ++i) orow[i] = __float_as_uint(__uint_as_float(orow[i]) * f);
           tmem_st32(t_o + c * 32, orow);
@@ -363,7 +363,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         uint32_t orow[32];
         if (n_t > 0) {
           tmem_ld32(t_o + c * 32, orow);
-          tmem_wait_ld();
+          tmem_wait_ld(orow);
         } else {
 #pragma unroll
           for (int i = 0; i < 32; ++i) orow[i] = 0u;

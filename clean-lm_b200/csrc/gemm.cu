@@ -149,7 +149,7 @@ __device__ __forceinline__ void store_tile_rows(const Params& p, uint32_t t_row,
     if (col0 >= p.N) break;  // warp-uniform
     uint32_t r[32];
     tmem_ld32(t_row + ch * 32, r);
-    tmem_wait_ld();
+    tmem_wait_ld(r);
     if (row_ok) {
       float v[32];
 #pragma unroll
@@ -326,7 +326,7 @@ __device__ __forceinline__ void store_tile_rows_rope(const Params& p, uint32_t t
     uint32_t lo[32], hi[32];
     tmem_ld32(t_row + pr * 32, lo);
     tmem_ld32(t_row + (pr + 2) * 32, hi);
-    tmem_wait_ld();
+    tmem_wait_ld(lo, hi);
     if (!row_ok) continue;
     uint32_t olo[16], ohi[16];
 #pragma unroll
@@ -445,9 +445,8 @@ __device__ __forceinline__ void store_tile_rows_swiglu(const Params& p, SwigluFe
     feed.phase ^= 1;
     feed.read(lane, 0, w0);
     if (TWO) feed.read(lane, 1, w1);
-    // (load and wait side by side: nothing ties the arithmetic on r to the wait but their order)
     tmem_ld32(t_row + ch * 32, r);
-    tmem_wait_ld();
+    tmem_wait_ld(r);
     __syncwarp();  // the buffer has been read
     if (ch + 1 < BN / 64 && col0 + 32 < p.N) feed.load(lane, row - lane, col0 + 32);
     uint32_t q1[16], q2[16];
@@ -498,7 +497,7 @@ __device__ __forceinline__ void add_tile_rows(const Params& p, const CUtensorMap
     if (col0 >= p.N) break;
     uint32_t r[32];
     tmem_ld32(t_row + ch * 32, r);
-    tmem_wait_ld();
+    tmem_wait_ld(r);
     if (lane == 0) tma_store_wait_read<0>();  // the buffer's last reduction has read it
     __syncwarp();
     add_chunk(tm_d, buf, r, p.alpha, lane, col0, row0, b);

@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(THREADS, STAGES == SHARED_STAGES ? 2 : 1)
       for (int c = half * 64; c < half * 64 + 64; c += 16) {
         uint32_t r[16];
         tmem_ld16(tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + c, r);
-        tmem_wait_ld();
+        tmem_wait_ld(r);
         float v[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
@@ -367,7 +367,7 @@ __global__ void __launch_bounds__(WALK_THREADS, 1)
           for (int c = half * 64; c < half * 64 + 64; c += 16) {
             uint32_t r[16];
             tmem_ld16(tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + acc * TILE_N + c, r);
-            tmem_wait_ld();
+            tmem_wait_ld(r);
             float v[16];
 #pragma unroll
             for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);

@@ -494,11 +494,11 @@ __global__ void __launch_bounds__(THREADS, 1)
         tmem_ld32(t_row + acc * TILE + c, r);
         if (g > 0) {
           tmem_ld32(t_row + 2 * TILE + c, t);
-          tmem_wait_ld();
+          tmem_wait_ld(r, t);
 #pragma unroll
           for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(t[j]) + __uint_as_float(r[j]));
         } else {
-          tmem_wait_ld();
+          tmem_wait_ld(r);
         }
         if (last) {
           // Every product is done and every stage read: the partial tile takes their place.
@@ -828,7 +828,7 @@ __global__ void __launch_bounds__(piece_threads<T>(), SLOTS == shared_slots(PAIR
       for (int c = 0; c < COLS; c += 16) {
         uint32_t r[16];
         tmem_ld16(t_row + acc * TILE + c, r);
-        tmem_wait_ld();
+        tmem_wait_ld(r);
 #pragma unroll
         for (int j = 0; j < 16; ++j) sum[c + j] = g == 0 ? __uint_as_float(r[j]) : sum[c + j] + __uint_as_float(r[j]);
       }

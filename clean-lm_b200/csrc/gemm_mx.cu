@@ -493,7 +493,8 @@ __global__ void __launch_bounds__(THREADS, 1)
         const int ch0 = backwards ? 3 : 0, ch1 = backwards ? 2 : 1;
         tmem_ld32(t_row + ch0 * 32, r0);
         if (C::OVL_CHUNKS == 2) tmem_ld32(t_row + ch1 * 32, r1);
-        tmem_wait_ld();
+        if constexpr (C::OVL_CHUNKS == 2) tmem_wait_ld(r0, r1);
+        else tmem_wait_ld(r0);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars->overlap_free);
@@ -506,7 +507,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         const int ch = backwards ? 3 - i : i;
         uint32_t r[32];
         tmem_ld32(t_row + ch * 32, r);
-        tmem_wait_ld();
+        tmem_wait_ld(r);
         emit(r, ch);
       }
       tc_fence_before();
@@ -763,7 +764,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
           uint32_t lo[32], hi[32];
           tmem_ld32(t_row + ch * 32, lo);
           tmem_ld32(t_row + (ch + 2) * 32, hi);
-          tmem_wait_ld();
+          tmem_wait_ld(lo, hi);
           if (owner && k == 0) {
             tc_fence_before();
             __syncwarp();
@@ -783,7 +784,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
         const int ch0 = backwards ? 3 : 0, ch1 = backwards ? 2 : 1;
         tmem_ld32(t_row + ch0 * 32, r0);
         if (C::OVL_CHUNKS == 2) tmem_ld32(t_row + ch1 * 32, r1);
-        tmem_wait_ld();
+        if constexpr (C::OVL_CHUNKS == 2) tmem_wait_ld(r0, r1);
+        else tmem_wait_ld(r0);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(ovl_leader);
@@ -796,7 +798,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
         const int ch = backwards ? 3 - i : i;
         uint32_t r[32];
         tmem_ld32(t_row + ch * 32, r);
-        tmem_wait_ld();
+        tmem_wait_ld(r);
         emit(r, ch);
       }
       tc_fence_before();
