@@ -116,8 +116,10 @@ if not LIB_PATH.exists():
     )
 
 lib = ctypes.CDLL(str(LIB_PATH))
+# The same library for callers that pass every `const cdl_tensor*` as the bytes of tensor_bytes(): nothing else is taken there.
+packed_lib = ctypes.CDLL(str(LIB_PATH))
 
-_T = ctypes.c_void_p  # const cdl_tensor*: what ref() gives, or byref() of a CdlTensor
+_T = ctypes.POINTER(CdlTensor)
 _MX = ctypes.POINTER(CdlMxTensor)
 _MO = ctypes.POINTER(CdlMatmulOptions)
 _NO = ctypes.POINTER(CdlNormOptions)
@@ -217,9 +219,10 @@ SIGNATURES = {
 }
 
 for _name, (_args, _res) in SIGNATURES.items():
-    _fn = getattr(lib, _name)
-    _fn.argtypes = _args
-    _fn.restype = _res
+    for _of, _tensor in ((lib, _T), (packed_lib, ctypes.c_char_p)):
+        _fn = getattr(_of, _name)
+        _fn.argtypes = [_tensor if a is _T else a for a in _args]
+        _fn.restype = _res
 
 
 def last_error() -> str:
@@ -237,12 +240,11 @@ _pack_tensor = _TENSOR_BYTES.pack
 _UNUSED = ((0, 0, 0, 0), (0, 0, 0), (0, 0), (0,), ())  # the dimensions a tensor of rank r leaves over
 
 
-def tensor_arg(t):
-    """A torch tensor (any strides) as the bytes of a cdl_tensor; None stays None (a NULL pointer).
+def tensor_bytes(t):
+    """A torch tensor (any strides) as the bytes of a cdl_tensor, for packed_lib; None stays None (a NULL pointer).
 
-    Bytes go to a `const cdl_tensor*` argument as they are.  A call of a small operator, which its host
-    time bounds, wraps three to eleven tensors: 0.8 us each, against 1.2 as a ctypes structure with a
-    byref() (field by field 2.7)."""
+    A call of a small operator, which its host time bounds, wraps three to eleven tensors: 0.8 us each, against
+    1.2 as a ctypes structure with a byref() (field by field 2.7)."""
     if t is None:
         return None
     dt = _dtype_codes().get(t.dtype)
@@ -256,6 +258,11 @@ def tensor_arg(t):
         raise CdlError(-1, f"rank {rank} exceeds 4")
     rest = _UNUSED[rank]
     return _pack_tensor(t.data_ptr(), dt, rank, *shape, *rest, *t.stride(), *rest)
+
+
+def tensor_arg(t):
+    """Wraps a torch tensor (any strides) as a cdl_tensor; None stays None (a NULL pointer)."""
+    return None if t is None else CdlTensor.from_buffer_copy(tensor_bytes(t))
 
 
 @functools.cache

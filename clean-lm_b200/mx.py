@@ -14,7 +14,7 @@ from typing import Optional
 import torch
 
 from . import _lib
-from ._lib import CdlMxTensor, check, current_stream, lib, ref, tensor_arg
+from ._lib import CdlMxTensor, check, current_stream, packed_lib, ref, tensor_bytes
 
 MXFP8, NVFP4 = _lib.CDL_MXFP8, _lib.CDL_NVFP4
 ROWWISE, COLWISE = _lib.CDL_MX_ROWWISE, _lib.CDL_MX_COLWISE
@@ -24,7 +24,7 @@ BLOCK = 32  # MXFP8; NVFP4 blocks hold 16 elements
 def layout_bytes(rows: int, cols: int, dim: int, fmt: int = MXFP8):
     """(values bytes, scale-factor bytes) of a block-scaled [rows, cols] tensor (`MxLayout::new`)."""
     v, s = ctypes.c_size_t(0), ctypes.c_size_t(0)
-    check(lib.cdl_b200_mx_layout(fmt, dim, rows, cols, ctypes.byref(v), ctypes.byref(s)))
+    check(packed_lib.cdl_b200_mx_layout(fmt, dim, rows, cols, ctypes.byref(v), ctypes.byref(s)))
     return v.value, s.value
 
 
@@ -78,28 +78,28 @@ def quantize(x: torch.Tensor, rowwise: bool = True, colwise: bool = False, fmt: 
     else:
         yr = MxTensor.empty(rows, cols, ROWWISE, x.device, zero_scales=True, fmt=fmt) if rowwise else None
         yc = MxTensor.empty(rows, cols, COLWISE, x.device, zero_scales=True, fmt=fmt) if colwise else None
-    tx, ar, ac = tensor_arg(x), _mx_arg(yr), _mx_arg(yc)
-    check(lib.cdl_b200_mx_quantize(ref(tx), ref(ar), ref(ac), current_stream()))
+    tx, ar, ac = tensor_bytes(x), _mx_arg(yr), _mx_arg(yc)
+    check(packed_lib.cdl_b200_mx_quantize(ref(tx), ref(ar), ref(ac), current_stream()))
     return yr, yc
 
 
 def swiglu_fwd(gate: torch.Tensor, up: torch.Tensor, out) -> None:
     """MXFP8 (rowwise, colwise) `out` = SiLU(gate) * up, rounded to bf16 in between."""
-    tg, tu, ar, ac = tensor_arg(gate), tensor_arg(up), out[0].arg(), out[1].arg()
-    check(lib.cdl_b200_mx_swiglu_fwd(ref(tg), ref(tu), ref(ar), ref(ac), current_stream()))
+    tg, tu, ar, ac = tensor_bytes(gate), tensor_bytes(up), out[0].arg(), out[1].arg()
+    check(packed_lib.cdl_b200_mx_swiglu_fwd(ref(tg), ref(tu), ref(ar), ref(ac), current_stream()))
 
 
 def swiglu_bwd(d_act: torch.Tensor, gate: torch.Tensor, up: torch.Tensor, d_gate, d_up) -> None:
     """The gradients of SwiGLU in the same form: `d_gate` and `d_up` are (rowwise, colwise) pairs."""
-    ts = [tensor_arg(t) for t in (d_act, gate, up)]
+    ts = [tensor_bytes(t) for t in (d_act, gate, up)]
     outs = [t.arg() for t in (*d_gate, *d_up)]
-    check(lib.cdl_b200_mx_swiglu_bwd(*(ref(t) for t in ts), *(ref(t) for t in outs), current_stream()))
+    check(packed_lib.cdl_b200_mx_swiglu_bwd(*(ref(t) for t in ts), *(ref(t) for t in outs), current_stream()))
 
 
 def dequantize(t: MxTensor, dtype: torch.dtype = torch.float32) -> torch.Tensor:
     y = torch.empty(t.rows, t.cols, dtype=dtype, device=t.values.device)
-    a, ty = t.arg(), tensor_arg(y)
-    check(lib.cdl_b200_mx_dequantize(ref(a), ref(ty), current_stream()))
+    a, ty = t.arg(), tensor_bytes(y)
+    check(packed_lib.cdl_b200_mx_dequantize(ref(a), ref(ty), current_stream()))
     return y
 
 
@@ -128,9 +128,9 @@ def norm_fwd_mx(x: torch.Tensor, scale: Optional[torch.Tensor] = None,
         yr = MxTensor.empty(rows, cols, ROWWISE, x.device, zero_scales=True, fmt=fmt)
         yc = MxTensor.empty(rows, cols, COLWISE, x.device, zero_scales=True, fmt=fmt) if colwise else None
         r_inv = torch.empty(rows, dtype=torch.float32, device=x.device) if save_stats else None
-    tx, ts, tb, tr = tensor_arg(x), tensor_arg(scale), tensor_arg(bias), tensor_arg(r_inv)
+    tx, ts, tb, tr = tensor_bytes(x), tensor_bytes(scale), tensor_bytes(bias), tensor_bytes(r_inv)
     ar, ac = _mx_arg(yr), _mx_arg(yc)
-    check(lib.cdl_b200_rmsnorm_fwd_mx(ref(tx), ref(ts), ref(tb), eps, ref(ar), ref(ac), ref(tr),
+    check(packed_lib.cdl_b200_rmsnorm_fwd_mx(ref(tx), ref(ts), ref(tb), eps, ref(ar), ref(ac), ref(tr),
                                       current_stream()))
     return NormMxOutputs(yr, yc, r_inv)
 
@@ -142,32 +142,32 @@ def matmul_mx(a: MxTensor, b: MxTensor, out_dtype: torch.dtype = torch.bfloat16,
     (accumulation in place).  `variant`: cdl_gemm_variant (0 = the library's heuristic)."""
     if out is None:
         out = torch.empty(a.rows, b.cols, dtype=out_dtype, device=a.values.device)
-    aa, ab, tc, td = a.arg(), b.arg(), tensor_arg(c), tensor_arg(out)
+    aa, ab, tc, td = a.arg(), b.arg(), tensor_bytes(c), tensor_bytes(out)
     if variant != 0:
         import ctypes
 
         from ._lib import CdlMatmulOptions
         mo = CdlMatmulOptions(int(variant), 0)
-        check(lib.cdl_b200_matmul_mx_opt(ref(aa), ref(ab), ref(tc), ref(td), alpha, beta,
+        check(packed_lib.cdl_b200_matmul_mx_opt(ref(aa), ref(ab), ref(tc), ref(td), alpha, beta,
                                          ctypes.byref(mo), current_stream()))
         return out
-    check(lib.cdl_b200_matmul_mx(ref(aa), ref(ab), ref(tc), ref(td), alpha, beta, current_stream()))
+    check(packed_lib.cdl_b200_matmul_mx(ref(aa), ref(ab), ref(tc), ref(td), alpha, beta, current_stream()))
     return out
 
 
 def matmul_mx_early(a: MxTensor, b: MxTensor, out: torch.Tensor, c: Optional[torch.Tensor] = None,
                     beta: float = 0.0) -> torch.Tensor:
     """`out` = A . B + beta * C beside the product enqueued just before on this stream, of which it is independent."""
-    aa, ab, tc, td = a.arg(), b.arg(), tensor_arg(c), tensor_arg(out)
-    check(lib.cdl_b200_matmul_mx_early(ref(aa), ref(ab), ref(tc), ref(td), 1.0, beta, current_stream()))
+    aa, ab, tc, td = a.arg(), b.arg(), tensor_bytes(c), tensor_bytes(out)
+    check(packed_lib.cdl_b200_matmul_mx_early(ref(aa), ref(ab), ref(tc), ref(td), 1.0, beta, current_stream()))
     return out
 
 
 def matmul_mx_rope(a: MxTensor, b: MxTensor, table: torch.Tensor, rot_heads: int, seqlen: int,
                    out: torch.Tensor) -> torch.Tensor:
     """bf16 `out` = A . B with the rotary embedding applied to its first `rot_heads` heads of 128 columns."""
-    aa, ab, tt, td = a.arg(), b.arg(), tensor_arg(table), tensor_arg(out)
-    check(lib.cdl_b200_matmul_mx_rope(ref(aa), ref(ab), ref(tt), rot_heads, seqlen, ref(td), current_stream()))
+    aa, ab, tt, td = a.arg(), b.arg(), tensor_bytes(table), tensor_bytes(out)
+    check(packed_lib.cdl_b200_matmul_mx_rope(ref(aa), ref(ab), ref(tt), rot_heads, seqlen, ref(td), current_stream()))
     return out
 
 
@@ -177,5 +177,5 @@ def matmul_mx_out(a: MxTensor, b: MxTensor, dim: int = ROWWISE, alpha: float = 1
     if out is None:
         out = MxTensor.empty(a.rows, b.cols, dim, a.values.device, zero_scales=True, fmt=fmt)
     aa, ab, ad = a.arg(), b.arg(), out.arg()
-    check(lib.cdl_b200_matmul_mx_out(ref(aa), ref(ab), ref(ad), alpha, current_stream()))
+    check(packed_lib.cdl_b200_matmul_mx_out(ref(aa), ref(ab), ref(ad), alpha, current_stream()))
     return out

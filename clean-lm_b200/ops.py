@@ -19,7 +19,7 @@ from typing import Optional
 import torch
 
 from . import _lib
-from ._lib import CdlAttnDesc, check, current_stream, lib, ref, tensor_arg
+from ._lib import CdlAttnDesc, check, current_stream, packed_lib, ref, tensor_bytes
 
 
 def _require_cuda(*tensors):
@@ -56,19 +56,19 @@ def matmul(a: torch.Tensor, b: torch.Tensor, opts: MatmulOpts | None = None,
         raise _lib.CdlError(-1, f"matmul contraction dimensions differ: {tuple(sa)} x {tuple(sb)}")
     if out is None:
         out = torch.empty(*sa[:-1], sb[-1], dtype=opts.out, device=a.device)
-    ta, tb, tc, td = tensor_arg(a), tensor_arg(b), tensor_arg(opts.c), tensor_arg(out)
+    ta, tb, tc, td = tensor_bytes(a), tensor_bytes(b), tensor_bytes(opts.c), tensor_bytes(out)
     scratch, scratch_bytes = None, 0
     if not (_on_grid(a) and _on_grid(b)):
         n = ctypes.c_size_t(0)
-        check(lib.cdl_b200_matmul_scratch_bytes(ta, tb, td, ctypes.byref(n)))
+        check(packed_lib.cdl_b200_matmul_scratch_bytes(ta, tb, td, ctypes.byref(n)))
         if n.value:
             block = torch.empty(n.value, dtype=torch.uint8, device=out.device)
             scratch, scratch_bytes = block.data_ptr(), n.value
     if opts.variant == _lib.GEMM_AUTO and not opts.deterministic:
-        check(lib.cdl_b200_matmul(ta, tb, tc, td, opts.alpha, opts.beta, scratch, scratch_bytes, current_stream()))
+        check(packed_lib.cdl_b200_matmul(ta, tb, tc, td, opts.alpha, opts.beta, scratch, scratch_bytes, current_stream()))
     else:
         mo = _lib.CdlMatmulOptions(int(opts.variant), 1 if opts.deterministic else 0)
-        check(lib.cdl_b200_matmul_opt(ta, tb, tc, td, opts.alpha, opts.beta, ctypes.byref(mo), scratch, scratch_bytes,
+        check(packed_lib.cdl_b200_matmul_opt(ta, tb, tc, td, opts.alpha, opts.beta, ctypes.byref(mo), scratch, scratch_bytes,
                                       current_stream()))
     return out
 
@@ -84,8 +84,8 @@ def matmul_candidates(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor) -> li
     (what an Executor would hand the tuner, op.rs:301-318)."""
     buf = (_lib.CdlMatmulOptions * 8)()
     n = ctypes.c_int32(0)
-    ta, tb, td = tensor_arg(a), tensor_arg(b), tensor_arg(out)
-    check(lib.cdl_b200_matmul_candidates(ref(ta), ref(tb), ref(td), buf, 8, ctypes.byref(n)))
+    ta, tb, td = tensor_bytes(a), tensor_bytes(b), tensor_bytes(out)
+    check(packed_lib.cdl_b200_matmul_candidates(ref(ta), ref(tb), ref(td), buf, 8, ctypes.byref(n)))
     return [(buf[i].variant, bool(buf[i].deterministic)) for i in range(n.value)]
 
 
@@ -119,27 +119,27 @@ def norm_fwd(x: torch.Tensor, opts: NormFwdOpts | None = None) -> NormFwdOutputs
         raise _lib.CdlError(-1, "norm_fwd: x must be a 2D tensor")
     y = torch.empty(x.shape, dtype=opts.out, device=x.device)
     r_inv = torch.empty(x.shape[0], dtype=torch.float32, device=x.device) if opts.save_stats else None
-    tx, ts, tb, ty, tr = (tensor_arg(t) for t in (x, opts.scale, opts.bias, y, r_inv))
+    tx, ts, tb, ty, tr = (tensor_bytes(t) for t in (x, opts.scale, opts.bias, y, r_inv))
     if opts.norm_type == "layer":
         mean = torch.empty(x.shape[0], dtype=torch.float32, device=x.device) if opts.save_stats else None
-        tm = tensor_arg(mean)
-        check(lib.cdl_b200_layernorm_fwd(ref(tx), ref(ts), ref(tb), opts.eps, ref(ty), ref(tm), ref(tr),
+        tm = tensor_bytes(mean)
+        check(packed_lib.cdl_b200_layernorm_fwd(ref(tx), ref(ts), ref(tb), opts.eps, ref(ty), ref(tm), ref(tr),
                                          current_stream()))
         return NormFwdOutputs(y, r_inv, mean)
     if opts.norm_type != "rms":
         raise _lib.CdlError(-1, f"norm_fwd: unknown norm type '{opts.norm_type}'")
     if opts.variant != _lib.NORM_AUTO:
         no = _lib.CdlNormOptions(int(opts.variant))
-        check(lib.cdl_b200_rmsnorm_fwd_opt(ref(tx), ref(ts), ref(tb), opts.eps, ref(ty), ref(tr),
+        check(packed_lib.cdl_b200_rmsnorm_fwd_opt(ref(tx), ref(ts), ref(tb), opts.eps, ref(ty), ref(tr),
                                            ctypes.byref(no), current_stream()))
         return NormFwdOutputs(y, r_inv)
-    check(lib.cdl_b200_rmsnorm_fwd(ref(tx), ref(ts), ref(tb), opts.eps, ref(ty), ref(tr), current_stream()))
+    check(packed_lib.cdl_b200_rmsnorm_fwd(ref(tx), ref(ts), ref(tb), opts.eps, ref(ty), ref(tr), current_stream()))
     return NormFwdOutputs(y, r_inv)
 
 
 def norm_bwd_scratch_bytes(rows: int, cols: int) -> int:
     n = ctypes.c_size_t(0)
-    check(lib.cdl_b200_rmsnorm_bwd_scratch_bytes(rows, cols, ctypes.byref(n)))
+    check(packed_lib.cdl_b200_rmsnorm_bwd_scratch_bytes(rows, cols, ctypes.byref(n)))
     return n.value
 
 
@@ -155,14 +155,14 @@ def norm_bwd(x, dy, scale, r_inv, dscale, residual_dy=None, scratch=None, dx=Non
     need = norm_bwd_scratch_bytes(x.shape[0], x.shape[1])
     if scratch is None:
         scratch = torch.empty(max(need, 16), dtype=torch.uint8, device=x.device)
-    args = [tensor_arg(t) for t in (x, dy, residual_dy, scale, r_inv, dx, dscale)]
+    args = [tensor_bytes(t) for t in (x, dy, residual_dy, scale, r_inv, dx, dscale)]
     if variant != _lib.NORM_AUTO:
         no = _lib.CdlNormOptions(int(variant))
-        check(lib.cdl_b200_rmsnorm_bwd_opt(*(ref(a) for a in args), ctypes.byref(no),
+        check(packed_lib.cdl_b200_rmsnorm_bwd_opt(*(ref(a) for a in args), ctypes.byref(no),
                                            ctypes.c_void_p(scratch.data_ptr()),
                                            scratch.numel() * scratch.element_size(), current_stream()))
         return dx
-    check(lib.cdl_b200_rmsnorm_bwd(*(ref(a) for a in args), ctypes.c_void_p(scratch.data_ptr()),
+    check(packed_lib.cdl_b200_rmsnorm_bwd(*(ref(a) for a in args), ctypes.c_void_p(scratch.data_ptr()),
                                    scratch.numel() * scratch.element_size(), current_stream()))
     return dx
 
@@ -219,9 +219,9 @@ def attention_fwd(q, k, v, opts: AttentionOpts | None = None, lse: bool = True,
         lse_t = (torch.empty(q.shape[1], q.shape[0], dtype=torch.float32, device=q.device)
                  if lse else None)
         desc = _attn_desc(opts)
-        a = [tensor_arg(t) for t in (q, k, v, opts.cu_seqlens_q, opts.cu_seqlens_k)]
-        b = [tensor_arg(t) for t in (out, lse_t)]
-        check(lib.cdl_b200_attn_fwd_packed(ctypes.byref(desc), *(ref(x) for x in a),
+        a = [tensor_bytes(t) for t in (q, k, v, opts.cu_seqlens_q, opts.cu_seqlens_k)]
+        b = [tensor_bytes(t) for t in (out, lse_t)]
+        check(packed_lib.cdl_b200_attn_fwd_packed(ctypes.byref(desc), *(ref(x) for x in a),
                                            int(opts.max_seqlen_q or 0), int(opts.max_seqlen_k or 0),
                                            *(ref(x) for x in b), current_stream()))
         return AttentionFwdOutputs(out, lse_t)
@@ -232,15 +232,15 @@ def attention_fwd(q, k, v, opts: AttentionOpts | None = None, lse: bool = True,
     lse_t = (torch.empty(q.shape[0], q.shape[2], q.shape[1], dtype=torch.float32, device=q.device)
              if lse else None)
     desc = _attn_desc(opts)
-    args = [tensor_arg(t) for t in (q, k, v, out, lse_t)]
-    check(lib.cdl_b200_attn_fwd(ctypes.byref(desc), *(ref(a) for a in args), current_stream()))
+    args = [tensor_bytes(t) for t in (q, k, v, out, lse_t)]
+    check(packed_lib.cdl_b200_attn_fwd(ctypes.byref(desc), *(ref(a) for a in args), current_stream()))
     return AttentionFwdOutputs(out, lse_t)
 
 
 def attention_bwd_scratch_bytes(q, k) -> int:
     n = ctypes.c_size_t(0)
-    tq, tk = tensor_arg(q), tensor_arg(k)
-    check(lib.cdl_b200_attn_bwd_scratch_bytes(ref(tq), ref(tk), ctypes.byref(n)))
+    tq, tk = tensor_bytes(q), tensor_bytes(k)
+    check(packed_lib.cdl_b200_attn_bwd_scratch_bytes(ref(tq), ref(tk), ctypes.byref(n)))
     return n.value
 
 
@@ -264,16 +264,16 @@ def attention_bwd(q, k, v, out, d_out, lse, opts: AttentionOpts | None = None, s
         batch = opts.cu_seqlens_q.shape[0] - 1
         max_q = int(opts.max_seqlen_q or 0)
         n = ctypes.c_size_t(0)
-        check(lib.cdl_b200_attn_bwd_packed_scratch_bytes(
+        check(packed_lib.cdl_b200_attn_bwd_packed_scratch_bytes(
             batch, max_q if 0 < max_q <= q.shape[0] else q.shape[0], q.shape[1], ctypes.byref(n)))
         if scratch is None:
             scratch = torch.empty(max(n.value, 16), dtype=torch.uint8, device=q.device)
         desc = _attn_desc(opts)
-        a = [tensor_arg(t) for t in (q, k, v, out, d_out, lse, opts.cu_seqlens_q, opts.cu_seqlens_k)]
-        b = [tensor_arg(t) for t in (dq, dk, dv)]
+        a = [tensor_bytes(t) for t in (q, k, v, out, d_out, lse, opts.cu_seqlens_q, opts.cu_seqlens_k)]
+        b = [tensor_bytes(t) for t in (dq, dk, dv)]
         if rope_table is not None:
-            b.insert(0, tensor_arg(rope_table))
-        fn = lib.cdl_b200_attn_bwd_packed if rope_table is None else lib.cdl_b200_attn_bwd_packed_rope
+            b.insert(0, tensor_bytes(rope_table))
+        fn = packed_lib.cdl_b200_attn_bwd_packed if rope_table is None else packed_lib.cdl_b200_attn_bwd_packed_rope
         check(fn(ctypes.byref(desc), *(ref(x) for x in a), max_q, int(opts.max_seqlen_k or 0),
                  *(ref(x) for x in b), ctypes.c_void_p(scratch.data_ptr()),
                  scratch.numel() * scratch.element_size(), current_stream()))
@@ -283,8 +283,8 @@ def attention_bwd(q, k, v, out, d_out, lse, opts: AttentionOpts | None = None, s
         scratch = torch.empty(max(need, 16), dtype=torch.uint8, device=q.device)
     desc = _attn_desc(opts)
     tensors = (q, k, v, out, d_out, lse) + (() if rope_table is None else (rope_table,)) + (dq, dk, dv)
-    args = [tensor_arg(t) for t in tensors]
-    fn = lib.cdl_b200_attn_bwd if rope_table is None else lib.cdl_b200_attn_bwd_rope
+    args = [tensor_bytes(t) for t in tensors]
+    fn = packed_lib.cdl_b200_attn_bwd if rope_table is None else packed_lib.cdl_b200_attn_bwd_rope
     check(fn(ctypes.byref(desc), *(ref(a) for a in args), ctypes.c_void_p(scratch.data_ptr()),
              scratch.numel() * scratch.element_size(), current_stream()))
     return dq, dk, dv

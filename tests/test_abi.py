@@ -4,6 +4,8 @@ import ctypes
 import re
 from pathlib import Path
 
+import pytest
+
 ROOT = Path(__file__).resolve().parent.parent
 
 
@@ -54,6 +56,28 @@ def test_host_validation_needs_no_gpu(cdl):
     x = L.CdlTensor(ptr=256, dtype=L.CDL_BF16, rank=3)
     st = L.lib.cdl_b200_rmsnorm_fwd(ctypes.byref(x), None, None, 1e-6, ctypes.byref(x), None, None)
     assert st == -1 and "2D" in L.last_error()
+
+
+def test_tensor_arguments_take_tensors_only(cdl):
+    """A `const cdl_tensor*` is a CdlTensor by reference (packed_lib: its bytes): an address or the descriptor of a
+    block-scaled tensor in its place is refused by the binding, not read as a tensor."""
+    import torch
+
+    L = cdl._lib
+    a, b = torch.zeros(8, 16, dtype=torch.bfloat16), torch.zeros(24, 8, dtype=torch.bfloat16)
+    ta, tb = L.tensor_arg(a), L.tensor_arg(b)
+    assert isinstance(ta, L.CdlTensor) and bytes(ta) == L.tensor_bytes(a)
+    assert (ta.ptr, ta.rank, list(ta.shape), list(ta.stride)) == (a.data_ptr(), 2, [8, 16, 0, 0], [16, 1, 0, 0])
+    rest = (1.0, 0.0, None, 0, None)
+    assert L.lib.cdl_b200_matmul(ctypes.byref(ta), L.ref(tb), None, ctypes.byref(ta), *rest) == -1
+    assert "contraction" in L.last_error()
+    pa, pb = L.tensor_bytes(a), L.tensor_bytes(b)
+    assert L.packed_lib.cdl_b200_matmul(pa, pb, None, pa, *rest) == -1 and "contraction" in L.last_error()
+    mx = L.CdlMxTensor(a.data_ptr(), b.data_ptr(), L.CDL_MXFP8, L.CDL_MX_ROWWISE, 8, 32)
+    for bad in (ctypes.byref(mx), ctypes.addressof(ta), 4096):
+        for f, good in ((L.lib.cdl_b200_matmul, ctypes.byref(ta)), (L.packed_lib.cdl_b200_matmul, pa)):
+            with pytest.raises(ctypes.ArgumentError):
+                f(good, bad, None, good, *rest)
 
 
 def test_candidates_need_no_gpu_and_put_the_heuristic_first(cdl):
