@@ -121,3 +121,17 @@ def test_candidates_need_no_gpu_and_put_the_heuristic_first(cdl):
     st = L.lib.cdl_b200_matmul_opt(ctypes.byref(a), ctypes.byref(b), None, ctypes.byref(d), 1.0, 0.0,
                                    ctypes.byref(mo), None, 0, None)
     assert st == -1 and "variant" in L.last_error()
+
+
+def test_current_stream_without_torch_internals(cdl, monkeypatch):
+    """The stream's handle comes from a private function of torch, and from the public one where that is missing."""
+    import types
+
+    import torch
+
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 3)
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda device: 40 + device, raising=False)
+    assert cdl._lib.current_stream() == 43
+    monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream")
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: types.SimpleNamespace(cuda_stream=77))
+    assert cdl._lib.current_stream() == 77
