@@ -45,7 +45,11 @@ class MatmulOpts:
 def matmul(a: torch.Tensor, b: torch.Tensor, opts: MatmulOpts | None = None,
            out: torch.Tensor | None = None) -> torch.Tensor:
     """D = alpha * A . B + beta * C.  `a`/`b` may be transposed views (`.mT`); `out` may be
-    given to write in place (e.g. out = c for accumulating wgrads)."""
+    given to write in place (e.g. out = c for accumulating wgrads).
+
+    f32 operands, and bf16 ones whose rows are off the 16-byte grid, are converted to bf16 pieces first where that is
+    faster: scratch of 6 bytes per f32 element and 2 per bf16 one, for the time of the call.  Where the memory is not
+    there the product runs without it."""
     opts = opts or MatmulOpts()
     _require_cuda(a, b, opts.c, out)
     sa, sb = a.shape, b.shape
@@ -62,8 +66,11 @@ def matmul(a: torch.Tensor, b: torch.Tensor, opts: MatmulOpts | None = None,
         n = ctypes.c_size_t(0)
         check(packed_lib.cdl_b200_matmul_scratch_bytes(ta, tb, td, ctypes.byref(n)))
         if n.value:
-            block = torch.empty(n.value, dtype=torch.uint8, device=out.device)
-            scratch, scratch_bytes = block.data_ptr(), n.value
+            try:
+                block = torch.empty(n.value, dtype=torch.uint8, device=out.device)
+                scratch, scratch_bytes = block.data_ptr(), n.value
+            except torch.cuda.OutOfMemoryError:
+                pass  # the product runs without it, slower
     if opts.variant == _lib.GEMM_AUTO and not opts.deterministic:
         check(packed_lib.cdl_b200_matmul(ta, tb, tc, td, opts.alpha, opts.beta, scratch, scratch_bytes, current_stream()))
     else:

@@ -643,3 +643,29 @@ def test_operands_laid_out_in_scratch(cdl, gpu_ok, dtype, batch, m, k, n, ta, tb
         assert bool(((d.double() - expected).abs() <= tol).all()), size
         assert bool((scratch[size:] == 0xff).all())
     assert L.device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_scratch_that_cannot_be_allocated(cdl, gpu_ok, dtype, monkeypatch):
+    """A product that would be faster with scratch runs without it where the memory is not there: the bits of the call that
+    lends none."""
+    L = cdl._lib
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    a, b = (torch.randn(*s, generator=gen, device="cuda").to(dtype) for s in ((1025, 2051), (2051, 1027)))
+    out, plain = torch.empty(1025, 1027, device="cuda"), torch.empty(1025, 1027, device="cuda")
+    need = ctypes.c_size_t(0)
+    args = [L.tensor_arg(t) for t in (a, b, plain)]
+    L.check(L.lib.cdl_b200_matmul_scratch_bytes(*(L.ref(t) for t in args), ctypes.byref(need)))
+    assert need.value > 0
+    L.check(L.lib.cdl_b200_matmul(L.ref(args[0]), L.ref(args[1]), None, L.ref(args[2]), 1.0, 0.0, None, 0, None))
+    asked = []
+
+    def empty(*size, dtype=None, **kw):
+        asked.append((size, dtype))
+        raise torch.cuda.OutOfMemoryError("no memory left")
+
+    monkeypatch.setattr(torch, "empty", empty)
+    cdl.ops.matmul(a, b, cdl.ops.MatmulOpts(out=torch.float32), out=out)
+    assert asked == [((need.value,), torch.uint8)]
+    assert torch.equal(out, plain)
+    assert L.device_status() == 0
