@@ -91,6 +91,12 @@ class CdlMxTensor(ctypes.Structure):
                 ("rows", ctypes.c_int64), ("cols", ctypes.c_int64)]
 
 
+class CdlMxProduct(ctypes.Structure):
+    _fields_ = [("a", ctypes.POINTER(CdlMxTensor)), ("b", ctypes.POINTER(CdlMxTensor)),
+                ("c", ctypes.POINTER(CdlTensor)), ("d", ctypes.POINTER(CdlTensor)),
+                ("alpha", ctypes.c_float), ("beta", ctypes.c_float)]
+
+
 CDL_MXFP8, CDL_NVFP4 = 0, 1
 CDL_MX_ROWWISE, CDL_MX_COLWISE = 0, 1
 
@@ -161,6 +167,7 @@ SIGNATURES = {
     "cdl_b200_mx_dequantize": ([_MX, _T, _vp], ctypes.c_int32),
     "cdl_b200_rmsnorm_fwd_mx": ([_T, _T, _T, ctypes.c_float, _MX, _MX, _T, _vp], ctypes.c_int32),
     "cdl_b200_matmul_mx": ([_MX, _MX, _T, _T, ctypes.c_float, ctypes.c_float, _vp], ctypes.c_int32),
+    "cdl_b200_matmul_mx_group": ([ctypes.POINTER(CdlMxProduct), ctypes.c_int32, _vp], ctypes.c_int32),
     "cdl_b200_matmul_mx_early": ([_MX, _MX, _T, _T, ctypes.c_float, ctypes.c_float, _vp], ctypes.c_int32),
     "cdl_b200_matmul_mx_rope": ([_MX, _MX, _T, ctypes.c_int32, ctypes.c_int32, _T, _vp], ctypes.c_int32),
     "cdl_b200_matmul_mx_opt": ([_MX, _MX, _T, _T, ctypes.c_float, ctypes.c_float, _MO, _vp],

@@ -100,7 +100,7 @@ struct Params {
   const float* rope_table;
   int rope_seqlen, rope_cols;
   int* status;
-  int early;  // 1 = starts before the kernel ahead of it has finished (see grid_dep_wait): block of 8 x 2048 3975 -> 3917 us
+  int early;  // 1 = starts before the kernel ahead of it has finished (see matmul_mx_group_execute)
 };
 
 struct Barriers {
@@ -1031,6 +1031,58 @@ int32_t matmul_mx_execute(const cdl_mx_tensor* a, const cdl_mx_tensor* b, const 
                        opts);
 }
 
+// The products of a group, one behind the other.  One that touches nothing the others since the last wait write, and
+// writes nothing they read, starts early (see grid_dep_wait): what else it reads was complete when that wait ended, and
+// the kernel ahead of it is one of the group's own.  (Asked of the caller instead, as a product that "may start early",
+// the same is wrong after any other kernel.)
+struct ProductSpans {  // memory that a product touches, [first byte, end)
+  uintptr_t at[6][2];  // values and scale factors of A and of B, D, C
+  int count;
+};
+static int32_t product_spans(const char* op, const cdl_mx_product& p, ProductSpans* s) {
+  if (!p.a || !p.b || !p.d) return fail(CDL_ERR_INVALID, "%s: a, b and d are required", op);
+  s->count = 0;
+  auto add = [&](const void* ptr, long long bytes) {
+    s->at[s->count][0] = reinterpret_cast<uintptr_t>(ptr);
+    s->at[s->count++][1] = reinterpret_cast<uintptr_t>(ptr) + bytes;
+  };
+  for (const cdl_mx_tensor* t : {p.a, p.b}) {
+    size_t values = 0, scales = 0;
+    CDL_CHECK(mx_layout(t->format, t->dim, t->rows, t->cols, &values, &scales));
+    add(t->values, static_cast<long long>(values));
+    add(t->scale_factors, static_cast<long long>(scales));
+  }
+  for (const cdl_tensor* t : {p.d, p.c}) {
+    if (!t) continue;
+    if (t->rank != 2) return fail(CDL_ERR_INVALID, "%s: c and d must have rank 2", op);
+    add(t->ptr, ((t->shape[0] - 1) * t->stride[0] + (t->shape[1] - 1) * t->stride[1] + 1) * dtype_size(t->dtype));
+  }
+  return CDL_OK;
+}
+static int32_t matmul_mx_group_execute(const cdl_mx_product* products, int32_t count, cudaStream_t stream) {
+  const char* op = "matmul (group of block-scaled products)";
+  if (count < 0 || (count > 0 && !products)) return fail(CDL_ERR_INVALID, "%s: products are required", op);
+  constexpr int D = 4;
+  auto meet = [](const uintptr_t (&s)[2], const uintptr_t (&t)[2]) { return s[0] < t[1] && t[0] < s[1]; };
+  auto no_kernel = [](const cdl_mx_product& p) { return p.a->rows == 0 || p.b->cols == 0; };
+  int32_t waited = -1;  // the last product that waits
+  for (int32_t i = 0; i < count; ++i) {
+    ProductSpans mine, other;
+    CDL_CHECK(product_spans(op, products[i], &mine));
+    bool early = waited >= 0;
+    for (int32_t j = waited; early && j < i; ++j) {
+      if (no_kernel(products[j])) continue;
+      CDL_CHECK(product_spans(op, products[j], &other));
+      for (int k = 0; k < mine.count; ++k) early = early && !meet(mine.at[k], other.at[D]);
+      for (int k = 0; k < other.count; ++k) early = early && !meet(mine.at[D], other.at[k]);
+    }
+    const cdl_mx_product& p = products[i];
+    CDL_CHECK(matmul_mx_run(op, p.a, p.b, p.c, p.d, nullptr, p.alpha, p.beta, stream, nullptr, nullptr, early));
+    if (!early && !no_kernel(p)) waited = i;
+  }
+  return CDL_OK;
+}
+
 int32_t matmul_mx_out_execute(const cdl_mx_tensor* a, const cdl_mx_tensor* b, const cdl_mx_tensor* d,
                               float alpha, cudaStream_t stream) {
   const char* op = "matmul (block-scaled operands and output)";
@@ -1061,10 +1113,13 @@ int32_t cdl_b200_matmul_mx(const cdl_mx_tensor* a, const cdl_mx_tensor* b, const
   return cdl::matmul_mx_execute(a, b, c, d, alpha, beta, static_cast<cudaStream_t>(stream));
 }
 
+int32_t cdl_b200_matmul_mx_group(const cdl_mx_product* products, int32_t count, cdl_stream stream) {
+  return cdl::matmul_mx_group_execute(products, count, static_cast<cudaStream_t>(stream));
+}
+
 int32_t cdl_b200_matmul_mx_early(const cdl_mx_tensor* a, const cdl_mx_tensor* b, const cdl_tensor* c,
                                  const cdl_tensor* d, float alpha, float beta, cdl_stream stream) {
-  return cdl::matmul_mx_run("matmul (block-scaled operands)", a, b, c, d, nullptr, alpha, beta,
-                            static_cast<cudaStream_t>(stream), nullptr, nullptr, true);
+  return cdl::matmul_mx_execute(a, b, c, d, alpha, beta, static_cast<cudaStream_t>(stream));
 }
 
 int32_t cdl_b200_matmul_mx_opt(const cdl_mx_tensor* a, const cdl_mx_tensor* b, const cdl_tensor* c,

@@ -155,12 +155,23 @@ def matmul_mx(a: MxTensor, b: MxTensor, out_dtype: torch.dtype = torch.bfloat16,
     return out
 
 
+def matmul_mx_group(*products) -> None:
+    """Products (a, b, out, c) as by `matmul_mx(a, b, out=out, c=c)`, c added unless it is None, in this order.  Those that are
+    independent of the ones ahead of them may run beside them."""
+    group = (_lib.CdlMxProduct * len(products))()
+    for p, (a, b, out, c) in zip(group, products):
+        p.a, p.b = ctypes.pointer(a.arg()), ctypes.pointer(b.arg())
+        p.d = ctypes.pointer(_lib.tensor_arg(out))
+        p.alpha, p.beta = 1.0, 0.0
+        if c is not None:
+            p.c, p.beta = ctypes.pointer(_lib.tensor_arg(c)), 1.0
+    check(packed_lib.cdl_b200_matmul_mx_group(group, len(products), current_stream()))
+
+
 def matmul_mx_early(a: MxTensor, b: MxTensor, out: torch.Tensor, c: Optional[torch.Tensor] = None,
                     beta: float = 0.0) -> torch.Tensor:
-    """`out` = A . B + beta * C beside the product enqueued just before on this stream, of which it is independent."""
-    aa, ab, tc, td = a.arg(), b.arg(), tensor_bytes(c), tensor_bytes(out)
-    check(packed_lib.cdl_b200_matmul_mx_early(ref(aa), ref(ab), ref(tc), ref(td), 1.0, beta, current_stream()))
-    return out
+    """The same as `matmul_mx` with `out` given.  (Products that may run beside one another: `matmul_mx_group`.)"""
+    return matmul_mx(a, b, out=out, c=c, beta=beta)
 
 
 def matmul_mx_rope(a: MxTensor, b: MxTensor, table: torch.Tensor, rot_heads: int, seqlen: int,

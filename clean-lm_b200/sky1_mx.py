@@ -75,24 +75,18 @@ class Sky1BlockMX:
         mx.quantize(x, rowwise=True, colwise=True, out=self.q[name])
         return self.q[name]
 
-    # `early`: beside the product enqueued just before, of which it is independent
+    # products for mx.matmul_mx_group
     @staticmethod
-    def _fwd(x_row, w_pair, out, c=None, early=False):    # Y = X . W (+ C)
-        if early:
-            return mx.matmul_mx_early(x_row, w_pair[1], out)
-        return mx.matmul_mx(x_row, w_pair[1], out=out, c=c, beta=1.0 if c is not None else 0.0)
+    def _fwd(x_row, w_pair, out, c=None):       # Y = X . W (+ C)
+        return x_row, w_pair[1], out, c
 
     @staticmethod
-    def _dgrad(dy_row, w_pair, out, c=None, early=False):  # dX = dY . W^T (+ C)
-        if early:
-            return mx.matmul_mx_early(dy_row, w_pair[0].transposed(), out)
-        return mx.matmul_mx(dy_row, w_pair[0].transposed(), out=out, c=c, beta=1.0 if c is not None else 0.0)
+    def _dgrad(dy_row, w_pair, out, c=None):    # dX = dY . W^T (+ C)
+        return dy_row, w_pair[0].transposed(), out, c
 
     @staticmethod
-    def _wgrad(x_col, dy_col, grad, early=False):         # dW += X^T . dY
-        if early:
-            return mx.matmul_mx_early(x_col.transposed(), dy_col, grad, c=grad, beta=1.0)
-        return mx.matmul_mx(x_col.transposed(), dy_col, out=grad, c=grad, beta=1.0)
+    def _wgrad(x_col, dy_col, grad):            # dW += X^T . dY
+        return x_col.transposed(), dy_col, grad, grad
 
     # ------------------------------------------------------------------ forward / backward
     def forward(self, x: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
@@ -106,35 +100,32 @@ class Sky1BlockMX:
                                 out=b["attn"].view(cfg.batch, cfg.seqlen, cfg.heads, cfg.head_dim))
         self.lse = att.lse
         qa = self._quant("attn", b["attn"])
-        self._fwd(qa[0], self.wq["wo"], b["o"], c=x)                       # o = attn Wo + x
+        mx.matmul_mx_group(self._fwd(qa[0], self.wq["wo"], b["o"], c=x))   # o = attn Wo + x
         n2 = mx.norm_fwd_mx(b["o"], p["norm2"], eps=cfg.eps, colwise=True, save_stats=True,
                             out=mx.NormMxOutputs(*self.q["h2"], self.r_inv[2]))
-        self._fwd(n2.y, self.wq["wup"], b["up"])
-        self._fwd(n2.y, self.wq["wgate"], b["gate"], early=True)
+        mx.matmul_mx_group(self._fwd(n2.y, self.wq["wup"], b["up"]), self._fwd(n2.y, self.wq["wgate"], b["gate"]))
         qact = self.q["act"]
         mx.swiglu_fwd(b["gate"], b["up"], qact)
-        self._fwd(qact[0], self.wq["wdown"], out, c=b["o"])                # out = act Wdown + o
+        mx.matmul_mx_group(self._fwd(qact[0], self.wq["wdown"], out, c=b["o"]))   # out = act Wdown + o
         return out
 
     def backward(self, dy: torch.Tensor, dx: torch.Tensor | None = None) -> torch.Tensor:
         cfg, b, p, g = self.cfg, self.buf, self.params, self.grads
         dx = torch.empty_like(dy) if dx is None else dx
         qdy = self._quant("dy", dy)
-        self._wgrad(self.q["act"][1], qdy[1], g["wdown"])
-        self._dgrad(qdy[0], self.wq["wdown"], b["d_act"], early=True)
+        mx.matmul_mx_group(self._wgrad(self.q["act"][1], qdy[1], g["wdown"]),
+                           self._dgrad(qdy[0], self.wq["wdown"], b["d_act"]))
         qdu, qdg = self.q["d_up"], self.q["d_gate"]
         mx.swiglu_bwd(b["d_act"], b["gate"], b["up"], qdg, qdu)
-        self._wgrad(self.q["h2"][1], qdu[1], g["wup"])
-        lo, hi = sorted((g["wup"], g["wgate"]), key=lambda t: t.data_ptr())
-        apart = lo.data_ptr() + 4 * lo.numel() <= hi.data_ptr()
-        self._wgrad(self.q["h2"][1], qdg[1], g["wgate"], early=apart)
-        self._dgrad(qdu[0], self.wq["wup"], b["dh"], early=True)
-        self._dgrad(qdg[0], self.wq["wgate"], b["dh"], c=b["dh"])
+        mx.matmul_mx_group(self._wgrad(self.q["h2"][1], qdu[1], g["wup"]),
+                           self._wgrad(self.q["h2"][1], qdg[1], g["wgate"]),
+                           self._dgrad(qdu[0], self.wq["wup"], b["dh"]),
+                           self._dgrad(qdg[0], self.wq["wgate"], b["dh"], c=b["dh"]))
         ops.norm_bwd(b["o"], b["dh"], p["norm2"], self.r_inv[2], g["norm2"], residual_dy=dy,
                      scratch=self.norm_scratch, dx=b["d_o"])
         qdo = self._quant("d_o", b["d_o"])
-        self._wgrad(self.q["attn"][1], qdo[1], g["wo"])
-        self._dgrad(qdo[0], self.wq["wo"], b["d_attn"], early=True)
+        mx.matmul_mx_group(self._wgrad(self.q["attn"][1], qdo[1], g["wo"]),
+                           self._dgrad(qdo[0], self.wq["wo"], b["d_attn"]))
         dqv = b["d_qkv"].view(cfg.batch, cfg.seqlen, cfg.heads + 2 * cfg.kv_heads, cfg.head_dim)
         h, kv = cfg.heads, cfg.kv_heads
         ops.attention_bwd(self._q, self._k, self._v, b["attn"].view(cfg.batch, cfg.seqlen, h, cfg.head_dim),
@@ -143,8 +134,8 @@ class Sky1BlockMX:
                           dq=dqv[:, :, :h], dk=dqv[:, :, h:h + kv], dv=dqv[:, :, h + kv:],
                           rope_table=self.table)  # d_q and d_k leave rotated back
         qdq = self._quant("d_qkv", b["d_qkv"])
-        self._wgrad(self.q["h1"][1], qdq[1], g["wqkv"])
-        self._dgrad(qdq[0], self.wq["wqkv"], b["dh"], early=True)
+        mx.matmul_mx_group(self._wgrad(self.q["h1"][1], qdq[1], g["wqkv"]),
+                           self._dgrad(qdq[0], self.wq["wqkv"], b["dh"]))
         ops.norm_bwd(self._x, b["dh"], p["norm1"], self.r_inv[1], g["norm1"], residual_dy=b["d_o"],
                      scratch=self.norm_scratch, dx=dx)
         return dx

@@ -314,9 +314,18 @@ int32_t cdl_b200_matmul_mx(const cdl_mx_tensor* a, const cdl_mx_tensor* b, const
 int32_t cdl_b200_matmul_mx_opt(const cdl_mx_tensor* a, const cdl_mx_tensor* b, const cdl_tensor* c,
                                const cdl_tensor* d, float alpha, float beta,
                                const cdl_matmul_options* options, cdl_stream stream);
-/* cdl_b200_matmul_mx that may run beside the product enqueued just before it on the stream (cdl_b200_matmul_mx or another of
- * these): the caller states that neither reads or writes what the other, or one of these ahead of it, writes.  Whatever is
- * enqueued next waits for both. */
+/* `count` products as by cdl_b200_matmul_mx, in this order and with its results.  One that touches nothing that those
+ * ahead of it in the group write, and writes nothing that they read, may run beside them; any other waits for them. */
+typedef struct {
+  const cdl_mx_tensor* a;
+  const cdl_mx_tensor* b;
+  const cdl_tensor* c; /* nullable */
+  const cdl_tensor* d;
+  float alpha;
+  float beta;
+} cdl_mx_product;
+int32_t cdl_b200_matmul_mx_group(const cdl_mx_product* products, int32_t count, cdl_stream stream);
+/* The same as cdl_b200_matmul_mx.  (Products that may run beside one another: cdl_b200_matmul_mx_group.) */
 int32_t cdl_b200_matmul_mx_early(const cdl_mx_tensor* a, const cdl_mx_tensor* b, const cdl_tensor* c,
                                  const cdl_tensor* d, float alpha, float beta, cdl_stream stream);
 /* D = RoPE(A . B) with MXFP8 operands: as cdl_b200_matmul_rope on dense sequences (bf16 [M, N], N % 128 == 0, 16-byte

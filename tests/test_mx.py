@@ -636,3 +636,58 @@ def test_matmul_mx_early_beside_the_product_ahead(cdl, gpu_ok, m, k, n):
         assert all(torch.equal(o, p) for o, p in zip(out, plain))
         assert torch.equal(got, ref) and torch.equal(last, total)
     assert cdl._lib.device_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,k,n", [(64, 64, 96), (256, 128, 256), (700, 1024, 520), (2048, 2048, 5632)])
+def test_matmul_mx_group(cdl, gpu_ok, m, k, n):
+    """Products of one call: independent ones; ones that read, overwrite or add to what another writes; two that share a
+    buffer without overlapping; one without rows.  Right behind kernels that write their operands, many times in a row: the
+    bits of the calls one by one."""
+    gen = torch.Generator(device="cuda").manual_seed(m + n)
+    r = lambda *s: torch.randn(*s, generator=gen, device="cuda").to(torch.bfloat16)
+    x, y = [r(m, k) for _ in range(3)], [r(n, k) for _ in range(3)]
+    qa = [cdl.mx.MxTensor.empty(m, k, cdl.mx.ROWWISE, zero_scales=True) for _ in range(3)]
+    b = [cdl.mx.quantize(t, rowwise=True)[0].transposed() for t in y]
+    none = cdl.mx.quantize(r(0, k), rowwise=True)[0]
+    grad = torch.randn(m, n, generator=gen, device="cuda")
+
+    def run(launch):
+        out = [torch.full((m, n), float("nan"), device="cuda", dtype=torch.bfloat16) for _ in range(3)]
+        wide, got = torch.full((2, m, n), float("nan"), device="cuda", dtype=torch.bfloat16), grad.clone()
+        empty = torch.empty(0, n, device="cuda", dtype=torch.bfloat16)
+        for t, q in zip(x, qa):
+            q.values.zero_()
+            cdl.mx.quantize(t, out=(q, None))
+        launch((none, b[0], empty, None), (qa[0], b[0], out[0], None), (qa[1], b[1], got, got), (none, b[1], empty, None),
+               (qa[1], b[0], wide[0], None), (qa[1], b[2], wide[1], None), (qa[2], b[2], out[1], None),
+               (qa[2], b[1], out[2], out[0]), (qa[0], b[1], out[2], out[2]), (qa[2], b[0], got, got), (qa[1], b[1], out[0], None))
+        return *out, wide, got
+
+    def one_by_one(*products):
+        for p, q, d, c in products:
+            cdl.mx.matmul_mx(p, q, out=d, c=c, beta=0.0 if c is None else 1.0)
+            torch.cuda.synchronize()
+
+    ref = run(one_by_one)
+    for _ in range(20):
+        assert all(torch.equal(g, e) for g, e in zip(run(cdl.mx.matmul_mx_group), ref))
+    assert cdl._lib.device_status() == 0
+
+
+@pytest.mark.gpu
+def test_matmul_mx_early_after_any_kernel(cdl, gpu_ok):
+    """matmul_mx_early right behind the quantiser that writes its operand, and behind a product that writes C."""
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.randn(8192, 2048, generator=gen, device="cuda").to(torch.bfloat16)
+    b = cdl.mx.quantize(torch.randn(1024, 2048, generator=gen, device="cuda").to(torch.bfloat16))[0].transposed()
+    ref = cdl.mx.matmul_mx(cdl.mx.quantize(x)[0], b)
+    for _ in range(10):
+        q = cdl.mx.quantize(torch.zeros_like(x))[0]
+        out, twice = torch.empty_like(ref), torch.empty_like(ref)
+        torch.cuda.synchronize()
+        cdl.mx.quantize(x, out=(q, None))
+        cdl.mx.matmul_mx_early(q, b, out)
+        cdl.mx.matmul_mx_early(q, b, twice, c=out, beta=1.0)
+        assert torch.equal(out, ref) and torch.equal(twice, cdl.mx.matmul_mx(q, b, c=ref, beta=1.0))
+    assert cdl._lib.device_status() == 0
