@@ -90,8 +90,10 @@ typedef struct {
   int32_t variant;       /* cdl_gemm_variant */
   int32_t deterministic; /* != 0: fixed f32 summation order.  The accumulate-in-place form
                           * (D = C in f32, beta = 1: the weight-gradient GEMM) otherwise cuts K into
-                          * slices that add into D with red.global.add, so its low-order bits can
-                          * differ from run to run. */
+                          * slices that add into D with atomics, so its low-order bits can differ from run
+                          * to run, and may make a value of D below 2^-126 (a subnormal) zero before or
+                          * after it is added to.  With this set subnormals are kept; infinities and
+                          * NaN in D always are. */
 } cdl_matmul_options;
 typedef enum {
   CDL_NORM_AUTO = 0,         /* heuristic (measured per form, see cdl_b200_rmsnorm_bwd) */
@@ -117,8 +119,8 @@ typedef struct {
  * largest products are summed; a short K takes plain FMAs, f32 products summed in f64.  The error of a
  * f32 product is at most that of a chain of f32 FMAs.  scratch (nullable; 16-byte aligned, as many bytes as
  * cdl_b200_matmul_scratch_bytes says, 0 for many products) lets the operands of such a product be converted
- * once instead of in every tile; without it, or with less, the result comes from the other kernel.  K == 0 is an error ("K is zero", matmul.rs
- * tests :825-843).  D may alias C. */
+ * once instead of in every tile; without it, or with less, the result comes from the other kernel.
+ * K == 0 is an error ("K is zero", matmul.rs tests :825-843).  D may alias C. */
 int32_t cdl_b200_matmul(const cdl_tensor* a, const cdl_tensor* b, const cdl_tensor* c,
                         const cdl_tensor* d, float alpha, float beta, void* scratch,
                         size_t scratch_bytes, cdl_stream stream);
@@ -310,7 +312,7 @@ int32_t cdl_b200_rmsnorm_fwd_mx(const cdl_tensor* x, const cdl_tensor* scale, co
 int32_t cdl_b200_matmul_mx(const cdl_mx_tensor* a, const cdl_mx_tensor* b, const cdl_tensor* c,
                            const cdl_tensor* d, float alpha, float beta, cdl_stream stream);
 /* The same with the kernel variant chosen by the caller (NULL options = the call above; the
- * block-scaled kernels are always bit-reproducible, `deterministic` is ignored). */
+ * block-scaled kernels are always bit-reproducible and keep subnormals, `deterministic` is ignored). */
 int32_t cdl_b200_matmul_mx_opt(const cdl_mx_tensor* a, const cdl_mx_tensor* b, const cdl_tensor* c,
                                const cdl_tensor* d, float alpha, float beta,
                                const cdl_matmul_options* options, cdl_stream stream);

@@ -669,3 +669,31 @@ def test_scratch_that_cannot_be_allocated(cdl, gpu_ok, dtype, monkeypatch):
     assert asked == [((need.value,), torch.uint8)]
     assert torch.equal(out, plain)
     assert L.device_status() == 0
+
+
+@pytest.mark.parametrize("m,k,n", [(64, 96, 200), (130, 64, 36), (512, 256, 512), (512, 4096, 264), (2048, 256, 2048), (2048, 1024, 5632)])
+def test_in_place_additions_of_small_and_non_finite_values(cdl, gpu_ok, m, k, n):
+    """D += alpha A^T B in f32 where D and the product are subnormal, multiples of 2^-149, whose sums are exact; and where D
+    holds infinities and NaN.  Kept bit by bit with `deterministic` and by the two tile variants, whose additions
+    are TMA reductions; without it a subnormal of D may count as zero."""
+    gen = torch.Generator(device="cuda").manual_seed(m + k)
+    whole = lambda high, *s: torch.randint(-high, high + 1, s, generator=gen, device="cuda")
+    a, b = whole(2, k, m).to(torch.bfloat16).T, whole(2, k, n).to(torch.bfloat16)
+    prod = a.double() @ b.double()  # whole numbers
+    c = (whole(1 << 20, m, n).double() * 2.0 ** -149)
+    special = c.clone()
+    special[0, 0], special[1, n - 1], special[m - 1, n // 2] = float("inf"), float("nan"), float("-inf")
+    for start in (c, special):
+        exact = (start + prod * 2.0 ** -149).float()
+        for variant in (cdl._lib.GEMM_AUTO, cdl._lib.GEMM_ONE_CTA, cdl._lib.GEMM_CTA_PAIR):
+            for deterministic in (False, True):
+                d = start.float()
+                cdl.ops.matmul(a, b, cdl.ops.MatmulOpts(out=torch.float32, c=d, alpha=2.0 ** -149, beta=1.0, variant=variant,
+                                                        deterministic=deterministic), out=d)
+                finite = torch.isfinite(exact)
+                assert torch.equal(d[~finite].nan_to_num(1.0), exact[~finite].nan_to_num(1.0))
+                if deterministic or variant != cdl._lib.GEMM_AUTO and m > 128:
+                    assert torch.equal(d[finite], exact[finite]), (variant, deterministic)
+                else:  # what was there, what was added or the sum is missing
+                    assert bool(((d - exact)[finite].abs() <= 2.0 ** -126).all())
+    assert cdl._lib.device_status() == 0

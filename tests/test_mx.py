@@ -691,3 +691,21 @@ def test_matmul_mx_early_after_any_kernel(cdl, gpu_ok):
         cdl.mx.matmul_mx_early(q, b, twice, c=out, beta=1.0)
         assert torch.equal(out, ref) and torch.equal(twice, cdl.mx.matmul_mx(q, b, c=ref, beta=1.0))
     assert cdl._lib.device_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,k,n", [(64, 96, 200), (300, 64, 36), (512, 4096, 264), (2048, 1024, 5632)])
+def test_matmul_mx_adds_to_small_and_non_finite_values(cdl, gpu_ok, m, k, n):
+    """D += alpha A . B in f32 where D and the product are subnormal, multiples of 2^-149 (exact sums), or D is infinite or
+    NaN: TMA reductions (more than 128 rows) and the one-CTA kernel keep every bit."""
+    gen = torch.Generator(device="cuda").manual_seed(m + k)
+    whole = lambda high, *s: torch.randint(-high, high + 1, s, generator=gen, device="cuda")
+    qa, qb = (cdl.mx.quantize(whole(2, r, k).to(torch.bfloat16))[0] for r in (m, n))
+    prod = cdl.mx.dequantize(qa).double() @ cdl.mx.dequantize(qb).double().T  # whole numbers
+    c = whole(1 << 20, m, n).double() * 2.0 ** -149
+    c[0, 0], c[1, n - 1], c[m - 1, n // 2] = float("inf"), float("nan"), float("-inf")
+    exact = (c + prod * 2.0 ** -149).float()
+    d = c.float()
+    cdl.mx.matmul_mx(qa, qb.transposed(), out=d, c=d, alpha=2.0 ** -149, beta=1.0)
+    assert torch.equal(d.isnan(), exact.isnan()) and torch.equal(d.nan_to_num(1.0), exact.nan_to_num(1.0))
+    assert cdl._lib.device_status() == 0
