@@ -640,6 +640,9 @@ struct PieceBarriers {
 static_assert(sizeof(PieceBarriers) <= 256, "barriers fit behind the slots");
 constexpr size_t piece_smem_bytes(int slots, bool pair) { return 1024 + slots * slot_bytes(pair) + 256; }
 static_assert(gemm::PART_BYTES <= shared_slots(true) * slot_bytes(true), "the partial tile takes the slots' place");
+static_assert(gemm::PART_BYTES + 2 * REDO_FLOATS * sizeof(float) <= alone_slots(false) * slot_bytes(false) &&
+                  gemm::PART_BYTES + 2 * REDO_FLOATS * sizeof(float) <= alone_slots(true) * slot_bytes(true),
+              "the FMA tiles fit behind it");
 template <typename T>
 constexpr int piece_threads() { return (2 + PieceTraits<T>::SUM_WARPS) * 32; }
 

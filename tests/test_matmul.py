@@ -697,3 +697,80 @@ def test_in_place_additions_of_small_and_non_finite_values(cdl, gpu_ok, m, k, n)
                 else:  # what was there, what was added or the sum is missing
                     assert bool(((d - exact)[finite].abs() <= 2.0 ** -126).all())
     assert cdl._lib.device_status() == 0
+
+
+def _lend_scratch(cdl, a, b, c, alpha, beta, out_dtype):
+    """The product with the scratch the library asks for, which has to be some: the operands are laid out first."""
+    L = cdl._lib
+    d = torch.full((*a.shape[:-1], b.shape[-1]), float("nan"), dtype=out_dtype, device="cuda")
+    need = ctypes.c_size_t(0)
+    args = [L.tensor_arg(t) for t in (a, b, c, d)]
+    L.check(L.lib.cdl_b200_matmul_scratch_bytes(L.ref(args[0]), L.ref(args[1]), L.ref(args[3]), ctypes.byref(need)))
+    assert need.value > 0, "this shape was meant to be laid out"
+    scratch = torch.full((need.value + 16,), 0xff, dtype=torch.uint8, device="cuda")  # (NaN patterns)
+    L.check(L.lib.cdl_b200_matmul(*(L.ref(t) for t in args), alpha, beta, scratch.data_ptr(), need.value, None))
+    assert bool((scratch[need.value:] == 0xff).all())
+    return d
+
+
+@pytest.mark.parametrize("batch,m,k,n", [(1, 1500, 1027, 2051), (1, 1025, 1027, 2051), (20, 100, 1027, 1027), (3, 600, 2051, 1030),
+                                         (1, 1100, 4099, 1500), (1, 64, 2049, 2049)])
+@pytest.mark.parametrize("ta,tb", [(False, False), (True, False), (False, True), (True, True)])
+@pytest.mark.parametrize("out", [torch.bfloat16, torch.float32])
+def test_laid_out_bf16_products(cdl, gpu_ok, batch, m, k, n, ta, tb, out):
+    """Products of operands that are laid out first, more than one CTA per SM (the first four: two share one, CTA pairs with and
+    without a second CTA past M, single CTAs in batches) and fewer, with and without C, against f64.  Bound: exact
+    products, sums that truncate over at most 8 K blocks of 4 steps at a time (2^-23 each) and are rounded once per
+    such group, and the result's own rounding."""
+    gen = torch.Generator(device="cuda").manual_seed(m + k)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda").to(torch.bfloat16)
+    a = rnd(batch, k, m + 1 + m % 2)[:, :, 1:m + 1].mT if ta else rnd(batch, m, k + 2)[:, :, 1:k + 1]
+    b = rnd(batch, n, (k + 7) // 8 * 8)[:, :, :k].mT if tb else rnd(batch, k, n + 1)[:, :, :n]  # (tb: aligned rows)
+    c = torch.randn(batch, m, n, generator=gen, device="cuda")
+    if batch == 1:
+        a, b, c = a[0], b[0], c[0]
+    prod, bound = a.double() @ b.double(), a.double().abs() @ b.double().abs()
+    tol = (32 * 2.0 ** -23 + (k / 64 + 2) * 2.0 ** -24) * bound
+    own = 2.0 ** -8 if out == torch.bfloat16 else 2.0 ** -23
+    for beta in (0.0, 1.0):
+        expected = 0.5 * prod + beta * c
+        d = _lend_scratch(cdl, a, b, c if beta else None, 0.5, beta, out)
+        assert bool(((d.double() - expected).abs() <= 0.5 * tol + own * (expected.abs() + 0.5 * tol) + 1e-30).all()), beta
+    assert cdl._lib.device_status() == 0
+
+
+@pytest.mark.parametrize("batch,m,k,n", [(1, 64, 2049, 2049), (16, 128, 515, 128), (1, 1025, 1027, 705), (1, 300, 700, 1500)])
+@pytest.mark.parametrize("ta,tb", [(False, False), (True, True)])
+@pytest.mark.parametrize("which", ["non-finite", "tiny", "overflow"])
+def test_laid_out_f32_values_without_pieces(cdl, gpu_ok, batch, m, k, n, ta, tb, which):
+    """Values that are not the sum of bf16 pieces, and sums that leave f32's range, where the operands are laid out first: single
+    CTAs in K slices, CTA pairs, a second CTA of the pair past M; in the last K block, row and column.  Results as
+    f32 arithmetic gives them; bounds as in the tests above of the same values."""
+    gen = torch.Generator(device="cuda").manual_seed(m + n)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    a = rnd(batch, k, m).mT if ta else rnd(batch, m, k)
+    b = rnd(batch, n, k).mT if tb else rnd(batch, k, n)
+    floor = k * 2.0 ** -149
+    if which == "non-finite":
+        a[-1, m - 1, k - 1], b[-1, k - 1, n - 1] = float("inf"), float("nan")
+        a[0, 0, k // 2], b[0, k // 2] = 3.4e38, b[0, k // 2] * 1e-3
+    elif which == "tiny":
+        a[-1, m - 1, k - 1] *= 1e-37
+        b[0, :, n // 2] = b[0, :, n // 2] * 1e-37 + 1e-30
+        b[-1, k - 1, n - 1] *= 1e-37
+    else:
+        sign = lambda *s: torch.where(rnd(*s) < 0, -1.0, 1.0)
+        a[-1, :, k - 1] = 1e30 * (1 + rnd(m).abs()) * sign(m)
+        b[-1, k - 1] = 1e30 * (1 + rnd(n).abs()) * sign(n)
+        b[-1, k - 1, ::3] = rnd(n)[::3]  # every third column stays in range
+        a[-1, m - 1, k - 1] = b[-1, k - 1, 1] = 1.8446742e19  # the square is in range, that of its bf16 rounding is not
+    if batch == 1:
+        a, b = a[0], b[0]
+    d = _lend_scratch(cdl, a, b, None, 1.0, 0.0, torch.float32).double()
+    expected, bound = a.double() @ b.double(), a.double().abs() @ b.double().abs()
+    expected = torch.where(expected.abs() > torch.finfo(torch.float32).max, expected * float("inf"), expected)
+    assert torch.equal(d.isnan(), expected.isnan()) and torch.equal(d.isinf(), expected.isinf())
+    assert torch.equal(d[d.isinf()], expected[d.isinf()])
+    ok = expected.isfinite()
+    assert bool(((d - expected).abs()[ok] <= (k + 10) * 2.0 ** -24 * bound[ok] + floor).all())
+    assert cdl._lib.device_status() == 0
