@@ -32,9 +32,10 @@
 //   mx_rowcol_tile_kernel     the norm's both outputs, 32 whole rows in shared memory
 //   mx_row_full_kernel,       cols % 256 == 0 and no bias: the same two schemes trimmed of every
 //   mx_rowcol_full_kernel     operation the arithmetic does not need
-//   mx_panel_kernel           both outputs by panels of 256 or 512 columns: of x, of its norm (the panels of a
-//                             row are a cluster that shares the row sums through distributed shared
-//                             memory), of SwiGLU and of its gradients
+//   mx_rowcol_wide_kernel     the norm's both outputs by panels of 1024 or 512 columns, rows up to 8192
+//   mx_panel_kernel           both outputs by panels of 256 or 512 columns: of x, of the norm of few rows, of
+//                             SwiGLU and of its gradients
+//   (the norm's panels of a row are a cluster that shares its statistic through distributed shared memory)
 //   nvfp4_rows_kernel, nvfp4_row_full_kernel   the NVFP4 rowwise output, general and trimmed
 #include "host.h"
 #include "ops.h"
@@ -66,6 +67,7 @@ struct Params {
   uint8_t* row_sf;
   uint8_t* col_values;  // [cols, rows]; nullable
   uint8_t* col_sf;
+  int panel_cols;  // mx_rowcol_wide_kernel
 };
 // Further operands of mx_panel_kernel's SwiGLU sources.
 struct Extra {
@@ -430,8 +432,8 @@ __global__ void __launch_bounds__(256, NCH <= 8 ? FULL_MIN_CTAS : 1) mx_row_full
 // (TILE [32][cols + 8] bf16): a CTA of 32 warps owns 32 rows.  A warp loads its row into the
 // tile while it sums the squares, replaces it by the bf16 result (writing the rowwise output on
 // the way), and after one barrier every thread quantises whole 32-row blocks of its columns.
-// x is read once; the colwise stores are one 32-byte sector per thread.  For what mx_panel_kernel does not
-// take: a bias, or rows that no eight panels make up.
+// x is read once; the colwise stores are one 32-byte sector per thread.  For what the kernels below do not
+// take: a bias, or a column count that is no multiple of 256.
 __global__ void __launch_bounds__(1024, 1) mx_rowcol_tile_kernel(const Params p) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   __nv_bfloat16* tile = reinterpret_cast<__nv_bfloat16*>(smem_raw);
@@ -592,12 +594,83 @@ __device__ __forceinline__ void st_shared_cluster_f32(uint32_t cluster_addr, flo
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(cluster_addr), "f"(v) : "memory");
 }
 
+// Both outputs of the norm of rows that do not fit a CTA's shared memory 32 at a time, no bias: CTA (blockIdx.x,
+// blockIdx.y) owns rows [32 y, +32) x columns [W x, +W), W = 1024 or 512, with W / 2 threads, so that two or more CTAs
+// share an SM.  The CTAs of a row (at most 8) are a cluster: each sums the squares of its part of the 32 rows, writes the 32
+// partial sums into every member's shared memory, and after a cluster barrier all of them add the parts in
+// rank order, so that every member normalises with the same bits.  ([4096, 8192] 51.3 us, with a
+// panel's part of the rows in registers, as in mx_panel_kernel, 66.6.)
+constexpr size_t wide_smem(int w) { return 64 * static_cast<size_t>(w + 8) + static_cast<size_t>(w) * 4 + 8 * 32 * 4; }
+__global__ void __launch_bounds__(512, 2) mx_rowcol_wide_kernel(const Params p) {
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  const int W = p.panel_cols, ld = W + 8;
+  __nv_bfloat16* tile = reinterpret_cast<__nv_bfloat16*>(smem_raw);
+  float4* s_gamma = reinterpret_cast<float4*>(smem_raw + 64 * ld);  // [W] f32
+  float* s_ss = reinterpret_cast<float*>(s_gamma + W / 4);          // [8][32]
+  const int pc0 = blockIdx.x * W;
+  const long long row0 = static_cast<long long>(blockIdx.y) * 32;
+  const int lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const int row_tiles = (p.cols / BLOCK + 3) >> 2;
+  const bool has_gamma = p.gamma != nullptr;
+  const bool rowwise = p.row_values != nullptr;
+  const uint32_t rank = cluster_ctarank(), members = gridDim.x;
+  if (has_gamma) stage_gamma(p.gamma + pc0, W, s_gamma);
+  cluster_sync_all();  // a member's shared memory may be written only once that member runs
+
+  for (int rr = warp; rr < 32; rr += warps) {
+    const __nv_bfloat16* xr = p.x + (row0 + rr) * p.ldx + pc0;
+    __nv_bfloat16* trow = tile + rr * ld;
+    float ss = 0.f;
+    for (int c = lane * 8; c < W; c += 256) {
+      const uint4 q = ld_nc_v4(xr + c);
+      *reinterpret_cast<uint4*>(trow + c) = q;
+      float f[8];
+      unpack8(q, f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) ss = fmaf(f[j], f[j], ss);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if (lane < members) st_shared_cluster_f32(mapa_shared(smem_u32(s_ss + rank * 32 + rr), lane), ss);
+  }
+  cluster_sync_all();  // every member's partial sums have landed; nothing remote after this
+
+  const int sf_lane = (lane >> 4) * 512 + ((lane >> 2) & 3);
+  for (int rr = warp; rr < 32; rr += warps) {
+    const long long row = row0 + rr;
+    __nv_bfloat16* trow = tile + rr * ld;
+    float ss = 0.f;
+    for (uint32_t k = 0; k < members; ++k) ss += s_ss[k * 32 + rr];
+    const float r = rsqrtf(ss * (1.0f / static_cast<float>(p.cols)) + p.eps);
+    if (rank == 0 && lane == 0 && p.r_inv != nullptr) p.r_inv[row * p.r_inv_stride] = r;
+    uint8_t* out = rowwise ? p.row_values + row * p.cols + pc0 + lane * 8 : nullptr;
+    uint8_t* sf = rowwise ? p.row_sf + ((row >> 7) * row_tiles + (pc0 >> 7)) * 512 + (row & 31) * 16 +
+                                ((row & 127) >> 5) * 4 + sf_lane
+                          : nullptr;
+    for (int c0 = 0; c0 < W; c0 += 256) {
+      const int c = c0 + lane * 8;
+      uint32_t q[4];
+      norm_packed8(*reinterpret_cast<const uint4*>(trow + c), r, has_gamma ? s_gamma + (c0 >> 2) + lane : nullptr, q);
+      *reinterpret_cast<uint4*>(trow + c) = make_uint4(q[0], q[1], q[2], q[3]);
+      if (rowwise) {  // CTA-uniform: the shuffles see whole warps
+        uint32_t e;
+        const uint2 o = quantize_packed8(q, e);
+        *reinterpret_cast<uint2*>(out + c0) = o;
+        if ((lane & 3) == 0) sf[(c0 >> 7) * 512] = static_cast<uint8_t>(e);
+      }
+    }
+  }
+  __syncthreads();
+  quantize_column_pair(p.col_values, p.col_sf, p.rows, tile, ld, threadIdx.x, pc0, row0);
+}
+
 // Rowwise and colwise outputs by panels: a CTA of W / 2 threads owns 32 rows x W columns, a lane 8 neighbouring
 // columns of 8 (row, 256-column chunk) units.  What is quantised is
 //   PLAIN       x
-//   NORM        x r gamma; the panels of a row (at most 8) are a cluster: each sums the squares of its part
-//               of the 32 rows, writes the 32 partial sums into every member's shared memory, and after a cluster
-//               barrier all add the parts in rank order, so that every member normalises with the same bits
+//   NORM        x r gamma; the panels of a row (at most 8) are a cluster: each reads every `panels`-th of the 32 rows
+//               whole, adds its squares up in the order of the kernels of whole rows and writes r to all members, so that the
+//               bytes of a row do not depend on how many rows there are
 //   SWIGLU      bf16(SiLU(gate) up)                                    x = gate, extra.x = {up}
 //   SWIGLU_BWD  the two gradients of that, d_up and d_gate, in bf16    x = gate, extra.x = {up, d_act}
 // (the values that the stand-alone kernels of elem.cu store: the SwiGLU tensors never exist in HBM).
@@ -609,7 +682,7 @@ enum Source { PLAIN, NORM, SWIGLU, SWIGLU_BWD };
 constexpr int panel_outputs(int src) { return src == SWIGLU_BWD ? 2 : 1; }
 constexpr int panel_inputs(int src) { return src == SWIGLU_BWD ? 3 : src == SWIGLU ? 2 : 1; }
 constexpr size_t panel_smem(int w, int src) {
-  return static_cast<size_t>(panel_outputs(src)) * 64 * (w + 8) + (src == NORM ? 8 * 32 * 4 : 0);
+  return static_cast<size_t>(panel_outputs(src)) * 64 * (w + 8) + (src == NORM ? 32 * 4 : 0);
 }
 constexpr int panel_ctas(int w, int src) { return (src == SWIGLU_BWD || src == NORM ? 3 : 4) * 512 / w; }
 
@@ -620,7 +693,7 @@ __global__ void __launch_bounds__(W / 2, panel_ctas(W, SRC)) mx_panel_kernel(con
   constexpr int IN = panel_inputs(SRC), OUT = panel_outputs(SRC);
   constexpr int BATCH = SRC == SWIGLU_BWD ? 2 : SRC == SWIGLU ? 4 : 8;  // units whose loads are in flight together
   __nv_bfloat16* tile = reinterpret_cast<__nv_bfloat16*>(smem_raw);    // [OUT][32][LD]
-  float* s_ss = reinterpret_cast<float*>(smem_raw + OUT * 64 * LD);    // NORM: [8][32]
+  float* s_r = reinterpret_cast<float*>(smem_raw + OUT * 64 * LD);     // NORM: [32]
   const int panels = (p.cols + W - 1) / W;
   const int panel = static_cast<int>(blockIdx.x) % panels;
   const long long row0 = static_cast<long long>(static_cast<int>(blockIdx.x) / panels) * 32;
@@ -671,23 +744,28 @@ __global__ void __launch_bounds__(W / 2, panel_ctas(W, SRC)) mx_panel_kernel(con
     if constexpr (SRC == NORM) {
       // A member's shared memory may be written only once that member runs.
       cluster_sync_all();
-      const uint32_t rank = cluster_ctarank();
-#pragma unroll
-      for (int rw = 0; rw < UNITS / CHUNKS; ++rw) {
+      for (int rr = static_cast<int>(cluster_ctarank()) + panels * warp; rr < 32; rr += panels * WARPS) {
+        const __nv_bfloat16* row = p.x + (row0 + rr) * p.ldx + lane * 8;
         float ss = 0.f;
+        for (int c0 = 0; c0 < p.cols; c0 += 1024) {  // (cols % 256 == 0; what lies beyond adds 0)
+          uint4 q[4];
 #pragma unroll
-        for (int c = 0; c < CHUNKS; ++c) {
-          float f[8];
-          unpack8(v[rw * CHUNKS + c][0], f);
+          for (int c = 0; c < 4; ++c)
+            q[c] = c0 + c * 256 < p.cols ? ld_nc_v4(row + c0 + c * 256) : make_uint4(0, 0, 0, 0);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) ss = fmaf(f[j], f[j], ss);
+          for (int c = 0; c < 4; ++c) {
+            float f[8];
+            unpack8(q[c], f);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) ss = fmaf(f[j], f[j], ss);
+          }
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        if (lane < panels)
-          st_shared_cluster_f32(mapa_shared(smem_u32(s_ss + rank * 32 + warp + WARPS * rw), lane), ss);
+        const float r = rsqrtf(ss * (1.0f / static_cast<float>(p.cols)) + p.eps);
+        if (lane < panels) st_shared_cluster_f32(mapa_shared(smem_u32(s_r + rr), lane), r);
       }
-      cluster_sync_all();  // every member's partial sums have landed; nothing remote after this
+      cluster_sync_all();  // every member's rows have landed; nothing remote after this
       uint4 gamma[CHUNKS];
 #pragma unroll
       for (int c = 0; c < CHUNKS; ++c)
@@ -695,9 +773,7 @@ __global__ void __launch_bounds__(W / 2, panel_ctas(W, SRC)) mx_panel_kernel(con
 #pragma unroll
       for (int rw = 0; rw < UNITS / CHUNKS; ++rw) {
         const int rr = warp + WARPS * rw;
-        float ss = 0.f;
-        for (int k = 0; k < panels; ++k) ss += s_ss[k * 32 + rr];
-        const float r = rsqrtf(ss * (1.0f / static_cast<float>(p.cols)) + p.eps);
+        const float r = s_r[rr];
         if (panel == 0 && lane == 0 && p.r_inv != nullptr) p.r_inv[(row0 + rr) * p.r_inv_stride] = r;
 #pragma unroll
         for (int c = 0; c < CHUNKS; ++c) {
@@ -1069,17 +1145,20 @@ static int32_t mx_rows_run(const char* op, const cdl_tensor* x, const cdl_tensor
 #undef CDL_FP4_FULL
   } else if (y_col) {
     if (!norm) return launch_panels<PLAIN>(p, Extra{}, stream);
-    // The norm: whole rows, where 32 of them fit a CTA's shared memory and there is work for two SMs in three (4096 x 2048
-    // 13 us, by panels 18); else panels that make up the row in a cluster of at most 8 (1024 x 2048 7.7 us, whole
-    // rows 11.6).
+    // The norm.  Rows of which 32 fit a CTA's shared memory: whole; by panels that add up in the same order where few rows
+    // leave SMs without work and the panels fit in one wave (1024 x 2048 11.6 us whole, 6.4; 3136 x 2048 11.8 and 10.4; the other
+    // way 3136 x 2560 14.0 and 17.2, 1024 x 512 4.8 and 6.4).  Wider rows: panels of their own.
     const size_t tile_bytes = 32 * static_cast<size_t>(cols + 8) * 2, gamma_bytes = scale ? static_cast<size_t>(cols) * 4 : 0;
     const bool full = cols % 256 == 0 && !bias && tile_bytes + gamma_bytes <= 227 * 1024;
-    if (!bias && !(full && rows / 32 * 3 >= 2 * sm_count())) {
-      if (cols % 256 == 0 && cols <= 2048 && (cols % 512 != 0 || rows / 32 * (cols / 512) < 2 * sm_count()))
+    const long long blocks = rows / 32, sms = sm_count();
+    if (full && cols >= 1024 && blocks * (cols / 512) <= 3 * sms &&
+        (blocks * 2 <= sms || (cols >= 2048 && blocks * 3 < 2 * sms))) {
+      if (cols <= 2048 && (cols % 512 != 0 || blocks * (cols / 512) < 2 * sms))
         return launch_panels<256, NORM>(p, Extra{}, stream);
-      if (cols % 512 == 0 && cols <= 4096) return launch_panels<512, NORM>(p, Extra{}, stream);
-      if (cols % 1024 == 0 && cols <= 8192) return launch_panels<1024, NORM>(p, Extra{}, stream);
+      if (cols % 512 == 0) return launch_panels<512, NORM>(p, Extra{}, stream);
     }
+    const int panel = cols % 1024 == 0 ? 1024 : cols % 512 == 0 ? 512 : 0;
+    const bool wide = !full && !bias && panel != 0 && cols / panel <= 8 && blocks <= 65535;
     int dev = 0;
     CDL_CUDA(cudaGetDevice(&dev));
     static std::once_flag once[64];
@@ -1091,11 +1170,28 @@ static int32_t mx_rows_run(const char* op, const cdl_tensor* x, const cdl_tensor
         err = cudaFuncSetAttribute(mx_rowcol_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
       if (err == cudaSuccess)
         err = cudaFuncSetAttribute(mx_rowcol_full_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+      if (err == cudaSuccess)
+        err = cudaFuncSetAttribute(mx_rowcol_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   static_cast<int>(wide_smem(1024)));
     });
     if (err != cudaSuccess)
       return fail(CDL_ERR_CUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(err));
     const unsigned grid = static_cast<unsigned>(rows / 32);
-    if (full) mx_rowcol_full_kernel<<<grid, 1024, tile_bytes + gamma_bytes, stream>>>(p);
+    if (wide) {
+      cudaLaunchConfig_t cfg{};
+      p.panel_cols = panel;
+      cfg.gridDim = dim3(static_cast<unsigned>(cols / panel), grid);
+      cfg.blockDim = dim3(static_cast<unsigned>(panel / 2));
+      cfg.dynamicSmemBytes = wide_smem(panel);
+      cfg.stream = stream;
+      cudaLaunchAttribute attr{};
+      attr.id = cudaLaunchAttributeClusterDimension;
+      attr.val.clusterDim.x = static_cast<unsigned>(cols / panel);
+      attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+      cfg.attrs = &attr;
+      cfg.numAttrs = 1;
+      CDL_CUDA(cudaLaunchKernelEx(&cfg, mx_rowcol_wide_kernel, p));
+    } else if (full) mx_rowcol_full_kernel<<<grid, 1024, tile_bytes + gamma_bytes, stream>>>(p);
     else if (tile_bytes <= 227 * 1024) mx_rowcol_tile_kernel<<<grid, 1024, tile_bytes, stream>>>(p);
     else mx_rows_kernel<true, true><<<grid, 1024, COL_SMEM_BYTES, stream>>>(p);
   } else {

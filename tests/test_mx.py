@@ -207,6 +207,44 @@ def test_norm_fwd_mx(cdl, gpu_ok, rows, cols, affine):
         assert np.array_equal(to_f32(cdl.mx.dequantize(t)), got)
 
 
+def _norm_in_order(x, scale, eps, width):
+    """(bf16 y, r_inv) with the squares of a row added in f32 in the kernels' order: a lane its 8 columns of every 256, one
+    after the other (FMAs), the 32 lanes by halves, panels of `width` columns one after the other."""
+    rows, cols = x.shape
+    sq = x.double().view(rows, cols // 256, 32, 8).square()
+    lanes, total = torch.arange(32, device="cuda"), torch.zeros(rows, device="cuda")
+    for c0 in range(0, cols // 256, width // 256):
+        ss = torch.zeros(rows, 32, device="cuda")
+        for c in range(c0, c0 + width // 256):
+            for j in range(8):
+                ss = (ss.double() + sq[:, c, :, j]).float()
+        for o in (16, 8, 4, 2, 1):
+            ss = ss + ss[:, lanes ^ o]
+        total = total + ss[:, 0]
+    inv, eps = float(np.float32(1.0) / np.float32(cols)), float(np.float32(eps))
+    r = torch.rsqrt((total.double() * inv + eps).float())
+    y = x.float() * r[:, None]
+    return (y if scale is None else y * scale.float()).to(torch.bfloat16), r
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [32, 1024, 3136, 3168])
+@pytest.mark.parametrize("cols,affine,width", [(256, 1, 256), (512, 1, 512), (768, 0, 768), (1536, 1, 1536), (2048, 0, 2048),
+                                               (2048, 1, 2048), (2304, 1, 2304), (3072, 1, 3072), (3584, 0, 3584),
+                                               (3584, 1, 512), (4096, 1, 1024), (5120, 0, 1024), (8192, 1, 1024)])
+def test_norm_fwd_mx_adds_in_one_order(cdl, gpu_ok, rows, cols, affine, width):
+    """The bytes of a row do not depend on how many rows there are: whole rows, panels of them where there are few, and the
+    panels of rows too wide for that add a row's squares in an order that its width alone decides."""
+    gen = torch.Generator(device="cuda").manual_seed(rows + cols)
+    x = torch.randn(rows, cols, generator=gen, device="cuda").to(torch.bfloat16)
+    scale = (torch.rand(cols, generator=gen, device="cuda") + 0.5).to(torch.bfloat16) if affine else None
+    y, r = _norm_in_order(x, scale, 1e-6, width)
+    got = cdl.mx.norm_fwd_mx(x, scale, eps=1e-6, colwise=True, save_stats=True)
+    assert torch.equal(got.r_inv, r)
+    for a, b in zip((got.y, got.y_col), cdl.mx.quantize(y, colwise=True)):
+        assert torch.equal(a.values, b.values) and torch.equal(a.scale_factors, b.scale_factors)
+
+
 MM_CASES = [(192, 256, 160), (128, 32, 64), (128, 128, 256), (256, 2048, 512), (100, 96, 24),
             (384, 416, 296), (1024, 1024, 2048)]
 
