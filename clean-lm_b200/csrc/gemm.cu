@@ -1080,6 +1080,26 @@ static int choose_cluster_splits(long long batch, long long M, long long N, long
   return splits;
 }
 
+// K slices of a CTA-pair product that adds into D.
+// time ~ waves * (K slice + a fixed per-unit cost of epilogue / ramp).  The fixed part is worth
+// ~6 K blocks without slices and ~10 with them, whose additions into D are reductions at the L2
+// (fitted to 47 shapes, 64 to 16384 deep; mean distance from the best slice count 0.4 %, worst
+// 6 %; with 6 for both 1.3 % and 25 %: 2048 x 5632 x 2048 takes 53 us whole and 66 us in two
+// slices, 2048 x 6144 x 16384 285 whole and 299 in three).
+static int choose_pair_slices(long long tiles, int k_blocks, long long clusters) {
+  int best_s = 1;
+  double best_cost = 1e30;
+  for (int sp = 1; sp <= 8 && sp * 8 <= k_blocks; ++sp) {
+    const long long waves = (tiles * sp + clusters - 1) / clusters;
+    const double cost = static_cast<double>(waves) * (static_cast<double>(k_blocks) / sp + (sp == 1 ? 6.0 : 10.0));
+    if (cost < best_cost * 0.97) {
+      best_cost = cost;
+      best_s = sp;
+    }
+  }
+  return best_s;
+}
+
 }  // namespace gemm
 
 static int32_t check_epi_operand(const char* name, const cdl_tensor* t, long long M, long long N) {
@@ -1175,9 +1195,18 @@ int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_t
                         d->stride[r - 2] >= N && c->stride[r - 2] == d->stride[r - 2] &&
                         (r == 2 || batch == 1 ||
                          (d->stride[0] % 4 == 0 && d->stride[0] > 0 && c->stride[0] == d->stride[0]));
-  const int cluster_splits =
-      variant == CDL_GEMM_AUTO ? choose_cluster_splits(batch, M, N, K, adds_f32, use_c && !adds_f32, may_slice, reduces, tma_adds)
-                               : 0;
+  auto splits_of = [&](bool tma) {
+    return choose_cluster_splits(batch, M, N, K, adds_f32, use_c && !adds_f32, may_slice, reduces, tma);
+  };
+  int cluster_splits = variant == CDL_GEMM_AUTO ? splits_of(tma_adds) : 0;
+  // The error of a sum in the tensor core grows with its length: a shorter store is no reason for fewer K slices (129 x
+  // 384 x 640 whole instead of in four slices: 4.7e-7 off, not 1.3e-7).  One in a thousand weight gradients.
+  if (variant == CDL_GEMM_AUTO && cluster_splits == 0 && tma_adds) {
+    const int sliced = splits_of(false);
+    const long long tiles = batch * ((M + PAIR_M - 1) / PAIR_M) * ((N + BN - 1) / BN);
+    if (sliced > (may_slice ? choose_pair_slices(tiles, static_cast<int>((K + BK - 1) / BK), sm_count() / 2) : 1))
+      cluster_splits = sliced;
+  }
   const bool use_cluster = cluster_splits > 0;
   const bool use_pair = !use_cluster && (variant == CDL_GEMM_AUTO ? M > BM : variant == CDL_GEMM_CTA_PAIR);
   const int tile_m = use_pair ? PAIR_M : BM;
@@ -1380,24 +1409,7 @@ int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_t
   // unordered f32 sum; the caller's `deterministic` option turns it off.
   if (use_pair && adds_in_place) {
     if (!(opts && opts->deterministic != 0)) {
-      const int nc = max_clusters[dev & 63];
-      int best_s = 1;
-      double best_cost = 1e30;
-      for (int sp = 1; sp <= 8 && sp * 8 <= p.k_blocks; ++sp) {
-        const long long units = static_cast<long long>(p.num_tiles) * sp;
-        const long long waves = (units + nc - 1) / nc;
-        // time ~ waves * (K slice + a fixed per-unit cost of epilogue / ramp).  The fixed part is worth
-        // ~6 K blocks without slices and ~10 with them, whose additions into D are reductions at the L2
-        // (fitted to 47 shapes, 64 to 16384 deep; mean distance from the best slice count 0.4 %, worst
-        // 6 %; with 6 for both 1.3 % and 25 %: 2048 x 5632 x 2048 takes 53 us whole and 66 us in two
-        // slices, 2048 x 6144 x 16384 285 whole and 299 in three).
-        const double cost = static_cast<double>(waves) *
-                            (static_cast<double>(p.k_blocks) / sp + (sp == 1 ? 6.0 : 10.0));
-        if (cost < best_cost * 0.97) {
-          best_cost = cost;
-          best_s = sp;
-        }
-      }
+      const int best_s = choose_pair_slices(p.num_tiles, p.k_blocks, max_clusters[dev & 63]);
       if (best_s > 1) {
         p.split_k = best_s;
         p.atomic_out = 1;

@@ -774,3 +774,23 @@ def test_laid_out_f32_values_without_pieces(cdl, gpu_ok, batch, m, k, n, ta, tb,
     ok = expected.isfinite()
     assert bool(((d - expected).abs()[ok] <= (k + 10) * 2.0 ** -24 * bound[ok] + floor).all())
     assert cdl._lib.device_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,k,deterministic", [(136, 384, 640, True), (320, 6400, 3328, False), (384, 6464, 3264, False),
+                                                 (2304, 2112, 7168, True)])
+def test_weight_gradients_keep_their_slices(cdl, gpu_ok, m, n, k, deterministic):
+    """D += A^T B in f32 of shapes that take two or more K slices in clusters where TMA additions are not to be had: with them
+    the sums are no longer.  The error grows with the length of a sum in the tensor core, so two slices halve that of
+    the CTA-pair kernel, which sums these whole; three quarters leave room for the additions' own rounding."""
+    gen = torch.Generator(device="cuda").manual_seed(m + k)
+    a, b = (torch.randn(k, w, generator=gen, device="cuda").to(torch.bfloat16) for w in (m, n))
+    exact = a.double().T @ b.double()
+    errors = []
+    for variant in (cdl._lib.GEMM_AUTO, cdl._lib.GEMM_CTA_PAIR):
+        d = torch.zeros(m, n, device="cuda")
+        opts = cdl.ops.MatmulOpts(out=torch.float32, c=d, beta=1.0, variant=variant,
+                                  deterministic=deterministic or variant != cdl._lib.GEMM_AUTO)
+        cdl.ops.matmul(a.T, b, opts, out=d)
+        errors.append(((d.double() - exact).norm() / exact.norm()).item())
+    assert errors[0] < 0.75 * errors[1], errors
