@@ -347,10 +347,10 @@ __device__ __noinline__ void partial_by_fma(const Operand oa, const Operand ob, 
   }
 }
 
-template <int S, int W, bool PAIR = false>
+template <int S, int W, bool PAIR, int ROWS>
 __device__ __forceinline__ void store_out(const Params& p, const float* part, int rank, int warp, int b, int m0,
                                           int n0) {
-  gemm::TileOut<S, W, PAIR> out;
+  gemm::TileOut<S, W, PAIR, ROWS> out;
   out.prefetch(p, rank, warp, b, m0, n0);
   out.finish(p, part, rank, warp, b, m0, n0);
 }
@@ -531,10 +531,10 @@ __global__ void __launch_bounds__(THREADS, 1)
   else __syncthreads();
   if (warp >= 1) {
     switch (p.split_k) {
-      case 1: store_out<1, WARPS - 1>(p, part, rank, warp - 1, b, m0, n0); break;
-      case 2: store_out<2, WARPS - 1>(p, part, rank, warp - 1, b, m0, n0); break;
-      case 4: store_out<4, WARPS - 1>(p, part, rank, warp - 1, b, m0, n0); break;
-      default: store_out<8, WARPS - 1>(p, part, rank, warp - 1, b, m0, n0); break;
+      case 1: store_out<1, WARPS - 1, false, 1>(p, part, rank, warp - 1, b, m0, n0); break;
+      case 2: store_out<2, WARPS - 1, false, 1>(p, part, rank, warp - 1, b, m0, n0); break;
+      case 4: store_out<4, WARPS - 1, false, 1>(p, part, rank, warp - 1, b, m0, n0); break;
+      default: store_out<8, WARPS - 1, false, 1>(p, part, rank, warp - 1, b, m0, n0); break;
     }
   }
   __syncwarp();
@@ -866,10 +866,10 @@ __global__ void __launch_bounds__(piece_threads<T>(), SLOTS == shared_slots(PAIR
   else __syncthreads();
   if (m0 < p.M) {
     switch (p.split_k) {
-      case 1: store_out<1, W, PAIR>(p, part, rank, warp, b, m0, n0); break;
-      case 2: store_out<2, W, PAIR>(p, part, rank, warp, b, m0, n0); break;
-      case 4: store_out<4, W, PAIR>(p, part, rank, warp, b, m0, n0); break;
-      default: store_out<PAIR ? 4 : 8, W, PAIR>(p, part, rank, warp, b, m0, n0); break;
+      case 1: store_out<1, W, PAIR, 4>(p, part, rank, warp, b, m0, n0); break;
+      case 2: store_out<2, W, PAIR, 4>(p, part, rank, warp, b, m0, n0); break;
+      case 4: store_out<4, W, PAIR, 4>(p, part, rank, warp, b, m0, n0); break;
+      default: store_out<PAIR ? 4 : 8, W, PAIR, 4>(p, part, rank, warp, b, m0, n0); break;
     }
   }
   __syncwarp();

@@ -167,7 +167,10 @@ __device__ __forceinline__ int rope_position(const Params& p, int row) {
 // the tile takes a tenth of it.
 //
 // PAIR: the cluster holds S pairs of CTAs; slice s of this CTA's 128 rows lies in CTA 2 s + (its rank & 1).
-template <int S, int W, bool PAIR = false>
+// ROWS: rows off the 16-byte grid that a warp takes at a time (finish_scalar).  Four pay where a CTA has 128 rows and many K
+// blocks (cluster kernel, 515 x 1030 x 2056: 21.6 -> 16.8 us); the general kernel's products, most of them small, take one
+// (16 x 515 x 515 7.2 us, four 9.6; 8 x 4097 x 4097 23.8 and 25.5).
+template <int S, int W, bool PAIR = false, int ROWS = 4>
 struct TileOut {
   static __device__ __forceinline__ uint32_t part_of(uint32_t at, int s) {
     return S == 1 ? at : mapa_shared(at, PAIR ? 2 * s + (cluster_ctarank() & 1) : s);
@@ -337,11 +340,10 @@ struct TileOut {
   }
 
   // Rows off the 16-byte grid or a column count that is no multiple of 4 (never a fused form): lane l
-  // takes columns l, l + 32, l + 64 and l + 96, so that every access of the warp is contiguous; four rows at a time,
-  // whose loads of C are in flight together.
+  // takes columns l, l + 32, l + 64 and l + 96, so that every access of the warp is contiguous; ROWS at a
+  // time, whose loads are in flight together.
   static __device__ __forceinline__ void finish_scalar(const Params& p, uint32_t base, int rank, int warp, int b,
                                                        int m0, int n0) {
-    constexpr int ROWS = 4;
     const int lane = threadIdx.x & 31;
     const int rows = min(128, p.M - m0);
     const long long at_c = b * p.c_batch + m0 * p.ldc + n0 + lane, at_d = b * p.d_batch + m0 * p.ldd + n0 + lane;
