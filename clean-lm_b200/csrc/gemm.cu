@@ -667,9 +667,15 @@ __global__ void __launch_bounds__(THREADS, 1)
 constexpr int PAIR_STAGES = 6;
 constexpr int PAIR_STAGE_BYTES = 2 * A_BYTES;  // A 128 x 64 and half of B 128 x 64
 constexpr int PAIR_M = 2 * BM;
-constexpr int PAIR_STAGING = EPI_WARPS * CHUNK_BYTES;  // a buffer per epilogue warp
 constexpr int PAIR_BARRIER_BYTES = 512;
-constexpr size_t PAIR_SMEM_BYTES = 1024 + PAIR_STAGES * PAIR_STAGE_BYTES + PAIR_STAGING + PAIR_BARRIER_BYTES;
+// One kernel per kind of store.  All of them in one, with the buffers that the plain ones do not need (they take room
+// from the L1, through which C is read), cost those 0.2 to 0.9 us (2048 x 5632 x
+// 256 12.3 instead of 11.9, with a bf16 C 18.8 instead of 18.0).
+enum PairStore { STORE, STORE_ADD, STORE_SWIGLU };  // D (with C, or rotated), D += by TMA, the fused SwiGLU forms
+constexpr int pair_staging(int kind) { return kind == STORE ? 0 : EPI_WARPS * CHUNK_BYTES; }  // a buffer per epilogue warp
+constexpr size_t pair_smem_bytes(int kind) {
+  return 1024 + PAIR_STAGES * PAIR_STAGE_BYTES + pair_staging(kind) + PAIR_BARRIER_BYTES;
+}
 
 // Work units are handed out at run time: a cluster's first unit is its index, every further one
 // comes from a global counter, so a cluster that finds its SMs late (another kernel, e.g. a
@@ -694,6 +700,7 @@ struct PairBarriers {
 };
 static_assert(sizeof(PairBarriers) <= PAIR_BARRIER_BYTES, "barriers fit behind the staging buffers");
 
+template <int KIND>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
     gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
                           const __grid_constant__ CUtensorMap tmap_b,
@@ -703,7 +710,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
   uint8_t* staging = smem + PAIR_STAGES * PAIR_STAGE_BYTES;
-  PairBarriers* bars = reinterpret_cast<PairBarriers*>(staging + PAIR_STAGING);
+  PairBarriers* bars = reinterpret_cast<PairBarriers*>(staging + pair_staging(KIND));
   volatile int* abort_word = &bars->abort_word;
 
   const int warp = threadIdx.x >> 5;
@@ -899,7 +906,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
     const int quad = warp & 3;
     const int half = (warp - 2) >> 2;
     uint8_t* buf = staging + (warp - 2) * CHUNK_BYTES;
-    const bool swiglu = p.epi_mode == 1 || p.epi_mode == 2;
     SwigluFeed feed{&tmap_e0, &tmap_e1, buf, &bars->extra_full[warp - 2], p.epi_mode == 2, 0};
     if (p.early == 2) grid_dep_wait();
     int t = 0;
@@ -916,20 +922,24 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
       const uint32_t acc_ph = (t >> 1) & 1;
       const int row = tm * PAIR_M + static_cast<int>(rank) * BM + quad * 32 + lane;
       const int col = tn * BN + half * (BN / 2);
-      if (swiglu && row - lane < p.M && col < p.N) feed.load(lane, row - lane, col);  // under the products
+      if (KIND == STORE_SWIGLU && row - lane < p.M && col < p.N) feed.load(lane, row - lane, col);  // under the products
       if (!mbar_wait(&bars->acc_full[acc], acc_ph, abort_word, 311)) break;
       tc_fence_after();
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BN + half * (BN / 2);
-      if (p.tma_add) add_tile_rows(p, &tmap_e0, buf, t_row, b, row - lane, col, lane);
-      else if (p.epi_mode == 1) store_tile_rows_swiglu<false>(p, feed, t_row, row, col, lane, abort_word);
-      else if (p.epi_mode == 2) store_tile_rows_swiglu<true>(p, feed, t_row, row, col, lane, abort_word);
-      else if (p.epi_mode == 3) store_tile_rows_rope(p, t_row, row, col);
-      else store_tile_rows(p, t_row, b, row, col);
+      if constexpr (KIND == STORE_ADD) {
+        add_tile_rows(p, &tmap_e0, buf, t_row, b, row - lane, col, lane);
+      } else if constexpr (KIND == STORE_SWIGLU) {
+        if (p.epi_mode == 1) store_tile_rows_swiglu<false>(p, feed, t_row, row, col, lane, abort_word);
+        else store_tile_rows_swiglu<true>(p, feed, t_row, row, col, lane, abort_word);
+      } else {
+        if (p.epi_mode == 3) store_tile_rows_rope(p, t_row, row, col);
+        else store_tile_rows(p, t_row, b, row, col);
+      }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&bars->acc_empty[acc]), 0));
     }
-    if (p.tma_add && lane == 0) tma_store_wait<0>();
+    if (KIND == STORE_ADD && lane == 0) tma_store_wait<0>();
   }
 
   // ------------------------------------------------------------ tear-down
@@ -1383,18 +1393,22 @@ int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_t
   std::call_once(attr_once[dev & 63], [&] {
     attr_err = cudaFuncSetAttribute(gemm_bf16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     static_cast<int>(SMEM_BYTES));
-    if (attr_err == cudaSuccess)
-      attr_err = cudaFuncSetAttribute(gemm_bf16_pair_kernel,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(PAIR_SMEM_BYTES));
+    auto pair = [&](auto kernel, int kind) {
+      if (attr_err == cudaSuccess)
+        attr_err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        static_cast<int>(pair_smem_bytes(kind)));
+    };
+    pair(gemm_bf16_pair_kernel<STORE>, STORE);
+    pair(gemm_bf16_pair_kernel<STORE_ADD>, STORE_ADD);
+    pair(gemm_bf16_pair_kernel<STORE_SWIGLU>, STORE_SWIGLU);
     // How many CTA pairs the device can hold at once (GPCs with an odd SM count lose one SM).
     int n = 0;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(sm_count() & ~1));
     cfg.blockDim = dim3(THREADS);
-    cfg.dynamicSmemBytes = PAIR_SMEM_BYTES;
+    cfg.dynamicSmemBytes = pair_smem_bytes(STORE);
     if (attr_err == cudaSuccess &&
-        cudaOccupancyMaxActiveClusters(&n, gemm_bf16_pair_kernel, &cfg) == cudaSuccess && n > 0)
+        cudaOccupancyMaxActiveClusters(&n, gemm_bf16_pair_kernel<STORE>, &cfg) == cudaSuccess && n > 0)
       max_clusters[dev & 63] = n;
     else
       max_clusters[dev & 63] = sm_count() / 2;
@@ -1432,8 +1446,12 @@ int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_t
     const long long units = static_cast<long long>(p.num_tiles) * p.split_k;
     const int clusters = units < max_clusters[dev & 63] ? static_cast<int>(units) : max_clusters[dev & 63];
     p.sched_counter = units > clusters ? sched_counter_for(gemm_counter_kind(early), dev, stream) : nullptr;
-    CDL_CUDA(launch_pdl(gemm_bf16_pair_kernel, dim3(2 * clusters), dim3(THREADS), PAIR_SMEM_BYTES, stream,
-                        tm_a, tm_b, tm_e0, tm_e1, p));
+    auto run = [&](auto kernel, int kind) {
+      return launch_pdl(kernel, dim3(2 * clusters), dim3(THREADS), pair_smem_bytes(kind), stream, tm_a, tm_b, tm_e0, tm_e1, p);
+    };
+    CDL_CUDA(p.tma_add                             ? run(gemm_bf16_pair_kernel<STORE_ADD>, STORE_ADD)
+             : p.epi_mode == 1 || p.epi_mode == 2 ? run(gemm_bf16_pair_kernel<STORE_SWIGLU>, STORE_SWIGLU)
+                                                  : run(gemm_bf16_pair_kernel<STORE>, STORE));
   } else {  // (this one always waits at its start)
     const int grid = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
     CDL_CUDA(launch_pdl(gemm_bf16_kernel, dim3(grid), dim3(THREADS), SMEM_BYTES, stream, tm_a, tm_b, p));
