@@ -671,7 +671,7 @@ constexpr int PAIR_BARRIER_BYTES = 512;
 // One kernel per kind of store.  All of them in one, with the buffers that the plain ones do not need (they take room
 // from the L1, through which C is read), cost those 0.2 to 0.9 us (2048 x 5632 x
 // 256 12.3 instead of 11.9, with a bf16 C 18.8 instead of 18.0).
-enum PairStore { STORE, STORE_ADD, STORE_SWIGLU };  // D (with C, or rotated), D += by TMA, the fused SwiGLU forms
+enum PairStore { STORE, STORE_ADD, STORE_SWIGLU };  // D in any form, D += by TMA, the SwiGLU forms whose operands TMA brings
 constexpr int pair_staging(int kind) { return kind == STORE ? 0 : EPI_WARPS * CHUNK_BYTES; }  // a buffer per epilogue warp
 constexpr size_t pair_smem_bytes(int kind) {
   return 1024 + PAIR_STAGES * PAIR_STAGE_BYTES + pair_staging(kind) + PAIR_BARRIER_BYTES;
@@ -1362,7 +1362,10 @@ int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_t
     CDL_CHECK(encode_tmap(&tm_e0, p.d, CDL_F32, 3, dims, strides, box, true));
     p.tma_add = 1;
   }
-  if (use_pair && (p.epi_mode == 1 || p.epi_mode == 2)) {
+  // (rows that overlap, one row for all of M for instance, are read by the store itself)
+  const bool feeds = use_pair && (p.epi_mode == 1 || p.epi_mode == 2) && aux0->stride[0] >= N &&
+                     (p.epi_mode == 1 || aux1->stride[0] >= N);
+  if (feeds) {
     const cdl_tensor* aux[2] = {aux0, aux1};
     for (int i = 0; i < p.epi_mode; ++i) {
       const uint64_t ld = static_cast<uint64_t>(aux[i]->stride[0]) * 2;
@@ -1449,9 +1452,9 @@ int32_t matmul_execute_epi(const cdl_tensor* a, const cdl_tensor* b, const cdl_t
     auto run = [&](auto kernel, int kind) {
       return launch_pdl(kernel, dim3(2 * clusters), dim3(THREADS), pair_smem_bytes(kind), stream, tm_a, tm_b, tm_e0, tm_e1, p);
     };
-    CDL_CUDA(p.tma_add                             ? run(gemm_bf16_pair_kernel<STORE_ADD>, STORE_ADD)
-             : p.epi_mode == 1 || p.epi_mode == 2 ? run(gemm_bf16_pair_kernel<STORE_SWIGLU>, STORE_SWIGLU)
-                                                  : run(gemm_bf16_pair_kernel<STORE>, STORE));
+    CDL_CUDA(p.tma_add ? run(gemm_bf16_pair_kernel<STORE_ADD>, STORE_ADD)
+             : feeds   ? run(gemm_bf16_pair_kernel<STORE_SWIGLU>, STORE_SWIGLU)
+                       : run(gemm_bf16_pair_kernel<STORE>, STORE));
   } else {  // (this one always waits at its start)
     const int grid = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
     CDL_CUDA(launch_pdl(gemm_bf16_kernel, dim3(grid), dim3(THREADS), SMEM_BYTES, stream, tm_a, tm_b, p));

@@ -794,3 +794,23 @@ def test_weight_gradients_keep_their_slices(cdl, gpu_ok, m, n, k, deterministic)
         cdl.ops.matmul(a.T, b, opts, out=d)
         errors.append(((d.double() - exact).norm() / exact.norm()).item())
     assert errors[0] < 0.75 * errors[1], errors
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,k", [(64, 136, 64), (300, 264, 128), (2048, 1024, 64)])
+def test_fused_swiglu_operands_may_share_a_row(cdl, gpu_ok, m, n, k):
+    """up, and gate of the backward, as one row for all of M (stride 0): the bits of the same operands laid out."""
+    L = cdl._lib
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda").to(torch.bfloat16)
+    a, b, gate, up = rnd(m, k), rnd(k, n), rnd(1, n), rnd(1, n)
+    results = []
+    for lay in (lambda t: t.expand(m, n), lambda t: t.expand(m, n).contiguous()):
+        d = [torch.empty(m, n, dtype=torch.bfloat16, device="cuda") for _ in range(4)]
+        fwd = [L.tensor_arg(t) for t in (a, b, lay(up), d[0], d[1])]
+        L.check(L.lib.cdl_b200_matmul_swiglu_gate(*(L.ref(t) for t in fwd), None))
+        bwd = [L.tensor_arg(t) for t in (a, b, lay(gate), lay(up), d[2], d[3])]
+        L.check(L.lib.cdl_b200_matmul_swiglu_dgrad(*(L.ref(t) for t in bwd), None))
+        results.append(d)
+    assert all(torch.equal(x, y) for x, y in zip(*results))
+    assert cdl._lib.device_status() == 0
