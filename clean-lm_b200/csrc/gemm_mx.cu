@@ -95,10 +95,6 @@ struct Params {
   uint8_t* out_values;
   uint8_t* out_sf;
   float alpha;
-  // Rotate-half RoPE of the heads (128 columns each) below rope_cols (bf16 outputs; null: none): f32 rows of cos | sin
-  // by position = row % rope_seqlen.
-  const float* rope_table;
-  int rope_seqlen, rope_cols;
   int* status;
   int early;  // 1 = starts before the kernel ahead of it has finished (see matmul_mx_group_execute)
 };
@@ -215,43 +211,6 @@ __device__ __forceinline__ uint32_t fp8x4(float a, float b, float c, float d) {
   const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(a, b), __NV_SATFINITE, __NV_E4M3);
   const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(c, d), __NV_SATFINITE, __NV_E4M3);
   return lo | (hi << 16);
-}
-
-// Two 32-column chunks of one output row, 64 columns apart in a head of 128, rotated by the row's position.  The product
-// is rounded to bf16 first, so that the results are those of the plain product and a rotation of what it stored.
-__device__ __forceinline__ void store_rope_pair(const Params& p, const uint32_t (&lo)[32], const uint32_t (&hi)[32], int row,
-                                                int col0) {
-  const float* cs = p.rope_table + static_cast<long long>(row % p.rope_seqlen) * 128 + (col0 & 63);
-  const bool rotate = col0 < p.rope_cols;
-  uint32_t olo[16], ohi[16];
-#pragma unroll
-  for (int g = 0; g < 8; ++g) {
-    float c[4] = {1.f, 1.f, 1.f, 1.f}, sn[4] = {0.f, 0.f, 0.f, 0.f};
-    if (rotate) {
-      const float4 cv = __ldg(reinterpret_cast<const float4*>(cs + g * 4));
-      const float4 sv = __ldg(reinterpret_cast<const float4*>(cs + 64 + g * 4));
-      c[0] = cv.x; c[1] = cv.y; c[2] = cv.z; c[3] = cv.w;
-      sn[0] = sv.x; sn[1] = sv.y; sn[2] = sv.z; sn[3] = sv.w;
-    }
-    float rl[4], rh[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float l = __bfloat162float(__float2bfloat16_rn(p.alpha * __uint_as_float(lo[g * 4 + e])));
-      const float h = __bfloat162float(__float2bfloat16_rn(p.alpha * __uint_as_float(hi[g * 4 + e])));
-      rl[e] = l * c[e] - h * sn[e];
-      rh[e] = h * c[e] + l * sn[e];
-    }
-    olo[g * 2] = pack_bf16x2(rl[0], rl[1]);
-    olo[g * 2 + 1] = pack_bf16x2(rl[2], rl[3]);
-    ohi[g * 2] = pack_bf16x2(rh[0], rh[1]);
-    ohi[g * 2 + 1] = pack_bf16x2(rh[2], rh[3]);
-  }
-  __nv_bfloat16* d = static_cast<__nv_bfloat16*>(p.d) + static_cast<long long>(row) * p.ldd + col0;
-#pragma unroll
-  for (int g = 0; g < 4; ++g) {
-    *reinterpret_cast<uint4*>(d + g * 8) = make_uint4(olo[g * 4], olo[g * 4 + 1], olo[g * 4 + 2], olo[g * 4 + 3]);
-    *reinterpret_cast<uint4*>(d + 64 + g * 8) = make_uint4(ohi[g * 4], ohi[g * 4 + 1], ohi[g * 4 + 2], ohi[g * 4 + 3]);
-  }
 }
 
 // The NVFP4 form of the block-scaled store: the 32 columns are two blocks of 16; scale = amax / 6
@@ -756,28 +715,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
           else store32_mx(p, r, row, col0);
         }
       };
-      if (!FP4 && !ADD && p.rope_table != nullptr) {
-        // chunk pairs (1, 3) and (0, 2), the one that holds the shared columns first
-#pragma unroll 1
-        for (int k = 0; k < 2; ++k) {
-          const int ch = backwards ? 1 - k : k;
-          uint32_t lo[32], hi[32];
-          tmem_ld32(t_row + ch * 32, lo);
-          tmem_ld32(t_row + (ch + 2) * 32, hi);
-          tmem_wait_ld(lo, hi);
-          if (owner && k == 0) {
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(ovl_leader);
-          }
-          if (row < p.M && col_base < p.N) store_rope_pair(p, lo, hi, row, col_base + ch * 32);
-          __syncwarp();
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&bars->acc_empty[acc]), 0));
-        continue;
-      }
       int i = 0;
       if (owner) {
         uint32_t r0[32], r1[32];
@@ -830,8 +767,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 static int32_t matmul_mx_run(const char* op, const cdl_mx_tensor* a, const cdl_mx_tensor* b,
                              const cdl_tensor* c, const cdl_tensor* d, const cdl_mx_tensor* d_mx,
                              float alpha, float beta, cudaStream_t stream,
-                             const cdl_matmul_options* opts = nullptr, const RopeEpilogue* rope = nullptr,
-                             bool early = false) {
+                             const cdl_matmul_options* opts = nullptr, bool early = false) {
   using namespace gemm_mx;
   if (!a || !b || (!d && !d_mx)) return fail(CDL_ERR_INVALID, "%s: a, b and d are required", op);
   const int variant = opts ? opts->variant : CDL_GEMM_AUTO;
@@ -945,16 +881,6 @@ static int32_t matmul_mx_run(const char* op, const cdl_mx_tensor* a, const cdl_m
                (M == 1 || (c->stride[0] * dtype_size(c->dtype)) % 32 == 0);
     }
   }
-  if (rope) {
-    if (fp4 || d->dtype != CDL_BF16 || p.c_mode != 0 || N % 128 != 0 || rope->rot_cols > N ||
-        (reinterpret_cast<uintptr_t>(d->ptr) & 15) != 0 || d->stride[0] % 8 != 0 ||
-        (reinterpret_cast<uintptr_t>(rope->table) & 15) != 0)
-      return fail(CDL_ERR_INVALID, "%s: MXFP8 operands, a bf16 output of whole heads of 128 columns with 16-byte aligned "
-                  "rows and a 16-byte aligned table are required", op);
-    p.rope_table = rope->table;
-    p.rope_seqlen = rope->seqlen;
-    p.rope_cols = rope->rot_cols;
-  }
   p.alpha = alpha;
   p.status = device_status_ptr();
   if (!p.status) return fail(CDL_ERR_CUDA, "cannot resolve the device status word");
@@ -973,7 +899,7 @@ static int32_t matmul_mx_run(const char* op, const cdl_mx_tensor* a, const cdl_m
     CDL_CHECK(encode_tmap(&tb, b->values, TMAP_U8, 3, dims, strides, box, true));
   }
   ProfileScope ps(PROF_GEMM, 2.0 * M * N * K, stream);
-  if (rope || (variant == CDL_GEMM_AUTO ? M > BM : variant == CDL_GEMM_CTA_PAIR)) {
+  if (variant == CDL_GEMM_AUTO ? M > BM : variant == CDL_GEMM_CTA_PAIR) {
     // CTA pairs over 256 x 256 tiles
     p.num_m_tiles = static_cast<int>((M + 2 * BM - 1) / (2 * BM));
     p.num_tiles = p.num_m_tiles * p.num_n_tiles;
@@ -1077,7 +1003,7 @@ static int32_t matmul_mx_group_execute(const cdl_mx_product* products, int32_t c
       for (int k = 0; k < other.count; ++k) early = early && !meet(mine.at[D], other.at[k]);
     }
     const cdl_mx_product& p = products[i];
-    CDL_CHECK(matmul_mx_run(op, p.a, p.b, p.c, p.d, nullptr, p.alpha, p.beta, stream, nullptr, nullptr, early));
+    CDL_CHECK(matmul_mx_run(op, p.a, p.b, p.c, p.d, nullptr, p.alpha, p.beta, stream, nullptr, early));
     if (!early && !no_kernel(p)) waited = i;
   }
   return CDL_OK;
@@ -1131,14 +1057,25 @@ int32_t cdl_b200_matmul_mx_opt(const cdl_mx_tensor* a, const cdl_mx_tensor* b, c
 int32_t cdl_b200_matmul_mx_rope(const cdl_mx_tensor* a, const cdl_mx_tensor* b, const cdl_tensor* cos_sin,
                                 int32_t rot_heads, int32_t seqlen, const cdl_tensor* d, cdl_stream stream) {
   using namespace cdl;
-  const char* op = "matmul (block-scaled operands, RoPE epilogue)";
+  const char* op = "matmul (block-scaled operands, RoPE)";
   if (!cos_sin || cos_sin->rank != 2 || cos_sin->dtype != CDL_F32 || cos_sin->shape[1] != 128 ||
       cos_sin->stride[1] != 1 || cos_sin->stride[0] != 128 || seqlen <= 0 || cos_sin->shape[0] < seqlen)
     return fail(CDL_ERR_INVALID, "%s: cos_sin must be packed f32 [>= seqlen, 128] (head_dim 128)", op);
   if (rot_heads < 0 || rot_heads > INT32_MAX / 128) return fail(CDL_ERR_INVALID, "%s: rot_heads out of range", op);
-  if (!d) return fail(CDL_ERR_INVALID, "%s: a, b and d are required", op);
-  const RopeEpilogue rope{static_cast<const float*>(cos_sin->ptr), seqlen, rot_heads * 128, nullptr, 0};
-  return matmul_mx_run(op, a, b, nullptr, d, nullptr, 1.0f, 0.0f, static_cast<cudaStream_t>(stream), nullptr, &rope);
+  if (!a || !b || !d) return fail(CDL_ERR_INVALID, "%s: a, b and d are required", op);
+  const long long M = d->shape[0], N = d->shape[1];
+  if (d->rank == 2 && M > 0 && N > 0 &&
+      (a->format != CDL_MXFP8 || d->dtype != CDL_BF16 || N % 128 != 0 || rot_heads * 128LL > N ||
+       (reinterpret_cast<uintptr_t>(d->ptr) & 15) != 0 || d->stride[0] % 8 != 0 ||
+       (reinterpret_cast<uintptr_t>(cos_sin->ptr) & 15) != 0))
+    return fail(CDL_ERR_INVALID, "%s: MXFP8 operands, a bf16 output of whole heads of 128 columns with 16-byte aligned "
+                "rows and a 16-byte aligned table are required", op);
+  // Two launches: rotated in the product's store, where a lane reads its own row of the table, the product took longer
+  // than both (block of 1 x 512 tokens 360 us, 355 like this; 1 x 1024 421 and 417; 8 x 2048 the same).
+  CDL_CHECK(matmul_mx_run(op, a, b, nullptr, d, nullptr, 1.0f, 0.0f, static_cast<cudaStream_t>(stream)));
+  if (M == 0 || N == 0) return CDL_OK;
+  const cdl_tensor heads{d->ptr, CDL_BF16, 3, {M, N / 128, 128}, {d->stride[0], 128, 1}};
+  return rope_execute(&heads, cos_sin, rot_heads, seqlen, 0, static_cast<cudaStream_t>(stream));
 }
 
 int32_t cdl_b200_matmul_mx_out(const cdl_mx_tensor* a, const cdl_mx_tensor* b, const cdl_mx_tensor* d,
