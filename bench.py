@@ -414,7 +414,7 @@ def run_ours(args) -> None:
         # kernels launched per step: 15 GEMM (SwiGLU fused into two of them, RoPE into the QKV
         # projection), 4 norm fwd, 2 x 2 norm bwd, 1 attn fwd, 3 attn bwd (the inverse RoPE in
         # their store epilogues), 1 embedding
-        launches_per_step = 15 + 4 + 4 + 1 + 3 + 1
+        launches_per_step = 15 + 2 + 4 + 1 + 3 + 1
         # DRAM traffic of the average GEMM launch.  The block's shapes are too large to capture
         # under Nsight Compute, so: the minimum bytes of each of the 15 GEMMs (operands read once,
         # outputs written once, accumulated outputs read and written, fused-epilogue operands

@@ -59,9 +59,9 @@ int sm_count() {
 // Work counters of the kernels that hand out their work at run time (the CTA-pair GEMM's units,
 // kind 0; the persistent attention forward's items, kind 1; the persistent attention backward
 // kernels' items, kinds 2 and 3; GEMMs that start early, kinds 4 to 7): one per kind, device and stream, zero
-// between launches (the kernel's last draw puts its counter back).  Launches on one stream run
-// one after the other, so they can share a counter; launches on different streams may overlap and
-// must not.  Inside the library's device image: nothing is allocated.  A launch that gets no
+// between launches (the kernel's last draw puts its counter back).  Launches that wait for one another
+// share a counter; those that may overlap must not: on different streams, and on one stream a GEMM that starts
+// early and what it starts beside, whose kinds therefore differ (a kind returns only behind a kernel that has waited).  Inside the library's device image: nothing is allocated.  A launch that gets no
 // counter (more than SCHED_STREAMS streams on a device) runs with its fixed assignment.
 #ifndef CDL_DYNAMIC_WORK
 #define CDL_DYNAMIC_WORK 1

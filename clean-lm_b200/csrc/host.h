@@ -54,7 +54,8 @@ int32_t encode_tmap(CUtensorMap* out, const void* base, int32_t dtype, int rank,
 
 // Launches `kernel` with the programmatic-serialization attribute (see grid_dep_wait in ptx.cuh):
 // the kernel may begin before the previous kernel of the stream has finished and MUST call
-// grid_dep_wait() before its first access to global memory.  CDL_PDL=0 builds launch normally.
+// grid_dep_wait() before its first access to global memory, or, where it starts early under the conditions given there, at
+// its end.  CDL_PDL=0 builds launch normally.
 #ifndef CDL_PDL
 #define CDL_PDL 1
 #endif

@@ -8,10 +8,10 @@
 //   forward   h1 = RMSNorm(x; g1); qkv = h1 Wqkv; RoPE(q, k); attn = causal FA(q, k, v);
 //             o = attn Wo + x; h2 = RMSNorm(o; g2); up = h2 Wup; gate = h2 Wgate;
 //             act = SiLU(gate) * up; out = act Wdown + o.        saved: qkv attn lse o up gate act
-//   backward  h1 and h2 are recomputed (decoder.rs:560-567, 660-667); weight gradients are
-//             accumulated into f32 buffers (beta = 1), residual gradients are fused into the
-//             RMSNorm backward (residual_dy), the second FFN dgrad accumulates into the first
-//             (decoder.rs:591-596).
+//   backward  h1 and h2 are recomputed (decoder.rs:560-567, 660-667) by the RMSNorm backward, ahead of
+//             the weight gradients that need them; those are accumulated into f32 buffers (beta = 1),
+//             residual gradients are fused into the RMSNorm backward (residual_dy), the second FFN dgrad
+//             accumulates into the first (decoder.rs:591-596).
 // Residual adds and gradient accumulation ride in the GEMM epilogue (C operand, beta = 1).
 // Weights are stored [in, out] (decoder.rs:166-173).  Everything runs on the caller's stream;
 // nothing is allocated: the caller passes one workspace sized by *_workspace_bytes.
